@@ -287,6 +287,22 @@ int msgl_build_attn_metadata(const int32_t* req, const int32_t* page_table, int6
                              void* status_word, void* stream);
 
 /*
+ * The same arrays with the requests' numbers in HOST memory: `req_host` (3 * batch int32, same order)
+ * is read before the call returns and travels as kernel parameters, so a step needs no copy, no
+ * staging buffer and no event.  batch <= MSGL_METADATA_HOST_MAX.  Also writes kv_lens (batch), the KV
+ * lengths, which the page-granular operators read.
+ */
+#define MSGL_METADATA_HOST_MAX 1024
+int msgl_build_attn_metadata_host(const int32_t* req_host, const int32_t* page_table,
+                                  int64_t table_row_stride, int64_t table_rows, int64_t table_cols,
+                                  int batch, int page_size, int split_chunk, int max_kv_splits,
+                                  int64_t total_q, int64_t total_kv, int64_t total_pages,
+                                  int32_t* qo_indptr, int32_t* kv_indptr, int32_t* prefix_lens,
+                                  int32_t* num_kv_splits, int32_t* positions, int32_t* kv_lens,
+                                  int32_t* kv_indices, int32_t* page_indptr, int32_t* page_indices,
+                                  void* status_word, void* stream);
+
+/*
  * Page-granular index entries.  The reference hard-wires one token per page
  * (mini_sglang_mlx/engine/engine.py:103) and hands the ops one slot id per token
  * (kv_indices, mini_sglang_mlx/attention/backend.py:239-244, 279-284).  A pool

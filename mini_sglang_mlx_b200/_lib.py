@@ -45,6 +45,9 @@ SIGNATURES = {
     "msgl_build_attn_metadata": (
         _i, [_vp, _vp, _i64, _i64, _i64, _i, _i, _i, _i, _i64, _i64, _i64, _vp, _vp, _vp, _vp, _vp,
              _vp, _vp, _vp, _vp, _vp]),
+    "msgl_build_attn_metadata_host": (
+        _i, [_vp, _vp, _i64, _i64, _i64, _i, _i, _i, _i, _i64, _i64, _i64, _vp, _vp, _vp, _vp, _vp,
+             _vp, _vp, _vp, _vp, _vp, _vp]),
     "msgl_prefill_workspace_bytes_p16": (_sz, [_i, _i, _i64, _i, _i, _i, _i, _i, _i]),
     "msgl_paged_prefill_attention_p16": (
         _i, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _sz, _i, _i, _i, _i, _i, _i64, _i,
@@ -73,6 +76,26 @@ def lib() -> C.CDLL:
         fn.restype = res
         fn.argtypes = args
     return handle
+
+
+class _Host:
+    """The native host module ``_host.so`` (``csrc/host_ops.cpp``), loaded at the first use of one of
+    its functions; they become plain attributes then."""
+
+    def __getattr__(self, name):
+        if name.startswith("__"):
+            raise AttributeError(name)
+        try:
+            from . import _host
+        except ImportError as e:
+            raise RuntimeError(
+                "_host.so is missing or does not load: build it with `python -m mini_sglang_mlx_b200.build` "
+                "(there is no fallback implementation)") from e
+        self.__dict__.update({k: v for k, v in vars(_host).items() if not k.startswith("__")})
+        return self.__dict__[name]
+
+
+host = _Host()
 
 
 def last_error() -> str:

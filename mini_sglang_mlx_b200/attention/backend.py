@@ -7,9 +7,10 @@ Differences, all inside the boundary:
 
 * every index array of a step (``qo_indptr``, ``kv_indptr``, ``kv_indices``,
   ``prefix_lens``, ``positions``, ``num_kv_splits``) comes from ONE launch over the
-  device-resident page table after ONE host-to-device copy of the per-request
-  lengths and table rows (pinned staging), instead of per-request loops and several
-  small copies on the host (reference lines 205-307).
+  device-resident page table, the per-request lengths and table rows travelling as its
+  parameters, instead of per-request loops and several small copies on the host
+  (reference lines 205-307).  A batch of more than 1024 requests sends them ahead in one
+  host-to-device copy from pinned staging.
 * ``page_size`` > 1 (the reference has one token per page,
   mini_sglang_mlx/engine/engine.py:103): the table rows hold page-structured slots
   (``CacheManager(page_size=...)``), the metadata also carries one id per page
@@ -27,10 +28,11 @@ import math
 from dataclasses import dataclass
 from typing import List, Optional, Sequence
 
+import numpy as np
 import torch
 
 from .. import _lib
-from ..kernel import (build_attn_metadata, paged_decode_attention, paged_decode_attention_p16,
+from ..kernel import (_ops, build_attn_metadata, paged_decode_attention, paged_decode_attention_p16,
                       paged_prefill_attention, paged_prefill_attention_p16, qk_norm_rope_store)
 
 MAX_KV_SPLITS = 32
@@ -127,6 +129,7 @@ class AttnBackend:
         # the page-granular operators are the fast path when their kernels can fetch whole
         # 16-row boxes; other page sizes keep the per-token ids
         self._paged_ops = self.page_size % 16 == 0
+        self._index_page = self.page_size if self._paged_ops else 1
         self._sm_count: Optional[int] = None
         self._staging: List[torch.Tensor] = []        # pinned (3, capacity) int32 buffers, in turn
         self._staging_events: List[torch.cuda.Event] = []
@@ -234,55 +237,60 @@ class AttnBackend:
         rows_np[2] = rows
         return req, self._staging_events[k]
 
-    def _index_arrays(self, reqs, extend_lens: Sequence[int], kv_lens: Sequence[int], split_chunk: int):
-        req, event = self._stage(extend_lens, kv_lens, [r.table_idx for r in reqs])
-        ps = self.page_size if self._paged_ops else 1
-        md = build_attn_metadata(req, self.page_table, total_q=sum(extend_lens), total_kv=sum(kv_lens),
-                                 page_size=ps, split_chunk=split_chunk, max_kv_splits=MAX_KV_SPLITS,
-                                 per_token_ids=not self._paged_ops,
-                                 total_pages=sum((l + ps - 1) // ps for l in kv_lens) if ps > 1 else 0)
+    def _index_arrays(self, packed: bytes, total_q: int, total_kv: int, total_pages: int, split_chunk: int):
+        """(qo_indptr, kv_indptr, prefix_lens, num_kv_splits, positions, kv_lens, kv_indices,
+        page_indptr, page_indices) of the requests whose numbers ``packed`` holds."""
+        ps = self._index_page
+        out = _ops.index_arrays(packed, self.page_table, total_q, total_kv, total_pages, ps,
+                                      split_chunk, MAX_KV_SPLITS, not self._paged_ops, None)
+        if out is not None:
+            return out
+        # a batch too large to travel with the launch (or a table on another device)
+        n = len(packed) // 12
+        lens = np.frombuffer(packed, dtype=np.int32).reshape(3, n)
+        req, event = self._stage(*lens)
+        md = build_attn_metadata(req, self.page_table, total_q=total_q, total_kv=total_kv, page_size=ps,
+                                 split_chunk=split_chunk, max_kv_splits=MAX_KV_SPLITS,
+                                 per_token_ids=not self._paged_ops, total_pages=total_pages if ps > 1 else 0)
         event.record()
-        return md
+        return tuple(md[k] for k in ("qo_indptr", "kv_indptr", "prefix_lens", "num_kv_splits", "positions",
+                                     "kv_lens", "kv_indices", "page_indptr", "page_indices"))
 
     def build_prefill_metadata(self, reqs, *, extend_lens: Optional[List[int]] = None,
                                kv_lens: Optional[List[int]] = None,
                                positions: Optional[torch.Tensor] = None) -> PrefillMetadata:
         """Reference lines 205-254; ``extend_lens`` / ``kv_lens`` overrides serve a
         virtual extend window such as a K+1-token verify."""
-        if extend_lens is None:
-            extend_lens = [req.extend_len for req in reqs]
-        if kv_lens is None:
-            kv_lens = [req.device_len for req in reqs]
-        md = self._index_arrays(reqs, extend_lens, kv_lens, 0)
-        return PrefillMetadata(positions=md["positions"] if positions is None else positions,
-                               qo_indptr=md["qo_indptr"], kv_indptr=md["kv_indptr"],
-                               kv_indices=md["kv_indices"], prefix_lens=md["prefix_lens"],
-                               max_len_extend=max(extend_lens), page_indptr=md["page_indptr"],
-                               page_indices=md["page_indices"], kv_lens=md["kv_lens"],
-                               page_size=self.page_size if self._paged_ops else 1)
+        packed, total_q, total_kv, pages, max_extend, _ = _ops.collect_lens(
+            reqs, extend_lens, kv_lens, False, self._index_page)
+        qo, kvp, prefix, _, pos, lens, ids, page_indptr, page_ids = self._index_arrays(
+            packed, total_q, total_kv, pages, 0)
+        return PrefillMetadata(positions=pos if positions is None else positions, qo_indptr=qo,
+                               kv_indptr=kvp, kv_indices=ids, prefix_lens=prefix,
+                               max_len_extend=max_extend, page_indptr=page_indptr, page_indices=page_ids,
+                               kv_lens=lens, page_size=self._index_page)
 
     def build_decode_metadata(self, reqs, *, kv_lens: Optional[List[int]] = None,
                               positions: Optional[torch.Tensor] = None) -> DecodeMetadata:
         """Reference lines 256-293."""
-        if kv_lens is None:
-            kv_lens = [req.device_len for req in reqs]
         if self._sm_count is None:
             with torch.cuda.device(self.page_table.device):
                 self._sm_count = max(1, _lib.lib().msgl_device_sm_count())
-        chunk = split_chunk_tokens(sum(kv_lens), self.config.num_kv_heads, sm_count=self._sm_count,
-                                   batch=len(kv_lens), policy=self.split_policy)
         # "new tokens" of a decode row = everything behind what the request has cached, so that
         # the kernel's prefix_lens are the reference's positions (req.cached_len, line 276)
-        extend = [max(1, min(kv_lens[i], kv_lens[i] - reqs[i].cached_len)) for i in range(len(reqs))]
-        md = self._index_arrays(reqs, extend, kv_lens, chunk)
+        packed, total_q, total_kv, pages, _, max_kv = _ops.collect_lens(
+            reqs, None, kv_lens, True, self._index_page)
+        chunk = split_chunk_tokens(total_kv, self.config.num_kv_heads, sm_count=self._sm_count,
+                                   batch=len(packed) // 12, policy=self.split_policy)
+        _, kvp, prefix, splits, _, lens, ids, page_indptr, page_ids = self._index_arrays(
+            packed, total_q, total_kv, pages, chunk)
         # the split dimension of the launch grid: what the longest sequence needs, not the cap
         # (CTAs of split slots no sequence uses would only start, look up a length and leave)
         # (the reference policy keeps the reference's constant, backend.py:293)
         max_splits = MAX_KV_SPLITS
-        if self.split_policy != "reference" and kv_lens:
-            max_splits = min(MAX_KV_SPLITS, max(1, -(-max(kv_lens) // chunk)))
-        return DecodeMetadata(positions=md["prefix_lens"] if positions is None else positions,
-                              kv_indptr=md["kv_indptr"], kv_indices=md["kv_indices"],
-                              num_kv_splits=md["num_kv_splits"], max_kv_splits=max_splits,
-                              page_indptr=md["page_indptr"], page_indices=md["page_indices"],
-                              kv_lens=md["kv_lens"], page_size=self.page_size if self._paged_ops else 1)
+        if self.split_policy != "reference":
+            max_splits = min(MAX_KV_SPLITS, max(1, -(-max_kv // chunk)))
+        return DecodeMetadata(positions=prefix if positions is None else positions, kv_indptr=kvp,
+                              kv_indices=ids, num_kv_splits=splits, max_kv_splits=max_splits,
+                              page_indptr=page_indptr, page_indices=page_ids, kv_lens=lens,
+                              page_size=self._index_page)

@@ -68,7 +68,6 @@ int static_scratch_for_current_device(void** out) {
 
 constexpr int kDecWarps = 4;
 constexpr int kDecStages = 3;
-constexpr int kDecCtaTokens = kDecWarps * msgl::kDecodeGroupTokens;
 
 int sm_count_cached() {
   static thread_local int cached_dev = -1;
@@ -84,9 +83,24 @@ int sm_count_cached() {
   return cached_sms;
 }
 
+// Dynamic shared memory of a kernel, set once per kernel, device and thread (the runtime call takes
+// longer than the rest of a launch's preparation).
 template <typename K>
 cudaError_t allow_smem(K kernel, int bytes) {
-  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  struct Done {
+    const void* fn;
+    int dev, bytes;
+  };
+  static thread_local Done done[64] = {};
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  const void* fn = reinterpret_cast<const void*>(kernel);
+  Done& d = done[((reinterpret_cast<uintptr_t>(fn) >> 4) ^ dev) % 64];
+  if (d.fn == fn && d.dev == dev && d.bytes == bytes) return cudaSuccess;
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (e == cudaSuccess) d = Done{fn, dev, bytes};
+  return e;
 }
 
 // ---- TMA tensor maps over a K or V pool (page-granular entries)
@@ -112,7 +126,8 @@ EncodeTiledFn tensor_map_encoder() {
 // 2-D map over a pool (num_slots rows of num_kv_heads * head_dim 16-bit elements): a box is
 // 16 token rows x 64 elements (128 bytes) of one head, written to shared memory with the
 // 128-byte swizzle, i.e. in the layout the tensor-core descriptors of the kernels expect.
-// Rows outside the pool read as zeros.  The last map per (pointer, shape) is kept per thread.
+// Rows outside the pool read as zeros.  The maps are kept per thread, one per hash of the pool's
+// address: a model's layers each have two pools and go through them in turn.
 bool make_pool_tensor_map(CUtensorMap* out, const void* base, int64_t num_slots, int num_kv_heads,
                           int head_dim, int dtype) {
   struct Cached {
@@ -121,14 +136,14 @@ bool make_pool_tensor_map(CUtensorMap* out, const void* base, int64_t num_slots,
     int hkv, hd, dtype;
     CUtensorMap map;
   };
-  static thread_local Cached cache[4] = {};
-  static thread_local int next = 0;
-  for (const Cached& c : cache)
-    if (c.base == base && c.num_slots == num_slots && c.hkv == num_kv_heads && c.hd == head_dim &&
-        c.dtype == dtype && base != nullptr) {
-      *out = c.map;
-      return true;
-    }
+  static thread_local Cached cache[256] = {};
+  const uintptr_t key = reinterpret_cast<uintptr_t>(base) >> 8;
+  Cached& c = cache[(key ^ (key >> 8) ^ (key >> 16) ^ (key >> 24)) % 256];
+  if (c.base == base && c.num_slots == num_slots && c.hkv == num_kv_heads && c.hd == head_dim &&
+      c.dtype == dtype && base != nullptr) {
+    *out = c.map;
+    return true;
+  }
   EncodeTiledFn enc = tensor_map_encoder();
   if (!enc || num_slots <= 0 || reinterpret_cast<uintptr_t>(base) % 16 != 0) return false;
   const cuuint64_t dims[2] = {static_cast<cuuint64_t>(num_kv_heads) * head_dim,
@@ -143,8 +158,7 @@ bool make_pool_tensor_map(CUtensorMap* out, const void* base, int64_t num_slots,
                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                          CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return false;
-  cache[next] = Cached{base, num_slots, num_kv_heads, head_dim, dtype, m};
-  next = (next + 1) % 4;
+  c = Cached{base, num_slots, num_kv_heads, head_dim, dtype, m};
   *out = m;
   return true;
 }
@@ -431,6 +445,63 @@ __global__ void __launch_bounds__(256) build_metadata_kernel(const MetadataParam
     }
   }
   for (int t = blockIdx.x * 256 + tid; t < e; t += stride) p.positions[q0 + t] = k - e + t;
+}
+
+// The same arrays when the host hands the lengths over with the launch: the requests travel as kernel
+// parameters with their prefix sums already taken (a few hundred additions on the host), so a step needs no
+// staging buffer, no copy and no event, and a CTA neither scans the batch nor waits for anything.
+// One decode step of 64 requests with 3 million cached tokens: 28 us for copy and launch before (a division
+// per cached token), see the page loop below.
+struct MetadataRecord {
+  int32_t extend, kv, row;       // new tokens, KV length, page-table row
+  int32_t q0, k0, g0;            // sums of the requests in front: new tokens, KV tokens, pages
+};
+template <int N>
+struct MetadataRecords {
+  MetadataRecord r[N];
+};
+
+template <int N>
+__global__ void __launch_bounds__(256)
+    build_metadata_host_kernel(const MetadataParams p, int32_t* __restrict__ kv_lens,
+                               const __grid_constant__ MetadataRecords<N> recs) {
+  const int b = blockIdx.y, tid = threadIdx.x;
+  const MetadataRecord m = recs.r[b];
+  const int e = max(m.extend, 0), k = max(m.kv, 0);
+  const int npg = (k + p.page_size - 1) / p.page_size;
+  const bool bad = m.extend < 0 || m.kv < 0 || e > k || m.row < 0 || m.row >= p.table_rows ||
+                   k > p.table_cols || static_cast<int64_t>(m.q0) + e > p.total_q ||
+                   static_cast<int64_t>(m.k0) + k > p.total_kv ||
+                   (p.page_indices && static_cast<int64_t>(m.g0) + npg > p.total_pages);
+  if (blockIdx.x == 0 && tid == 0) {
+    p.qo_indptr[b] = m.q0;
+    p.kv_indptr[b] = m.k0;
+    if (p.page_indptr) p.page_indptr[b] = m.g0;
+    if (b == p.batch - 1) {
+      p.qo_indptr[p.batch] = m.q0 + e;
+      p.kv_indptr[p.batch] = m.k0 + k;
+      if (p.page_indptr) p.page_indptr[p.batch] = m.g0 + npg;
+    }
+    p.prefix_lens[b] = k - e;
+    kv_lens[b] = m.kv;
+    const int chunk = p.split_chunk > 0 ? p.split_chunk : 128;
+    p.num_kv_splits[b] = min(p.max_kv_splits, max(1, (k + chunk - 1) / chunk));
+    if (bad && p.status) atomicExch(p.status, 2);
+  }
+  if (bad) return;
+  const int32_t* row = p.page_table + static_cast<int64_t>(m.row) * p.row_stride;
+  const int stride = gridDim.x * 256, first = blockIdx.x * 256 + tid;
+  if (p.kv_indices)
+    for (int t = first; t < k; t += stride) p.kv_indices[m.k0 + t] = row[t];
+  if (p.page_indices) {
+    for (int g = first; g < npg; g += stride) {
+      const int32_t slot = row[static_cast<int64_t>(g) * p.page_size];
+      const bool off = slot < 0 || slot % p.page_size != 0;   // pages must start on page boundaries
+      if (off && p.status) atomicExch(p.status, 2);
+      p.page_indices[m.g0 + g] = off ? -1 : slot / p.page_size;
+    }
+  }
+  for (int t = first; t < e; t += stride) p.positions[m.q0 + t] = k - e + t;
 }
 
 // Page-granular index entries: kv_indptr = exclusive scan of the sequence lengths (one CTA),
@@ -1273,6 +1344,77 @@ int msgl_build_attn_metadata(const int32_t* req, const int32_t* page_table, int6
   if (bx < 1) bx = 1;
   build_metadata_kernel<<<dim3(bx, batch), 256, 0, static_cast<cudaStream_t>(stream)>>>(p);
   cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return cuda_fail("build_attn_metadata", e);
+  return MSGL_OK;
+}
+
+int msgl_build_attn_metadata_host(const int32_t* req_host, const int32_t* page_table, int64_t table_row_stride,
+                                  int64_t table_rows, int64_t table_cols, int batch, int page_size,
+                                  int split_chunk, int max_kv_splits, int64_t total_q, int64_t total_kv,
+                                  int64_t total_pages, int32_t* qo_indptr, int32_t* kv_indptr,
+                                  int32_t* prefix_lens, int32_t* num_kv_splits, int32_t* positions,
+                                  int32_t* kv_lens, int32_t* kv_indices, int32_t* page_indptr,
+                                  int32_t* page_indices, void* status_word, void* stream) {
+  const char* op = "build_attn_metadata: ";
+  if (batch < 0 || table_rows < 0 || table_cols < 0 || table_row_stride < 0 || total_q < 0 || total_kv < 0 ||
+      total_pages < 0)
+    return fail(MSGL_BAD_SHAPE, std::string(op) + "negative size");
+  if (page_size < 1 || max_kv_splits < 1 || split_chunk < 0)
+    return fail(MSGL_BAD_ARG, std::string(op) + "page_size and max_kv_splits must be >= 1, split_chunk >= 0");
+  if (batch > MSGL_METADATA_HOST_MAX)
+    return fail(MSGL_BAD_SHAPE, std::string(op) + "batch must be <= " + std::to_string(MSGL_METADATA_HOST_MAX) +
+                                    " when the lengths are host memory");
+  if (total_q >= (1ll << 31) || total_kv >= (1ll << 31))
+    return fail(MSGL_BAD_SHAPE, std::string(op) + "totals must be < 2^31");
+  if (batch == 0) return MSGL_OK;
+  if (!req_host || !page_table || !qo_indptr || !kv_indptr || !prefix_lens || !num_kv_splits || !kv_lens ||
+      (total_q > 0 && !positions) || (page_indptr && total_pages > 0 && !page_indices))
+    return fail(MSGL_BAD_ARG, std::string(op) + "null tensor pointer");
+  MetadataParams p{};
+  p.page_table = page_table;
+  p.row_stride = table_row_stride;
+  p.table_rows = table_rows;
+  p.table_cols = table_cols;
+  p.batch = batch;
+  p.page_size = page_size;
+  p.split_chunk = split_chunk;
+  p.max_kv_splits = max_kv_splits;
+  p.total_q = total_q;
+  p.total_kv = total_kv;
+  p.total_pages = total_pages;
+  p.qo_indptr = qo_indptr;
+  p.kv_indptr = kv_indptr;
+  p.prefix_lens = prefix_lens;
+  p.num_kv_splits = num_kv_splits;
+  p.positions = positions;
+  p.kv_indices = kv_indices;
+  p.page_indptr = page_indptr;
+  p.page_indices = page_indptr ? page_indices : nullptr;
+  p.status = static_cast<int*>(status_word);
+  // entries the longest request writes decide how many CTAs each request gets
+  int64_t widest = 0;
+  auto launch = [&](auto tag) -> cudaError_t {
+    constexpr int N = decltype(tag)::value;
+    MetadataRecords<N> recs;
+    int64_t q0 = 0, k0 = 0, g0 = 0;
+    for (int b = 0; b < batch; ++b) {
+      const int32_t e = req_host[b], k = req_host[batch + b];
+      recs.r[b] = MetadataRecord{e, k, req_host[2 * batch + b], static_cast<int32_t>(q0),
+                                 static_cast<int32_t>(k0), static_cast<int32_t>(g0)};
+      const int64_t pages = (static_cast<int64_t>(std::max(k, 0)) + page_size - 1) / page_size;
+      q0 += std::max(e, 0);
+      k0 += std::max(k, 0);
+      g0 += pages;
+      widest = std::max<int64_t>(widest, std::max<int64_t>(kv_indices ? k : pages, e));
+    }
+    const unsigned bx = static_cast<unsigned>(std::min<int64_t>(32, std::max<int64_t>(1, (widest + 255) / 256)));
+    build_metadata_host_kernel<N><<<dim3(bx, batch), 256, 0, static_cast<cudaStream_t>(stream)>>>(p, kv_lens, recs);
+    return cudaGetLastError();
+  };
+  // the parameter block is copied with every launch: 0.8, 6 or 24 KB of it
+  const cudaError_t e = batch <= 32    ? launch(std::integral_constant<int, 32>{})
+                        : batch <= 256 ? launch(std::integral_constant<int, 256>{})
+                                       : launch(std::integral_constant<int, MSGL_METADATA_HOST_MAX>{});
   if (e != cudaSuccess) return cuda_fail("build_attn_metadata", e);
   return MSGL_OK;
 }

@@ -88,6 +88,39 @@ def _workspace(nbytes: int, device: torch.device, stream_handle: int, kind: str)
     return ws
 
 
+def _make_workspace(nbytes: int, index: int, stream_handle: int, kind: str) -> torch.Tensor:
+    return _workspace(nbytes, torch.device("cuda", index), stream_handle, kind)
+
+
+class _HostOps:
+    """The native operators (``csrc/host_ops.cpp``), told at their first use how scratch is made."""
+
+    def __getattr__(self, name):
+        fn = getattr(_lib.host, name)
+        _lib.host.set_workspace_maker(_make_workspace)
+        setattr(self, name, fn)
+        return fn
+
+
+_ops = _HostOps()
+
+
+def _handle(stream) -> Optional[int]:
+    """``stream=`` of an operator as the native calls take it: None (torch's current) or a handle."""
+    if stream is None:
+        return None
+    return stream.cuda_stream if isinstance(stream, torch.cuda.Stream) else int(stream)
+
+
+def _again(op: str, fn, device: torch.device, *args):
+    """A native call that was declined although the arguments are in order: the tensors' device is
+    not the current one."""
+    with torch.cuda.device(device):
+        out = fn(*args)
+    _require(out is not None, f"{op}: arguments the operator does not take")
+    return out
+
+
 def device_status(device=None) -> int:
     """Synchronise and return the OR of the device status words of every
     workspace on ``device`` (0 = no kernel reported an out-of-range slot),
@@ -142,6 +175,11 @@ def paged_decode_attention(q, k_cache, v_cache, kv_indptr, kv_indices, num_kv_sp
     reference op; same shape as q) fuses the ``* sigmoid(gate)`` of the reference's Qwen3.5
     attention layer (models/qwen3_5.py:110) into the final write.
     """
+    args = (q, k_cache, v_cache, kv_indptr, kv_indices, num_kv_splits, sm_scale, max_kv_splits, gate,
+            None if stream is None else _handle(stream))
+    out = _ops.decode(*args)
+    if out is not None:
+        return out
     op = "paged_decode_attention"
     _check_common(op, q, k_cache, v_cache, (kv_indptr, kv_indices, num_kv_splits),
                   "kv_indptr, kv_indices, num_kv_splits must be 1D",
@@ -150,22 +188,9 @@ def paged_decode_attention(q, k_cache, v_cache, kv_indptr, kv_indices, num_kv_sp
     _require(k_cache.shape[2] == d, f"{op}: cache head_dim must match q head_dim")
     _require(kv_indptr.numel() == batch + 1 and num_kv_splits.numel() == batch,
              f"{op}: kv_indptr must have batch+1 and num_kv_splits batch entries")
-    out = torch.empty_like(q)
-    sh = _stream_handle(stream, q.device)
-    lib = _lib.lib()
-    with _on_device(q.device):
-        need = lib.msgl_decode_workspace_bytes(batch, hq, d, int(max_kv_splits))
-        ws = _workspace(need, q.device, sh, "decode")
-        tail = (out.data_ptr(), ws.data_ptr(), ws.numel(), batch, hq, k_cache.shape[1], d,
-                k_cache.shape[0], _DTYPES[q.dtype], float(sm_scale), int(max_kv_splits), sh)
-        head = (q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), kv_indptr.data_ptr(),
-                kv_indices.data_ptr(), num_kv_splits.data_ptr())
-        if gate is None:
-            _lib.check(lib.msgl_paged_decode_attention(*head, *tail))
-        else:
-            _check_gate(op, gate, q)
-            _lib.check(lib.msgl_paged_decode_attention_gated(*head, gate.data_ptr(), *tail))
-    return out
+    if gate is not None:
+        _check_gate(op, gate, q)
+    return _again(op, _ops.decode, q.device, *args)
 
 
 def paged_prefill_attention(q, k_cache, v_cache, qo_indptr, kv_indptr, kv_indices, prefix_lens,
@@ -181,35 +206,23 @@ def paged_prefill_attention(q, k_cache, v_cache, qo_indptr, kv_indptr, kv_indice
     Signature of the reference op: mini-sglang-mlx-kernel/csrc/bindings.cpp:45-55.
     ``gate`` (not in the reference op; same shape as q): out = attention * sigmoid(gate).
     """
+    args = (q, k_cache, v_cache, qo_indptr, kv_indptr, kv_indices, prefix_lens, sm_scale, max_len_extend,
+            is_cross_attention, sliding_window_size, gate, None if stream is None else _handle(stream))
+    out = _ops.prefill(*args)
+    if out is not None:
+        return out
     op = "paged_prefill_attention"
     _check_common(op, q, k_cache, v_cache, (qo_indptr, kv_indptr, kv_indices, prefix_lens),
                   "qo_indptr, kv_indptr, kv_indices, prefix_lens must be 1D",
                   "q must be 3D (total_q_tokens, num_q_heads, head_dim)")
-    total_q, hq, d = q.shape
-    _require(k_cache.shape[2] == d, f"{op}: cache head_dim must match q head_dim")
+    _require(k_cache.shape[2] == q.shape[2], f"{op}: cache head_dim must match q head_dim")
     batch = qo_indptr.numel() - 1
     _require(batch > 0, f"{op}: batch must be > 0")
     _require(kv_indptr.numel() == batch + 1 and prefix_lens.numel() == batch,
              f"{op}: kv_indptr must have batch+1 and prefix_lens batch entries")
-    out = torch.empty_like(q)
-    sh = _stream_handle(stream, q.device)
-    lib = _lib.lib()
-    total_kv = kv_indices.numel()
-    with _on_device(q.device):
-        need = lib.msgl_prefill_workspace_bytes(batch, total_q, total_kv, hq, k_cache.shape[1], d,
-                                                int(max_len_extend), int(sliding_window_size))
-        ws = _workspace(need, q.device, sh, "prefill")
-        head = (q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), qo_indptr.data_ptr(),
-                kv_indptr.data_ptr(), kv_indices.data_ptr(), prefix_lens.data_ptr())
-        tail = (out.data_ptr(), ws.data_ptr(), ws.numel(), batch, total_q, total_kv, hq, k_cache.shape[1],
-                d, k_cache.shape[0], _DTYPES[q.dtype], float(sm_scale), int(max_len_extend),
-                int(bool(is_cross_attention)), int(sliding_window_size), sh)
-        if gate is None:
-            _lib.check(lib.msgl_paged_prefill_attention(*head, *tail))
-        else:
-            _check_gate(op, gate, q)
-            _lib.check(lib.msgl_paged_prefill_attention_gated(*head, gate.data_ptr(), *tail))
-    return out
+    if gate is not None:
+        _check_gate(op, gate, q)
+    return _again(op, _ops.prefill, q.device, *args)
 
 
 def paged_decode_attention_p16(q, k_cache, v_cache, page_indptr, page_indices, kv_lens, num_kv_splits,
@@ -221,6 +234,11 @@ def paged_decode_attention_p16(q, k_cache, v_cache, page_indptr, page_indices, k
     ``kv_indptr`` / ``kv_indices`` of the reference op (the reference hard-wires one token per
     page, mini_sglang_mlx/engine/engine.py:103).  No host synchronisation: the per-token ids
     are built on the device in front of the same kernels."""
+    args = (q, k_cache, v_cache, page_indptr, page_indices, kv_lens, num_kv_splits, sm_scale, max_kv_splits,
+            page_size, gate, None if stream is None else _handle(stream))
+    out = _ops.decode_paged(*args)
+    if out is not None:
+        return out
     op = "paged_decode_attention_p16"
     _check_common(op, q, k_cache, v_cache, (page_indptr, page_indices, kv_lens, num_kv_splits),
                   "page_indptr, page_indices, kv_lens, num_kv_splits must be 1D",
@@ -231,23 +249,9 @@ def paged_decode_attention_p16(q, k_cache, v_cache, page_indptr, page_indices, k
              and num_kv_splits.numel() == batch,
              f"{op}: page_indptr must have batch+1, kv_lens and num_kv_splits batch entries")
     _require(int(page_size) > 0, f"{op}: page_size must be > 0")
-    out = torch.empty_like(q)
-    sh = _stream_handle(stream, q.device)
-    lib = _lib.lib()
-    total_pages = page_indices.numel()
-    with _on_device(q.device):
-        need = ((lib.msgl_decode_workspace_bytes(batch, hq, d, int(max_kv_splits)) + 255) // 256 * 256
-                + lib.msgl_page_index_workspace_bytes(batch, total_pages, int(page_size)))
-        ws = _workspace(need, q.device, sh, "decode")
-        if gate is not None:
-            _check_gate(op, gate, q)
-        _lib.check(lib.msgl_paged_decode_attention_p16(
-            q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), page_indptr.data_ptr(),
-            page_indices.data_ptr(), kv_lens.data_ptr(), num_kv_splits.data_ptr(),
-            gate.data_ptr() if gate is not None else None, out.data_ptr(),
-            ws.data_ptr(), ws.numel(), batch, hq, k_cache.shape[1], d, k_cache.shape[0],
-            _DTYPES[q.dtype], float(sm_scale), int(max_kv_splits), int(page_size), total_pages, sh))
-    return out
+    if gate is not None:
+        _check_gate(op, gate, q)
+    return _again(op, _ops.decode_paged, q.device, *args)
 
 
 def paged_prefill_attention_p16(q, k_cache, v_cache, qo_indptr, page_indptr, page_indices, kv_lens,
@@ -256,37 +260,26 @@ def paged_prefill_attention_p16(q, k_cache, v_cache, qo_indptr, page_indptr, pag
                                 sliding_window_size: int = 0, gate=None, stream=None) -> torch.Tensor:
     """``paged_prefill_attention`` with one id per page of ``page_size`` tokens instead of one
     per token; see ``paged_decode_attention_p16``."""
+    args = (q, k_cache, v_cache, qo_indptr, page_indptr, page_indices, kv_lens, prefix_lens, sm_scale,
+            max_len_extend, page_size, is_cross_attention, sliding_window_size, gate,
+            None if stream is None else _handle(stream))
+    out = _ops.prefill_paged(*args)
+    if out is not None:
+        return out
     op = "paged_prefill_attention_p16"
     _check_common(op, q, k_cache, v_cache, (qo_indptr, page_indptr, page_indices, kv_lens, prefix_lens),
                   "qo_indptr, page_indptr, page_indices, kv_lens, prefix_lens must be 1D",
                   "q must be 3D (total_q_tokens, num_q_heads, head_dim)")
-    total_q, hq, d = q.shape
-    _require(k_cache.shape[2] == d, f"{op}: cache head_dim must match q head_dim")
+    _require(k_cache.shape[2] == q.shape[2], f"{op}: cache head_dim must match q head_dim")
     batch = qo_indptr.numel() - 1
     _require(batch > 0, f"{op}: batch must be > 0")
     _require(page_indptr.numel() == batch + 1 and kv_lens.numel() == batch
              and prefix_lens.numel() == batch,
              f"{op}: page_indptr must have batch+1, kv_lens and prefix_lens batch entries")
     _require(int(page_size) > 0, f"{op}: page_size must be > 0")
-    out = torch.empty_like(q)
-    sh = _stream_handle(stream, q.device)
-    lib = _lib.lib()
-    total_pages = page_indices.numel()
-    with _on_device(q.device):
-        need = lib.msgl_prefill_workspace_bytes_p16(batch, total_q, total_pages, int(page_size), hq,
-                                                    k_cache.shape[1], d, int(max_len_extend),
-                                                    int(sliding_window_size))
-        ws = _workspace(need, q.device, sh, "prefill")
-        if gate is not None:
-            _check_gate(op, gate, q)
-        _lib.check(lib.msgl_paged_prefill_attention_p16(
-            q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), qo_indptr.data_ptr(),
-            page_indptr.data_ptr(), page_indices.data_ptr(), kv_lens.data_ptr(), prefix_lens.data_ptr(),
-            gate.data_ptr() if gate is not None else None,
-            out.data_ptr(), ws.data_ptr(), ws.numel(), batch, total_q, hq, k_cache.shape[1], d,
-            k_cache.shape[0], _DTYPES[q.dtype], float(sm_scale), int(max_len_extend),
-            int(bool(is_cross_attention)), int(sliding_window_size), int(page_size), total_pages, sh))
-    return out
+    if gate is not None:
+        _check_gate(op, gate, q)
+    return _again(op, _ops.prefill_paged, q.device, *args)
 
 
 def store_kv_cache(k_cache, v_cache, indices, k, v, *, stream=None) -> None:
@@ -295,6 +288,9 @@ def store_kv_cache(k_cache, v_cache, indices, k, v, *, stream=None) -> None:
     Signature and checks of the reference op:
     mini-sglang-mlx-kernel/csrc/bindings.cpp:27-32, csrc/store_kv_cache.cpp:22-63.
     """
+    args = (k_cache, v_cache, indices, k, v, None if stream is None else _handle(stream))
+    if _ops.store_kv(*args) is not None:
+        return
     op = "store_kv_cache"
     _require(k_cache.dim() == 3 and v_cache.dim() == 3,
              f"{op}: k_cache and v_cache must be 3D (num_pages, num_kv_heads, head_dim)")
@@ -318,13 +314,7 @@ def store_kv_cache(k_cache, v_cache, indices, k, v, *, stream=None) -> None:
     _require(k.stride(0) == v.stride(0) and k_cache.stride(0) == v_cache.stride(0),
              f"{op}: k/v (and the two caches) must share their row stride")
     _require(indices.is_contiguous(), f"{op}: indices must be contiguous")
-    sh = _stream_handle(stream, k_cache.device)
-    with _on_device(k_cache.device):
-        status = _workspace(256, k_cache.device, sh, "decode")   # dropped rows are reported there
-        _lib.check(_lib.lib().msgl_store_kv_cache(
-            k_cache.data_ptr(), v_cache.data_ptr(), indices.data_ptr(), k.data_ptr(), v.data_ptr(),
-            length, hkv, d, num_slots, k_cache.stride(0), k.stride(0), _DTYPES[k_cache.dtype],
-            status.data_ptr(), sh))
+    _again(op, _ops.store_kv, k_cache.device, *args)
 
 
 def qk_norm_rope_store(q, k, v, q_weight, k_weight, positions, out_loc, k_cache, v_cache, *,
@@ -340,6 +330,10 @@ def qk_norm_rope_store(q, k, v, q_weight, k_weight, positions, out_loc, k_cache,
     into one fused projection output (dense heads, any token stride).  ``q_weight`` /
     ``k_weight``: (head_dim,) or None to skip that norm.
     """
+    args = (q, k, v, q_weight, k_weight, positions, out_loc, k_cache, v_cache, rope_base, eps,
+            rotary_dim, None if stream is None else _handle(stream))
+    if _ops.qk_norm_rope_store(*args) is not None:
+        return q
     op = "qk_norm_rope_store"
     _require(q.dim() == 3 and k.dim() == 3 and v.dim() == 3,
              f"{op}: q must be (n_tokens, num_q_heads, head_dim), k and v (n_tokens, num_kv_heads, head_dim)")
@@ -363,16 +357,7 @@ def qk_norm_rope_store(q, k, v, q_weight, k_weight, positions, out_loc, k_cache,
     _require(k_cache.stride(0) == v_cache.stride(0), f"{op}: the two caches must share their row stride")
     _require(q.is_cuda and all(t.device == q.device for t in (k, v, positions, out_loc, k_cache, v_cache)),
              f"{op}: tensors must live on the same CUDA device")
-    rd = d if rotary_dim is None else int(rotary_dim)
-    sh = _stream_handle(stream, q.device)
-    with _on_device(q.device):
-        _lib.check(_lib.lib().msgl_qk_norm_rope_store(
-            q.data_ptr(), k.data_ptr(), v.data_ptr(),
-            q_weight.data_ptr() if q_weight is not None else None,
-            k_weight.data_ptr() if k_weight is not None else None,
-            positions.data_ptr(), out_loc.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(),
-            n, hq, hkv, d, rd, float(rope_base), float(eps), k_cache.shape[0],
-            q.stride(0), k.stride(0), v.stride(0), k_cache.stride(0), _DTYPES[q.dtype], sh))
+    _again(op, _ops.qk_norm_rope_store, q.device, *args)
     return q
 
 
