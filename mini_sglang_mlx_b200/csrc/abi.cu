@@ -188,20 +188,21 @@ bool make_query_tensor_map(CUtensorMap* out, const void* q, int total_q, int num
 
 // Launches `kernel` so that its CTAs may be scheduled while the previous kernel of the
 // stream drains (programmatic dependent launch); the kernel itself waits for the previous
-// kernel's memory with griddepcontrol.wait before it reads anything that kernel wrote.
-template <typename P, typename K>
-cudaError_t launch_dependent(K kernel, dim3 grid, dim3 block, cudaStream_t s, const P& params) {
+// kernel's memory with griddepcontrol.wait before it touches global memory.
+template <typename... P, typename... A>
+cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                             const A&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
-  cfg.dynamicSmemBytes = 0;
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kernel, params);
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
 // ---- prefill scheduling decision (shared by the workspace query and the launch)
@@ -315,6 +316,8 @@ __global__ void store_kv_kernel(unsigned char* __restrict__ kc, unsigned char* _
                                 int64_t cache_row_bytes, int64_t input_row_bytes,
                                 int64_t num_slots, int* status) {
   using V = typename std::conditional<VEC_BYTES == 16, uint4, uint2>::type;
+  msgl::grid_dependency_wait();
+  msgl::grid_dependency_launch();
   const int64_t total = static_cast<int64_t>(length) * vec_per_row;
   for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < total;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
@@ -585,8 +588,7 @@ int launch_decode(const msgl::DecodeParams& p, int head_dim, cudaStream_t s, con
   auto launch = [&](auto k1, int smem) -> int {
     cudaError_t e = allow_smem(k1, smem);
     if (e != cudaSuccess) return cuda_fail("paged_decode_attention", e);
-    k1<<<grid1, kDecWarps * 32, smem, s>>>(p, tm_k, tm_v);
-    e = cudaGetLastError();
+    e = launch_dependent(k1, grid1, dim3(kDecWarps * 32), smem, s, p, tm_k, tm_v);
     if (e != cudaSuccess) return cuda_fail("paged_decode_attention", e);
     return MSGL_OK;
   };
@@ -927,9 +929,10 @@ static int prefill_impl(const void* q, const void* k_cache, const void* v_cache,
   auto launch = [&](auto kernel, auto merge, int threads, int smem) -> cudaError_t {
     cudaError_t err = allow_smem(kernel, smem);
     if (err != cudaSuccess) return err;
-    kernel<<<grid, threads, smem, s>>>(p, tm_k, tm_v, tm_q);
+    err = launch_dependent(kernel, grid, dim3(threads), smem, s, p, tm_k, tm_v, tm_q);
+    if (err != cudaSuccess) return err;
     if (pl.kv_chunk > 0 && !pl.fused_merge)
-      return launch_dependent(merge, dim3(grid.x, msgl::kMergeSlices), dim3(msgl::kMergeWarps * 32), s, p);
+      return launch_dependent(merge, dim3(grid.x, msgl::kMergeSlices), dim3(msgl::kMergeWarps * 32), 0, s, p);
     return cudaSuccess;
   };
   // per element type: head_dim 256 / short query blocks / long chunks, each per-token or paged
@@ -1025,17 +1028,11 @@ int msgl_store_kv_cache(void* k_cache, void* v_cache, const int32_t* indices, co
   if (sms <= 0) sms = 148;
   int64_t blocks = (total + threads - 1) / threads;
   if (blocks > static_cast<int64_t>(sms) * 16) blocks = static_cast<int64_t>(sms) * 16;
-  if (vec16)
-    store_kv_kernel<16><<<static_cast<unsigned>(blocks), threads, 0, s>>>(
-        static_cast<unsigned char*>(k_cache), static_cast<unsigned char*>(v_cache), indices,
-        static_cast<const unsigned char*>(k), static_cast<const unsigned char*>(v), length,
-        vec_per_row, crb, irb, num_slots, static_cast<int*>(status_word));
-  else
-    store_kv_kernel<8><<<static_cast<unsigned>(blocks), threads, 0, s>>>(
-        static_cast<unsigned char*>(k_cache), static_cast<unsigned char*>(v_cache), indices,
-        static_cast<const unsigned char*>(k), static_cast<const unsigned char*>(v), length,
-        vec_per_row, crb, irb, num_slots, static_cast<int*>(status_word));
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = launch_dependent(
+      vec16 ? store_kv_kernel<16> : store_kv_kernel<8>, dim3(static_cast<unsigned>(blocks)), dim3(threads), 0, s,
+      static_cast<unsigned char*>(k_cache), static_cast<unsigned char*>(v_cache), indices,
+      static_cast<const unsigned char*>(k), static_cast<const unsigned char*>(v), length, vec_per_row, crb, irb,
+      num_slots, static_cast<int*>(status_word));
   if (e != cudaSuccess) return cuda_fail("store_kv_cache", e);
   return MSGL_OK;
 }
@@ -1106,17 +1103,11 @@ int msgl_qk_norm_rope_store(void* q, const void* k, const void* v, const void* q
   if (items >= (1ll << 31)) return fail(MSGL_BAD_ARG, "qk_norm_rope_store: too many rows for one call");
   const int64_t want = (items + 15) / 16;
   const int n_ctas = static_cast<int>(std::min<int64_t>(want, static_cast<int64_t>(sms) * 16));
-  if (head_dim == 256) {
-    if (dtype == MSGL_DTYPE_BF16)
-      msgl::qk_norm_rope_store_kernel<__nv_bfloat16, 256><<<n_ctas, threads, 0, s>>>(p);
-    else
-      msgl::qk_norm_rope_store_kernel<__half, 256><<<n_ctas, threads, 0, s>>>(p);
-  } else if (dtype == MSGL_DTYPE_BF16) {
-    msgl::qk_norm_rope_store_kernel<__nv_bfloat16, 128><<<n_ctas, threads, 0, s>>>(p);
-  } else {
-    msgl::qk_norm_rope_store_kernel<__half, 128><<<n_ctas, threads, 0, s>>>(p);
-  }
-  cudaError_t e = cudaGetLastError();
+  auto* kernel = head_dim == 256 ? (dtype == MSGL_DTYPE_BF16 ? msgl::qk_norm_rope_store_kernel<__nv_bfloat16, 256>
+                                                             : msgl::qk_norm_rope_store_kernel<__half, 256>)
+                                 : (dtype == MSGL_DTYPE_BF16 ? msgl::qk_norm_rope_store_kernel<__nv_bfloat16, 128>
+                                                             : msgl::qk_norm_rope_store_kernel<__half, 128>);
+  cudaError_t e = launch_dependent(kernel, dim3(n_ctas), dim3(threads), 0, s, p);
   if (e != cudaSuccess) return cuda_fail("qk_norm_rope_store", e);
   return MSGL_OK;
 }

@@ -284,10 +284,17 @@ __device__ __forceinline__ void fence_proxy_async_smem() {
 __device__ __forceinline__ void fence_mbar_init() {
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
-// Programmatic dependent launch: block until the kernel this one depends on has finished
-// and its writes are visible (no-op when launched without the attribute).
+// Programmatic dependent launch.  Every kernel here is launched so that its CTAs may be resident
+// while the kernel in front of it in the stream drains: it sets up what is its own (shared memory,
+// barriers, tensor memory), then grid_dependency_wait() blocks until the kernel in front has
+// finished and its writes are visible (no-op when launched without the attribute), and only then
+// does it touch global memory or let the kernel behind it in (grid_dependency_launch).  So a kernel
+// that has started knows that everything but the one kernel in front of it is complete.
 __device__ __forceinline__ void grid_dependency_wait() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+__device__ __forceinline__ void grid_dependency_launch() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
 __host__ __device__ __forceinline__ int ceil_div(int a, int b) { return (a + b - 1) / b; }

@@ -112,6 +112,19 @@ __global__ void __launch_bounds__(NWARPS * 32)
 
   const int G = p.group;
   const T* __restrict__ q = static_cast<const T*>(p.q);
+  // ---- this warp group's own set-up, then the kernel in front
+  __shared__ uint64_t s_bar[PAGED ? NWARPS * NSTAGES : 1];
+  if constexpr (PAGED) {
+    if (threadIdx.x == 0) {
+      for (int i = 0; i < NWARPS * NSTAGES; ++i) mbar_init(smem_u32(&s_bar[i]), 1);
+      fence_mbar_init();
+      prefetch_tensormap(&tm_k);
+      prefetch_tensormap(&tm_v);
+    }
+    __syncthreads();
+  }
+  grid_dependency_wait();
+  grid_dependency_launch();
   // (issued before the sequence's length is looked up: the two round trips to memory overlap)
   // ---- Q fragments: rows = query heads of this KV head (rows >= G are zero)
   uint32_t qf[KSTEPS][4];
@@ -165,17 +178,6 @@ __global__ void __launch_bounds__(NWARPS * 32)
     else
       return swz_offset<CH>(row, chunk);
   };
-  __shared__ uint64_t s_bar[PAGED ? NWARPS * NSTAGES : 1];
-  if constexpr (PAGED) {
-    if (threadIdx.x == 0) {
-      for (int i = 0; i < NWARPS * NSTAGES; ++i) mbar_init(smem_u32(&s_bar[i]), 1);
-      fence_mbar_init();
-      prefetch_tensormap(&tm_k);
-      prefetch_tensormap(&tm_v);
-    }
-    __syncthreads();
-  }
-
   // group g of this warp covers tokens [t_begin + (g*NWARPS + warp)*16, +16)
   const int first = t_begin + warp * kDecodeGroupTokens;
   const int nsteps = first < t_end ? ceil_div(t_end - first, CTA_TOKENS) : 0;

@@ -475,6 +475,8 @@ __global__ void __launch_bounds__(TcShape<NSUB, HD, PAGED>::kThreads,
     tmem_relinquish();
   }
 
+  grid_dependency_wait();
+  grid_dependency_launch();
   ItemCoord it;
   const bool have_item =
       find_item<kTcThreads>(p, static_cast<int>(blockIdx.x), BM, reinterpret_cast<int*>(smem_raw), it);
@@ -1171,6 +1173,7 @@ template <typename T, int HD, int BM>
 __global__ void __launch_bounds__(kMergeWarps * 32) prefill_merge_kernel(const PrefillParams p) {
   __shared__ int s_scratch[4 * kSortedBatchMax];
   grid_dependency_wait();   // the partials come from the attention kernel
+  grid_dependency_launch();
   ItemCoord it;
   if (!find_item<kMergeWarps * 32>(p, static_cast<int>(blockIdx.x), BM, s_scratch, it)) return;
   const SeqShape sq = load_seq_shape(p, it.b, BM);

@@ -112,6 +112,8 @@ __global__ void __launch_bounds__(256) qk_norm_rope_store_kernel(const QkNormRop
 #pragma unroll
     for (int e = 0; e < E; ++e) freq[e] = exp2f(-p.log2_base * (static_cast<float>(2 * (f0 + e)) * inv_rd));
   }
+  grid_dependency_wait();
+  grid_dependency_launch();
   auto word = [](const Vec& v, int i) -> uint32_t { return reinterpret_cast<const uint32_t*>(&v)[i]; };
   auto from_bits2 = [](uint32_t v) -> uint64_t {
     const float2 f = Pair16<T>::from_bits(v);
