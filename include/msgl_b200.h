@@ -92,6 +92,14 @@ int msgl_device_sm_count(void);
 size_t msgl_decode_workspace_bytes(int batch, int num_q_heads, int head_dim, int max_kv_splits);
 
 /*
+ * As many bytes of scratch as the decode op can use for a batch of total_kv cached tokens (0 = not
+ * known).  The op lays the sequences of a KV head end to end and cuts them into equal shares, one or
+ * more per SM; with less scratch (down to msgl_decode_workspace_bytes) it makes fewer shares.
+ */
+size_t msgl_decode_workspace_bytes_full(int batch, int num_q_heads, int num_kv_heads, int head_dim,
+                                        int max_kv_splits, int64_t total_kv);
+
+/*
  * Paged decode attention: one query token per sequence over all of its KV
  * tokens, split over the KV range; the piece of a (sequence, KV head) that
  * finishes last merges the partials by log-sum-exp (one launch).
@@ -177,6 +185,18 @@ int msgl_paged_decode_attention_gated(
     const void* gate, void* out, void* workspace, size_t workspace_bytes,
     int batch, int num_q_heads, int num_kv_heads, int head_dim, int64_t num_slots,
     int dtype, float sm_scale, int max_kv_splits, void* stream);
+
+/*
+ * The same op told how many KV tokens the batch has (total_kv = kv_indptr[batch], which the entries
+ * above cannot know on the host): a long batch is then cut into more shares than the GPU takes at once,
+ * so that the launch ends evenly.  gate may be NULL.
+ */
+int msgl_paged_decode_attention_sized(const void* q, const void* k_cache, const void* v_cache,
+                                      const int32_t* kv_indptr, const int32_t* kv_indices, const void* gate,
+                                      void* out, void* workspace, size_t workspace_bytes, int batch,
+                                      int num_q_heads, int num_kv_heads, int head_dim, int64_t num_slots,
+                                      int dtype, float sm_scale, int max_kv_splits, int64_t total_kv,
+                                      void* stream);
 
 /*
  * Bytes of scratch the prefill op needs for the given problem (split-KV
@@ -387,6 +407,48 @@ int msgl_qk_norm_rope_store(void* q, const void* k, const void* v, const void* q
                             float rope_base, float eps, int64_t num_slots, int64_t q_token_stride,
                             int64_t k_token_stride, int64_t v_token_stride,
                             int64_t cache_row_stride, int dtype, void* stream);
+
+/*
+ * One attention layer's work on a step's new tokens as one call: their K/V rows go into the pool
+ * (plainly, or after the q/k RMSNorm and rotary embedding of msgl_qk_norm_rope_store), then the
+ * attention op runs.  Same results as the two calls one after the other; the attention kernel,
+ * knowing what is in front of it, finds its work and starts on the older K/V rows while the rows are
+ * being stored.  The index arrays, out_loc and positions must be complete when the call's kernels
+ * reach the front of the stream, i.e. written by earlier work of that stream (or synchronised with it).
+ */
+typedef struct msgl_new_rows {
+  const void* k;                 /* (n_tokens, num_kv_heads, head_dim), dense heads */
+  const void* v;
+  const int32_t* out_loc;        /* (n_tokens) pool slots */
+  int n_tokens;
+  int64_t k_token_stride, v_token_stride; /* elements */
+  int project;                   /* 0: store k and v; 1: normalise and rotate q (in place) and k first */
+  const void* q_weight;          /* project: norm weights (head_dim) or NULL */
+  const void* k_weight;
+  const int32_t* positions;      /* project: (n_tokens) */
+  int rotary_dim;
+  float rope_base, eps;
+} msgl_new_rows;
+
+/*
+ * kv_lens NULL: indptr / indices are kv_indptr / per-token kv_indices and `total` is the number of KV
+ * tokens (page_size is ignored).  kv_lens given: page_indptr / page_indices of pages of page_size
+ * tokens (a multiple of 16), `total` is the number of pages.  gate may be NULL.  Workspace as for
+ * msgl_decode_workspace_bytes(_full).
+ */
+int msgl_decode_layer(const msgl_new_rows* rows, void* q, void* k_cache, void* v_cache,
+                      const int32_t* indptr, const int32_t* indices, const int32_t* kv_lens,
+                      const void* gate, void* out, void* workspace, size_t workspace_bytes, int batch,
+                      int num_q_heads, int num_kv_heads, int head_dim, int64_t num_slots, int dtype,
+                      float sm_scale, int max_kv_splits, int page_size, int64_t total, void* stream);
+
+int msgl_prefill_layer(const msgl_new_rows* rows, void* q, void* k_cache, void* v_cache,
+                       const int32_t* qo_indptr, const int32_t* indptr, const int32_t* indices,
+                       const int32_t* kv_lens, const int32_t* prefix_lens, const void* gate, void* out,
+                       void* workspace, size_t workspace_bytes, int batch, int total_q, int num_q_heads,
+                       int num_kv_heads, int head_dim, int64_t num_slots, int dtype, float sm_scale,
+                       int max_len_extend, int is_cross_attention, int sliding_window_size,
+                       int page_size, int64_t total, void* stream);
 
 #ifdef __cplusplus
 }

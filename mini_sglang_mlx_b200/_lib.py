@@ -25,6 +25,9 @@ SIGNATURES = {
     "msgl_last_error_string": (C.c_char_p, []),
     "msgl_device_sm_count": (_i, []),
     "msgl_decode_workspace_bytes": (_sz, [_i, _i, _i, _i]),
+    "msgl_decode_workspace_bytes_full": (_sz, [_i, _i, _i, _i, _i, _i64]),
+    "msgl_paged_decode_attention_sized": (
+        _i, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _sz, _i, _i, _i, _i, _i64, _i, _f, _i, _i64, _vp]),
     "msgl_paged_decode_attention": (
         _i, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _sz, _i, _i, _i, _i, _i64, _i, _f, _i, _vp]),
     "msgl_paged_decode_attention_gated": (
@@ -55,6 +58,12 @@ SIGNATURES = {
     "msgl_paged_prefill_attention": (
         _i, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _sz, _i, _i, _i64, _i, _i, _i, _i64,
              _i, _f, _i, _i, _i, _vp]),
+    "msgl_decode_layer": (
+        _i, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _sz, _i, _i, _i, _i, _i64, _i, _f, _i, _i,
+             _i64, _vp]),
+    "msgl_prefill_layer": (
+        _i, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _sz, _i, _i, _i, _i, _i, _i64, _i,
+             _f, _i, _i, _i, _i, _i64, _vp]),
     "msgl_store_kv_cache": (_i, [_vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i64, _i64, _i64, _i, _vp, _vp]),
     "msgl_gather_kv_indices": (_i, [_vp, _i64, _vp, _vp, _vp, _i, _i64, _i64, _i64, _vp, _vp]),
     "msgl_fast_compare_key": (_i64, [_vp, _vp, _i64, _i64, _i]),

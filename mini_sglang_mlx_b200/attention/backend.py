@@ -34,6 +34,7 @@ import torch
 from .. import _lib
 from ..kernel import (_ops, build_attn_metadata, paged_decode_attention, paged_decode_attention_p16,
                       paged_prefill_attention, paged_prefill_attention_p16, qk_norm_rope_store)
+from ..kvcache.mha_pool import MHAKVCache
 
 MAX_KV_SPLITS = 32
 
@@ -130,6 +131,7 @@ class AttnBackend:
         # 16-row boxes; other page sizes keep the per-token ids
         self._paged_ops = self.page_size % 16 == 0
         self._index_page = self.page_size if self._paged_ops else 1
+        self._own_pool = type(kvcache) is MHAKVCache   # a pool of another class keeps its own store_kv
         self._sm_count: Optional[int] = None
         self._staging: List[torch.Tensor] = []        # pinned (3, capacity) int32 buffers, in turn
         self._staging_events: List[torch.cuda.Event] = []
@@ -151,10 +153,36 @@ class AttnBackend:
         assert sliding_window_size >= 0, (
             f"sliding_window_size must be >= 0, got {sliding_window_size}")
         metadata = batch.attn_metadata
+        if self._own_pool:
+            k_cache = self.kvcache.k_cache(layer_id)
+            v_cache = self.kvcache.v_cache(layer_id)
+            out = self._layer(q, k, v, k_cache, v_cache, batch.out_loc, None, metadata, is_cross_attention,
+                              sliding_window_size, gate)
+            if out is not None:
+                return out
         self.kvcache.store_kv(k, v, batch.out_loc, layer_id)
         k_cache = self.kvcache.k_cache(layer_id)
         v_cache = self.kvcache.v_cache(layer_id)
         return self._attend(q, k_cache, v_cache, metadata, is_cross_attention, sliding_window_size, gate)
+
+    def _layer(self, q, k, v, k_cache, v_cache, out_loc, projection, metadata, is_cross_attention: bool,
+               sliding_window_size: int, gate):
+        """K/V store and attention as one native call (the attention kernel starts while the rows
+        are being stored); None where it does not take the arguments."""
+        ps = metadata.page_size
+        paged = self._paged_ops and metadata.page_indices is not None
+        if paged:
+            indptr, indices, lens = metadata.page_indptr, metadata.page_indices, metadata.kv_lens
+        else:
+            indptr, indices, lens = metadata.kv_indptr, metadata.kv_indices, None
+        if isinstance(metadata, PrefillMetadata):
+            return _ops.prefill_layer(q, k, v, k_cache, v_cache, out_loc, projection, metadata.qo_indptr, indptr,
+                                      indices, lens, metadata.prefix_lens, self.sm_scale, metadata.max_len_extend,
+                                      ps, is_cross_attention, sliding_window_size, gate)
+        if is_cross_attention or sliding_window_size:
+            return None
+        return _ops.decode_layer(q, k, v, k_cache, v_cache, out_loc, projection, indptr, indices, lens,
+                                 self.sm_scale, metadata.max_kv_splits, ps, gate)
 
     def _attend(self, q, k_cache, v_cache, metadata, is_cross_attention: bool,
                 sliding_window_size: int, gate=None) -> torch.Tensor:
@@ -199,6 +227,11 @@ class AttnBackend:
         metadata = batch.attn_metadata
         k_cache = self.kvcache.k_cache(layer_id)
         v_cache = self.kvcache.v_cache(layer_id)
+        out = self._layer(q, k, v, k_cache, v_cache, batch.out_loc,
+                          (q_norm_weight, k_norm_weight, metadata.positions, rope_base, rms_norm_eps, rotary_dim),
+                          metadata, is_cross_attention, sliding_window_size, gate)
+        if out is not None:
+            return out
         qk_norm_rope_store(q, k, v, q_norm_weight, k_norm_weight, metadata.positions, batch.out_loc,
                            k_cache, v_cache, rope_base=rope_base, eps=rms_norm_eps, rotary_dim=rotary_dim)
         return self._attend(q, k_cache, v_cache, metadata, is_cross_attention, sliding_window_size, gate)

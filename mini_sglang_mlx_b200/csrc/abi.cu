@@ -310,14 +310,16 @@ __global__ void bounded_wait_selftest_kernel(int* status, long long limit_cycles
 // ---- small data-movement kernels
 template <int VEC_BYTES>
 __global__ void store_kv_kernel(unsigned char* __restrict__ kc, unsigned char* __restrict__ vc,
-                                const int32_t* __restrict__ indices,
-                                const unsigned char* __restrict__ k,
-                                const unsigned char* __restrict__ v, int length, int vec_per_row,
+                                const int32_t* indices, const unsigned char* k,
+                                const unsigned char* v, int length, int vec_per_row,
                                 int64_t cache_row_bytes, int64_t input_row_bytes,
                                 int64_t num_slots, int* status) {
   using V = typename std::conditional<VEC_BYTES == 16, uint4, uint2>::type;
   msgl::grid_dependency_wait();
   msgl::grid_dependency_launch();
+  indices = msgl::after_wait(indices);
+  k = msgl::after_wait(k);
+  v = msgl::after_wait(v);
   const int64_t total = static_cast<int64_t>(length) * vec_per_row;
   for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < total;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
@@ -580,29 +582,44 @@ __global__ void expand_page_indices_kernel(const int32_t* __restrict__ page_indp
   }
 }
 
+// ---- decode scheduling (shared by the workspace query and the launch), in groups of 16 tokens
+constexpr int kDecMinShare = 8;      // below, a warp has one group or two and the merge dominates
+constexpr int kDecMaxShare = 256;
+// A segment's end (merge of the warps, partial, next Q) takes about as long as two groups of each of
+// the four warps, five at head_dim 256 with its twice as long rows and one CTA per SM.
+constexpr int kDecPad128 = 8, kDecPad256 = 20;
+
+// Shares per KV head that fill the GPU's CTA slots once (two CTAs per SM, one at head_dim 256) ...
+int decode_wave(int num_kv_heads, int head_dim, int sms) {
+  return std::max(1, sms * (head_dim == 256 ? 1 : 2) / num_kv_heads);
+}
+// ... and at most: more where a share would exceed kDecMaxShare, because a long launch then ends
+// evenly (the hardware hands the next share to whichever SM is done).
+int64_t decode_shares(int num_kv_heads, int head_dim, int batch, int64_t total_kv, int sms) {
+  const int64_t groups = total_kv / msgl::kDecodeGroupTokens + static_cast<int64_t>(batch) * (1 + kDecPad256);
+  return std::max<int64_t>(decode_wave(num_kv_heads, head_dim, sms), (groups + kDecMaxShare - 1) / kDecMaxShare);
+}
+
 template <typename T>
 int launch_decode(const msgl::DecodeParams& p, int head_dim, cudaStream_t s, const CUtensorMap& tm_k,
                   const CUtensorMap& tm_v) {
-  dim3 grid1(p.max_splits, p.hkv, p.batch);
+  const dim3 grid(static_cast<unsigned>((p.num_shares > 0 ? p.num_shares : p.batch) * p.hkv));
   const bool paged = p.kv_lens != nullptr;
-  auto launch = [&](auto k1, int smem) -> int {
-    cudaError_t e = allow_smem(k1, smem);
+  auto launch = [&](auto kernel) -> int {
+    const int smem = msgl::decode_smem_bytes(head_dim, kDecWarps, kDecStages);
+    cudaError_t e = allow_smem(kernel, smem);
     if (e != cudaSuccess) return cuda_fail("paged_decode_attention", e);
-    e = launch_dependent(k1, grid1, dim3(kDecWarps * 32), smem, s, p, tm_k, tm_v);
+    e = launch_dependent(kernel, grid, dim3(kDecWarps * 32), smem, s, p, tm_k, tm_v);
     if (e != cudaSuccess) return cuda_fail("paged_decode_attention", e);
     return MSGL_OK;
   };
-  // page-granular: the same ring plus the slack that puts it on a 1024-byte boundary
-  if (head_dim == 128) {
-    constexpr int smem = kDecWarps * kDecStages * 2 * msgl::kDecodeGroupTokens * 256;
-    return paged ? launch(msgl::decode_partial_kernel<T, 128, kDecWarps, kDecStages, true>, smem + 1024)
-                 : launch(msgl::decode_partial_kernel<T, 128, kDecWarps, kDecStages>, smem);
-  }
-  // head_dim 256: 512-byte token rows, 16 KB per stage
-  constexpr int kStages256 = 3;   // 192 KB of the 227 KB: one CTA per SM, three 16-token groups in flight per warp
-  constexpr int smem = kDecWarps * kStages256 * 2 * msgl::kDecodeGroupTokens * 512;
-  return paged ? launch(msgl::decode_partial_kernel<T, 256, kDecWarps, kStages256, true>, smem + 1024)
-               : launch(msgl::decode_partial_kernel<T, 256, kDecWarps, kStages256>, smem);
+  // three 16-token groups in flight per warp: 96 KB of ring and two CTAs per SM at head_dim 128,
+  // 192 KB and one CTA at 256
+  if (head_dim == 128)
+    return paged ? launch(msgl::decode_kernel<T, 128, kDecWarps, kDecStages, true>)
+                 : launch(msgl::decode_kernel<T, 128, kDecWarps, kDecStages, false>);
+  return paged ? launch(msgl::decode_kernel<T, 256, kDecWarps, kDecStages, true>)
+               : launch(msgl::decode_kernel<T, 256, kDecWarps, kDecStages, false>);
 }
 
 // Page-granular addressing of a call (null: per-token kv_indptr / kv_indices).
@@ -641,12 +658,26 @@ size_t msgl_decode_workspace_bytes(int batch, int num_q_heads, int head_dim, int
          rows * sizeof(float);
 }
 
+// As many bytes as a call can use: with fewer (down to msgl_decode_workspace_bytes) it cuts the
+// sequences into fewer shares.
+size_t msgl_decode_workspace_bytes_full(int batch, int num_q_heads, int num_kv_heads, int head_dim,
+                                        int max_kv_splits, int64_t total_kv) {
+  const size_t least = msgl_decode_workspace_bytes(batch, num_q_heads, head_dim, max_kv_splits);
+  if (batch <= 0 || num_q_heads <= 0 || num_kv_heads <= 0 || head_dim <= 0 || max_kv_splits <= 0) return least;
+  const int sms = sm_count_cached();
+  const size_t rows = static_cast<size_t>(decode_shares(num_kv_heads, head_dim, batch, total_kv,
+                                                        sms > 0 ? sms : 148) + batch) *
+                      num_q_heads;
+  return std::max(least, kStatusBytes + decode_ticket_bytes(batch, num_q_heads) + rows * msgl::decode_partial_floats(head_dim) * sizeof(float));
+}
+
 static int decode_impl(const void* q, const void* k_cache, const void* v_cache,
                        const int32_t* kv_indptr, const int32_t* kv_indices,
-                       const int32_t* num_kv_splits, const void* gate, void* out, void* workspace,
-                       size_t workspace_bytes, int batch, int num_q_heads, int num_kv_heads,
+                       const void* gate, void* out, void* workspace, size_t workspace_bytes,
+                       int batch, int num_q_heads, int num_kv_heads,
                        int head_dim, int64_t num_slots, int dtype, float sm_scale,
-                       int max_kv_splits, void* stream, const PageIndex* pages = nullptr) {
+                       int max_kv_splits, int64_t total_kv, void* stream, const PageIndex* pages = nullptr,
+                       const msgl_new_rows* new_rows = nullptr) {
   const char* op = "paged_decode_attention: ";
   if (batch < 0 || num_q_heads <= 0 || num_kv_heads <= 0 || num_slots < 0)
     return fail(MSGL_BAD_SHAPE, std::string(op) + "q must be 3D (batch, num_q_heads, head_dim)");
@@ -679,25 +710,39 @@ static int decode_impl(const void* q, const void* k_cache, const void* v_cache,
   if (!workspace || workspace_bytes < need)
     return fail(MSGL_BAD_ARG, std::string(op) + "workspace too small");
 
+  const int sms = sm_count_cached();
+  if (sms <= 0) return fail(MSGL_CUDA_ERROR, std::string(op) + "cannot query the device");
+
   msgl::DecodeParams p{};
   p.q = q;
   p.k_cache = k_cache;
   p.v_cache = v_cache;
-  p.kv_indptr = kv_indptr;
-  p.kv_indices = kv_indices;
-  p.num_kv_splits = num_kv_splits;
-  if (pages) {
-    p.page_indptr = pages->page_indptr;
-    p.page_indices = pages->page_indices;
-    p.kv_lens = pages->kv_lens;
-    p.page_size = pages->page_size;
-  }
+  p.indptr = pages ? pages->page_indptr : kv_indptr;
+  p.indices = pages ? pages->page_indices : kv_indices;
+  p.kv_lens = pages ? pages->kv_lens : nullptr;
+  p.page_size = pages ? pages->page_size : 1;
   p.out = out;
   p.gate = gate;
+  p.batch = batch;
+  p.hq = num_q_heads;
+  p.hkv = num_kv_heads;
+  p.group = num_q_heads / num_kv_heads;
+  p.num_slots = num_slots;
+  p.scale_log2 = sm_scale * msgl::kLog2e;
+  p.min_share = kDecMinShare;
+  p.max_share = kDecMaxShare;
+  p.pad = head_dim == 256 ? kDecPad256 : kDecPad128;
+  p.wave = decode_wave(num_kv_heads, head_dim, sms);
   unsigned char* ws = static_cast<unsigned char*>(workspace);
   p.status = reinterpret_cast<int*>(ws);
   const size_t own_tickets = decode_ticket_bytes(batch, num_q_heads);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  // (counters of its own are cleared in between: then the store is not the kernel in front)
+  p.num_new = -1;
+  if (new_rows && new_rows->n_tokens <= msgl::kDecodeNewMax && own_tickets == 0) {
+    p.new_slots = new_rows->out_loc;
+    p.num_new = new_rows->n_tokens;
+  }
   if (own_tickets == 0) {
     p.tickets = reinterpret_cast<int*>(ws + 256);
   } else {
@@ -705,15 +750,18 @@ static int decode_impl(const void* q, const void* k_cache, const void* v_cache,
     cudaError_t e = cudaMemsetAsync(p.tickets, 0, own_tickets, s);
     if (e != cudaSuccess) return cuda_fail("paged_decode_attention", e);
   }
-  p.part_o = reinterpret_cast<float*>(ws + kStatusBytes + own_tickets);
-  p.part_lse = p.part_o + static_cast<size_t>(batch) * num_q_heads * max_kv_splits * head_dim;
-  p.batch = batch;
-  p.hq = num_q_heads;
-  p.hkv = num_kv_heads;
-  p.group = num_q_heads / num_kv_heads;
-  p.max_splits = max_kv_splits;
-  p.num_slots = num_slots;
-  p.scale_log2 = sm_scale * msgl::kLog2e;
+  // one partial row per query head, share and sequence (see the kernel's slot numbers): as many
+  // shares as the scratch holds; a scratch of one row per sequence takes whole sequences
+  const int64_t rows = static_cast<int64_t>((workspace_bytes - kStatusBytes - own_tickets) /
+                                            (msgl::decode_partial_floats(head_dim) * sizeof(float)));
+  const int64_t want = decode_shares(num_kv_heads, head_dim, batch, total_kv, sms);
+  const int64_t room = rows / num_q_heads - batch;
+  int64_t shares = std::min(want, room);
+  if (shares < want && shares < batch) shares = 0;
+  if (std::max<int64_t>(shares, batch) * num_kv_heads > 0x7fffffffLL)
+    return fail(MSGL_BAD_SHAPE, std::string(op) + "problem too large for one launch");
+  p.num_shares = static_cast<int>(shares);
+  p.part = reinterpret_cast<float*>(ws + kStatusBytes + own_tickets);
   if (dtype == MSGL_DTYPE_BF16) return launch_decode<__nv_bfloat16>(p, head_dim, s, tm_k, tm_v);
   return launch_decode<__half>(p, head_dim, s, tm_k, tm_v);
 }
@@ -724,9 +772,10 @@ int msgl_paged_decode_attention(const void* q, const void* k_cache, const void* 
                                 size_t workspace_bytes, int batch, int num_q_heads,
                                 int num_kv_heads, int head_dim, int64_t num_slots, int dtype,
                                 float sm_scale, int max_kv_splits, void* stream) {
-  return decode_impl(q, k_cache, v_cache, kv_indptr, kv_indices, num_kv_splits, nullptr, out, workspace,
+  (void)num_kv_splits;   // hints: the shares take their place
+  return decode_impl(q, k_cache, v_cache, kv_indptr, kv_indices, nullptr, out, workspace,
                      workspace_bytes, batch, num_q_heads, num_kv_heads, head_dim, num_slots, dtype,
-                     sm_scale, max_kv_splits, stream);
+                     sm_scale, max_kv_splits, 0, stream);
 }
 
 int msgl_paged_decode_attention_gated(const void* q, const void* k_cache, const void* v_cache,
@@ -736,10 +785,23 @@ int msgl_paged_decode_attention_gated(const void* q, const void* k_cache, const 
                                       int num_q_heads, int num_kv_heads, int head_dim,
                                       int64_t num_slots, int dtype, float sm_scale,
                                       int max_kv_splits, void* stream) {
+  (void)num_kv_splits;
   if (!gate && batch > 0) return fail(MSGL_BAD_ARG, "paged_decode_attention: null gate pointer");
-  return decode_impl(q, k_cache, v_cache, kv_indptr, kv_indices, num_kv_splits, gate, out, workspace,
+  return decode_impl(q, k_cache, v_cache, kv_indptr, kv_indices, gate, out, workspace,
                      workspace_bytes, batch, num_q_heads, num_kv_heads, head_dim, num_slots, dtype,
-                     sm_scale, max_kv_splits, stream);
+                     sm_scale, max_kv_splits, 0, stream);
+}
+
+int msgl_paged_decode_attention_sized(const void* q, const void* k_cache, const void* v_cache,
+                                      const int32_t* kv_indptr, const int32_t* kv_indices, const void* gate,
+                                      void* out, void* workspace, size_t workspace_bytes, int batch,
+                                      int num_q_heads, int num_kv_heads, int head_dim, int64_t num_slots,
+                                      int dtype, float sm_scale, int max_kv_splits, int64_t total_kv,
+                                      void* stream) {
+  if (total_kv < 0) return fail(MSGL_BAD_ARG, "paged_decode_attention: total_kv must be >= 0");
+  return decode_impl(q, k_cache, v_cache, kv_indptr, kv_indices, gate, out, workspace, workspace_bytes, batch,
+                     num_q_heads, num_kv_heads, head_dim, num_slots, dtype, sm_scale, max_kv_splits, total_kv,
+                     stream);
 }
 
 int msgl_paged_decode_attention_static(const void* q, const void* k_cache, const void* v_cache,
@@ -841,7 +903,7 @@ static int prefill_impl(const void* q, const void* k_cache, const void* v_cache,
                         int64_t total_kv, int num_q_heads, int num_kv_heads, int head_dim,
                         int64_t num_slots, int dtype, float sm_scale, int max_len_extend,
                         int is_cross_attention, int sliding_window_size, void* stream,
-                        const PageIndex* pages = nullptr) {
+                        const PageIndex* pages = nullptr, bool behind_store = false) {
   const char* op = "paged_prefill_attention: ";
   if (total_q < 0 || num_q_heads <= 0 || num_kv_heads <= 0 || num_slots < 0 || total_kv < 0)
     return fail(MSGL_BAD_SHAPE,
@@ -921,6 +983,7 @@ static int prefill_impl(const void* q, const void* k_cache, const void* v_cache,
   p.is_cross = is_cross_attention ? 1 : 0;
   p.window = sliding_window_size;
   p.kv_chunk = pl.kv_chunk;
+  p.early = behind_store ? 1 : 0;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
 
   dim3 grid(static_cast<unsigned>(pl.items * num_kv_heads));
@@ -1162,6 +1225,7 @@ int msgl_paged_decode_attention_p16(const void* q, const void* k_cache, const vo
                                     int64_t num_slots, int dtype, float sm_scale, int max_kv_splits,
                                     int page_size, int64_t total_pages, void* stream) {
   const char* op = "paged_decode_attention_p16";
+  (void)num_kv_splits;   // hints: the shares take their place
   if (batch < 0 || num_q_heads <= 0 || head_dim <= 0 || max_kv_splits <= 0 || total_pages < 0 ||
       page_size <= 0)
     return fail(MSGL_BAD_SHAPE, std::string(op) + ": bad sizes");
@@ -1179,9 +1243,9 @@ int msgl_paged_decode_attention_p16(const void* q, const void* k_cache, const vo
     if (total_pages * page_size >= (1ll << 31))
       return fail(MSGL_BAD_SHAPE, std::string(op) + ": total_pages * page_size must be < 2^31");
     const PageIndex pages{page_indptr, page_indices, kv_lens, page_size};
-    return decode_impl(q, k_cache, v_cache, nullptr, nullptr, num_kv_splits, gate, out, workspace,
-                       op_ws, batch, num_q_heads, num_kv_heads, head_dim, num_slots, dtype, sm_scale,
-                       max_kv_splits, stream, &pages);
+    return decode_impl(q, k_cache, v_cache, nullptr, nullptr, gate, out, workspace, workspace_bytes, batch,
+                       num_q_heads, num_kv_heads, head_dim, num_slots, dtype, sm_scale, max_kv_splits,
+                       total_pages * page_size, stream, &pages);
   }
   const int32_t *kv_indptr = nullptr, *kv_indices = nullptr;
   int64_t bound = 0;
@@ -1189,9 +1253,9 @@ int msgl_paged_decode_attention_p16(const void* q, const void* k_cache, const vo
                              num_slots, static_cast<unsigned char*>(workspace) + op_ws,
                              static_cast<int*>(workspace), &kv_indptr, &kv_indices, &bound, stream);
   if (rc != MSGL_OK) return rc;
-  return decode_impl(q, k_cache, v_cache, kv_indptr, kv_indices, num_kv_splits, gate, out, workspace,
-                     op_ws, batch, num_q_heads, num_kv_heads, head_dim, num_slots, dtype, sm_scale,
-                     max_kv_splits, stream);
+  return decode_impl(q, k_cache, v_cache, kv_indptr, kv_indices, gate, out, workspace, op_ws, batch,
+                     num_q_heads, num_kv_heads, head_dim, num_slots, dtype, sm_scale, max_kv_splits, bound,
+                     stream);
 }
 
 size_t msgl_prefill_workspace_bytes_p16(int batch, int total_q, int64_t total_pages, int page_size,
@@ -1431,6 +1495,68 @@ int msgl_gather_kv_indices(const int32_t* page_table, int64_t table_row_stride,
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail("gather_kv_indices", e);
   return MSGL_OK;
+}
+
+// The K/V store of a layer call.
+static int store_new_rows(const msgl_new_rows* r, void* q, void* k_cache, void* v_cache, int num_q_heads,
+                          int num_kv_heads, int head_dim, int64_t num_slots, int dtype, void* status,
+                          void* stream) {
+  const int64_t row = static_cast<int64_t>(num_kv_heads) * head_dim;
+  if (r->project)
+    return msgl_qk_norm_rope_store(q, r->k, r->v, r->q_weight, r->k_weight, r->positions, r->out_loc, k_cache,
+                                   v_cache, r->n_tokens, num_q_heads, num_kv_heads, head_dim, r->rotary_dim,
+                                   r->rope_base, r->eps, num_slots, static_cast<int64_t>(num_q_heads) * head_dim,
+                                   r->k_token_stride, r->v_token_stride, row, dtype, stream);
+  if (r->k_token_stride != r->v_token_stride)
+    return fail(MSGL_BAD_SHAPE, "store_kv_cache: k/v must share their row stride");
+  return msgl_store_kv_cache(k_cache, v_cache, r->out_loc, r->k, r->v, r->n_tokens, num_kv_heads, head_dim,
+                             num_slots, row, r->k_token_stride, dtype, status, stream);
+}
+
+int msgl_decode_layer(const msgl_new_rows* rows, void* q, void* k_cache, void* v_cache, const int32_t* indptr,
+                      const int32_t* indices, const int32_t* kv_lens, const void* gate, void* out,
+                      void* workspace, size_t workspace_bytes, int batch, int num_q_heads, int num_kv_heads,
+                      int head_dim, int64_t num_slots, int dtype, float sm_scale, int max_kv_splits,
+                      int page_size, int64_t total, void* stream) {
+  if (!rows) return fail(MSGL_BAD_ARG, "paged_decode_attention: null rows");
+  if (total < 0) return fail(MSGL_BAD_SHAPE, "paged_decode_attention: negative size");
+  if (kv_lens && (page_size <= 0 || page_size % msgl::kTmaBoxRows != 0 || total * page_size >= (1ll << 31)))
+    return fail(MSGL_BAD_ARG, "paged_decode_attention: page_size must be a multiple of 16, with fewer than 2^31 "
+                              "tokens in all pages");
+  if (kv_lens && batch > 0 && (!indptr || (total > 0 && !indices)))
+    return fail(MSGL_BAD_ARG, "paged_decode_attention: null tensor pointer");
+  const int rc = store_new_rows(rows, q, k_cache, v_cache, num_q_heads, num_kv_heads, head_dim, num_slots, dtype,
+                                workspace, stream);
+  if (rc != MSGL_OK) return rc;
+  const PageIndex pages{indptr, indices, kv_lens, page_size};
+  return decode_impl(q, k_cache, v_cache, indptr, indices, gate, out, workspace, workspace_bytes, batch,
+                     num_q_heads, num_kv_heads, head_dim, num_slots, dtype, sm_scale, max_kv_splits,
+                     kv_lens ? total * page_size : total, stream, kv_lens ? &pages : nullptr,
+                     rows->n_tokens > 0 ? rows : nullptr);
+}
+
+int msgl_prefill_layer(const msgl_new_rows* rows, void* q, void* k_cache, void* v_cache,
+                       const int32_t* qo_indptr, const int32_t* indptr, const int32_t* indices,
+                       const int32_t* kv_lens, const int32_t* prefix_lens, const void* gate, void* out,
+                       void* workspace, size_t workspace_bytes, int batch, int total_q, int num_q_heads,
+                       int num_kv_heads, int head_dim, int64_t num_slots, int dtype, float sm_scale,
+                       int max_len_extend, int is_cross_attention, int sliding_window_size, int page_size,
+                       int64_t total, void* stream) {
+  if (!rows) return fail(MSGL_BAD_ARG, "paged_prefill_attention: null rows");
+  if (total < 0) return fail(MSGL_BAD_SHAPE, "paged_prefill_attention: negative size");
+  if (kv_lens && (page_size <= 0 || page_size % msgl::kTmaBoxRows != 0 || total * page_size >= (1ll << 31)))
+    return fail(MSGL_BAD_ARG, "paged_prefill_attention: page_size must be a multiple of 16, with fewer than 2^31 "
+                              "tokens in all pages");
+  if (kv_lens && batch > 0 && (!indptr || (total > 0 && !indices)))
+    return fail(MSGL_BAD_ARG, "paged_prefill_attention: null tensor pointer");
+  const int rc = store_new_rows(rows, q, k_cache, v_cache, num_q_heads, num_kv_heads, head_dim, num_slots, dtype,
+                                workspace, stream);
+  if (rc != MSGL_OK) return rc;
+  const PageIndex pages{indptr, indices, kv_lens, page_size};
+  return prefill_impl(q, k_cache, v_cache, qo_indptr, indptr, indices, prefix_lens, gate, out, workspace,
+                      workspace_bytes, batch, total_q, kv_lens ? total * page_size : total, num_q_heads,
+                      num_kv_heads, head_dim, num_slots, dtype, sm_scale, max_len_extend, is_cross_attention,
+                      sliding_window_size, stream, kv_lens ? &pages : nullptr, rows->n_tokens > 0);
 }
 
 }  // extern "C"

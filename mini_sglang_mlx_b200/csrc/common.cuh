@@ -44,6 +44,19 @@ __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
 }
 
+// All cp.async copies of this thread have landed.
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
+__device__ __forceinline__ void prefetch_l2(const void* p) {
+  asm volatile("prefetch.global.L2 [%0];" ::"l"(p) : "memory");
+}
+// Counts an arrival: what the CTA wrote before (this thread is behind a CTA barrier) is visible to
+// whoever sees the count, and what was written before the counts seen is visible here.
+__device__ __forceinline__ int atomic_add_acq_rel(int* p, int v) {
+  int old;
+  asm volatile("atom.add.acq_rel.gpu.global.s32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(v) : "memory");
+  return old;
+}
+
 // ---------------------------------------------------------------- ldmatrix / mma
 __device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], uint32_t addr) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
@@ -292,6 +305,13 @@ __device__ __forceinline__ void fence_mbar_init() {
 // that has started knows that everything but the one kernel in front of it is complete.
 __device__ __forceinline__ void grid_dependency_wait() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+// A pointer as it is known after the wait: no read through it moves in front of the wait, not even
+// one that the compiler takes for a read of constant memory.
+template <typename T>
+__device__ __forceinline__ T* after_wait(T* p) {
+  asm volatile("" : "+l"(p)::"memory");
+  return p;
 }
 __device__ __forceinline__ void grid_dependency_launch() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

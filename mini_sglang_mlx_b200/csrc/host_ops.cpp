@@ -176,19 +176,15 @@ PyObject* decode(PyObject*, PyObject* const* a, Py_ssize_t n) {
   size_t ws_bytes;
   if (!stream_of(a[9], s.device, &stream) ||
       !scratch_for(s.device, stream, kDecode,
-                   msgl_decode_workspace_bytes(s.n, s.hq, s.d, static_cast<int>(max_splits)), &ws, &ws_bytes))
+                   msgl_decode_workspace_bytes_full(s.n, s.hq, s.hkv, s.d, static_cast<int>(max_splits),
+                                                    indices.numel()),
+                   &ws, &ws_bytes))
     return nullptr;
   Tensor out = empty_like_rows(q);
-  void* st = reinterpret_cast<void*>(stream);
-  const int rc =
-      gate ? msgl_paged_decode_attention_gated(q.data_ptr(), kc.data_ptr(), vc.data_ptr(), i32(indptr),
-                                               i32(indices), i32(splits), gate, out.data_ptr(), ws, ws_bytes,
-                                               s.n, s.hq, s.hkv, s.d, s.num_slots, s.dtype,
-                                               static_cast<float>(scale), static_cast<int>(max_splits), st)
-           : msgl_paged_decode_attention(q.data_ptr(), kc.data_ptr(), vc.data_ptr(), i32(indptr), i32(indices),
-                                         i32(splits), out.data_ptr(), ws, ws_bytes, s.n, s.hq, s.hkv, s.d,
-                                         s.num_slots, s.dtype, static_cast<float>(scale),
-                                         static_cast<int>(max_splits), st);
+  const int rc = msgl_paged_decode_attention_sized(
+      q.data_ptr(), kc.data_ptr(), vc.data_ptr(), i32(indptr), i32(indices), gate, out.data_ptr(), ws, ws_bytes,
+      s.n, s.hq, s.hkv, s.d, s.num_slots, s.dtype, static_cast<float>(scale), static_cast<int>(max_splits),
+      indices.numel(), reinterpret_cast<void*>(stream));
   return rc ? raise_status(rc) : THPVariable_Wrap(std::move(out));
 }
 
@@ -212,7 +208,8 @@ PyObject* decode_paged(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (page_size <= 0) Py_RETURN_NONE;
   const int64_t total_pages = pages.numel();
   const size_t need =
-      (msgl_decode_workspace_bytes(s.n, s.hq, s.d, static_cast<int>(max_splits)) + 255) / 256 * 256 +
+      (msgl_decode_workspace_bytes_full(s.n, s.hq, s.hkv, s.d, static_cast<int>(max_splits),
+                                        total_pages * page_size) + 255) / 256 * 256 +
       msgl_page_index_workspace_bytes(s.n, total_pages, static_cast<int>(page_size));
   int64_t stream;
   void* ws;
@@ -395,6 +392,148 @@ PyObject* qk_norm_rope_store(PyObject*, PyObject* const* a, Py_ssize_t n) {
   Py_RETURN_TRUE;
 }
 
+// ------------------------------------------------------------------ a layer's new tokens, store and attention
+// k, v, out_loc and projection (None, or (q_weight, k_weight, positions, rope_base, eps, rotary_dim or
+// None)) of a layer call -> *rows.  1: fine, 0: not what the native call takes, -1: a Python error.
+int new_rows(PyObject* ko, PyObject* vo, PyObject* loco, PyObject* proj, const Tensor& q, const Shapes& s,
+             msgl_new_rows* r) {
+  if (!is_tensor(ko) || !is_tensor(vo) || !is_tensor(loco)) return 0;
+  const Tensor &k = THPVariable_Unpack(ko), &v = THPVariable_Unpack(vo), &loc = THPVariable_Unpack(loco);
+  const c10::Device dev = q.device();
+  if (k.dim() != 3 || v.sizes() != k.sizes() || k.size(1) != s.hkv || k.size(2) != s.d ||
+      k.scalar_type() != q.scalar_type() || v.scalar_type() != q.scalar_type() || k.device() != dev ||
+      v.device() != dev || !rows_dense(k, s.d) || !rows_dense(v, s.d) || !index_ok(loc, dev) ||
+      loc.numel() != k.size(0))
+    return 0;
+  *r = msgl_new_rows{};
+  r->k = k.data_ptr();
+  r->v = v.data_ptr();
+  r->out_loc = i32(loc);
+  r->n_tokens = static_cast<int>(k.size(0));
+  r->k_token_stride = k.stride(0);
+  r->v_token_stride = v.stride(0);
+  if (proj == Py_None) return r->k_token_stride == r->v_token_stride ? 1 : 0;
+  if (!PyTuple_Check(proj) || PyTuple_GET_SIZE(proj) != 6 || k.size(0) != s.n) return 0;
+  r->project = 1;
+  const void** weights[2] = {&r->q_weight, &r->k_weight};
+  for (int i = 0; i < 2; ++i) {
+    PyObject* o = PyTuple_GET_ITEM(proj, i);
+    if (o == Py_None) continue;
+    if (!is_tensor(o)) return 0;
+    const Tensor& w = THPVariable_Unpack(o);
+    if (w.scalar_type() != q.scalar_type() || w.device() != dev || w.dim() != 1 || w.size(0) != s.d ||
+        !w.is_contiguous())
+      return 0;
+    *weights[i] = w.data_ptr();
+  }
+  if (!is_tensor(PyTuple_GET_ITEM(proj, 2))) return 0;
+  const Tensor& pos = THPVariable_Unpack(PyTuple_GET_ITEM(proj, 2));
+  if (!index_ok(pos, dev) || pos.numel() != s.n) return 0;
+  r->positions = i32(pos);
+  r->rope_base = static_cast<float>(PyFloat_AsDouble(PyTuple_GET_ITEM(proj, 3)));
+  r->eps = static_cast<float>(PyFloat_AsDouble(PyTuple_GET_ITEM(proj, 4)));
+  PyObject* rd = PyTuple_GET_ITEM(proj, 5);
+  r->rotary_dim = rd == Py_None ? s.d : static_cast<int>(PyLong_AsLong(rd));
+  return PyErr_Occurred() ? -1 : 1;
+}
+
+// (q, k, v, k_cache, v_cache, out_loc, projection, indptr, indices, kv_lens or None, sm_scale,
+//  max_kv_splits, page_size, gate)
+PyObject* decode_layer(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  if (n != 14) return PyErr_Format(PyExc_TypeError, "decode_layer takes 14 arguments");
+  if (!is_tensor(a[0]) || !is_tensor(a[3]) || !is_tensor(a[4]) || !is_tensor(a[7]) || !is_tensor(a[8]))
+    Py_RETURN_NONE;
+  const Tensor &q = THPVariable_Unpack(a[0]), &kc = THPVariable_Unpack(a[3]), &vc = THPVariable_Unpack(a[4]),
+               &indptr = THPVariable_Unpack(a[7]), &indices = THPVariable_Unpack(a[8]);
+  Shapes s;
+  const void* gate;
+  if (!attention_shapes(q, kc, vc, &s) || !index_ok(indptr, q.device()) || !index_ok(indices, q.device()) ||
+      indptr.numel() != s.n + 1 || !gate_ptr(a[13], q, &gate))
+    Py_RETURN_NONE;
+  const int32_t* lens = nullptr;
+  if (a[9] != Py_None) {
+    if (!is_tensor(a[9])) Py_RETURN_NONE;
+    const Tensor& t = THPVariable_Unpack(a[9]);
+    if (!index_ok(t, q.device()) || t.numel() != s.n) Py_RETURN_NONE;
+    lens = i32(t);
+  }
+  msgl_new_rows rows;
+  const int fine = new_rows(a[1], a[2], a[5], a[6], q, s, &rows);
+  if (fine < 0) return nullptr;
+  if (fine == 0) Py_RETURN_NONE;
+  ARG_FLOAT(scale, a[10]);
+  ARG_INT(max_splits, a[11]);
+  ARG_INT(page_size, a[12]);
+  const int64_t total = indices.numel();
+  int64_t stream;
+  void* ws;
+  size_t ws_bytes;
+  if (!stream_of(Py_None, s.device, &stream) ||
+      !scratch_for(s.device, stream, kDecode,
+                   msgl_decode_workspace_bytes_full(s.n, s.hq, s.hkv, s.d, static_cast<int>(max_splits),
+                                                    lens ? total * page_size : total),
+                   &ws, &ws_bytes))
+    return nullptr;
+  Tensor out = empty_like_rows(q);
+  const int rc = msgl_decode_layer(&rows, q.data_ptr(), kc.data_ptr(), vc.data_ptr(), i32(indptr), i32(indices),
+                                   lens, gate, out.data_ptr(), ws, ws_bytes, s.n, s.hq, s.hkv, s.d, s.num_slots,
+                                   s.dtype, static_cast<float>(scale), static_cast<int>(max_splits),
+                                   static_cast<int>(page_size), total, reinterpret_cast<void*>(stream));
+  return rc ? raise_status(rc) : THPVariable_Wrap(std::move(out));
+}
+
+// (q, k, v, k_cache, v_cache, out_loc, projection, qo_indptr, indptr, indices, kv_lens or None,
+//  prefix_lens, sm_scale, max_len_extend, page_size, is_cross_attention, sliding_window_size, gate)
+PyObject* prefill_layer(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  if (n != 18) return PyErr_Format(PyExc_TypeError, "prefill_layer takes 18 arguments");
+  for (int i : {0, 3, 4, 7, 8, 9, 11})
+    if (!is_tensor(a[i])) Py_RETURN_NONE;
+  const Tensor &q = THPVariable_Unpack(a[0]), &kc = THPVariable_Unpack(a[3]), &vc = THPVariable_Unpack(a[4]),
+               &qo = THPVariable_Unpack(a[7]), &indptr = THPVariable_Unpack(a[8]),
+               &indices = THPVariable_Unpack(a[9]), &prefix = THPVariable_Unpack(a[11]);
+  Shapes s;
+  const void* gate;
+  if (!attention_shapes(q, kc, vc, &s) || !index_ok(qo, q.device()) || !index_ok(indptr, q.device()) ||
+      !index_ok(indices, q.device()) || !index_ok(prefix, q.device()) || qo.numel() < 2 ||
+      indptr.numel() != qo.numel() || prefix.numel() + 1 != qo.numel() || !gate_ptr(a[17], q, &gate))
+    Py_RETURN_NONE;
+  const int batch = static_cast<int>(prefix.numel());
+  const int32_t* lens = nullptr;
+  if (a[10] != Py_None) {
+    if (!is_tensor(a[10])) Py_RETURN_NONE;
+    const Tensor& t = THPVariable_Unpack(a[10]);
+    if (!index_ok(t, q.device()) || t.numel() != batch) Py_RETURN_NONE;
+    lens = i32(t);
+  }
+  msgl_new_rows rows;
+  const int fine = new_rows(a[1], a[2], a[5], a[6], q, s, &rows);
+  if (fine < 0) return nullptr;
+  if (fine == 0) Py_RETURN_NONE;
+  ARG_FLOAT(scale, a[12]);
+  ARG_INT(max_ext, a[13]);
+  ARG_INT(page_size, a[14]);
+  ARG_INT(window, a[16]);
+  const int cross = PyObject_IsTrue(a[15]);
+  if (cross < 0) return nullptr;
+  const int64_t total = indices.numel();
+  int64_t stream;
+  void* ws;
+  size_t ws_bytes;
+  if (!stream_of(Py_None, s.device, &stream) ||
+      !scratch_for(s.device, stream, kPrefill,
+                   msgl_prefill_workspace_bytes(batch, s.n, lens ? total * page_size : total, s.hq, s.hkv, s.d,
+                                                static_cast<int>(max_ext), static_cast<int>(window)),
+                   &ws, &ws_bytes))
+    return nullptr;
+  Tensor out = empty_like_rows(q);
+  const int rc = msgl_prefill_layer(
+      &rows, q.data_ptr(), kc.data_ptr(), vc.data_ptr(), i32(qo), i32(indptr), i32(indices), lens, i32(prefix), gate,
+      out.data_ptr(), ws, ws_bytes, batch, s.n, s.hq, s.hkv, s.d, s.num_slots, s.dtype, static_cast<float>(scale),
+      static_cast<int>(max_ext), cross, static_cast<int>(window), static_cast<int>(page_size), total,
+      reinterpret_cast<void*>(stream));
+  return rc ? raise_status(rc) : THPVariable_Wrap(std::move(out));
+}
+
 // ------------------------------------------------------------------ index arrays of a step
 PyObject *g_s_row, *g_s_cached, *g_s_device, *g_s_extend;   // interned attribute names
 
@@ -560,7 +699,8 @@ PyObject* set_workspace_maker(PyObject*, PyObject* fn) {
 #define FAST(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(name)), METH_FASTCALL, nullptr}
 PyMethodDef kMethods[] = {FAST(decode),       FAST(decode_paged),       FAST(prefill),
                           FAST(prefill_paged), FAST(store_kv),          FAST(qk_norm_rope_store),
-                          FAST(collect_lens), FAST(index_arrays),
+                          FAST(decode_layer), FAST(prefill_layer),     FAST(collect_lens),
+                          FAST(index_arrays),
                           {"set_workspace_maker", set_workspace_maker, METH_O, nullptr},
                           {nullptr, nullptr, 0, nullptr}};
 PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_host", "Host side of the operators.", -1, kMethods,

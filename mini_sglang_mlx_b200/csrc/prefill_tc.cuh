@@ -475,11 +475,12 @@ __global__ void __launch_bounds__(TcShape<NSUB, HD, PAGED>::kThreads,
     tmem_relinquish();
   }
 
-  grid_dependency_wait();
-  grid_dependency_launch();
+  if (!p.early) grid_dependency_wait();
   ItemCoord it;
   const bool have_item =
       find_item<kTcThreads>(p, static_cast<int>(blockIdx.x), BM, reinterpret_cast<int*>(smem_raw), it);
+  if (p.early) grid_dependency_wait();   // the item is found while the K/V store drains
+  grid_dependency_launch();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();

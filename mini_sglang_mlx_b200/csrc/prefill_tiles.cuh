@@ -51,6 +51,7 @@ struct PrefillParams {
   float scale_log2;
   int is_cross, window;
   int kv_chunk;  // tokens per kv split; 0 = never split
+  int early;     // the kernel in front is this call's own K/V store: the index arrays are complete
 };
 
 struct SeqShape {
