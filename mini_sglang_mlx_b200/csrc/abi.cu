@@ -14,6 +14,7 @@
 
 #include "../../include/msgl_b200.h"
 #include "decode_splitkv.cuh"
+#include "prefill_pair.cuh"
 #include "prefill_tc.cuh"
 #include "qk_norm_rope.cuh"
 
@@ -190,19 +191,27 @@ bool make_query_tensor_map(CUtensorMap* out, const void* q, int total_q, int num
 // stream drains (programmatic dependent launch); the kernel itself waits for the previous
 // kernel's memory with griddepcontrol.wait before it touches global memory.
 template <typename... P, typename... A>
-cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
-                             const A&... args) {
+cudaError_t launch_clusters(int cluster, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                            const A&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = cluster;
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
   return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+template <typename... P, typename... A>
+cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                             const A&... args) {
+  return launch_clusters(1, kernel, grid, block, smem, s, args...);
 }
 
 // ---- prefill scheduling decision (shared by the workspace query and the launch)
@@ -220,6 +229,16 @@ struct PrefillPlan {
 // output accumulator alone takes 256 of the 512 TMEM columns), one CTA per SM.
 bool prefill_short_q(int max_len_extend, int group, int head_dim) {
   return head_dim == 256 || static_cast<int64_t>(max_len_extend) * group <= msgl::kTcSub;
+}
+
+// Pairs of CTAs: head_dim 256, query blocks of more than one 128-row tile, key range not split.
+bool prefill_pairs(int max_len_extend, int group, int head_dim, int kv_chunk) {
+#ifdef MSGL_PAIR128
+  const bool hd = true;
+#else
+  const bool hd = head_dim == 256;
+#endif
+  return hd && kv_chunk == 0 && static_cast<int64_t>(max_len_extend) * group > msgl::kTcSub;
 }
 
 PrefillPlan plan_prefill(int batch, int total_q, int64_t total_kv, int hq, int hkv, int head_dim,
@@ -987,6 +1006,12 @@ static int prefill_impl(const void* q, const void* k_cache, const void* v_cache,
   cudaStream_t s = static_cast<cudaStream_t>(stream);
 
   dim3 grid(static_cast<unsigned>(pl.items * num_kv_heads));
+  const bool pair = prefill_pairs(max_len_extend, p.group, head_dim, pl.kv_chunk);
+  if (pair) {
+    const int64_t pairs = msgl::prefill_item_bound(batch, total_q, total_kv, p.group, 256, max_len_extend, 0) * num_kv_heads;
+    if (pairs * 2 > 0x7fffffffLL) return fail(MSGL_BAD_SHAPE, std::string(op) + "problem too large for one launch");
+    grid = dim3(static_cast<unsigned>(pairs * 2));
+  }
   const bool short_q = prefill_short_q(max_len_extend, p.group, head_dim);
   cudaError_t e;
   auto launch = [&](auto kernel, auto merge, int threads, int smem) -> cudaError_t {
@@ -1007,6 +1032,21 @@ static int prefill_impl(const void* q, const void* k_cache, const void* v_cache,
     using P1 = msgl::TcShape<1, 128, true>;
     using P2 = msgl::TcShape<2, 128, true>;
     using P1w = msgl::TcShape<1, 256, true>;
+    if (pair) {
+      auto go = [&](auto kernel, auto shape) -> cudaError_t {
+        using S = decltype(shape);
+        const cudaError_t err = allow_smem(kernel, S::kSmemBytes);
+        if (err != cudaSuccess) return err;
+        return launch_clusters(2, kernel, grid, dim3(S::kThreads), S::kSmemBytes, s, p, tm_k, tm_v, tm_q);
+      };
+#ifdef MSGL_PAIR128
+      if (head_dim == 128)
+        return pages ? go(msgl::prefill_pair_kernel<T, 128, true>, msgl::PairShape<128, true>{})
+                     : go(msgl::prefill_pair_kernel<T, 128, false>, msgl::PairShape<128, false>{});
+#endif
+      return pages ? go(msgl::prefill_pair_kernel<T, 256, true>, msgl::PairShape<256, true>{})
+                   : go(msgl::prefill_pair_kernel<T, 256, false>, msgl::PairShape<256, false>{});
+    }
     auto m1w = msgl::prefill_merge_kernel<T, 256, S1w::kBM>;
     auto m1 = msgl::prefill_merge_kernel<T, 128, S1::kBM>;
     auto m2 = msgl::prefill_merge_kernel<T, 128, S2::kBM>;

@@ -151,7 +151,9 @@ __device__ __forceinline__ float to_f32(__half x) { return __half2float(x); }
 template <typename T>
 __device__ __forceinline__ T apply_gate(float out, T gate) {
   const float o = to_f32(MmaOp<T>::from_float(out));
-  const float s = to_f32(MmaOp<T>::from_float(1.f / (1.f + __expf(-to_f32(gate)))));
+  // (a fast division, two units in the last place of fp32, in front of a rounding to 16 bits: the exact one
+  // took most of a 128-row epilogue, 38 us at head_dim 256)
+  const float s = to_f32(MmaOp<T>::from_float(__fdividef(1.f, 1.f + __expf(-to_f32(gate)))));
   return MmaOp<T>::from_float(o * s);
 }
 
@@ -203,6 +205,9 @@ __device__ __forceinline__ void mbar_inval(uint32_t bar) {
 }
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive_n(uint32_t bar, uint32_t count) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(count) : "memory");
 }
 __device__ __forceinline__ uint32_t mbar_try_wait(uint32_t bar, uint32_t parity) {
   uint32_t ok;
@@ -315,6 +320,18 @@ __device__ __forceinline__ T* after_wait(T* p) {
 }
 __device__ __forceinline__ void grid_dependency_launch() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+// One lane of a converged warp (the same lane every time for a full mask).
+__device__ __forceinline__ uint32_t elect_one() {
+  uint32_t pred = 0;
+  asm volatile(
+      "{\n\t.reg .b32 rx;\n\t.reg .pred px;\n\t"
+      "elect.sync rx|px, %1;\n\t"
+      "@px mov.s32 %0, 1;\n\t}"
+      : "+r"(pred)
+      : "r"(0xFFFFFFFFu));
+  return pred;
 }
 
 __host__ __device__ __forceinline__ int ceil_div(int a, int b) { return (a + b - 1) / b; }

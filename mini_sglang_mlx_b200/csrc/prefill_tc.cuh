@@ -218,18 +218,6 @@ __device__ __forceinline__ void tmem_ld32_at(uint32_t taddr, uint32_t (&r)[N]) {
       : "memory");
 }
 
-// One lane of a converged warp (the same lane every time for a full mask).
-__device__ __forceinline__ uint32_t elect_one() {
-  uint32_t pred = 0;
-  asm volatile(
-      "{\n\t.reg .b32 rx;\n\t.reg .pred px;\n\t"
-      "elect.sync rx|px, %1;\n\t"
-      "@px mov.s32 %0, 1;\n\t}"
-      : "+r"(pred)
-      : "r"(0xFFFFFFFFu));
-  return pred;
-}
-
 // Shared-memory matrix descriptor, 128-byte swizzle, descriptor version 1.
 // lbo / sbo are byte offsets (leading / stride dimension).
 __device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t addr, uint32_t lbo, uint32_t sbo) {
@@ -454,9 +442,9 @@ __global__ void __launch_bounds__(TcShape<NSUB, HD, PAGED>::kThreads,
     mbar_init(bar_q, q_tma ? 1 : NPROD);
     mbar_init(smem_u32(&bars.idx_sync), NPROD);
     for (int bf = 0; bf < kTcBufs; ++bf) {
-      // PAGED: the 32 lanes of the copying warp (their cp.async arrivals) + the arrival that
+      // PAGED: per copying warp its 32 lanes (their cp.async arrivals) + the arrival that
       // announces the TMA bytes
-      mbar_init(bar_full(bf), PAGED ? 33 : NPROD);
+      mbar_init(bar_full(bf), PAGED ? (NPROD / 32) * 33 : NPROD);
       mbar_init(bar_empty(bf), 1);
     }
     for (int i = 0; i < NSUB; ++i) {
@@ -587,7 +575,13 @@ __global__ void __launch_bounds__(TcShape<NSUB, HD, PAGED>::kThreads,
     bool alive = true;
     if constexpr (PAGED) {
       // ------------------------------------------------ page-granular: TMA boxes from the page ids
-      if (warp == kTcProducerWarp0) {
+      // All producer warps issue, a share of a tile's boxes each, one elected lane with warp-uniform
+      // operands: one warp gets a 2 KB box in every 67 cycles (31 B/clk per SM, measured from L2 with
+      // 1 or 148 SMs at work alike; 93 cycles when every lane issues its own box), two warps 63 B/clk,
+      // four 74 to 80, and a 128-key step of two sub-tiles wants 64 KB in about 2500 cycles.
+      {
+        constexpr int NPW = Shape::kWarps - kTcProducerWarp0;   // producer warps
+        const int pw = warp - kTcProducerWarp0;
         constexpr int PPT = BN / kTmaBoxRows;            // boxes (= lanes at work) per tile
         constexpr int NQ = HD / 64;                      // 128-byte column blocks of a token row
         constexpr uint32_t kBoxBytes = kTmaBoxRows * 128;
@@ -623,19 +617,34 @@ __global__ void __launch_bounds__(TcShape<NSUB, HD, PAGED>::kThreads,
           if (!alive) return;
           const uint32_t dst = ring + bf * kTcKvTileBytes;
           const uint32_t bar = bar_full(bf);
-          const bool full = n == kTmaBoxRows;
-          const uint32_t full_mask = __ballot_sync(0xffffffffu, full);
-          if (lane == 0) mbar_arrive_expect_tx(bar, __popc(full_mask) * (kTmaBoxRows * HD * 2));
-          __syncwarp();
-          if (full) {
-#pragma unroll
-            for (int c = 0; c < NQ; ++c)
-              tma_load_2d(dst + c * (BN * 128) + lane * kBoxBytes, tm, x0 + c * 64, y, bar);
-          }
+          const uint32_t full_mask = __ballot_sync(0xffffffffu, n == kTmaBoxRows);
           uint32_t rest = ~full_mask & ((1u << PPT) - 1u);
+          // box k of this warp: page (pw + k * NPW) % PPT, column block (pw + k * NPW) / PPT
+          constexpr int MINE = (PPT * NQ + NPW - 1) / NPW;
+          int yk[MINE], boxes = 0;
+#pragma unroll
+          for (int k = 0; k < MINE; ++k) {
+            const int id = pw + k * NPW;
+            yk[k] = __shfl_sync(0xffffffffu, y, id % PPT);
+            if (id >= PPT * NQ || ((full_mask >> (id % PPT)) & 1u) == 0) yk[k] = -1;
+            boxes += yk[k] >= 0 ? 1 : 0;
+          }
+          if (elect_one()) {
+            mbar_arrive_expect_tx(bar, boxes * kBoxBytes);
+#pragma unroll
+            for (int k = 0; k < MINE; ++k) {
+              const int id = pw + k * NPW;
+              if (yk[k] >= 0)
+                tma_load_2d(dst + (id / PPT) * (BN * 128) + (id % PPT) * kBoxBytes, tm, x0 + (id / PPT) * 64, yk[k], bar);
+            }
+            if (rest == 0) mbar_arrive_n(bar, 32);     // (else the lanes arrive behind their own copies)
+          }
+          __syncwarp();
+          const bool ragged = rest != 0;
           while (rest) {   // warp-uniform
             const int i = __ffs(rest) - 1;
             rest &= rest - 1;
+            if (i % NPW != pw) continue;
             const int yi = __shfl_sync(0xffffffffu, y, i), ni = __shfl_sync(0xffffffffu, n, i);
 #pragma unroll
             for (int k = 0; k < kTmaBoxRows * CPR / 32; ++k) {
@@ -648,7 +657,7 @@ __global__ void __launch_bounds__(TcShape<NSUB, HD, PAGED>::kThreads,
                           ok ? 16 : 0);
             }
           }
-          cp_async_mbar_arrive(bar);
+          if (ragged) cp_async_mbar_arrive(bar);
           issued_seq = seq;
         };
         // window of the boxes of tiles j .. j+LA (tile j: V next, tile j+LA: K next)
