@@ -125,23 +125,23 @@ EncodeTiledFn tensor_map_encoder() {
 }
 
 // 2-D map over a pool (num_slots rows of num_kv_heads * head_dim 16-bit elements): a box is
-// 16 token rows x 64 elements (128 bytes) of one head, written to shared memory with the
+// box_rows (16, or 1 for tile::gather4) token rows x 64 elements (128 bytes) of one head, written to shared memory with the
 // 128-byte swizzle, i.e. in the layout the tensor-core descriptors of the kernels expect.
 // Rows outside the pool read as zeros.  The maps are kept per thread, one per hash of the pool's
 // address: a model's layers each have two pools and go through them in turn.
 bool make_pool_tensor_map(CUtensorMap* out, const void* base, int64_t num_slots, int num_kv_heads,
-                          int head_dim, int dtype) {
+                          int head_dim, int dtype, int box_rows = msgl::kTmaBoxRows) {
   struct Cached {
     const void* base;
     int64_t num_slots;
-    int hkv, hd, dtype;
+    int hkv, hd, dtype, rows;
     CUtensorMap map;
   };
   static thread_local Cached cache[256] = {};
   const uintptr_t key = reinterpret_cast<uintptr_t>(base) >> 8;
-  Cached& c = cache[(key ^ (key >> 8) ^ (key >> 16) ^ (key >> 24)) % 256];
+  Cached& c = cache[(key ^ (key >> 8) ^ (key >> 16) ^ (key >> 24) ^ (box_rows * 8)) % 256];
   if (c.base == base && c.num_slots == num_slots && c.hkv == num_kv_heads && c.hd == head_dim &&
-      c.dtype == dtype && base != nullptr) {
+      c.dtype == dtype && c.rows == box_rows && base != nullptr) {
     *out = c.map;
     return true;
   }
@@ -150,7 +150,7 @@ bool make_pool_tensor_map(CUtensorMap* out, const void* base, int64_t num_slots,
   const cuuint64_t dims[2] = {static_cast<cuuint64_t>(num_kv_heads) * head_dim,
                               static_cast<cuuint64_t>(num_slots)};
   const cuuint64_t strides[1] = {static_cast<cuuint64_t>(num_kv_heads) * head_dim * 2};
-  const cuuint32_t box[2] = {64, static_cast<cuuint32_t>(msgl::kTmaBoxRows)};
+  const cuuint32_t box[2] = {64, static_cast<cuuint32_t>(box_rows)};
   const cuuint32_t elem_strides[2] = {1, 1};
   CUtensorMap m;
   const CUresult r = enc(&m, dtype == MSGL_DTYPE_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16
@@ -159,7 +159,7 @@ bool make_pool_tensor_map(CUtensorMap* out, const void* base, int64_t num_slots,
                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                          CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return false;
-  c = Cached{base, num_slots, num_kv_heads, head_dim, dtype, m};
+  c = Cached{base, num_slots, num_kv_heads, head_dim, dtype, box_rows, m};
   *out = m;
   return true;
 }
@@ -185,6 +185,21 @@ bool make_query_tensor_map(CUtensorMap* out, const void* q, int total_q, int num
                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                          CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS;
+}
+
+// 2-D map over the query rows (tokens x heads, head_dim) for tile::gather4: a box is one row x 64 elements.
+bool make_query_row_map(CUtensorMap* out, const void* q, int total_q, int num_q_heads, int head_dim, int dtype) {
+  EncodeTiledFn enc = tensor_map_encoder();
+  const int64_t rows = static_cast<int64_t>(total_q) * num_q_heads;
+  if (!enc || rows <= 0 || rows >= (1ll << 31) || reinterpret_cast<uintptr_t>(q) % 16 != 0) return false;
+  const cuuint64_t dims[2] = {static_cast<cuuint64_t>(head_dim), static_cast<cuuint64_t>(rows)};
+  const cuuint64_t strides[1] = {static_cast<cuuint64_t>(head_dim) * 2};
+  const cuuint32_t box[2] = {64, 1};
+  const cuuint32_t elem_strides[2] = {1, 1};
+  return enc(out, dtype == MSGL_DTYPE_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2,
+             const_cast<void*>(q), dims, strides, box, elem_strides, CU_TENSOR_MAP_INTERLEAVE_NONE,
+             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 // Launches `kernel` so that its CTAs may be scheduled while the previous kernel of the
@@ -1006,7 +1021,17 @@ static int prefill_impl(const void* q, const void* k_cache, const void* v_cache,
   cudaStream_t s = static_cast<cudaStream_t>(stream);
 
   dim3 grid(static_cast<unsigned>(pl.items * num_kv_heads));
-  const bool pair = prefill_pairs(max_len_extend, p.group, head_dim, pl.kv_chunk);
+  bool pair = prefill_pairs(max_len_extend, p.group, head_dim, pl.kv_chunk) && num_slots < (1ll << 31);
+  CUtensorMap tg_k, tg_v;
+  if (pair) {
+    // everything by TMA: boxes of pages, rows of pools and queries by gather
+    pair = make_pool_tensor_map(&tg_k, k_cache, num_slots, num_kv_heads, head_dim, dtype, 1) &&
+           make_pool_tensor_map(&tg_v, v_cache, num_slots, num_kv_heads, head_dim, dtype, 1);
+    if (pair && !pages)
+      p.q_tma = make_query_tensor_map(&tm_q, q, total_q, num_q_heads, p.group, head_dim, dtype) ? 1 : 0;
+    if (pair && !p.q_tma) pair = make_query_row_map(&tm_q, q, total_q, num_q_heads, head_dim, dtype);
+    if (!pair && !pages) p.q_tma = 0;
+  }
   if (pair) {
     const int64_t pairs = msgl::prefill_item_bound(batch, total_q, total_kv, p.group, 256, max_len_extend, 0) * num_kv_heads;
     if (pairs * 2 > 0x7fffffffLL) return fail(MSGL_BAD_SHAPE, std::string(op) + "problem too large for one launch");
@@ -1037,7 +1062,7 @@ static int prefill_impl(const void* q, const void* k_cache, const void* v_cache,
         using S = decltype(shape);
         const cudaError_t err = allow_smem(kernel, S::kSmemBytes);
         if (err != cudaSuccess) return err;
-        return launch_clusters(2, kernel, grid, dim3(S::kThreads), S::kSmemBytes, s, p, tm_k, tm_v, tm_q);
+        return launch_clusters(2, kernel, grid, dim3(S::kThreads), S::kSmemBytes, s, p, tm_k, tm_v, tg_k, tg_v, tm_q);
       };
 #ifdef MSGL_PAIR128
       if (head_dim == 128)

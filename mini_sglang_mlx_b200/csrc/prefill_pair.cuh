@@ -11,14 +11,28 @@
 //   O   += P[j] V_j   M 256, N head_dim: CTA r holds columns [r head_dim / 2, ...) of the V tile
 //
 // The MMAs are issued by the leader (rank 0) and fill both CTAs' tensor memory; a commit signals both.
-// S has two buffers and runs two key tiles ahead of PV, so the softmax warps never wait for the tensor
-// pipe.  TMEM columns: S[b] at 128 b, O at 256.
+// S has LA buffers and runs LA key tiles ahead of PV, so the softmax warps do not wait for the tensor
+// pipe.  TMEM columns: S[b] at 128 b, O behind them: LA = 2 at head_dim 256, 3 at 128.
 //
-//   warps 0-3   softmax: thread r owns row r of this CTA's half (TMEM lane r)
-//   warp 4      MMA issuer (leader)
-//   warp 5      relay: a buffer that is full here is announced to the leader, behind the proxy fence
-//               that its generic-proxy copies (ragged pages, per-token rows) need
-//   warps 6 ..  producers: one warp issues TMA boxes (PAGED), ten gather per-token rows
+// At head_dim 128 two softmax groups take the tiles in turn: the 128 x 128 exponentials of a tile are
+// 1024 cycles of the special-function unit, and one group alone needs 2140 for the tile (score load 240,
+// row maximum 240, exponentials 1290, hand-over and waits 370), twice what the tensor pipe does.  Both
+// add to one O, so a row's reference maximum goes from tile to tile: a group publishes it as soon as it
+// has the tile's row maximum, and the other group, which is half a tile behind, picks it up.  (With an O
+// and an S buffer for each group there is no third S buffer, and a group waits 1440 cycles per tile for
+// PV and the next S: 1995 cycles per tile.)  At head_dim 256 one group keeps up with the tensor pipe (2048
+// cycles per tile).
+//
+//   warps 0-3 (0-7)   softmax: thread r of a group owns row r of this CTA's half (TMEM lane r)
+//   next warp         MMA issuer (leader)
+//   next six warps    producers, three for the K tiles and three for the V tiles
+//
+// Everything arrives by TMA and is counted in bytes on the leader's barrier, from both CTAs
+// (.cta_group::2): full pages as boxes of 16 rows, anything else (per-token slots, a sequence's ragged
+// last page, query rows whose heads do not divide 128) as tile::gather4 loads of four rows, where an
+// absent row is one past the end of the tensor and reads as zeros.  Six producers because a warp
+// issues one TMA instruction in about 67 cycles: with two, and the tiles announced to the leader by a
+// relay warp, the MMA warp waited 1200 cycles per tile for K and V.
 //
 // Tile layouts are those of prefill_tc.cuh (128-byte swizzle; K tile [head_dim/64][64 rows][128 B],
 // V tile [head_dim/128][128 rows][128 B], Q tile [head_dim/64][128 rows][128 B]).  Every wait is bounded.
@@ -37,10 +51,16 @@ struct PairShape {
   static constexpr int kBufBytes = kBN * HD;              // half a K (or V) tile
   static constexpr int kBufs = 128 * 1024 / kBufBytes;    // 4 at head_dim 256, 8 at 128
   static constexpr int kSmemBytes = kQBytes + kBufs * kBufBytes + 1024;
-  static constexpr int kMmaWarp = 4, kRelayWarp = 5, kProducerWarp0 = 6;
-  static constexpr int kWarps = PAGED ? 8 : 16;
+  static constexpr int kGroups = HD == 128 ? 2 : 1;       // softmax groups
+  static constexpr int kMmaWarp = 4 * kGroups, kProducerWarp0 = kMmaWarp + 1;
+  static constexpr int kKindWarps = 3;                    // producers of K, and of V
+  static constexpr int kWarps = kMmaWarp + 8;             // (one idle: whole warpgroups for setmaxnreg)
+  // registers moved from the other warps to the softmax warps: 512 threads at 128, 384 at 168
+  static constexpr int kSoftRegs = kGroups == 2 ? 192 : 200;
+  static constexpr int kOtherRegs = kGroups == 2 ? 64 : 144;
   static constexpr int kThreads = kWarps * 32;
-  static constexpr int kOCol = 2 * kBN;
+  static constexpr int kLA = kGroups == 2 ? 3 : 2;        // S buffers = tiles S runs ahead
+  static constexpr int kOCol = kLA * kBN;
 };
 
 // ---------------------------------------------------------------- cluster and cta_group::2 wrappers
@@ -52,41 +72,47 @@ __device__ __forceinline__ uint32_t cluster_rank() {
 __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-// Arrival on the barrier at this address in CTA `rank` of the cluster.
-__device__ __forceinline__ void mbar_arrive_at(uint32_t bar, uint32_t rank) {
+// Address of this shared-memory address in CTA `rank` of the cluster.
+__device__ __forceinline__ uint32_t cluster_addr(uint32_t addr, uint32_t rank) {
+  uint32_t ra;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(addr), "r"(rank));
+  return ra;
+}
+// Arrivals on a barrier of either CTA, without memory ordering of their own (a release at cluster scope
+// took 600 to 1300 cycles): tensor memory is ordered by the tcgen05 fences on both sides, and bytes
+// that TMA counts on the barrier itself.
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_bar) {
+  asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive_expect_tx_cluster(uint32_t cluster_bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.relaxed.cluster.shared::cluster.b64 _, [%0], %1;" ::"r"(cluster_bar), "r"(bytes)
+               : "memory");
+}
+// TMA into this CTA's shared memory, counted on a barrier of either CTA of the pair.
+__device__ __forceinline__ void tma_pair_2d(uint32_t dst, const CUtensorMap* tmap, int x, int y, uint32_t cluster_bar) {
   asm volatile(
-      "{\n\t.reg .b32 ra;\n\t"
-      "mapa.shared::cluster.u32 ra, %0, %1;\n\t"
-      "mbarrier.arrive.release.cluster.shared::cluster.b64 _, [ra];\n\t}" ::"r"(bar),
-      "r"(rank)
+      "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2 "
+      "[%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
+      "l"(reinterpret_cast<uint64_t>(tmap)), "r"(x), "r"(y), "r"(cluster_bar)
       : "memory");
 }
-__device__ __forceinline__ uint32_t mbar_try_wait_cluster(uint32_t bar, uint32_t parity) {
-  uint32_t ok;
+__device__ __forceinline__ void tma_pair_3d(uint32_t dst, const CUtensorMap* tmap, int x, int y, int z,
+                                            uint32_t cluster_bar) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.b32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
+      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2 "
+      "[%0], [%1, {%2, %3, %4}], [%5];" ::"r"(dst),
+      "l"(reinterpret_cast<uint64_t>(tmap)), "r"(x), "r"(y), "r"(z), "r"(cluster_bar)
       : "memory");
-  return ok;
 }
-// Bounded, warp-uniform wait for arrivals from either CTA (see mbar_wait_limit).
-__device__ __forceinline__ bool mbar_wait_warp_cluster(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
-  bool ok = mbar_try_wait_cluster(bar, parity) != 0;
-  if (!ok) {
-    const long long t0 = clock64();
-    while (true) {
-      ok = mbar_try_wait_cluster(bar, parity) != 0;
-      if (ok) break;
-      if (*abort_flag != 0 || clock64() - t0 > kTcWaitCycles) {
-        *abort_flag = 1;
-        break;
-      }
-    }
-  }
-  return __all_sync(0xffffffffu, ok ? 1 : 0) != 0;
+// four rows of 64 elements (one-row boxes), 512 bytes
+__device__ __forceinline__ void tma_pair_gather4(uint32_t dst, const CUtensorMap* tmap, int x, const int (&rows)[4],
+                                                 uint32_t cluster_bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.shared::cluster.global.tile::gather4.mbarrier::complete_tx::bytes.cta_group::2 "
+      "[%0], [%1, {%2, %3, %4, %5, %6}], [%7];" ::"r"(dst),
+      "l"(reinterpret_cast<uint64_t>(tmap)), "r"(x), "r"(rows[0]), "r"(rows[1]), "r"(rows[2]), "r"(rows[3]),
+      "r"(cluster_bar)
+      : "memory");
 }
 __device__ __forceinline__ void tmem_alloc_pair(uint32_t smem_dst, uint32_t ncols) {
   asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_dst), "r"(ncols)
@@ -129,55 +155,56 @@ __device__ __forceinline__ uint32_t idesc_m256(uint32_t n, uint32_t b_mn) {
   return (idesc_m128<T>(n, b_mn) & ~(0x1fu << 24)) | ((256u >> 4) << 24);
 }
 
+// Barrier of the 256 threads of both softmax groups.
+__device__ __forceinline__ void softmax_groups_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
+
 struct PairBarriers {
-  uint64_t q_full, q_pair;               // Q of this CTA / of both (leader)
-  uint64_t full[8], pair_full[8], empty[8];
-  uint64_t s_full[2], p_full[2], pv_done[2];
-  uint64_t idx_sync;                     // per-token form: the producers' own barrier
+  uint64_t q_full, full[8];              // leader: both CTAs' copies
+  uint64_t empty[8];
+  uint64_t s_full[3], p_full[3], pv_done[3];
+  uint64_t m_ref[2][4];                  // [tile parity][warp of the group]: the reference maxima are published
 };
 
 template <typename T, int HD, bool PAGED>
 __global__ void __launch_bounds__(PairShape<HD, PAGED>::kThreads, 1)
     prefill_pair_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap tm_k,
-                        const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_q) {
+                        const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tg_k,
+                        const __grid_constant__ CUtensorMap tg_v, const __grid_constant__ CUtensorMap tm_q) {
   using Shape = PairShape<HD, PAGED>;
   constexpr int BM = Shape::kBM, BN = Shape::kBN, ROWS = Shape::kRows, NB = Shape::kBufs;
   constexpr int KEYS = BN / 2;                  // keys of a K tile in this CTA
   constexpr int CH = HD / 8;                    // 16-byte chunks of a token row
-  constexpr int VCH = CH / 2;                   // ... of its half of a V row
-  constexpr int NPROD = (Shape::kWarps - Shape::kProducerWarp0) * 32;
+  constexpr int NKW = Shape::kKindWarps;
+  constexpr int NG = Shape::kGroups, LA = Shape::kLA;
 
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ PairBarriers bars;
   __shared__ uint32_t s_tmem_base;
   __shared__ int s_abort;
-  __shared__ int s_slots[PAGED ? 1 : 3 * BN];   // slot ids of the key tiles being copied / next to copy
+  __shared__ float2 s_ml[NG == 2 ? 2 * ROWS : 1];        // (reference maximum, sum) of the rows, per group
+  __shared__ float s_mref[NG == 2 ? 2 * ROWS : 1];       // reference maxima after the even / odd tiles
 
   const int tid = threadIdx.x;
   const int warp = tid >> 5, lane = tid & 31;
   const int G = p.group;
   const int rank = static_cast<int>(cluster_rank());
-  const bool q_tma = PAGED && p.q_tma != 0;
 
   auto bar_full = [&](int bf) { return smem_u32(&bars.full[bf]); };
-  auto bar_pair = [&](int bf) { return smem_u32(&bars.pair_full[bf]); };
   auto bar_empty = [&](int bf) { return smem_u32(&bars.empty[bf]); };
   auto bar_s = [&](int b) { return smem_u32(&bars.s_full[b]); };
   auto bar_p = [&](int b) { return smem_u32(&bars.p_full[b]); };
   auto bar_pv = [&](int b) { return smem_u32(&bars.pv_done[b]); };
-  const uint32_t bar_q = smem_u32(&bars.q_full), bar_qp = smem_u32(&bars.q_pair);
+  const uint32_t bar_q = smem_u32(&bars.q_full);
 
   if (tid == 0) {
     s_abort = 0;
-    mbar_init(bar_q, q_tma ? 1 : Shape::kThreads);
-    mbar_init(bar_qp, 2);
-    mbar_init(smem_u32(&bars.idx_sync), NPROD);
+    mbar_init(bar_q, 2 * 2 * NKW);
     for (int bf = 0; bf < NB; ++bf) {
-      mbar_init(bar_full(bf), PAGED ? (NPROD / 32) * 33 : NPROD);   // (33: see prefill_tc.cuh)
-      mbar_init(bar_pair(bf), 2);
+      mbar_init(bar_full(bf), 2 * NKW);         // the producers of its kind in both CTAs
       mbar_init(bar_empty(bf), 1);
     }
-    for (int b = 0; b < 2; ++b) {
+    for (int e = 0; e < 8; ++e) mbar_init(smem_u32(&bars.m_ref[e >> 2][e & 3]), 1);
+    for (int b = 0; b < LA; ++b) {
       mbar_init(bar_s(b), 1);
       mbar_init(bar_p(b), 2 * (ROWS / 32));
       mbar_init(bar_pv(b), 1);
@@ -227,260 +254,167 @@ __global__ void __launch_bounds__(PairShape<HD, PAGED>::kThreads, 1)
   const uint32_t ring = smem0 + Shape::kQBytes;
   volatile int* abort_flag = &s_abort;
 
-  // ---- Q: TMA boxes where a box holds whole tokens (128 rows divide by the group), else 16-byte
-  // copies by all threads (by the two producer warps alone they took 24000 cycles at head_dim 256)
-  if (q_tma) {
-    // (rows past the sequence's last query token hold a neighbour's rows: computed on, never written)
-    if (warp == Shape::kProducerWarp0 && elect_one()) {
-      prefetch_tensormap(&tm_q);
-      mbar_arrive_expect_tx(bar_q, Shape::kQBytes);
-#pragma unroll
-      for (int c = 0; c < HD / 64; ++c)
-        tma_load_3d(q_smem + c * (ROWS * 128), &tm_q, c * 64, h * G, sq.q_begin + tok_first + rank * (ROWS / G), bar_q);
-    }
-    __syncwarp();
-  } else {
-    const T* q = static_cast<const T*>(p.q);
-    const int chunk = tid % CH;
-    for (int row = tid / CH; row < ROWS; row += Shape::kThreads / CH) {
-      const int pk = pk0 + rank * ROWS + row;
-      const int tl = pk / G, g = pk - tl * G;
-      const bool ok = row < rows_valid;
-      const int64_t off =
-          ok ? ((static_cast<int64_t>(sq.q_begin + tl) * p.hq + static_cast<int64_t>(h) * G + g) * HD) : 0;
-      cp_async_16(q_smem + tc_tile_offset<ROWS>(row, chunk),
-                  reinterpret_cast<const unsigned char*>(q + off) + chunk * 16, ok ? 16 : 0);
-    }
-    cp_async_mbar_arrive(bar_q);
-  }
-  // the gate's rows on their way into L2: the epilogue wants them
-  if (p.gate && warp == Shape::kRelayWarp) {
-    for (int e = lane; e < rows_valid * (HD / 64); e += 32) {
-      const int pk = pk0 + rank * ROWS + e / (HD / 64);
-      const int tl = pk / G, g = pk - tl * G;
-      prefetch_l2(static_cast<const T*>(p.gate) +
-                  (static_cast<int64_t>(sq.q_begin + tl) * p.hq + static_cast<int64_t>(h) * G + g) * HD +
-                  e % (HD / 64) * 64);
-    }
-  }
-
   if (warp >= Shape::kMmaWarp) {
-    if constexpr (!PAGED) reg_dec<88>();
-    if (warp >= Shape::kProducerWarp0) {
+    reg_dec<Shape::kOtherRegs>();
+    if (warp >= Shape::kProducerWarp0 && warp < Shape::kProducerWarp0 + 2 * NKW) {
       // =========================================================== producers
-      const int ptid = tid - Shape::kProducerWarp0 * 32;
-      const unsigned char* kbase = static_cast<const unsigned char*>(p.k_cache);
-      const unsigned char* vbase = static_cast<const unsigned char*>(p.v_cache);
-      const int64_t slot_stride = static_cast<int64_t>(p.hkv) * (HD * 2);
-      const int64_t head_off = static_cast<int64_t>(h) * (HD * 2);
-      const int64_t v_off = head_off + rank * HD;          // this CTA's half of the V columns, bytes
-      bool alive = true;
-      if constexpr (PAGED) {
-        {
-          // (the boxes of a tile are dealt to both producer warps: one alone issues 31 B/clk)
-          constexpr int NPW = NPROD / 32;
-          const int pw = warp - Shape::kProducerWarp0;
-          constexpr int PPT = BN / kTmaBoxRows;            // 8 pages of a tile, a lane each
-          constexpr uint32_t kBoxBytes = kTmaBoxRows * 128;
-          const int32_t* pages = p.page_indices + sq.kv_begin;
-          if (lane == 0) {
-            prefetch_tensormap(&tm_k);
-            prefetch_tensormap(&tm_v);
+      const int pid = warp - Shape::kProducerWarp0;
+      const bool is_k = pid < NKW;
+      const int pw = is_k ? pid : pid - NKW;            // among the warps of its kind
+      const uint32_t q_bar = cluster_addr(bar_q, 0);
+      if (lane == 0) {
+        prefetch_tensormap(&tm_q);
+        prefetch_tensormap(is_k ? &tg_k : &tg_v);
+        if (PAGED) prefetch_tensormap(is_k ? &tm_k : &tm_v);
+      }
+      // ---- Q, dealt to all producers: boxes of 64 columns x 128 rows where a box holds whole tokens
+      // (rows past the sequence's last query token hold a neighbour's rows then: computed on, never
+      // written), else four rows at a time
+      if (ntiles > 0) {
+        if (p.q_tma) {
+          if (elect_one()) {
+            int mine = 0;
+            for (int c = pid; c < HD / 64; c += 2 * NKW) ++mine;
+            mbar_arrive_expect_tx_cluster(q_bar, mine * (ROWS * 128));
+            for (int c = pid; c < HD / 64; c += 2 * NKW)
+              tma_pair_3d(q_smem + c * (ROWS * 128), &tm_q, c * 64, h * G, sq.q_begin + tok_first + rank * (ROWS / G), q_bar);
           }
-          // y = first pool row of the lane's page, n = rows of it that belong to the sequence
-          auto fetch_box = [&](int tile, int& y, int& n) {
-            y = 0;
-            n = 0;
-            const int t0 = kv_lo + tile * BN + lane * kTmaBoxRows;
-            if (lane < PPT && tile < ntiles && t0 < kv_hi) {
-              const int pg = __ldg(pages + t0 / p.page_size);
-              const int64_t row0 = static_cast<int64_t>(pg) * p.page_size + t0 % p.page_size;
-              const int nv = min(kTmaBoxRows, sq.L - t0);
-              if (pg < 0 || row0 + nv > p.num_slots) {
-                if (p.status) atomicExch(p.status, 2);     // page outside the pool: rows read as zeros
-              } else {
-                y = static_cast<int>(row0);
-                n = nv;
-              }
-            }
-          };
-          int issued_seq = -1;
-          auto produce = [&](int seq, bool is_k, int y, int n) {
-            const int bf = seq % NB;
-            alive = mbar_wait_warp(bar_empty(bf), ((seq / NB) & 1) ^ 1, abort_flag);
-            if (!alive) return;
-            const uint32_t dst = ring + bf * Shape::kBufBytes;
-            const uint32_t bar = bar_full(bf);
-            // K: this CTA's half of the pages, all columns; V: all pages, its half of the columns
-            const uint32_t full_mask = __ballot_sync(0xffffffffu, n == kTmaBoxRows);
-            const int page0 = is_k ? rank * (PPT / 2) : 0, npages = is_k ? PPT / 2 : PPT;
-            const uint32_t mine = ((1u << npages) - 1u) << page0;
-            uint32_t rest = mine & ~full_mask;
-            constexpr int MINE = (PPT / 2) * (HD / 64) / NPW;   // boxes of a warp
-            int yk[MINE], boxes = 0;
+        } else {
+          // lane l knows the rows 4 l .. 4 l + 3; the groups l = pid, pid + 6, ... are this warp's
+          int rows[4];
 #pragma unroll
-            for (int k = 0; k < MINE; ++k) {
-              const int i = page0 + (pw + k * NPW) % npages;
-              yk[k] = __shfl_sync(0xffffffffu, y, i);
-              if (((full_mask >> i) & 1u) == 0) yk[k] = -1;
-              boxes += yk[k] >= 0 ? 1 : 0;
-            }
-            const uint32_t block_bytes = (is_k ? KEYS : BN) * 128;
+          for (int e = 0; e < 4; ++e) {
+            const int row = lane * 4 + e;
+            const int pk = pk0 + rank * ROWS + row;
+            const int tl = pk / G, g = pk - tl * G;
+            rows[e] = row < rows_valid ? (sq.q_begin + tl) * p.hq + h * G + g : p.total_q * p.hq;
+          }
+          if (elect_one()) mbar_arrive_expect_tx_cluster(q_bar, (32 - pid + 2 * NKW - 1) / (2 * NKW) * (HD * 8));
+          __syncwarp();
+          for (int l = pid; l < 32; l += 2 * NKW) {
+            int r4[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) r4[e] = __shfl_sync(0xffffffffu, rows[e], l);
             if (elect_one()) {
-              const CUtensorMap* tm = is_k ? &tm_k : &tm_v;
-              const int x0 = h * HD + (is_k ? 0 : rank * (HD / 2));
-              mbar_arrive_expect_tx(bar, boxes * kBoxBytes);
 #pragma unroll
-              for (int k = 0; k < MINE; ++k) {
-                const int id = pw + k * NPW;
-                if (yk[k] >= 0)
-                  tma_load_2d(dst + (id / npages) * block_bytes + (id % npages) * kBoxBytes, tm,
-                              x0 + (id / npages) * 64, yk[k], bar);
-              }
-              if (rest == 0) mbar_arrive_n(bar, 32);     // (else the lanes arrive behind their own copies)
+              for (int c = 0; c < HD / 64; ++c)
+                tma_pair_gather4(q_smem + c * (ROWS * 128) + l * 512, &tm_q, c * 64, r4, q_bar);
             }
             __syncwarp();
-            const bool ragged = rest != 0;
-            const unsigned char* src = is_k ? kbase + head_off : vbase + v_off;
-            const int ch = is_k ? CH : VCH;
-            while (rest) {   // warp-uniform: ragged or out-of-range pages, row by row, zeros behind the end
-              const int i = __ffs(rest) - 1;
-              rest &= rest - 1;
-              if (i % NPW != pw) continue;
-              const int yi = __shfl_sync(0xffffffffu, y, i), ni = __shfl_sync(0xffffffffu, n, i);
-              const int row_i = (i - page0) * kTmaBoxRows;
-              for (int e = lane; e < kTmaBoxRows * ch; e += 32) {
-                const int row = e / ch, chunk = e % ch;
-                const bool ok = row < ni;
-                const int64_t off = (ok ? static_cast<int64_t>(yi + row) * slot_stride : 0) + chunk * 16;
-                const uint32_t so = is_k ? tc_tile_offset<KEYS>(row_i + row, chunk) : tc_tile_offset<BN>(row_i + row, chunk);
-                cp_async_16(dst + so, src + off, ok ? 16 : 0);
-              }
-            }
-            if (ragged) cp_async_mbar_arrive(bar);
-            issued_seq = seq;
-          };
-          int wy[3], wn[3];
-#pragma unroll
-          for (int t = 0; t < 3; ++t) fetch_box(t, wy[t], wn[t]);
-#pragma unroll 1
-          for (int j = -2; j < ntiles && alive; ++j) {     // K two tiles ahead of V
-            int ny = 0, nn = 0;
-            if (j >= 0) {
-              fetch_box(j + 3, ny, nn);                     // in flight while this step's copies are issued
-              produce(ring_seq_v<2>(j), false, wy[0], wn[0]);
-              if (!alive) break;
-            }
-            if (j + 2 < ntiles) {
-              const int k = j < 0 ? j + 2 : 2;
-              produce(ring_seq_k<2>(j + 2), true, k == 0 ? wy[0] : k == 1 ? wy[1] : wy[2],
-                      k == 0 ? wn[0] : k == 1 ? wn[1] : wn[2]);
-            }
-            if (j >= 0) {
-              wy[0] = wy[1];
-              wn[0] = wn[1];
-              wy[1] = wy[2];
-              wn[1] = wn[2];
-              wy[2] = ny;
-              wn[2] = nn;
-            }
-          }
-          if (!alive) {
-            // gave up: let the bulk copies still in flight land before the shared memory goes away; bounded
-            const long long t0 = clock64();
-            for (int i = max(0, issued_seq - NB + 1); i <= issued_seq; ++i) {
-              while (!mbar_try_wait(bar_full(i % NB), (i / NB) & 1) && clock64() - t0 < 2000000LL) {
-              }
-            }
           }
         }
-      } else {
-        // slot ids of a tile: one coalesced load, two tiles ahead of their use, staged in shared memory
-        const int32_t* idx = p.kv_indices + sq.kv_begin;
-        auto fetch_slot = [&](int tile) -> int {
-          const int t = kv_lo + tile * BN + ptid;
-          return (ptid < BN && tile < ntiles && t < kv_hi) ? __ldg(idx + t) : -1;
-        };
-        auto stage_slot = [&](int tile, int slot) {
-          if (ptid < BN) {
-            if (slot < -1 || static_cast<int64_t>(slot) >= p.num_slots) {
-              if (p.status) atomicExch(p.status, 2);
-              slot = -1;
-            }
-            s_slots[(tile % 3) * BN + ptid] = slot;
-          }
-        };
-        uint32_t idx_phase = 0;
-        const uint32_t bar_idx = smem_u32(&bars.idx_sync);
-        auto producers_sync = [&]() {
-          mbar_arrive(bar_idx);
-          alive = mbar_wait_warp(bar_idx, idx_phase, abort_flag);
-          idx_phase ^= 1;
-        };
-        auto produce = [&](int seq, bool is_k, int tile) {
-          const int bf = seq % NB;
-          alive = mbar_wait_warp(bar_empty(bf), ((seq / NB) & 1) ^ 1, abort_flag);
-          if (!alive) return;
-          const uint32_t dst = ring + bf * Shape::kBufBytes;
-          const int* slots = s_slots + (tile % 3) * BN;
-          if (is_k) {
-            for (int e = ptid; e < KEYS * CH; e += NPROD) {
-              const int row = e / CH, chunk = e % CH;
-              const int slot = slots[rank * KEYS + row];
-              const int64_t off = (slot >= 0 ? static_cast<int64_t>(slot) * slot_stride + head_off : 0) + chunk * 16;
-              cp_async_16(dst + tc_tile_offset<KEYS>(row, chunk), kbase + off, slot >= 0 ? 16 : 0);
-            }
-          } else {
-            for (int e = ptid; e < BN * VCH; e += NPROD) {
-              const int row = e / VCH, chunk = e % VCH;
-              const int slot = slots[row];
-              const int64_t off = (slot >= 0 ? static_cast<int64_t>(slot) * slot_stride + v_off : 0) + chunk * 16;
-              cp_async_16(dst + tc_tile_offset<BN>(row, chunk), vbase + off, slot >= 0 ? 16 : 0);
-            }
-          }
-          cp_async_mbar_arrive(bar_full(bf));
-        };
-        for (int t = 0; t < 3; ++t) stage_slot(t, fetch_slot(t));
-        producers_sync();
-#pragma unroll 1
-        for (int j = -2; j < ntiles && alive; ++j) {
-          const int next_slot = j >= 0 ? fetch_slot(j + 3) : -1;
-          if (j >= 0) produce(ring_seq_v<2>(j), false, j);
-          if (alive && j + 2 < ntiles) produce(ring_seq_k<2>(j + 2), true, j + 2);
-          if (!alive) break;
-          if (j >= 0) {
-            producers_sync();                   // every producer is done reading tile j's ids
-            if (!alive) break;
-            stage_slot(j + 3, next_slot);       // takes tile j's place
-            producers_sync();
-          }
-        }
+        __syncwarp();
       }
-      cp_async_wait<0>();
-      if (!alive && p.status && ptid == 0) atomicExch(p.status, 1);
-    } else if (warp == Shape::kRelayWarp) {
-      // =========================================================== relay
-      bool alive = true;
-      if (ntiles > 0) {
-        alive = mbar_wait_warp(bar_q, 0, abort_flag);
-        if (alive) {
-          fence_proxy_async_smem();
-          if (lane == 0) mbar_arrive_at(bar_qp, 0);
-        }
-      }
-      auto announce = [&](int seq) {
-        const int bf = seq % NB;
-        alive = mbar_wait_warp(bar_full(bf), (seq / NB) & 1, abort_flag);
-        if (!alive) return;
-        fence_proxy_async_smem();
-        if (lane == 0) mbar_arrive_at(bar_pair(bf), 0);
+      // ---- key tiles.  K: this CTA's 64 keys, all columns; V: all 128 keys, its half of the columns.
+      const int rows_tile = is_k ? KEYS : BN;
+      const int cols = is_k ? HD / 64 : HD / 128;                 // blocks of 64 columns
+      const int x0 = h * HD + (is_k ? 0 : rank * (HD / 2));
+      const int key0 = is_k ? rank * KEYS : 0;                    // first key of the tile copied here
+      const CUtensorMap* tm = is_k ? &tm_k : &tm_v;
+      const CUtensorMap* tg = is_k ? &tg_k : &tg_v;
+      const int absent = static_cast<int>(p.num_slots);
+      const int32_t* ids = (PAGED ? p.page_indices : p.kv_indices) + sq.kv_begin;
+      // PAGED: lane i = page i of the copied keys: a = its first pool row, n = rows of it that belong to
+      // the sequence.  Per-token: lane l = keys 4 l .. 4 l + 3: their slots.
+      struct Ids {
+        int a[PAGED ? 1 : 4], n;
       };
+      auto fetch = [&](int tile, Ids& d) {
+        const int t0 = kv_lo + tile * BN + key0;
+        if constexpr (PAGED) {
+          d.a[0] = absent;
+          d.n = 0;
+          const int t = t0 + lane * kTmaBoxRows;
+          if (lane * kTmaBoxRows < rows_tile && tile < ntiles && t < kv_hi) {
+            const int pg = __ldg(ids + t / p.page_size);
+            const int64_t row0 = static_cast<int64_t>(pg) * p.page_size + t % p.page_size;
+            const int nv = min(kTmaBoxRows, sq.L - t);
+            if (pg < 0 || row0 + nv > p.num_slots) {
+              if (p.status) atomicExch(p.status, 2);     // page outside the pool: rows read as zeros
+            } else {
+              d.a[0] = static_cast<int>(row0);
+              d.n = nv;
+            }
+          }
+        } else {
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int t = t0 + lane * 4 + e;
+            int slot = -1;
+            if (lane * 4 < rows_tile && tile < ntiles && t < kv_hi) {
+              slot = __ldg(ids + t);
+              if ((slot < -1 || static_cast<int64_t>(slot) >= p.num_slots) && p.status) atomicExch(p.status, 2);
+            }
+            d.a[e] = slot < 0 || static_cast<int64_t>(slot) >= p.num_slots ? absent : slot;
+          }
+        }
+      };
+      const int block_bytes = rows_tile * 128;
+      bool alive = true;
+      Ids cur, nxt;
+      fetch(0, cur);
+      const uint32_t full0 = cluster_addr(bar_full(0), 0);
 #pragma unroll 1
-      for (int j = -2; j < ntiles && alive; ++j) {
-        if (j >= 0) announce(ring_seq_v<2>(j));
-        if (alive && j + 2 < ntiles) announce(ring_seq_k<2>(j + 2));
+      for (int t = 0; t < ntiles; ++t) {
+        fetch(t + 1, nxt);                                        // in flight while this tile's copies are issued
+        const int seq = is_k ? ring_seq_k<LA>(t) : ring_seq_v<LA>(t);
+        const int bf = seq % NB;
+        alive = mbar_wait_warp(bar_empty(bf), ((seq / NB) & 1) ^ 1, abort_flag);
+        if (!alive) break;
+        const uint32_t dst = ring + bf * Shape::kBufBytes;
+        const uint32_t bar = full0 + bf * 8;
+        if constexpr (PAGED) {
+          // a page is four groups of four rows; page i is warp i % NKW's, one box per column block
+          const int npages = rows_tile / kTmaBoxRows;
+          if (elect_one())
+            mbar_arrive_expect_tx_cluster(bar, (npages - pw + NKW - 1) / NKW * (kTmaBoxRows * 128) * cols);
+          __syncwarp();
+#pragma unroll 1
+          for (int i = pw; i < npages; i += NKW) {
+            const int y = __shfl_sync(0xffffffffu, cur.a[0], i), n = __shfl_sync(0xffffffffu, cur.n, i);
+            const uint32_t at = dst + i * (kTmaBoxRows * 128);
+            if (elect_one()) {
+              if (n == kTmaBoxRows) {
+#pragma unroll 1
+                for (int c = 0; c < cols; ++c) tma_pair_2d(at + c * block_bytes, tm, x0 + c * 64, y, bar);
+              } else {
+#pragma unroll 1
+                for (int r = 0; r < kTmaBoxRows; r += 4) {
+                  int r4[4];
+#pragma unroll
+                  for (int e = 0; e < 4; ++e) r4[e] = r + e < n ? y + r + e : absent;
+#pragma unroll 1
+                  for (int c = 0; c < cols; ++c)
+                    tma_pair_gather4(at + r * 128 + c * block_bytes, tg, x0 + c * 64, r4, bar);
+                }
+              }
+            }
+            __syncwarp();
+          }
+        } else {
+          const int ngroups = rows_tile / 4;
+          if (elect_one()) mbar_arrive_expect_tx_cluster(bar, (ngroups - pw + NKW - 1) / NKW * 512 * cols);
+          __syncwarp();
+#pragma unroll 2
+          for (int i = pw; i < ngroups; i += NKW) {
+            int r4[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) r4[e] = __shfl_sync(0xffffffffu, cur.a[e], i);
+            if (elect_one()) {
+              for (int c = 0; c < cols; ++c) tma_pair_gather4(dst + i * 512 + c * block_bytes, tg, x0 + c * 64, r4, bar);
+            }
+            __syncwarp();
+          }
+        }
+        cur = nxt;
       }
-      if (!alive && p.status && lane == 0) atomicExch(p.status, 1);
+      if (!alive) {
+        if (p.status && lane == 0) atomicExch(p.status, 1);
+        // gave up: let the copies still in flight land before the shared memory goes away
+        const long long t0 = clock64();
+        while (clock64() - t0 < 2000000LL) {
+        }
+      }
     } else if (warp == Shape::kMmaWarp && rank == 0) {
       // =========================================================== MMA issuer
       const uint32_t idesc_s = idesc_m256<T>(BN, 0);
@@ -488,25 +422,26 @@ __global__ void __launch_bounds__(PairShape<HD, PAGED>::kThreads, 1)
       const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem, 0);
       const uint64_t desc_k = smem_desc_sw128(0, 16, 1024);                 // Q / K: K-major
       const uint64_t desc_v = smem_desc_sw128(0, BN * 128, 1024);           // V: MN-major
-      const int last_seq = ring_seq_v<2>(ntiles - 1);
+      const int last_seq = ring_seq_v<LA>(ntiles - 1);
       bool alive = true;
       auto acquire = [&](int seq) {
-        alive = mbar_wait_warp_cluster(bar_pair(seq % NB), (seq / NB) & 1, abort_flag);
+        alive = mbar_wait_warp(bar_full(seq % NB), (seq / NB) & 1, abort_flag);
         if (alive) tc_fence_after();
       };
       // frees a ring buffer in both CTAs (only while somebody will fill it again)
       auto release = [&](int seq) {
         if (seq + NB <= last_seq) tc_commit_pair(bar_empty(seq % NB));
       };
-      if (ntiles > 0) alive = mbar_wait_warp_cluster(bar_qp, 0, abort_flag);
+      if (ntiles > 0) alive = mbar_wait_warp(bar_q, 0, abort_flag);
 #pragma unroll 1
-      for (int j = -2; j < ntiles && alive; ++j) {
-        const bool do_pv = j >= 0, do_s = j + 2 < ntiles;
-        const int sv = ring_seq_v<2>(j), sk = ring_seq_k<2>(j + 2);
+      for (int j = -LA; j < ntiles && alive; ++j) {
+        const bool do_pv = j >= 0, do_s = j + LA < ntiles;
+        const int sv = ring_seq_v<LA>(j), sk = ring_seq_k<LA>(j + LA);
+        const int sb = (j + LA) % LA;                       // buffer of P of tile j and of S of tile j + LA
         if (do_pv) acquire(sv);
         if (alive && do_s) acquire(sk);
         if (alive && do_pv) {
-          alive = mbar_wait_warp_cluster(bar_p(j & 1), (j >> 1) & 1, abort_flag);
+          alive = mbar_wait_warp(bar_p(sb), (j / LA) & 1, abort_flag);
           tc_fence_after();
         }
         if (!alive) break;
@@ -514,14 +449,14 @@ __global__ void __launch_bounds__(PairShape<HD, PAGED>::kThreads, 1)
         const uint32_t kb = (ring + (do_s ? sk % NB : 0) * Shape::kBufBytes) >> 4;
         const uint32_t qa = q_smem >> 4;
         const uint32_t o_tm = tmem_u + Shape::kOCol;
-        const uint32_t ps_tm = tmem_u + (j & 1) * BN;       // P of tile j, then S of tile j + 2
+        const uint32_t ps_tm = tmem_u + sb * BN;
         if (elect_one()) {
           if (do_pv) {
 #pragma unroll
             for (int ks = 0; ks < BN / 16; ++ks)
               tc_mma_pair_ts(o_tm, ps_tm + ks * 8, desc_v | (vb + ks * (2048 >> 4)), idesc_pv,
                              (j == 0 && ks == 0) ? 0u : 1u);
-            tc_commit_pair(bar_pv(j & 1));
+            tc_commit_pair(bar_pv(sb));
             release(sv);
           }
           if (do_s) {
@@ -531,7 +466,7 @@ __global__ void __launch_bounds__(PairShape<HD, PAGED>::kThreads, 1)
               const uint32_t koff = ((ks >> 2) * (KEYS * 128) + (ks & 3) * 32) >> 4;
               tc_mma_pair_ss(ps_tm, desc_k | (qa + qoff), desc_k | (kb + koff), idesc_s, ks > 0 ? 1u : 0u);
             }
-            tc_commit_pair(bar_s(j & 1));
+            tc_commit_pair(bar_s(sb));
             release(sk);
           }
         }
@@ -541,9 +476,10 @@ __global__ void __launch_bounds__(PairShape<HD, PAGED>::kThreads, 1)
     }
   } else {
     // =========================================================== softmax
-    if constexpr (!PAGED) reg_inc<232>();
-    const int r = tid;                                     // row of this CTA's half == TMEM lane
-    const uint32_t lane_base = static_cast<uint32_t>(warp * 32) << 16;
+    reg_inc<Shape::kSoftRegs>();
+    const int grp = warp >> 2;                             // takes tiles grp, grp + NG, ...
+    const int r = tid & (ROWS - 1);                        // row of this CTA's half == TMEM lane
+    const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
     const uint32_t s_tm = tmem + lane_base;
     const uint32_t o_tm = tmem + lane_base + Shape::kOCol;
     const int tl = (pk0 + rank * ROWS + r) / G;
@@ -555,10 +491,21 @@ __global__ void __launch_bounds__(PairShape<HD, PAGED>::kThreads, 1)
     const bool sc_neg = !(p.scale_log2 > 0.f);
     const float sc = sc_neg ? 1.f : p.scale_log2;
 
+    const uint32_t p_bar = cluster_addr(bar_p(0), 0);
+    // the gate's rows on their way into L2: the epilogue wants them
+    if (p.gate) {
+      for (int e = warp * 32 + lane; e < rows_valid * (HD / 64); e += NG * ROWS) {
+        const int pk = pk0 + rank * ROWS + e / (HD / 64);
+        const int tle = pk / G, g = pk - tle * G;
+        prefetch_l2(static_cast<const T*>(p.gate) +
+                    (static_cast<int64_t>(sq.q_begin + tle) * p.hq + static_cast<int64_t>(h) * G + g) * HD +
+                    e % (HD / 64) * 64);
+      }
+    }
 #pragma unroll 1
-    for (int j = 0; j < ntiles; ++j) {
-      const int sb = j & 1;
-      alive = mbar_wait_warp_cluster(bar_s(sb), (j >> 1) & 1, abort_flag);
+    for (int j = grp; j < ntiles; j += NG) {
+      const int sb = j % LA;
+      alive = mbar_wait_warp(bar_s(sb), (j / LA) & 1, abort_flag);
       if (!alive) break;
       tc_fence_after();
       const int k0 = kv_lo + j * BN;
@@ -589,18 +536,29 @@ __global__ void __launch_bounds__(PairShape<HD, PAGED>::kThreads, 1)
           mx[c] = max3(mx[c], __uint_as_float(v[e + 2 * c]), __uint_as_float(v[e + 2 * c + 1]));
       }
       const float mt = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * sc;
-      // ---- lazy rescale of the accumulator
-      float alpha = 1.f;
-      bool resc = false;
-      if (mt > m_ref + 8.f) {
-        if (m_ref != -INFINITY) {
-          alpha = fast_exp2(m_ref - mt);
-          resc = true;
+      // ---- the row's reference maximum: the one after tile j - 1, raised (and O rescaled) only when the
+      // maximum has grown by more than 2^8
+      float alpha = 1.f;                      // of this group's sum
+      float m_old = m_ref;
+      if constexpr (NG == 2) {
+        if (j > 0) {
+          alive = mbar_wait_warp(smem_u32(&bars.m_ref[(j - 1) & 1][warp & 3]), ((j - 1) >> 1) & 1, abort_flag);
+          if (!alive) break;
+          m_old = s_mref[((j - 1) & 1) * ROWS + r];
         }
-        m_ref = mt;
       }
+      const float m_new = mt > m_old + 8.f ? mt : m_old;
+      if constexpr (NG == 2) {
+        s_mref[(j & 1) * ROWS + r] = m_new;
+        __syncwarp();
+        if (lane == 0) mbar_arrive(smem_u32(&bars.m_ref[j & 1][warp & 3]));
+      }
+      if (m_new != m_ref && m_ref != -INFINITY) alpha = fast_exp2(m_ref - m_new);
+      const bool resc = m_new != m_old && m_old != -INFINITY;
+      const float o_scale = resc ? fast_exp2(m_old - m_new) : 1.f;
+      m_ref = m_new;
       if (j > 0 && __any_sync(0xffffffffu, resc)) {
-        alive = mbar_wait_warp_cluster(bar_pv((j - 1) & 1), ((j - 1) >> 1) & 1, abort_flag);
+        alive = mbar_wait_warp(bar_pv((j - 1) % LA), ((j - 1) / LA) & 1, abort_flag);
         if (!alive) break;
         tc_fence_after();
 #pragma unroll 1
@@ -610,7 +568,7 @@ __global__ void __launch_bounds__(PairShape<HD, PAGED>::kThreads, 1)
           tmem_wait_ld();
           reg_fence(o);
 #pragma unroll
-          for (int e = 0; e < 32; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * alpha);
+          for (int e = 0; e < 32; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * o_scale);
           tmem_st32(o_tm + c * 32, o);
         }
         tmem_wait_st();
@@ -644,60 +602,89 @@ __global__ void __launch_bounds__(PairShape<HD, PAGED>::kThreads, 1)
       tmem_wait_st();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive_at(bar_p(sb), 0);
+      if (lane == 0) mbar_arrive_cluster(p_bar + sb * 8);
     }
 
-    // ---- epilogue: rows through the Q buffer (free: every S MMA is done), out as whole rows
-    if (alive && ntiles > 0) {
-      alive = mbar_wait_warp_cluster(bar_pv((ntiles - 1) & 1), ((ntiles - 1) >> 1) & 1, abort_flag);
+    // ---- epilogue
+    const bool any = ntiles > 0;
+    if (alive && any) {
+      alive = mbar_wait_warp(bar_pv((ntiles - 1) % LA), ((ntiles - 1) / LA) & 1, abort_flag);
       if (alive) tc_fence_after();
     }
-    if (alive && warp * 32 < rows_valid) {
-      const float inv = l > 0.f ? 1.f / l : 0.f;
-      constexpr int RB = HD * 2;
-      unsigned char* stage = smem_raw + (q_smem - smem_u32(smem_raw));
+    // Output rows are packed in the Q buffer (free: every S MMA is done; chunk c of row r sits at chunk
+    // position c ^ (r & 15)) and leave as whole rows, by all softmax warps.
+    constexpr int RB = HD * 2;
+    unsigned char* stage = smem_raw + (q_smem - smem_u32(smem_raw));
+    float inv = l > 0.f ? 1.f / l : 0.f;
+    if constexpr (NG == 2) {
+      // O is relative to the last tile's reference maximum, each group's sum to that of its own last tile
+      s_ml[grp * ROWS + r] = make_float2(m_ref, l);
+      softmax_groups_sync();
+      const float2 peer = s_ml[(grp ^ 1) * ROWS + r];
+      const float M = fmaxf(m_ref, peer.x);   // (it only grows)
+      const float L = (m_ref == -INFINITY ? 0.f : l * fast_exp2(m_ref - M)) +
+                      (peer.x == -INFINITY ? 0.f : peer.y * fast_exp2(peer.x - M));
+      inv = L > 0.f ? 1.f / L : 0.f;
+    }
 #pragma unroll 1
-      for (int c = 0; c < HD / 32; ++c) {
-        uint32_t v[32];
-        if (ntiles > 0) {
-          tmem_ld32(o_tm + c * 32, v);
-          tmem_wait_ld();
-          reg_fence(v);
-        } else {
+    for (int c = grp * (HD / 32 / NG); c < (grp + 1) * (HD / 32 / NG); ++c) {   // a group's share of the columns
+      uint32_t v[32];
+      if (any && alive) {
+        tmem_ld32(o_tm + c * 32, v);
+        tmem_wait_ld();
+        reg_fence(v);
+      } else {
 #pragma unroll
-          for (int e = 0; e < 32; ++e) v[e] = 0u;
-        }
-#pragma unroll
-        for (int e = 0; e < 32; e += 8) {
-          uint4 w;
-          w.x = MmaOp<T>::pack(__uint_as_float(v[e]) * inv, __uint_as_float(v[e + 1]) * inv);
-          w.y = MmaOp<T>::pack(__uint_as_float(v[e + 2]) * inv, __uint_as_float(v[e + 3]) * inv);
-          w.z = MmaOp<T>::pack(__uint_as_float(v[e + 4]) * inv, __uint_as_float(v[e + 5]) * inv);
-          w.w = MmaOp<T>::pack(__uint_as_float(v[e + 6]) * inv, __uint_as_float(v[e + 7]) * inv);
-          const int chunk = c * 4 + (e >> 3);
-          *reinterpret_cast<uint4*>(stage + r * RB + ((chunk ^ (r & 15)) << 4)) = w;
-        }
+        for (int e = 0; e < 32; ++e) v[e] = 0u;
       }
-      __syncwarp();
+#pragma unroll
+      for (int e = 0; e < 32; e += 8) {
+        uint4 w;
+        w.x = MmaOp<T>::pack(__uint_as_float(v[e]) * inv, __uint_as_float(v[e + 1]) * inv);
+        w.y = MmaOp<T>::pack(__uint_as_float(v[e + 2]) * inv, __uint_as_float(v[e + 3]) * inv);
+        w.z = MmaOp<T>::pack(__uint_as_float(v[e + 4]) * inv, __uint_as_float(v[e + 5]) * inv);
+        w.w = MmaOp<T>::pack(__uint_as_float(v[e + 6]) * inv, __uint_as_float(v[e + 7]) * inv);
+        const int chunk = c * 4 + (e >> 3);
+        *reinterpret_cast<uint4*>(stage + r * RB + ((chunk ^ (r & 15)) << 4)) = w;
+      }
+    }
+    if constexpr (NG == 2) softmax_groups_sync();
+    __syncwarp();
+    // whole rows, 32 per warp of a group (with two groups each warp takes half of them); a lane knows
+    // the place of one row, and the loads of four rows are in flight together
+    {
+      const int row_l = (warp & 3) * 32 + lane;
+      const int pkr = pk0 + rank * ROWS + row_l;
+      const int tlr = pkr / G, gr = pkr - tlr * G;
+      const int64_t off_l = row_l < rows_valid && alive
+                                ? (static_cast<int64_t>(sq.q_begin + tlr) * p.hq + static_cast<int64_t>(h) * G + gr) * HD
+                                : -1;
+      constexpr int RPI = 32 / CH == 0 ? 1 : 32 / CH;         // rows of an iteration
+      constexpr int N = 32 / NG;                              // rows of this warp
       const int chunk = lane % CH;
-#pragma unroll 8
-      for (int rr = lane / CH; rr < 32; rr += 32 / CH) {
-        const int row = warp * 32 + rr;
-        if (row < rows_valid) {
-          const int pkr = pk0 + rank * ROWS + row;
-          const int tlr = pkr / G, gr = pkr - tlr * G;
-          T* dst = static_cast<T*>(p.out) +
-                   (static_cast<int64_t>(sq.q_begin + tlr) * p.hq + static_cast<int64_t>(h) * G + gr) * HD;
-          uint4 w = *reinterpret_cast<const uint4*>(stage + row * RB + ((chunk ^ (row & 15)) << 4));
+#pragma unroll 1
+      for (int r0 = grp * (32 - N); r0 < grp * (32 - N) + N; r0 += 4 * RPI) {
+        int64_t off[4];
+        uint4 w[4], gv[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const int rr = r0 + k * RPI + lane / CH;
+          off[k] = __shfl_sync(0xffffffffu, off_l, rr);
+          if (p.gate && off[k] >= 0)
+            gv[k] = *reinterpret_cast<const uint4*>(static_cast<const T*>(p.gate) + off[k] + chunk * 8);
+          const int row = (warp & 3) * 32 + rr;
+          w[k] = *reinterpret_cast<const uint4*>(stage + row * RB + ((chunk ^ (row & 15)) << 4));
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          if (off[k] < 0) continue;
           if (p.gate) {
-            const T* grow = static_cast<const T*>(p.gate) + (dst - static_cast<T*>(p.out));
-            const uint4 gv = *reinterpret_cast<const uint4*>(grow + chunk * 8);
-            T* wo = reinterpret_cast<T*>(&w);
-            const T* wg = reinterpret_cast<const T*>(&gv);
+            T* wo = reinterpret_cast<T*>(&w[k]);
+            const T* wg = reinterpret_cast<const T*>(&gv[k]);
 #pragma unroll
             for (int e = 0; e < 8; ++e) wo[e] = apply_gate<T>(to_f32(wo[e]), wg[e]);
           }
-          *reinterpret_cast<uint4*>(reinterpret_cast<unsigned char*>(dst) + chunk * 16) = w;
+          *reinterpret_cast<uint4*>(static_cast<T*>(p.out) + off[k] + chunk * 8) = w[k];
         }
       }
     }
