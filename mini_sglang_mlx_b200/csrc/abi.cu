@@ -246,14 +246,15 @@ bool prefill_short_q(int max_len_extend, int group, int head_dim) {
   return head_dim == 256 || static_cast<int64_t>(max_len_extend) * group <= msgl::kTcSub;
 }
 
-// Pairs of CTAs: head_dim 256, query blocks of more than one 128-row tile, key range not split.
-bool prefill_pairs(int max_len_extend, int group, int head_dim, int kv_chunk) {
-#ifdef MSGL_PAIR128
-  const bool hd = true;
-#else
-  const bool hd = head_dim == 256;
-#endif
-  return hd && kv_chunk == 0 && static_cast<int64_t>(max_len_extend) * group > msgl::kTcSub;
+// Pairs of CTAs (prefill_pair.cuh) serve query blocks of more than one 128-row tile whose key range is
+// not split.  Not head_dim 128 with per-token slots over longer contexts: there four-row gathers are all
+// the copies, and TMA moves them slower (about 45 cycles per 512 bytes) than the copying warps of the
+// 256-row CTA do (2000-token prompts over 8000 cached tokens: 1450 us against 1095); short contexts
+// gain from the faster start all the same (six prompts of up to 300 tokens: 117 us against 135).
+bool prefill_pairs(int max_len_extend, int group, int head_dim, int kv_chunk, bool paged, int batch,
+                   int64_t total_kv) {
+  if (kv_chunk != 0 || static_cast<int64_t>(max_len_extend) * group <= msgl::kTcSub) return false;
+  return head_dim == 256 || paged || total_kv <= static_cast<int64_t>(batch) * 512;
 }
 
 PrefillPlan plan_prefill(int batch, int total_q, int64_t total_kv, int hq, int hkv, int head_dim,
@@ -1021,7 +1022,8 @@ static int prefill_impl(const void* q, const void* k_cache, const void* v_cache,
   cudaStream_t s = static_cast<cudaStream_t>(stream);
 
   dim3 grid(static_cast<unsigned>(pl.items * num_kv_heads));
-  bool pair = prefill_pairs(max_len_extend, p.group, head_dim, pl.kv_chunk) && num_slots < (1ll << 31);
+  bool pair = prefill_pairs(max_len_extend, p.group, head_dim, pl.kv_chunk, pages != nullptr, batch, total_kv) &&
+              num_slots < (1ll << 31);
   CUtensorMap tg_k, tg_v;
   if (pair) {
     // everything by TMA: boxes of pages, rows of pools and queries by gather
@@ -1064,11 +1066,9 @@ static int prefill_impl(const void* q, const void* k_cache, const void* v_cache,
         if (err != cudaSuccess) return err;
         return launch_clusters(2, kernel, grid, dim3(S::kThreads), S::kSmemBytes, s, p, tm_k, tm_v, tg_k, tg_v, tm_q);
       };
-#ifdef MSGL_PAIR128
       if (head_dim == 128)
         return pages ? go(msgl::prefill_pair_kernel<T, 128, true>, msgl::PairShape<128, true>{})
                      : go(msgl::prefill_pair_kernel<T, 128, false>, msgl::PairShape<128, false>{});
-#endif
       return pages ? go(msgl::prefill_pair_kernel<T, 256, true>, msgl::PairShape<256, true>{})
                    : go(msgl::prefill_pair_kernel<T, 256, false>, msgl::PairShape<256, false>{});
     }

@@ -155,6 +155,14 @@ __device__ __forceinline__ uint32_t idesc_m256(uint32_t n, uint32_t b_mn) {
   return (idesc_m128<T>(n, b_mn) & ~(0x1fu << 24)) | ((256u >> 4) << 24);
 }
 
+__device__ __forceinline__ uint2 ld_shared_volatile2(uint32_t addr) {
+  uint2 v;
+  asm volatile("ld.volatile.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(addr) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_shared_volatile2(uint32_t addr, uint2 v) {
+  asm volatile("st.volatile.shared.v2.u32 [%0], {%1, %2};" ::"r"(addr), "r"(v.x), "r"(v.y) : "memory");
+}
 // Barrier of the 256 threads of both softmax groups.
 __device__ __forceinline__ void softmax_groups_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
 
@@ -162,7 +170,6 @@ struct PairBarriers {
   uint64_t q_full, full[8];              // leader: both CTAs' copies
   uint64_t empty[8];
   uint64_t s_full[3], p_full[3], pv_done[3];
-  uint64_t m_ref[2][4];                  // [tile parity][warp of the group]: the reference maxima are published
 };
 
 template <typename T, int HD, bool PAGED>
@@ -182,7 +189,8 @@ __global__ void __launch_bounds__(PairShape<HD, PAGED>::kThreads, 1)
   __shared__ uint32_t s_tmem_base;
   __shared__ int s_abort;
   __shared__ float2 s_ml[NG == 2 ? 2 * ROWS : 1];        // (reference maximum, sum) of the rows, per group
-  __shared__ float s_mref[NG == 2 ? 2 * ROWS : 1];       // reference maxima after the even / odd tiles
+  // reference maxima after the even / odd tiles, each with its tile's number
+  __shared__ __align__(16) uint2 s_mref[NG == 2 ? 2 * ROWS : 1];
 
   const int tid = threadIdx.x;
   const int warp = tid >> 5, lane = tid & 31;
@@ -203,7 +211,6 @@ __global__ void __launch_bounds__(PairShape<HD, PAGED>::kThreads, 1)
       mbar_init(bar_full(bf), 2 * NKW);         // the producers of its kind in both CTAs
       mbar_init(bar_empty(bf), 1);
     }
-    for (int e = 0; e < 8; ++e) mbar_init(smem_u32(&bars.m_ref[e >> 2][e & 3]), 1);
     for (int b = 0; b < LA; ++b) {
       mbar_init(bar_s(b), 1);
       mbar_init(bar_p(b), 2 * (ROWS / 32));
@@ -211,6 +218,7 @@ __global__ void __launch_bounds__(PairShape<HD, PAGED>::kThreads, 1)
     }
     fence_mbar_init();
   }
+  if (NG == 2 && tid < 2 * ROWS) s_mref[tid] = make_uint2(0u, 0xffffffffu);
   if (warp == Shape::kMmaWarp) {
     tmem_alloc_pair(smem_u32(&s_tmem_base), 512);
     tmem_relinquish_pair();
@@ -306,108 +314,107 @@ __global__ void __launch_bounds__(PairShape<HD, PAGED>::kThreads, 1)
         __syncwarp();
       }
       // ---- key tiles.  K: this CTA's 64 keys, all columns; V: all 128 keys, its half of the columns.
-      const int rows_tile = is_k ? KEYS : BN;
-      const int cols = is_k ? HD / 64 : HD / 128;                 // blocks of 64 columns
-      const int x0 = h * HD + (is_k ? 0 : rank * (HD / 2));
-      const int key0 = is_k ? rank * KEYS : 0;                    // first key of the tile copied here
-      const CUtensorMap* tm = is_k ? &tm_k : &tm_v;
-      const CUtensorMap* tg = is_k ? &tg_k : &tg_v;
       const int absent = static_cast<int>(p.num_slots);
       const int32_t* ids = (PAGED ? p.page_indices : p.kv_indices) + sq.kv_begin;
-      // PAGED: lane i = page i of the copied keys: a = its first pool row, n = rows of it that belong to
-      // the sequence.  Per-token: lane l = keys 4 l .. 4 l + 3: their slots.
-      struct Ids {
-        int a[PAGED ? 1 : 4], n;
-      };
-      auto fetch = [&](int tile, Ids& d) {
-        const int t0 = kv_lo + tile * BN + key0;
-        if constexpr (PAGED) {
-          d.a[0] = absent;
-          d.n = 0;
-          const int t = t0 + lane * kTmaBoxRows;
-          if (lane * kTmaBoxRows < rows_tile && tile < ntiles && t < kv_hi) {
-            const int pg = __ldg(ids + t / p.page_size);
-            const int64_t row0 = static_cast<int64_t>(pg) * p.page_size + t % p.page_size;
-            const int nv = min(kTmaBoxRows, sq.L - t);
-            if (pg < 0 || row0 + nv > p.num_slots) {
-              if (p.status) atomicExch(p.status, 2);     // page outside the pool: rows read as zeros
-            } else {
-              d.a[0] = static_cast<int>(row0);
-              d.n = nv;
-            }
-          }
-        } else {
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const int t = t0 + lane * 4 + e;
-            int slot = -1;
-            if (lane * 4 < rows_tile && tile < ntiles && t < kv_hi) {
-              slot = __ldg(ids + t);
-              if ((slot < -1 || static_cast<int64_t>(slot) >= p.num_slots) && p.status) atomicExch(p.status, 2);
-            }
-            d.a[e] = slot < 0 || static_cast<int64_t>(slot) >= p.num_slots ? absent : slot;
-          }
-        }
-      };
-      const int block_bytes = rows_tile * 128;
-      bool alive = true;
-      Ids cur, nxt;
-      fetch(0, cur);
       const uint32_t full0 = cluster_addr(bar_full(0), 0);
-#pragma unroll 1
-      for (int t = 0; t < ntiles; ++t) {
-        fetch(t + 1, nxt);                                        // in flight while this tile's copies are issued
-        const int seq = is_k ? ring_seq_k<LA>(t) : ring_seq_v<LA>(t);
-        const int bf = seq % NB;
-        alive = mbar_wait_warp(bar_empty(bf), ((seq / NB) & 1) ^ 1, abort_flag);
-        if (!alive) break;
-        const uint32_t dst = ring + bf * Shape::kBufBytes;
-        const uint32_t bar = full0 + bf * 8;
-        if constexpr (PAGED) {
-          // a page is four groups of four rows; page i is warp i % NKW's, one box per column block
-          const int npages = rows_tile / kTmaBoxRows;
-          if (elect_one())
-            mbar_arrive_expect_tx_cluster(bar, (npages - pw + NKW - 1) / NKW * (kTmaBoxRows * 128) * cols);
-          __syncwarp();
-#pragma unroll 1
-          for (int i = pw; i < npages; i += NKW) {
-            const int y = __shfl_sync(0xffffffffu, cur.a[0], i), n = __shfl_sync(0xffffffffu, cur.n, i);
-            const uint32_t at = dst + i * (kTmaBoxRows * 128);
-            if (elect_one()) {
-              if (n == kTmaBoxRows) {
-#pragma unroll 1
-                for (int c = 0; c < cols; ++c) tma_pair_2d(at + c * block_bytes, tm, x0 + c * 64, y, bar);
+      bool alive = true;
+      auto produce = [&](auto kind, const CUtensorMap* tm, const CUtensorMap* tg) {
+        constexpr bool K = decltype(kind)::value;
+        constexpr int RT = K ? KEYS : BN;                         // rows of the tile copied here
+        constexpr int COLS = K ? HD / 64 : HD / 128;              // blocks of 64 columns
+        // what is dealt to the warps: boxes, or groups of four rows with all their column blocks
+        constexpr int UNITS = PAGED ? RT / kTmaBoxRows * COLS : RT / 4;
+        constexpr int MINE = (UNITS + NKW - 1) / NKW;             // of this warp: pw, pw + NKW, ...
+        constexpr int UB = PAGED ? kTmaBoxRows * 128 : 512 * COLS;     // bytes
+        const uint32_t my_bytes = static_cast<uint32_t>((UNITS - pw + NKW - 1) / NKW) * UB;
+        const int x0 = h * HD + (K ? 0 : rank * (HD / 2));
+        const int key0 = K ? rank * KEYS : 0;                     // first key of the tile copied here
+        // PAGED: lane i = page i of the copied keys: a = its first pool row, n = rows of it that belong
+        // to the sequence.  Per-token: lane l = keys 4 l .. 4 l + 3: their slots.
+        struct Ids {
+          int a[PAGED ? 1 : 4], n;
+        };
+        auto fetch = [&](int tile, Ids& d) {
+          const int t0 = kv_lo + tile * BN + key0;
+          if constexpr (PAGED) {
+            d.a[0] = absent;
+            d.n = 0;
+            const int t = t0 + lane * kTmaBoxRows;
+            if (lane * kTmaBoxRows < RT && tile < ntiles && t < kv_hi) {
+              const int pg = __ldg(ids + t / p.page_size);
+              const int64_t row0 = static_cast<int64_t>(pg) * p.page_size + t % p.page_size;
+              const int nv = min(kTmaBoxRows, sq.L - t);
+              if (pg < 0 || row0 + nv > p.num_slots) {
+                if (p.status) atomicExch(p.status, 2);     // page outside the pool: rows read as zeros
               } else {
-#pragma unroll 1
-                for (int r = 0; r < kTmaBoxRows; r += 4) {
-                  int r4[4];
+                d.a[0] = static_cast<int>(row0);
+                d.n = nv;
+              }
+            }
+          } else {
 #pragma unroll
-                  for (int e = 0; e < 4; ++e) r4[e] = r + e < n ? y + r + e : absent;
+            for (int e = 0; e < 4; ++e) {
+              const int t = t0 + lane * 4 + e;
+              int slot = -1;
+              if (lane * 4 < RT && tile < ntiles && t < kv_hi) {
+                slot = __ldg(ids + t);
+                if ((slot < -1 || static_cast<int64_t>(slot) >= p.num_slots) && p.status) atomicExch(p.status, 2);
+              }
+              d.a[e] = slot < 0 || static_cast<int64_t>(slot) >= p.num_slots ? absent : slot;
+            }
+          }
+        };
+        Ids cur, nxt;
+        fetch(0, cur);
 #pragma unroll 1
-                  for (int c = 0; c < cols; ++c)
-                    tma_pair_gather4(at + r * 128 + c * block_bytes, tg, x0 + c * 64, r4, bar);
+        for (int t = 0; t < ntiles; ++t) {
+          fetch(t + 1, nxt);                                      // in flight while this tile's copies are issued
+          const int seq = K ? ring_seq_k<LA>(t) : ring_seq_v<LA>(t);
+          const int bf = seq % NB;
+          alive = mbar_wait_warp(bar_empty(bf), ((seq / NB) & 1) ^ 1, abort_flag);
+          if (!alive) break;
+          const uint32_t dst = ring + bf * Shape::kBufBytes;
+          const uint32_t bar = full0 + bf * 8;
+          if (elect_one()) mbar_arrive_expect_tx_cluster(bar, my_bytes);
+          __syncwarp();
+#pragma unroll(PAGED ? MINE : 2)
+          for (int k = 0; k < MINE; ++k) {
+            const int id = pw + k * NKW;
+            if (UNITS % NKW != 0 && id >= UNITS) break;
+            if constexpr (PAGED) {
+              constexpr int PAGES = RT / kTmaBoxRows;
+              const int i = id % PAGES, c = id / PAGES;
+              const uint32_t at = dst + c * (RT * 128) + i * UB;
+              const int y = __shfl_sync(0xffffffffu, cur.a[0], i), n = __shfl_sync(0xffffffffu, cur.n, i);
+              if (elect_one()) {
+                if (n == kTmaBoxRows) {
+                  tma_pair_2d(at, tm, x0 + c * 64, y, bar);
+                } else {
+#pragma unroll 1
+                  for (int r = 0; r < kTmaBoxRows; r += 4) {
+                    int r4[4];
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) r4[e] = r + e < n ? y + r + e : absent;
+                    tma_pair_gather4(at + r * 128, tg, x0 + c * 64, r4, bar);
+                  }
                 }
+              }
+            } else {
+              int r4[4];
+#pragma unroll
+              for (int e = 0; e < 4; ++e) r4[e] = __shfl_sync(0xffffffffu, cur.a[e], id);
+              if (elect_one()) {
+#pragma unroll
+                for (int c = 0; c < COLS; ++c) tma_pair_gather4(dst + c * (RT * 128) + id * 512, tg, x0 + c * 64, r4, bar);
               }
             }
             __syncwarp();
           }
-        } else {
-          const int ngroups = rows_tile / 4;
-          if (elect_one()) mbar_arrive_expect_tx_cluster(bar, (ngroups - pw + NKW - 1) / NKW * 512 * cols);
-          __syncwarp();
-#pragma unroll 2
-          for (int i = pw; i < ngroups; i += NKW) {
-            int r4[4];
-#pragma unroll
-            for (int e = 0; e < 4; ++e) r4[e] = __shfl_sync(0xffffffffu, cur.a[e], i);
-            if (elect_one()) {
-              for (int c = 0; c < cols; ++c) tma_pair_gather4(dst + i * 512 + c * block_bytes, tg, x0 + c * 64, r4, bar);
-            }
-            __syncwarp();
-          }
+          cur = nxt;
         }
-        cur = nxt;
-      }
+      };
+      if (is_k) produce(std::true_type{}, &tm_k, &tg_k);
+      else produce(std::false_type{}, &tm_v, &tg_v);
       if (!alive) {
         if (p.status && lane == 0) atomicExch(p.status, 1);
         // gave up: let the copies still in flight land before the shared memory goes away
@@ -542,16 +549,27 @@ __global__ void __launch_bounds__(PairShape<HD, PAGED>::kThreads, 1)
       float m_old = m_ref;
       if constexpr (NG == 2) {
         if (j > 0) {
-          alive = mbar_wait_warp(smem_u32(&bars.m_ref[(j - 1) & 1][warp & 3]), ((j - 1) >> 1) & 1, abort_flag);
+          // (a value tagged with its tile: the reader polls its own row, no barrier in between)
+          const uint32_t at = smem_u32(&s_mref[((j - 1) & 1) * ROWS + r]);
+          uint2 got = ld_shared_volatile2(at);
+          if (got.y != static_cast<uint32_t>(j - 1)) {
+            const long long t0 = clock64();
+            while ((got = ld_shared_volatile2(at)).y != static_cast<uint32_t>(j - 1)) {
+              if (*abort_flag != 0 || clock64() - t0 > kTcWaitCycles) {
+                *abort_flag = 1;
+                alive = false;
+                break;
+              }
+            }
+          }
+          alive = __all_sync(0xffffffffu, alive ? 1 : 0) != 0;
           if (!alive) break;
-          m_old = s_mref[((j - 1) & 1) * ROWS + r];
+          m_old = __uint_as_float(got.x);
         }
       }
       const float m_new = mt > m_old + 8.f ? mt : m_old;
       if constexpr (NG == 2) {
-        s_mref[(j & 1) * ROWS + r] = m_new;
-        __syncwarp();
-        if (lane == 0) mbar_arrive(smem_u32(&bars.m_ref[j & 1][warp & 3]));
+        st_shared_volatile2(smem_u32(&s_mref[(j & 1) * ROWS + r]), make_uint2(__float_as_uint(m_new), j));
       }
       if (m_new != m_ref && m_ref != -INFINITY) alpha = fast_exp2(m_ref - m_new);
       const bool resc = m_new != m_old && m_old != -INFINITY;
@@ -583,9 +601,9 @@ __global__ void __launch_bounds__(PairShape<HD, PAGED>::kThreads, 1)
         uint32_t pk16[16];
 #pragma unroll
         for (int e = 0; e < 32; e += 2) {
+          const uint64_t x = fma_f32x2(pack_f32x2(__uint_as_float(v[c * 32 + e]), __uint_as_float(v[c * 32 + e + 1])), sc2, nmu2);
           float x0, x1;
-          unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(v[c * 32 + e]), __uint_as_float(v[c * 32 + e + 1])),
-                                 sc2, nmu2), x0, x1);
+          unpack_f32x2(x, x0, x1);
           const float p0 = fast_exp2(x0);
           const float p1 = fast_exp2(x1);
           if (e & 2) lb = add_f32x2(lb, pack_f32x2(p0, p1));
