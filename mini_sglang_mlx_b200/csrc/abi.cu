@@ -254,6 +254,9 @@ bool prefill_short_q(int max_len_extend, int group, int head_dim) {
 bool prefill_pairs(int max_len_extend, int group, int head_dim, int kv_chunk, bool paged, int batch,
                    int64_t total_kv) {
   if (kv_chunk != 0 || static_cast<int64_t>(max_len_extend) * group <= msgl::kTcSub) return false;
+#ifdef MSGL_TOKALL
+  return true;
+#endif
   return head_dim == 256 || paged || total_kv <= static_cast<int64_t>(batch) * 512;
 }
 

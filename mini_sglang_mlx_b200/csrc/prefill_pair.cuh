@@ -54,7 +54,8 @@ struct PairShape {
   static constexpr int kGroups = HD == 128 ? 2 : 1;       // softmax groups
   static constexpr int kMmaWarp = 4 * kGroups, kProducerWarp0 = kMmaWarp + 1;
   static constexpr int kKindWarps = 3;                    // producers of K, and of V
-  static constexpr int kWarps = kMmaWarp + 8;             // (one idle: whole warpgroups for setmaxnreg)
+  static constexpr int kVWarps = PAGED ? 3 : 4;
+  static constexpr int kWarps = kMmaWarp + 8;             // (whole warpgroups for setmaxnreg)
   // registers moved from the other warps to the softmax warps: 512 threads at 128, 384 at 168
   static constexpr int kSoftRegs = kGroups == 2 ? 192 : 200;
   static constexpr int kOtherRegs = kGroups == 2 ? 64 : 144;
@@ -163,6 +164,11 @@ __device__ __forceinline__ uint2 ld_shared_volatile2(uint32_t addr) {
 __device__ __forceinline__ void st_shared_volatile2(uint32_t addr, uint2 v) {
   asm volatile("st.volatile.shared.v2.u32 [%0], {%1, %2};" ::"r"(addr), "r"(v.x), "r"(v.y) : "memory");
 }
+// Barrier of all threads of the CTA that may be reached from several places in the code.
+template <int N>
+__device__ __forceinline__ void cta_threads_sync() {
+  asm volatile("bar.sync 2, %0;" ::"n"(N) : "memory");
+}
 // Barrier of the 256 threads of both softmax groups.
 __device__ __forceinline__ void softmax_groups_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
 
@@ -208,7 +214,7 @@ __global__ void __launch_bounds__(PairShape<HD, PAGED>::kThreads, 1)
     s_abort = 0;
     mbar_init(bar_q, 2 * 2 * NKW);
     for (int bf = 0; bf < NB; ++bf) {
-      mbar_init(bar_full(bf), 2 * NKW);         // the producers of its kind in both CTAs
+      mbar_init(bar_full(bf), 2 * Shape::kVWarps);   // both CTAs' producers (K: the first arrives for two)
       mbar_init(bar_empty(bf), 1);
     }
     for (int b = 0; b < LA; ++b) {
@@ -262,9 +268,48 @@ __global__ void __launch_bounds__(PairShape<HD, PAGED>::kThreads, 1)
   const uint32_t ring = smem0 + Shape::kQBytes;
   volatile int* abort_flag = &s_abort;
 
+  // Output rows are packed in the Q buffer (free then: every S MMA is done; chunk c of row r sits at chunk
+  // position c ^ (r & 15)) and leave as whole rows, by all warps of the CTA: the gate's reads and
+  // exponentials took four softmax warps 20000 cycles at head_dim 256.
+  constexpr int RB = HD * 2;
+  unsigned char* stage = smem_raw + (q_smem - smem_u32(smem_raw));
+  auto write_rows = [&]() {
+    cta_threads_sync<Shape::kThreads>();
+    if (s_abort != 0) return;
+    constexpr int RPI = 32 / CH;                              // rows of a warp's access
+    constexpr int STEP = Shape::kWarps * RPI;
+    constexpr int FLY = 2;                                    // accesses in flight
+    const int chunk = lane % CH;
+#pragma unroll 1
+    for (int r0 = warp * RPI + lane / CH; r0 < rows_valid; r0 += FLY * STEP) {
+      T* dst[FLY];
+      uint4 w[FLY], gv[FLY];
+#pragma unroll
+      for (int k = 0; k < FLY; ++k) {
+        const int row = min(r0 + k * STEP, rows_valid - 1);   // (the last row again instead of a row behind it)
+        const int pk = pk0 + rank * ROWS + row;
+        const int tl = pk / G, g = pk - tl * G;
+        const int64_t off = (static_cast<int64_t>(sq.q_begin + tl) * p.hq + static_cast<int64_t>(h) * G + g) * HD + chunk * 8;
+        dst[k] = static_cast<T*>(p.out) + off;
+        if (p.gate) gv[k] = *reinterpret_cast<const uint4*>(static_cast<const T*>(p.gate) + off);
+        w[k] = *reinterpret_cast<const uint4*>(stage + row * RB + ((chunk ^ (row & 15)) << 4));
+      }
+#pragma unroll
+      for (int k = 0; k < FLY; ++k) {
+        if (p.gate) {
+          T* wo = reinterpret_cast<T*>(&w[k]);
+          const T* wg = reinterpret_cast<const T*>(&gv[k]);
+#pragma unroll
+          for (int e = 0; e < 8; ++e) wo[e] = apply_gate<T>(to_f32(wo[e]), wg[e]);
+        }
+        *reinterpret_cast<uint4*>(dst[k]) = w[k];
+      }
+    }
+  };
+
   if (warp >= Shape::kMmaWarp) {
     reg_dec<Shape::kOtherRegs>();
-    if (warp >= Shape::kProducerWarp0 && warp < Shape::kProducerWarp0 + 2 * NKW) {
+    if (warp >= Shape::kProducerWarp0 && warp < Shape::kProducerWarp0 + NKW + Shape::kVWarps) {
       // =========================================================== producers
       const int pid = warp - Shape::kProducerWarp0;
       const bool is_k = pid < NKW;
@@ -278,7 +323,7 @@ __global__ void __launch_bounds__(PairShape<HD, PAGED>::kThreads, 1)
       // ---- Q, dealt to all producers: boxes of 64 columns x 128 rows where a box holds whole tokens
       // (rows past the sequence's last query token hold a neighbour's rows then: computed on, never
       // written), else four rows at a time
-      if (ntiles > 0) {
+      if (ntiles > 0 && pid < 2 * NKW) {
         if (p.q_tma) {
           if (elect_one()) {
             int mine = 0;
@@ -375,7 +420,10 @@ __global__ void __launch_bounds__(PairShape<HD, PAGED>::kThreads, 1)
           if (!alive) break;
           const uint32_t dst = ring + bf * Shape::kBufBytes;
           const uint32_t bar = full0 + bf * 8;
-          if (elect_one()) mbar_arrive_expect_tx_cluster(bar, my_bytes);
+          if (elect_one()) {
+            mbar_arrive_expect_tx_cluster(bar, my_bytes);
+            if (Shape::kVWarps > NKW && pw == 0) mbar_arrive_cluster(bar);
+          }
           __syncwarp();
 #pragma unroll(PAGED ? MINE : 2)
           for (int k = 0; k < MINE; ++k) {
@@ -413,8 +461,60 @@ __global__ void __launch_bounds__(PairShape<HD, PAGED>::kThreads, 1)
           cur = nxt;
         }
       };
-      if (is_k) produce(std::true_type{}, &tm_k, &tg_k);
-      else produce(std::false_type{}, &tm_v, &tg_v);
+      if (is_k) {
+        produce(std::true_type{}, &tm_k, &tg_k);
+      } else if constexpr (PAGED) {
+        produce(std::false_type{}, &tm_v, &tg_v);
+      } else {
+        // V of per-token slots: 16-byte copies, the other path into shared memory (a gather of four
+        // 128-byte rows takes about 66 cycles of TMA, a copy instruction of 512 bytes about 47 of the
+        // load/store unit: K by one and V by the other nearly add up).  A tile is handed over, behind the
+        // proxy fence, when the next one has been issued.
+        constexpr int VCH = CH / 2;                               // 16-byte chunks of half a row
+        constexpr int RPA = 32 / VCH;                             // rows of an access
+        const unsigned char* vbase = static_cast<const unsigned char*>(p.v_cache) + static_cast<int64_t>(h) * (HD * 2) + rank * HD;
+        const int64_t slot_stride = static_cast<int64_t>(p.hkv) * (HD * 2);
+        const int row0 = pw * 32;                                 // 32 of the tile's 128 keys
+        auto slot_of = [&](int tile) -> int {
+          const int t = kv_lo + tile * BN + row0 + lane;
+          int slot = tile < ntiles && t < kv_hi ? __ldg(ids + t) : -1;
+          if (slot < -1 || static_cast<int64_t>(slot) >= p.num_slots) {
+            if (p.status) atomicExch(p.status, 2);
+            slot = -1;
+          }
+          return slot;
+        };
+        auto hand_over = [&](int tile) {
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) mbar_arrive_cluster(full0 + ring_seq_v<LA>(tile) % NB * 8);
+        };
+        int slot = slot_of(0);
+#pragma unroll 1
+        for (int t = 0; t < ntiles; ++t) {
+          const int next = slot_of(t + 1);
+          const int seq = ring_seq_v<LA>(t), bf = seq % NB;
+          alive = mbar_wait_warp(bar_empty(bf), ((seq / NB) & 1) ^ 1, abort_flag);
+          if (!alive) break;
+          const uint32_t dst = ring + bf * Shape::kBufBytes;
+          const int chunk = lane % VCH;
+#pragma unroll
+          for (int i = 0; i < 32 / RPA; ++i) {
+            const int row = i * RPA + lane / VCH;
+            const int sl = __shfl_sync(0xffffffffu, slot, row);
+            cp_async_16(dst + tc_tile_offset<BN>(row0 + row, chunk),
+                        vbase + (sl >= 0 ? sl * slot_stride : 0) + chunk * 16, sl >= 0 ? 16 : 0);
+          }
+          cp_async_commit();
+          if (t > 0) {
+            cp_async_wait<1>();
+            hand_over(t - 1);
+          }
+          slot = next;
+        }
+        cp_async_wait<0>();
+        if (alive && ntiles > 0) hand_over(ntiles - 1);
+      }
       if (!alive) {
         if (p.status && lane == 0) atomicExch(p.status, 1);
         // gave up: let the copies still in flight land before the shared memory goes away
@@ -481,6 +581,8 @@ __global__ void __launch_bounds__(PairShape<HD, PAGED>::kThreads, 1)
       }
       if (!alive && p.status && lane == 0) atomicExch(p.status, 1);
     }
+    __syncwarp();
+    write_rows();
   } else {
     // =========================================================== softmax
     reg_inc<Shape::kSoftRegs>();
@@ -629,10 +731,6 @@ __global__ void __launch_bounds__(PairShape<HD, PAGED>::kThreads, 1)
       alive = mbar_wait_warp(bar_pv((ntiles - 1) % LA), ((ntiles - 1) / LA) & 1, abort_flag);
       if (alive) tc_fence_after();
     }
-    // Output rows are packed in the Q buffer (free: every S MMA is done; chunk c of row r sits at chunk
-    // position c ^ (r & 15)) and leave as whole rows, by all softmax warps.
-    constexpr int RB = HD * 2;
-    unsigned char* stage = smem_raw + (q_smem - smem_u32(smem_raw));
     float inv = l > 0.f ? 1.f / l : 0.f;
     if constexpr (NG == 2) {
       // O is relative to the last tile's reference maximum, each group's sum to that of its own last tile
@@ -666,46 +764,7 @@ __global__ void __launch_bounds__(PairShape<HD, PAGED>::kThreads, 1)
         *reinterpret_cast<uint4*>(stage + r * RB + ((chunk ^ (r & 15)) << 4)) = w;
       }
     }
-    if constexpr (NG == 2) softmax_groups_sync();
-    __syncwarp();
-    // whole rows, 32 per warp of a group (with two groups each warp takes half of them); a lane knows
-    // the place of one row, and the loads of four rows are in flight together
-    {
-      const int row_l = (warp & 3) * 32 + lane;
-      const int pkr = pk0 + rank * ROWS + row_l;
-      const int tlr = pkr / G, gr = pkr - tlr * G;
-      const int64_t off_l = row_l < rows_valid && alive
-                                ? (static_cast<int64_t>(sq.q_begin + tlr) * p.hq + static_cast<int64_t>(h) * G + gr) * HD
-                                : -1;
-      constexpr int RPI = 32 / CH == 0 ? 1 : 32 / CH;         // rows of an iteration
-      constexpr int N = 32 / NG;                              // rows of this warp
-      const int chunk = lane % CH;
-#pragma unroll 1
-      for (int r0 = grp * (32 - N); r0 < grp * (32 - N) + N; r0 += 4 * RPI) {
-        int64_t off[4];
-        uint4 w[4], gv[4];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const int rr = r0 + k * RPI + lane / CH;
-          off[k] = __shfl_sync(0xffffffffu, off_l, rr);
-          if (p.gate && off[k] >= 0)
-            gv[k] = *reinterpret_cast<const uint4*>(static_cast<const T*>(p.gate) + off[k] + chunk * 8);
-          const int row = (warp & 3) * 32 + rr;
-          w[k] = *reinterpret_cast<const uint4*>(stage + row * RB + ((chunk ^ (row & 15)) << 4));
-        }
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          if (off[k] < 0) continue;
-          if (p.gate) {
-            T* wo = reinterpret_cast<T*>(&w[k]);
-            const T* wg = reinterpret_cast<const T*>(&gv[k]);
-#pragma unroll
-            for (int e = 0; e < 8; ++e) wo[e] = apply_gate<T>(to_f32(wo[e]), wg[e]);
-          }
-          *reinterpret_cast<uint4*>(static_cast<T*>(p.out) + off[k] + chunk * 8) = w[k];
-        }
-      }
-    }
+    write_rows();
     if (!alive && p.status && r == 0) atomicExch(p.status, 1);
   }
 
