@@ -247,16 +247,14 @@ bool prefill_short_q(int max_len_extend, int group, int head_dim) {
 }
 
 // Pairs of CTAs (prefill_pair.cuh) serve query blocks of more than one 128-row tile whose key range is
-// not split.  Not head_dim 128 with per-token slots over longer contexts: there four-row gathers are all
-// the copies, and TMA moves them slower (about 45 cycles per 512 bytes) than the copying warps of the
-// 256-row CTA do (2000-token prompts over 8000 cached tokens: 1450 us against 1095); short contexts
-// gain from the faster start all the same (six prompts of up to 300 tokens: 117 us against 135).
+// not split.  Not head_dim 128 with per-token slots over longer contexts: there every row is a copy of
+// its own, and the pair has four copying warps and gathers of four rows against seven copying warps of the
+// 256-row CTA (two layers of 2000-token prompts over 8000 cached tokens: 1168 us against 1109; with
+// gathers for K and V alike 1450); short contexts gain from the faster start all the same (eight layers of
+// six prompts of up to 300 tokens: 116 us against 135).
 bool prefill_pairs(int max_len_extend, int group, int head_dim, int kv_chunk, bool paged, int batch,
                    int64_t total_kv) {
   if (kv_chunk != 0 || static_cast<int64_t>(max_len_extend) * group <= msgl::kTcSub) return false;
-#ifdef MSGL_TOKALL
-  return true;
-#endif
   return head_dim == 256 || paged || total_kv <= static_cast<int64_t>(batch) * 512;
 }
 

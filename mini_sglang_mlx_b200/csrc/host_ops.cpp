@@ -87,6 +87,16 @@ inline bool index_ok(const Tensor& t, const c10::Device& dev) {
 
 const int32_t* i32(const Tensor& t) { return static_cast<const int32_t*>(t.data_ptr()); }
 
+// A call of the C ABI without the GIL: a launch waits when the stream's queue is full.  (Its error
+// message is per thread.)
+template <typename F>
+int unlocked(F&& call) {
+  PyThreadState* state = PyEval_SaveThread();
+  const int rc = call();
+  PyEval_RestoreThread(state);
+  return rc;
+}
+
 PyObject* raise_status(int rc) {
   PyErr_Format(PyExc_RuntimeError, "%s [msgl status %d]", msgl_last_error_string(), rc);
   return nullptr;
@@ -181,10 +191,12 @@ PyObject* decode(PyObject*, PyObject* const* a, Py_ssize_t n) {
                    &ws, &ws_bytes))
     return nullptr;
   Tensor out = empty_like_rows(q);
-  const int rc = msgl_paged_decode_attention_sized(
+  const int rc = unlocked([&] {
+    return msgl_paged_decode_attention_sized(
       q.data_ptr(), kc.data_ptr(), vc.data_ptr(), i32(indptr), i32(indices), gate, out.data_ptr(), ws, ws_bytes,
       s.n, s.hq, s.hkv, s.d, s.num_slots, s.dtype, static_cast<float>(scale), static_cast<int>(max_splits),
       indices.numel(), reinterpret_cast<void*>(stream));
+  });
   return rc ? raise_status(rc) : THPVariable_Wrap(std::move(out));
 }
 
@@ -217,10 +229,12 @@ PyObject* decode_paged(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (!stream_of(a[11], s.device, &stream) || !scratch_for(s.device, stream, kDecode, need, &ws, &ws_bytes))
     return nullptr;
   Tensor out = empty_like_rows(q);
-  const int rc = msgl_paged_decode_attention_p16(
+  const int rc = unlocked([&] {
+    return msgl_paged_decode_attention_p16(
       q.data_ptr(), kc.data_ptr(), vc.data_ptr(), i32(indptr), i32(pages), i32(lens), i32(splits), gate,
       out.data_ptr(), ws, ws_bytes, s.n, s.hq, s.hkv, s.d, s.num_slots, s.dtype, static_cast<float>(scale),
       static_cast<int>(max_splits), static_cast<int>(page_size), total_pages, reinterpret_cast<void*>(stream));
+  });
   return rc ? raise_status(rc) : THPVariable_Wrap(std::move(out));
 }
 
@@ -256,8 +270,8 @@ PyObject* prefill(PyObject*, PyObject* const* a, Py_ssize_t n) {
     return nullptr;
   Tensor out = empty_like_rows(q);
   void* st = reinterpret_cast<void*>(stream);
-  const int rc =
-      gate ? msgl_paged_prefill_attention_gated(q.data_ptr(), kc.data_ptr(), vc.data_ptr(), i32(qo), i32(indptr),
+  const int rc = unlocked([&] {
+    return gate ? msgl_paged_prefill_attention_gated(q.data_ptr(), kc.data_ptr(), vc.data_ptr(), i32(qo), i32(indptr),
                                                 i32(indices), i32(prefix), gate, out.data_ptr(), ws, ws_bytes,
                                                 batch, s.n, total_kv, s.hq, s.hkv, s.d, s.num_slots, s.dtype,
                                                 static_cast<float>(scale), static_cast<int>(max_ext), cross,
@@ -267,6 +281,7 @@ PyObject* prefill(PyObject*, PyObject* const* a, Py_ssize_t n) {
                                           total_kv, s.hq, s.hkv, s.d, s.num_slots, s.dtype,
                                           static_cast<float>(scale), static_cast<int>(max_ext), cross,
                                           static_cast<int>(window), st);
+  });
   return rc ? raise_status(rc) : THPVariable_Wrap(std::move(out));
 }
 
@@ -306,11 +321,13 @@ PyObject* prefill_paged(PyObject*, PyObject* const* a, Py_ssize_t n) {
                    &ws, &ws_bytes))
     return nullptr;
   Tensor out = empty_like_rows(q);
-  const int rc = msgl_paged_prefill_attention_p16(
+  const int rc = unlocked([&] {
+    return msgl_paged_prefill_attention_p16(
       q.data_ptr(), kc.data_ptr(), vc.data_ptr(), i32(qo), i32(indptr), i32(pages), i32(lens), i32(prefix), gate,
       out.data_ptr(), ws, ws_bytes, batch, s.n, s.hq, s.hkv, s.d, s.num_slots, s.dtype, static_cast<float>(scale),
       static_cast<int>(max_ext), cross, static_cast<int>(window), static_cast<int>(page_size), total_pages,
       reinterpret_cast<void*>(stream));
+  });
   return rc ? raise_status(rc) : THPVariable_Wrap(std::move(out));
 }
 
@@ -339,9 +356,11 @@ PyObject* store_kv(PyObject*, PyObject* const* a, Py_ssize_t n) {
   size_t ws_bytes;
   if (!stream_of(a[5], dev.index(), &stream) || !scratch_for(dev.index(), stream, kDecode, 256, &ws, &ws_bytes))
     return nullptr;
-  const int rc = msgl_store_kv_cache(kc.data_ptr(), vc.data_ptr(), i32(idx), k.data_ptr(), v.data_ptr(),
+  const int rc = unlocked([&] {
+    return msgl_store_kv_cache(kc.data_ptr(), vc.data_ptr(), i32(idx), k.data_ptr(), v.data_ptr(),
                                      static_cast<int>(len), static_cast<int>(hkv), static_cast<int>(d), kc.size(0),
                                      kc.stride(0), k.stride(0), dt, ws, reinterpret_cast<void*>(stream));
+  });
   if (rc) return raise_status(rc);
   Py_RETURN_TRUE;
 }
@@ -383,11 +402,13 @@ PyObject* qk_norm_rope_store(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (rd == -1 && PyErr_Occurred()) return nullptr;
   int64_t stream;
   if (!stream_of(a[12], dev.index(), &stream)) return nullptr;
-  const int rc = msgl_qk_norm_rope_store(
+  const int rc = unlocked([&] {
+    return msgl_qk_norm_rope_store(
       q.data_ptr(), k.data_ptr(), v.data_ptr(), wt[0], wt[1], i32(pos), i32(loc), kc.data_ptr(), vc.data_ptr(),
       static_cast<int>(nt), static_cast<int>(hq), static_cast<int>(hkv), static_cast<int>(d), static_cast<int>(rd),
       static_cast<float>(base), static_cast<float>(eps), kc.size(0), q.stride(0), k.stride(0), v.stride(0),
       kc.stride(0), dt, reinterpret_cast<void*>(stream));
+  });
   if (rc) return raise_status(rc);
   Py_RETURN_TRUE;
 }
@@ -475,10 +496,12 @@ PyObject* decode_layer(PyObject*, PyObject* const* a, Py_ssize_t n) {
                    &ws, &ws_bytes))
     return nullptr;
   Tensor out = empty_like_rows(q);
-  const int rc = msgl_decode_layer(&rows, q.data_ptr(), kc.data_ptr(), vc.data_ptr(), i32(indptr), i32(indices),
+  const int rc = unlocked([&] {
+    return msgl_decode_layer(&rows, q.data_ptr(), kc.data_ptr(), vc.data_ptr(), i32(indptr), i32(indices),
                                    lens, gate, out.data_ptr(), ws, ws_bytes, s.n, s.hq, s.hkv, s.d, s.num_slots,
                                    s.dtype, static_cast<float>(scale), static_cast<int>(max_splits),
                                    static_cast<int>(page_size), total, reinterpret_cast<void*>(stream));
+  });
   return rc ? raise_status(rc) : THPVariable_Wrap(std::move(out));
 }
 
@@ -526,11 +549,13 @@ PyObject* prefill_layer(PyObject*, PyObject* const* a, Py_ssize_t n) {
                    &ws, &ws_bytes))
     return nullptr;
   Tensor out = empty_like_rows(q);
-  const int rc = msgl_prefill_layer(
+  const int rc = unlocked([&] {
+    return msgl_prefill_layer(
       &rows, q.data_ptr(), kc.data_ptr(), vc.data_ptr(), i32(qo), i32(indptr), i32(indices), lens, i32(prefix), gate,
       out.data_ptr(), ws, ws_bytes, batch, s.n, s.hq, s.hkv, s.d, s.num_slots, s.dtype, static_cast<float>(scale),
       static_cast<int>(max_ext), cross, static_cast<int>(window), static_cast<int>(page_size), total,
       reinterpret_cast<void*>(stream));
+  });
   return rc ? raise_status(rc) : THPVariable_Wrap(std::move(out));
 }
 
@@ -662,12 +687,14 @@ PyObject* index_arrays(PyObject*, PyObject* const* a, Py_ssize_t n) {
     buf = at::empty({off[9]}, at::TensorOptions().dtype(at::kInt).device(table.device()));
   }
   int32_t* p = static_cast<int32_t*>(buf.data_ptr());
-  const int rc = msgl_build_attn_metadata_host(
+  const int rc = unlocked([&] {
+    return msgl_build_attn_metadata_host(
       reinterpret_cast<const int32_t*>(PyBytes_AS_STRING(a[0])), i32(table), table.stride(0), table.size(0),
       table.size(1), static_cast<int>(batch), static_cast<int>(ps), static_cast<int>(chunk),
       static_cast<int>(max_splits), tq, tkv, paged ? tp : 0, p + off[0], p + off[1], p + off[2], p + off[3],
       tq ? p + off[4] : nullptr, p + off[5], size[6] ? p + off[6] : nullptr, paged ? p + off[7] : nullptr,
       size[8] ? p + off[8] : nullptr, ws, reinterpret_cast<void*>(stream));
+  });
   if (rc) return raise_status(rc);
   PyObject* out = PyTuple_New(9);
   if (out == nullptr) return nullptr;

@@ -83,7 +83,10 @@ def _workspace(nbytes: int, device: torch.device, stream_handle: int, kind: str)
         # allocated and zero-filled on the stream the kernels will run on, so that the fill is
         # ordered before them even when that stream is not torch's current one
         with torch.cuda.stream(torch.cuda.ExternalStream(stream_handle, device=device)):
-            ws = torch.zeros(max(nbytes, 1 << 20), dtype=torch.uint8, device=device)
+            # (a power of two: the need of a decode batch grows with its tokens, and the outgrown
+            # buffers of a doubling series together stay below the buffer in use)
+            size = 1 << (max(nbytes, 1 << 20) - 1).bit_length()
+            ws = torch.zeros(size, dtype=torch.uint8, device=device)
         _workspaces[key] = ws
     return ws
 

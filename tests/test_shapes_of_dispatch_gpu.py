@@ -1,0 +1,121 @@
+"""Shapes where the kernels' work splits and dispatch rules change: pairs of CTAs for prefill (query blocks
+around one 128-row half and one 256-row pair, key ranges around a 128-key tile, heads that do and do not
+divide 128), equal shares of a decode batch (share and sequence boundaries, batches above a warp's 32
+sequences, more pieces than one merge holds), and a layer's store and attention as one call."""
+import math
+
+import pytest
+import torch
+
+from oracle import paged_attention_oracle as O
+from tests.helpers import assert_close_to_oracle
+from tests.test_page_granular_gpu import make_pool
+
+pytestmark = pytest.mark.gpu
+
+
+def _i32(x):
+    return torch.tensor(x, dtype=torch.int32).cuda()
+
+
+def _problem(q_lens, prefixes, hkv, hq, d, seed, dtype=torch.bfloat16):
+    kv_lens = [a + b for a, b in zip(q_lens, prefixes)]
+    kc, vc, pip, pidx, slots = make_pool(kv_lens, 16, hkv, seed=seed, d=d, dtype=dtype)
+    g = torch.Generator().manual_seed(seed + 1)
+    q = torch.randn(sum(q_lens), hq, d, generator=g).to(dtype).cuda()
+    gate = torch.randn(sum(q_lens), hq, d, generator=g).to(dtype).cuda()
+    return q, gate, kc, vc, pip, pidx, slots, kv_lens
+
+
+@pytest.mark.parametrize("d,hkv,hq", [(128, 2, 8), (128, 1, 6), (256, 1, 8), (256, 2, 12)])
+@pytest.mark.parametrize("q_lens,prefixes,cross,window", [
+    ([129], [0], False, 0), ([22, 43, 65], [0, 128, 127], False, 0), ([64, 33, 1], [129, 640, 300], False, 0),
+    ([85, 171], [1000, 0], False, 200), ([100, 70], [513, 15], True, 0)], ids=str)
+def test_prefill_pairs(d, hkv, hq, q_lens, prefixes, cross, window):
+    """Through page ids, per-token slots and with a gate; the three agree with the oracle."""
+    from mini_sglang_mlx_b200 import paged_prefill_attention, paged_prefill_attention_p16
+    q, gate, kc, vc, pip, pidx, slots, kv_lens = _problem(q_lens, prefixes, hkv, hq, d, sum(q_lens) + hq)
+    qo, kvp, pre = _i32(O.build_indptr(q_lens).tolist()), _i32(O.build_indptr(kv_lens).tolist()), _i32(prefixes)
+    kw = dict(is_cross_attention=cross, sliding_window_size=window)
+    sc, n = 1 / math.sqrt(d), max(q_lens)
+    ref = O.paged_prefill_attention_oracle(q, kc, vc, qo, kvp, slots, pre, sc, **kw)
+    paged = (q, kc, vc, qo, pip, pidx, _i32(kv_lens), pre, sc, n)
+    out = paged_prefill_attention_p16(*paged, page_size=16, **kw)
+    assert_close_to_oracle(out, ref, "pages")
+    assert_close_to_oracle(paged_prefill_attention(q, kc, vc, qo, kvp, slots, pre, sc, n, **kw), ref, "slots")
+    gated = paged_prefill_attention_p16(*paged, page_size=16, gate=gate, **kw)
+    assert_close_to_oracle(gated, out.float().cpu() * torch.sigmoid(gate.float()).cpu(), "gate")
+
+
+@pytest.mark.parametrize("d,hkv,hq", [(128, 8, 16), (128, 2, 32), (256, 2, 16), (256, 1, 2)])
+@pytest.mark.parametrize("kv_lens", [[64], [1, 0, 63, 64, 65, 4097], [20000], [0] * 5 + [17] * 31 + [900],
+                                     [7, 300, 0, 1500] * 33], ids=lambda x: f"{len(x)}x{sum(x)}")
+def test_decode_shares(d, hkv, hq, kv_lens):
+    """(20000 tokens of one or two KV heads: more pieces than fit the merge at once.)"""
+    from mini_sglang_mlx_b200 import paged_decode_attention, paged_decode_attention_p16
+    q, gate, kc, vc, pip, pidx, slots, _ = _problem([1] * len(kv_lens), [max(l - 1, 0) for l in kv_lens], hkv, hq, d, 3)
+    need = [max(l, 1) for l in kv_lens]       # (an empty sequence keeps its page, unread)
+    kept, at = [], 0
+    for l, n in zip(kv_lens, need):
+        kept.append(slots[at:at + l])
+        at += n
+    slots, kvp, sc = torch.cat(kept), _i32(O.build_indptr(kv_lens).tolist()), 1 / math.sqrt(d)
+    splits = _i32([4] * len(kv_lens))
+    ref = O.paged_decode_attention_oracle(q, kc, vc, kvp, slots, sc)
+    out = paged_decode_attention_p16(q, kc, vc, pip, pidx, _i32(kv_lens), splits, sc, 4, page_size=16)
+    assert_close_to_oracle(out, ref, "pages")
+    assert torch.equal(paged_decode_attention(q, kc, vc, kvp, slots, splits, sc, 4), out)
+    gated = paged_decode_attention_p16(q, kc, vc, pip, pidx, _i32(kv_lens), splits, sc, 4, page_size=16, gate=gate)
+    assert_close_to_oracle(gated, out.float().cpu() * torch.sigmoid(gate.float()).cpu(), "gate")
+
+
+@pytest.mark.parametrize("page_size", [1, 16])
+@pytest.mark.parametrize("phase,batch", [("DECODE", 1), ("DECODE", 40), ("DECODE", 129), ("PREFILL", 6)])
+def test_a_layer_call_equals_store_then_attention(phase, batch, page_size):
+    """A pool of another class keeps the separate calls; layers run back to back, with nothing between."""
+    from mini_sglang_mlx_b200.attention import AttnBackend
+    from mini_sglang_mlx_b200.core import Batch, BatchPhase, Req
+    from mini_sglang_mlx_b200.kvcache import MHAKVCache
+
+    class OtherPool(MHAKVCache):
+        pass
+
+    class Cfg:
+        head_dim, num_kv_heads = 128, 2
+
+    g = torch.Generator().manual_seed(batch)
+    pages = torch.randperm(batch * (640 // page_size), generator=g).int().view(batch, -1)
+    table = (pages[:, :, None] * page_size + torch.arange(page_size, dtype=torch.int32)).reshape(batch, -1).cuda()
+    new = 1 if phase == "DECODE" else 70
+    cached = torch.randint(0, 500, (batch,), generator=g).tolist()
+    reqs = [Req(table_idx=i, cached_len=c, device_len=c + new) for i, c in enumerate(cached)]
+    loc = torch.cat([table[i, c:c + new] for i, c in enumerate(cached)])
+    n = loc.numel()
+    x = [[torch.randn(n, h, 128, generator=g).bfloat16().cuda() for h in (8, 2, 2)] for _ in range(4)]
+    w = [torch.randn(128, generator=g).bfloat16().cuda() for _ in range(2)]
+    got = []
+    for cls in (MHAKVCache, OtherPool):
+        pool = cls(2, 4, 128, table.numel(), torch.bfloat16)
+        pool._buffer.copy_(torch.randn(pool._buffer.shape, generator=torch.Generator().manual_seed(9)))
+        be = AttnBackend(Cfg, pool, table, page_size=page_size)
+        b = Batch(reqs=reqs, phase=BatchPhase[phase], out_loc=loc)
+        be.prepare_metadata(b)
+        outs = []
+        for i, (q, k, v) in enumerate(x):
+            outs.append(be.forward(q, k, v, i, b) if i % 2 else be.forward_from_projections(
+                q.clone(), k, v, i, b, q_norm_weight=w[0], k_norm_weight=w[1], rope_base=1e6)
+                if cls is MHAKVCache else _separate(be, pool, q, k, v, i, b, w))
+        got.append((outs, pool._buffer.clone()))
+    assert all(torch.equal(a, c) for a, c in zip(got[0][0], got[1][0]))
+    assert torch.equal(got[0][1], got[1][1])
+
+
+def _separate(be, pool, q, k, v, i, b, w):
+    from mini_sglang_mlx_b200.kernel import qk_norm_rope_store
+    if i % 2:
+        return be.forward(q, k, v, i, b)
+    md = b.attn_metadata
+    q = qk_norm_rope_store(q.clone(), k, v, w[0], w[1], md.positions, b.out_loc, pool.k_cache(i), pool.v_cache(i),
+                           rope_base=1e6)
+    torch.cuda.synchronize()
+    return be._attend(q, pool.k_cache(i), pool.v_cache(i), md, False, 0)
