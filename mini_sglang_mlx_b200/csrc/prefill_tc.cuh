@@ -293,7 +293,6 @@ __device__ __noinline__ void merge_kv_splits(const MergeArgs p, int nsp, int64_t
   // 16-byte chunk c of row r sits at chunk position c ^ (r & 31) of the row
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int G = p.group;
-  __threadfence();
   constexpr int VPL = HD / 32;          // output columns per lane
   constexpr int NV = VPL / 4;           // 16-byte pieces per lane
   // RU rows a warp works on at a time, SU splits whose loads are issued together
@@ -384,6 +383,83 @@ __device__ __noinline__ void merge_kv_splits(const MergeArgs p, int nsp, int64_t
       else
         *reinterpret_cast<uint4*>(out + oi) = *reinterpret_cast<const uint4*>(vals);
     }
+  }
+}
+
+// The same by the CTA that arrived last, NSW of its warps: the rows of all splits are copied into shared
+// memory with everything in flight at once, then a warp reduces a row at a time.  Straight from scratch, 8
+// rows in flight per warp, 64 rows x 2 splits took 6.7 us.  `buf`: `bytes` of free shared memory, holding
+// at least a row of every split.
+template <int N>
+__device__ __forceinline__ void mergers_sync() {
+  asm volatile("bar.sync 3, %0;" ::"n"(N) : "memory");
+}
+template <typename T, int HD, int NSW, int BM>
+__device__ __noinline__ void merge_kv_splits_cta(const MergeArgs p, int nsp, int64_t slot0, int64_t slot_stride,
+                                                 int rows, int pk0, int q_begin, int h, unsigned char* buf,
+                                                 int bytes) {
+  constexpr int RB = HD * 4, CPR = RB / 16;     // bytes and 16-byte chunks of a row
+  constexpr int VPL = HD / 32, NV = VPL / 4;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int G = p.group;
+  const int block = min(rows, bytes / (nsp * (RB + 8)));   // rows at a time
+  float2* ml = reinterpret_cast<float2*>(buf + static_cast<int64_t>(nsp) * block * RB);
+  T* out = static_cast<T*>(p.out);
+  const T* gate = static_cast<const T*>(p.gate);
+  for (int r0 = 0; r0 < rows; r0 += block) {
+    const int n = min(block, rows - r0);
+    for (int s = 0; s < nsp; ++s) {
+      const int64_t row0 = (slot0 + s * slot_stride) * BM + r0;
+      const unsigned char* src = reinterpret_cast<const unsigned char*>(p.part_o + row0 * HD);
+      const uint32_t dst = smem_u32(buf) + s * block * RB;
+      for (int c = tid; c < n * CPR; c += NSW * 32) cp_async_16(dst + c * 16, src + static_cast<int64_t>(c) * 16, 16);
+      for (int r = tid; r < n; r += NSW * 32)
+        ml[s * block + r] = __ldcg(reinterpret_cast<const float2*>(p.part_ml + (row0 + r) * 2));
+    }
+    cp_async_wait_all();
+    mergers_sync<NSW * 32>();
+#pragma unroll 2
+    for (int r = warp; r < n; r += NSW) {
+      float M = -INFINITY, L = 0.f;
+      for (int s = 0; s < nsp; ++s) M = fmaxf(M, ml[s * block + r].x);
+      float4 acc[NV];
+#pragma unroll
+      for (int e4 = 0; e4 < NV; ++e4) acc[e4] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 2
+      for (int s = 0; s < nsp; ++s) {
+        const float2 m = ml[s * block + r];
+        const float w = m.x == -INFINITY ? 0.f : fast_exp2(m.x - M);
+        L += w * m.y;
+        const unsigned char* row = buf + (static_cast<int64_t>(s) * block + r) * RB;
+#pragma unroll
+        for (int e4 = 0; e4 < NV; ++e4) {
+          // (chunk c of a row sits at chunk position c ^ (row of the unit & 31))
+          const float4 x = *reinterpret_cast<const float4*>(row + (((lane * NV + e4) ^ ((r0 + r) & 31)) << 4));
+          acc[e4].x += w * x.x;
+          acc[e4].y += w * x.y;
+          acc[e4].z += w * x.z;
+          acc[e4].w += w * x.w;
+        }
+      }
+      const float inv = L > 0.f ? 1.f / L : 0.f;
+      const int pk = pk0 + r0 + r;
+      const int tl = pk / G, g = pk - tl * G;
+      const int64_t oi =
+          (static_cast<int64_t>(q_begin + tl) * p.hq + static_cast<int64_t>(h) * G + g) * HD + lane * VPL;
+      alignas(16) T vals[VPL];
+#pragma unroll
+      for (int e4 = 0; e4 < NV; ++e4) {
+        const float f[4] = {acc[e4].x * inv, acc[e4].y * inv, acc[e4].z * inv, acc[e4].w * inv};
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          vals[4 * e4 + e] = gate ? apply_gate<T>(f[e], gate[oi + 4 * e4 + e]) : MmaOp<T>::from_float(f[e]);
+      }
+      if constexpr (VPL == 4)
+        *reinterpret_cast<uint2*>(out + oi) = *reinterpret_cast<const uint2*>(vals);
+      else
+        *reinterpret_cast<uint4*>(out + oi) = *reinterpret_cast<const uint4*>(vals);
+    }
+    mergers_sync<NSW * 32>();
   }
 }
 
@@ -1102,14 +1178,13 @@ __global__ void __launch_bounds__(TcShape<NSUB, HD, PAGED>::kThreads,
             bulk_commit();
             bulk_wait_all();            // the copy has read the buffer and written scratch
             fence_proxy_async_all();
-            __threadfence();            // ... device-wide, before this CTA's arrival is counted
           }
           __syncwarp();
           if (lane == 0) mbar_arrive(bar_st);
           alive = mbar_wait_warp(bar_st, st_phase, abort_flag);
           st_phase ^= 1;
         }
-        __threadfence();                // (m, l) of this row
+        // (made visible device-wide, with (m, l), by the release of this CTA's arrival)
 #ifdef MSGL_TRACE
         if (tid == 0) MSGL_TR(15, clock64());
 #endif
@@ -1145,8 +1220,7 @@ __global__ void __launch_bounds__(TcShape<NSUB, HD, PAGED>::kThreads,
     if (tid == 0) {
       MSGL_TR(11, clock64());
       int* ticket = p.tickets + (it.qt_base + qt) * p.hkv + h;
-      __threadfence();
-      const int arrived = atomicAdd(ticket, 1);
+      const int arrived = atomic_add_acq_rel(ticket, 1);
       s_last = (arrived == nsp - 1) ? 1 : 0;
       if (s_last) *ticket = 0;
     }
@@ -1160,12 +1234,17 @@ __global__ void __launch_bounds__(TcShape<NSUB, HD, PAGED>::kThreads,
     // (where the register pool was re-balanced only the softmax warps have the registers)
     constexpr int kMergers = Shape::kRebalanceRegs ? kMmaWarp : Shape::kWarps;
     if (s_last != 0 && warp < kMergers) {
-      // the softmax warps merge (a function of its own: its registers do not weigh on the main loop)
+      // the softmax warps merge (functions of their own: their registers do not weigh on the main loop)
       const MergeArgs ma{p.part_o, p.part_ml, p.out, p.gate, p.hq, p.group};
       // (rows x 2 splits in flight per lane: what the register cap of the main kernel holds)
       constexpr int kMergeRows = (!Shape::kRebalanceRegs && HD == 128) ? 4 : 2;
-      merge_kv_splits<T, HD, kMergers, BM, kMergeRows, 2>(ma, nsp, slot0, p.hkv, 0, rows_valid,
-                                                                    pk0, sq.q_begin, h);
+      constexpr int kFree = Shape::kSmemBytes - 1024;       // Q and the ring
+      if (NSUB == 1 && nsp * (HD * 4 + 8) * 16 <= kFree)    // (else: less than 16 rows at a time)
+        merge_kv_splits_cta<T, HD, kMergers, BM>(ma, nsp, slot0, p.hkv, rows_valid, pk0, sq.q_begin, h,
+                                                 smem_raw + (smem0 - smem_u32(smem_raw)), kFree);
+      else
+        merge_kv_splits<T, HD, kMergers, BM, kMergeRows, 2>(ma, nsp, slot0, p.hkv, 0, rows_valid, pk0,
+                                                            sq.q_begin, h);
 #ifdef MSGL_TRACE
       if (tid == 0) MSGL_TR(14, clock64());
 #endif
