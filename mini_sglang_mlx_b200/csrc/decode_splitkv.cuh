@@ -61,7 +61,7 @@ struct DecodeParams {
   int batch, hq, hkv, group;
   int num_shares;    // shares per head at most (= gridDim.x / hkv); 0: a share is a whole sequence
   int wave;          // shares per head that fill the GPU once
-  int min_share, max_share;  // groups a share holds at least, and at most while num_shares allows it
+  int min_share, max_share;  // groups a share holds at least; at most, while num_shares allows another wave
   int pad;           // what the end of a segment costs, in groups
   int64_t num_slots;
   float scale_log2;  // sm_scale * log2(e)
@@ -237,7 +237,9 @@ __global__ void __launch_bounds__(NWARPS * 32, HD == 256 ? 1 : 2)
     }
     int incl = scan(sum);
     int total = __shfl_sync(0xffffffffu, incl, 31);
-    share = min(max(ceil_div(total, p.wave), p.min_share), p.max_share);
+    // whole waves of CTAs: 1.2 waves of equal shares take as long as two
+    const int waves = max(1, min(ceil_div(total, p.wave * p.max_share), p.num_shares / p.wave));
+    share = max(ceil_div(total, p.wave * waves), p.min_share);
     share = max(share, ceil_div(total, p.num_shares));
     share = ceil_div(share, NWARPS) * NWARPS;
     if (run == 1) {
