@@ -1224,14 +1224,16 @@ int msgl_qk_norm_rope_store(void* q, const void* k, const void* v, const void* q
   p.log2_base = log2f(rope_base);
   p.eps = eps;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const int threads = 256;                          // sixteen half-warps, an item each per pass
+  const int threads = 256;                          // sixteen half-warps (or eight warps), an item each per pass
+  const int per_cta = threads / msgl::qk_lanes(head_dim);
   int sms = sm_count_cached();
   if (sms <= 0) sms = 148;
-  const int kR = msgl::qk_rows_per_item(head_dim);
+  constexpr int kR = msgl::kQkRowsPerItem;
   const int64_t items = static_cast<int64_t>(n_tokens) *
                         ((num_q_heads + kR - 1) / kR + 2 * ((num_kv_heads + kR - 1) / kR));
   if (items >= (1ll << 31)) return fail(MSGL_BAD_ARG, "qk_norm_rope_store: too many rows for one call");
-  const int64_t want = (items + 15) / 16;
+  const int64_t want = (items + per_cta - 1) / per_cta;
+  // (16 CTAs per SM at most; 8, 64, or as many items for each CTA: the same within 3 %)
   const int n_ctas = static_cast<int>(std::min<int64_t>(want, static_cast<int64_t>(sms) * 16));
   auto* kernel = head_dim == 256 ? (dtype == MSGL_DTYPE_BF16 ? msgl::qk_norm_rope_store_kernel<__nv_bfloat16, 256>
                                                              : msgl::qk_norm_rope_store_kernel<__half, 256>)
