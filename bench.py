@@ -50,10 +50,10 @@ FALLBACK_PEAKS = {"hbm_gbs": 6650.0, "bf16_tflops": 1590.0, "bf16_tflops_sustain
 # reduced batch and scale with the tokens read).  A workload without a capture reports no traffic.
 TRAFFIC_PER_ALGORITHMIC_BYTE = {
     "cfg1": (1.00, "profiles/dram_traffic_cfg1_cfg3.md"),
-    "cfg2": (0.83, "profiles/prefill_tc_kernel_cfg2.md"),
+    "cfg2": (0.84, "profiles/prefill_pair_kernel_cfg2.md"),
     "cfg3": (1.03, "profiles/dram_traffic_cfg1_cfg3.md"),
     "cfg4": (1.02, "profiles/prefill_tc_kernel_cfg4_batch8.md"),
-    "cfg5a": (1.005, "profiles/decode_partial_kernel_cfg5a_batch16.md"),
+    "cfg5a": (1.001, "profiles/decode_kernel_cfg5a_batch16.md"),
 }
 
 
