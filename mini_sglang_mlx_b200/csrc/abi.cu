@@ -247,15 +247,36 @@ bool prefill_short_q(int max_len_extend, int group, int head_dim) {
 }
 
 // Pairs of CTAs (prefill_pair.cuh) serve query blocks of more than one 128-row tile whose key range is
-// not split.  Not head_dim 128 with per-token slots over longer contexts: there every row is a copy of
-// its own, and the pair has four copying warps and gathers of four rows against seven copying warps of the
-// 256-row CTA (two layers of 2000-token prompts over 8000 cached tokens: 1168 us against 1109; with
-// gathers for K and V alike 1450); short contexts gain from the faster start all the same (eight layers of
-// six prompts of up to 300 tokens: 116 us against 135).
-bool prefill_pairs(int max_len_extend, int group, int head_dim, int kv_chunk, bool paged, int batch,
-                   int64_t total_kv) {
+// not split: head_dim 256 always, head_dim 128 where they are the faster of two forms.  A pair takes
+// about 17000 cycles for a 256-row item's start and end and 1900 per 128-key tile, a one-CTA item 20000
+// and 4000, and the GPU holds half as many pairs.  So pairs win on long key ranges, and where there are
+// few items (they finish one in half the time, and a second, partial wave costs them half).  The item and
+// tile counts are what the host knows: bounds and averages.  The line was fitted to 26 shapes (one to
+// twelve sequences, 300 to 4096 new tokens, 0 to 32768 cached, 4 and 8 KV heads), of which it decides one
+// wrongly, by 4 %; pairs everywhere were up to 33 % slower (twelve prompts of 500 tokens: 139 us against
+// 105), one-CTA tiles everywhere up to 23 % (one prompt of 600 tokens: 27 us against 21; 4096 tokens over
+// 32768: 2300 against 2043).
+// Per-token slots over longer contexts stay with the one-CTA form at head_dim 128: there every row is a
+// copy of its own, and the pair has four copying warps and gathers of four rows against seven copying
+// warps (two layers of 2000-token prompts over 8000 cached tokens: 1168 us against 1109; with gathers for
+// K and V alike 1450).
+bool prefill_pairs(int batch, int total_q, int64_t total_kv, int group, int num_kv_heads, int head_dim,
+                   int max_len_extend, bool cross, int window, int kv_chunk, bool paged, int sms) {
   if (kv_chunk != 0 || static_cast<int64_t>(max_len_extend) * group <= msgl::kTcSub) return false;
-  return head_dim == 256 || paged || total_kv <= static_cast<int64_t>(batch) * 512;
+  if (head_dim == 256) return true;
+  if (!paged && total_kv > static_cast<int64_t>(batch) * 512) return false;
+  const int64_t per_seq = (static_cast<int64_t>(max_len_extend) * group + 255) / 256;
+  const int64_t tiles_q = std::min<int64_t>(static_cast<int64_t>(total_q) * group / 256 + batch, per_seq * batch);
+  const double items = static_cast<double>(tiles_q) * num_kv_heads;
+  double keys = static_cast<double>(total_kv) / batch;
+  if (window > 0) keys = std::min(keys, static_cast<double>(window) + 256. / group);
+  else if (!cross) keys -= 0.5 * total_q / batch;
+  const double key_tiles = std::max(1., keys / 128);
+  auto waves = [&](double slots) {   // up to two waves end together, more of them overlap
+    const double x = items / slots;
+    return x <= 2 ? std::max(1., std::ceil(x)) : 0.75 * x + 0.25 * std::ceil(x);
+  };
+  return waves(sms / 2) * (17. + 1.9 * key_tiles) < waves(sms) * (20. + 4. * key_tiles);
 }
 
 PrefillPlan plan_prefill(int batch, int total_q, int64_t total_kv, int hq, int hkv, int head_dim,
@@ -303,7 +324,7 @@ PrefillPlan plan_prefill(int batch, int total_q, int64_t total_kv, int hq, int h
     // (sized for a sequence of average length: the lengths themselves are device data)
     const int64_t rows = std::min<int64_t>(BM, static_cast<int64_t>(max_len_extend) * G);
     const int64_t pieces_used = (visible / batch + chunk - 1) / chunk;
-    pl.fused_merge = pieces_used * rows * head_dim * 4 <= 64 * 1024;
+    pl.fused_merge = short_q && pieces_used * rows * head_dim * 4 <= 64 * 1024;
   }
 #ifdef MSGL_TRACE
   // development builds only: a key-range piece length to try instead of the policy's
@@ -1024,7 +1045,8 @@ static int prefill_impl(const void* q, const void* k_cache, const void* v_cache,
   cudaStream_t s = static_cast<cudaStream_t>(stream);
 
   dim3 grid(static_cast<unsigned>(pl.items * num_kv_heads));
-  bool pair = prefill_pairs(max_len_extend, p.group, head_dim, pl.kv_chunk, pages != nullptr, batch, total_kv) &&
+  bool pair = prefill_pairs(batch, total_q, total_kv, p.group, num_kv_heads, head_dim, max_len_extend,
+                            is_cross_attention != 0, sliding_window_size, pl.kv_chunk, pages != nullptr, sms) &&
               num_slots < (1ll << 31);
   CUtensorMap tg_k, tg_v;
   if (pair) {

@@ -1213,6 +1213,8 @@ __global__ void __launch_bounds__(TcShape<NSUB, HD, PAGED>::kThreads,
   // ---- kv splits: the CTA that arrives last at the unit's counter merges the partials
   // (out = sum_s 2^(m_s - M) O_s / sum_s 2^(m_s - M) l_s) and writes the output rows; no second
   // launch.  The counter goes back to zero for the next call.
+  // (Units of the two-sub-tile shape are always too large for that: its merge is a second launch.)
+  if constexpr (NSUB == 1)
   if (p.kv_chunk > 0 && sq.nsplit > 1 && p.tickets != nullptr) {
     __shared__ int s_last;
     const int nsp = sq.nsplit;
@@ -1239,7 +1241,7 @@ __global__ void __launch_bounds__(TcShape<NSUB, HD, PAGED>::kThreads,
       // (rows x 2 splits in flight per lane: what the register cap of the main kernel holds)
       constexpr int kMergeRows = (!Shape::kRebalanceRegs && HD == 128) ? 4 : 2;
       constexpr int kFree = Shape::kSmemBytes - 1024;       // Q and the ring
-      if (NSUB == 1 && nsp * (HD * 4 + 8) * 16 <= kFree)    // (else: less than 16 rows at a time)
+      if (nsp * (HD * 4 + 8) * 16 <= kFree)    // (else: less than 16 rows at a time)
         merge_kv_splits_cta<T, HD, kMergers, BM>(ma, nsp, slot0, p.hkv, rows_valid, pk0, sq.q_begin, h,
                                                  smem_raw + (smem0 - smem_u32(smem_raw)), kFree);
       else

@@ -30,9 +30,11 @@ def _problem(q_lens, prefixes, hkv, hq, d, seed, dtype=torch.bfloat16):
 @pytest.mark.parametrize("d,hkv,hq", [(128, 2, 8), (128, 1, 6), (256, 1, 8), (256, 2, 12)])
 @pytest.mark.parametrize("q_lens,prefixes,cross,window", [
     ([129], [0], False, 0), ([22, 43, 65], [0, 128, 127], False, 0), ([64, 33, 1], [129, 640, 300], False, 0),
-    ([85, 171], [1000, 0], False, 200), ([100, 70], [513, 15], True, 0)], ids=str)
+    ([85, 171], [1000, 0], False, 200), ([100, 70], [513, 15], True, 0),
+    ([300, 131, 217] * 12, [0, 5, 40] * 12, False, 0)], ids=lambda x: str(x)[:40])
 def test_prefill_pairs(d, hkv, hq, q_lens, prefixes, cross, window):
-    """Through page ids, per-token slots and with a gate; the three agree with the oracle."""
+    """Through page ids, per-token slots and with a gate; the three agree with the oracle.  (The last: enough
+    short items at head_dim 128 for the one-CTA form.)"""
     from mini_sglang_mlx_b200 import paged_prefill_attention, paged_prefill_attention_p16
     q, gate, kc, vc, pip, pidx, slots, kv_lens = _problem(q_lens, prefixes, hkv, hq, d, sum(q_lens) + hq)
     qo, kvp, pre = _i32(O.build_indptr(q_lens).tolist()), _i32(O.build_indptr(kv_lens).tolist()), _i32(prefixes)
