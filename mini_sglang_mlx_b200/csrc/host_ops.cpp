@@ -9,14 +9,17 @@
 // Contract with the Python wrappers: a call whose arguments are not what the operator takes, or
 // whose tensors live on a device that is not current, returns None and launches nothing; the
 // wrapper then names the fault (or makes the device current and calls again).  An error of the C
-// ABI is raised as RuntimeError with the library's message.
+// ABI is raised as RuntimeError with the library's message, and what C++ throws as the exception that
+// torch raises for it (see `guarded`).
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 
 #include <ATen/ATen.h>
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/utils/object_ptr.h>
 
 #include <algorithm>
 #include <cmath>
@@ -53,12 +56,12 @@ bool scratch_for(int device, int64_t stream, int kind, size_t need, void** ptr, 
       break;
     }
   if (found == nullptr || found->bytes < need) {
-    PyObject* t = PyObject_CallFunction(g_make_workspace, "niLs", static_cast<Py_ssize_t>(need), device,
-                                        static_cast<long long>(stream), kKindNames[kind]);
-    if (t == nullptr) return false;
-    const Tensor& ws = THPVariable_Unpack(t);
+    // (the Python side keeps the tensor alive)
+    THPObjectPtr t(PyObject_CallFunction(g_make_workspace, "niLs", static_cast<Py_ssize_t>(need), device,
+                                         static_cast<long long>(stream), kKindNames[kind]));
+    if (!t) return false;
+    const Tensor& ws = THPVariable_Unpack(t.get());
     const Scratch s{device, stream, kind, ws.data_ptr(), static_cast<size_t>(ws.numel())};
-    Py_DECREF(t);   // (the Python side keeps it alive)
     found = nullptr;
     for (Scratch& e : g_scratch)
       if (e.stream == stream && e.kind == kind && e.device == device) found = &e;
@@ -88,13 +91,26 @@ inline bool index_ok(const Tensor& t, const c10::Device& dev) {
 const int32_t* i32(const Tensor& t) { return static_cast<const int32_t*>(t.data_ptr()); }
 
 // A call of the C ABI without the GIL: a launch waits when the stream's queue is full.  (Its error
-// message is per thread.)
+// message is per thread.)  The GIL is taken back however the call ends.
 template <typename F>
 int unlocked(F&& call) {
-  PyThreadState* state = PyEval_SaveThread();
-  const int rc = call();
-  PyEval_RestoreThread(state);
-  return rc;
+  struct NoGil {
+    PyThreadState* state = PyEval_SaveThread();
+    ~NoGil() { PyEval_RestoreThread(state); }
+  } no_gil;
+  return call();
+}
+
+// The form in which a function of this module is handed to Python: torch turns what it throws into the
+// Python exception.  Above all an allocation that finds no memory is torch.OutOfMemoryError, which a
+// serving loop answers by giving cache back and calling again: every function allocates before its first
+// launch, so the call that failed has changed nothing.  (Left alone, a C++ exception that leaves a
+// CPython function ends the process.)
+template <PyObject* (*F)(PyObject*, PyObject* const*, Py_ssize_t)>
+PyObject* guarded(PyObject* self, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  return F(self, a, n);
+  END_HANDLE_TH_ERRORS
 }
 
 PyObject* raise_status(int rc) {
@@ -696,8 +712,8 @@ PyObject* index_arrays(PyObject*, PyObject* const* a, Py_ssize_t n) {
       size[8] ? p + off[8] : nullptr, ws, reinterpret_cast<void*>(stream));
   });
   if (rc) return raise_status(rc);
-  PyObject* out = PyTuple_New(9);
-  if (out == nullptr) return nullptr;
+  THPObjectPtr out(PyTuple_New(9));
+  if (!out) return nullptr;
   for (int i = 0; i < 9; ++i) {
     PyObject* t;
     if ((i == 6 && !per_token) || (i >= 7 && !paged)) {
@@ -705,14 +721,11 @@ PyObject* index_arrays(PyObject*, PyObject* const* a, Py_ssize_t n) {
       Py_INCREF(t);
     } else {
       t = piece(buf, off[i], size[i]);
-      if (t == nullptr) {
-        Py_DECREF(out);
-        return nullptr;
-      }
+      if (t == nullptr) return nullptr;
     }
-    PyTuple_SET_ITEM(out, i, t);
+    PyTuple_SET_ITEM(out.get(), i, t);
   }
-  return out;
+  return out.release();
 }
 
 // (callable): how scratch is made, see g_make_workspace
@@ -723,7 +736,8 @@ PyObject* set_workspace_maker(PyObject*, PyObject* fn) {
   Py_RETURN_NONE;
 }
 
-#define FAST(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(name)), METH_FASTCALL, nullptr}
+#define FAST(name) \
+  {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(&guarded<name>)), METH_FASTCALL, nullptr}
 PyMethodDef kMethods[] = {FAST(decode),       FAST(decode_paged),       FAST(prefill),
                           FAST(prefill_paged), FAST(store_kv),          FAST(qk_norm_rope_store),
                           FAST(decode_layer), FAST(prefill_layer),     FAST(collect_lens),
