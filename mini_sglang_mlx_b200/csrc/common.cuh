@@ -209,38 +209,53 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
 __device__ __forceinline__ void mbar_arrive_n(uint32_t bar, uint32_t count) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(count) : "memory");
 }
+// CLUSTER: what was written before a release at cluster scope is visible once its count is seen (else:
+// before a release of this CTA's threads).
+template <bool CLUSTER = false>
 __device__ __forceinline__ uint32_t mbar_try_wait(uint32_t bar, uint32_t parity) {
   uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.b32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
-      : "memory");
+  if constexpr (CLUSTER)
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.b32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+  else
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.b32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
   return ok;
 }
 // Bounded wait: false after `limit` SM cycles or once another thread has given up.
+template <bool CLUSTER = false>
 __device__ __forceinline__ bool mbar_wait_limit(uint32_t bar, uint32_t parity, volatile int* abort_flag,
                                                 long long limit) {
-  if (mbar_try_wait(bar, parity)) return true;
+  if (mbar_try_wait<CLUSTER>(bar, parity)) return true;
   const long long t0 = clock64();
   while (true) {
-    if (mbar_try_wait(bar, parity)) return true;
+    if (mbar_try_wait<CLUSTER>(bar, parity)) return true;
     if (*abort_flag != 0 || clock64() - t0 > limit) {
       *abort_flag = 1;
       return false;
     }
   }
 }
+template <bool CLUSTER = false>
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
-  return mbar_wait_limit(bar, parity, abort_flag, kTcWaitCycles);
+  return mbar_wait_limit<CLUSTER>(bar, parity, abort_flag, kTcWaitCycles);
 }
 // Warp-uniform form: every lane waits, the warp agrees on the outcome, so that the
 // warp-collective instructions that follow are executed by all lanes or by none.
+template <bool CLUSTER = false>
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity,
                                                volatile int* abort_flag) {
-  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag) ? 1 : 0) != 0;
+  return __all_sync(0xffffffffu, mbar_wait<CLUSTER>(bar, parity, abort_flag) ? 1 : 0) != 0;
 }
 // Arrive on `bar` once all cp.async copies issued so far by this thread have landed.
 __device__ __forceinline__ void cp_async_mbar_arrive(uint32_t bar) {

@@ -27,8 +27,9 @@
 //   next warp         MMA issuer (leader)
 //   next six warps    producers, three for the K tiles and three for the V tiles
 //
-// Everything arrives by TMA and is counted in bytes on the leader's barrier, from both CTAs
-// (.cta_group::2): full pages as boxes of 16 rows, anything else (per-token slots, a sequence's ragged
+// With per-token slots V comes by 16-byte copies, of four warps, and the warp that issues the MMAs in the
+// leader hands the peer's over.  Everything else arrives by TMA and is counted in bytes on the leader's
+// barrier, from both CTAs (.cta_group::2): full pages as boxes of 16 rows, anything else (per-token slots, a sequence's ragged
 // last page, query rows whose heads do not divide 128) as tile::gather4 loads of four rows, where an
 // absent row is one past the end of the tensor and reads as zeros.  Six producers because a warp
 // issues one TMA instruction in about 67 cycles: with two, and the tiles announced to the leader by a
@@ -80,10 +81,15 @@ __device__ __forceinline__ uint32_t cluster_addr(uint32_t addr, uint32_t rank) {
   return ra;
 }
 // Arrivals on a barrier of either CTA, without memory ordering of their own (a release at cluster scope
-// took 600 to 1300 cycles): tensor memory is ordered by the tcgen05 fences on both sides, and bytes
-// that TMA counts on the barrier itself.
+// took 600 to 1300 cycles), for what is ordered otherwise: tensor memory by the tcgen05 fences on both
+// sides, bytes that TMA counts by the barrier itself.  Ordinary writes to shared memory are neither:
+// those of the peer are handed over by mbar_arrive_release_cluster.
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_bar) {
   asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive_release_cluster(uint32_t cluster_bar, uint32_t count) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0], %1;" ::"r"(cluster_bar), "r"(count)
+               : "memory");
 }
 __device__ __forceinline__ void mbar_arrive_expect_tx_cluster(uint32_t cluster_bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.relaxed.cluster.shared::cluster.b64 _, [%0], %1;" ::"r"(cluster_bar), "r"(bytes)
@@ -175,6 +181,7 @@ __device__ __forceinline__ void softmax_groups_sync() { asm volatile("bar.sync 1
 struct PairBarriers {
   uint64_t q_full, full[8];              // leader: both CTAs' copies
   uint64_t empty[8];
+  uint64_t v_here[4];                    // per-token slots: this CTA's half of a V tile (16-byte copies)
   uint64_t s_full[3], p_full[3], pv_done[3];
 };
 
@@ -209,14 +216,18 @@ __global__ void __launch_bounds__(PairShape<HD, PAGED>::kThreads, 1)
   auto bar_p = [&](int b) { return smem_u32(&bars.p_full[b]); };
   auto bar_pv = [&](int b) { return smem_u32(&bars.pv_done[b]); };
   const uint32_t bar_q = smem_u32(&bars.q_full);
+  // (every second buffer of the ring holds V tiles, so a barrier's next use is behind the buffer's)
+  auto bar_v = [&](int tile) { return smem_u32(&bars.v_here[tile % (NB / 2)]); };
 
   if (tid == 0) {
     s_abort = 0;
     mbar_init(bar_q, 2 * 2 * NKW);
     for (int bf = 0; bf < NB; ++bf) {
-      mbar_init(bar_full(bf), 2 * Shape::kVWarps);   // both CTAs' producers (K: the first arrives for two)
+      mbar_init(bar_full(bf), 2 * NKW);      // both CTAs' producers (V of per-token slots: the peer's relay)
       mbar_init(bar_empty(bf), 1);
     }
+    if (!PAGED)
+      for (int i = 0; i < NB / 2; ++i) mbar_init(smem_u32(&bars.v_here[i]), Shape::kVWarps * 32);
     for (int b = 0; b < LA; ++b) {
       mbar_init(bar_s(b), 1);
       mbar_init(bar_p(b), 2 * (ROWS / 32));
@@ -420,10 +431,7 @@ __global__ void __launch_bounds__(PairShape<HD, PAGED>::kThreads, 1)
           if (!alive) break;
           const uint32_t dst = ring + bf * Shape::kBufBytes;
           const uint32_t bar = full0 + bf * 8;
-          if (elect_one()) {
-            mbar_arrive_expect_tx_cluster(bar, my_bytes);
-            if (Shape::kVWarps > NKW && pw == 0) mbar_arrive_cluster(bar);
-          }
+          if (elect_one()) mbar_arrive_expect_tx_cluster(bar, my_bytes);
           __syncwarp();
 #pragma unroll(PAGED ? MINE : 2)
           for (int k = 0; k < MINE; ++k) {
@@ -468,8 +476,9 @@ __global__ void __launch_bounds__(PairShape<HD, PAGED>::kThreads, 1)
       } else {
         // V of per-token slots: 16-byte copies, the other path into shared memory (a gather of four
         // 128-byte rows takes about 66 cycles of TMA, a copy instruction of 512 bytes about 47 of the
-        // load/store unit: K by one and V by the other nearly add up).  A tile is handed over, behind the
-        // proxy fence, when the next one has been issued.
+        // load/store unit: K by one and V by the other nearly add up).  They are ordinary writes: a tile's
+        // copies arrive on a barrier of this CTA as they land, and who hands them to the tensor pipe
+        // (the leader its own half, the relay below the peer's) puts the proxy fence behind it.
         constexpr int VCH = CH / 2;                               // 16-byte chunks of half a row
         constexpr int RPA = 32 / VCH;                             // rows of an access
         const unsigned char* vbase = static_cast<const unsigned char*>(p.v_cache) + static_cast<int64_t>(h) * (HD * 2) + rank * HD;
@@ -483,11 +492,6 @@ __global__ void __launch_bounds__(PairShape<HD, PAGED>::kThreads, 1)
             slot = -1;
           }
           return slot;
-        };
-        auto hand_over = [&](int tile) {
-          fence_proxy_async_smem();
-          __syncwarp();
-          if (lane == 0) mbar_arrive_cluster(full0 + ring_seq_v<LA>(tile) % NB * 8);
         };
         int slot = slot_of(0);
 #pragma unroll 1
@@ -505,15 +509,10 @@ __global__ void __launch_bounds__(PairShape<HD, PAGED>::kThreads, 1)
             cp_async_16(dst + tc_tile_offset<BN>(row0 + row, chunk),
                         vbase + (sl >= 0 ? sl * slot_stride : 0) + chunk * 16, sl >= 0 ? 16 : 0);
           }
-          cp_async_commit();
-          if (t > 0) {
-            cp_async_wait<1>();
-            hand_over(t - 1);
-          }
+          cp_async_mbar_arrive(bar_v(t));
           slot = next;
         }
-        cp_async_wait<0>();
-        if (alive && ntiles > 0) hand_over(ntiles - 1);
+        cp_async_wait_all();
       }
       if (!alive) {
         if (p.status && lane == 0) atomicExch(p.status, 1);
@@ -535,6 +534,15 @@ __global__ void __launch_bounds__(PairShape<HD, PAGED>::kThreads, 1)
         alive = mbar_wait_warp(bar_full(seq % NB), (seq / NB) & 1, abort_flag);
         if (alive) tc_fence_after();
       };
+      // V of per-token slots: the copies of this CTA's threads, and those of the peer's by its relay
+      auto acquire_written = [&](int seq, int tile) {
+        alive = mbar_wait_warp(bar_v(tile), (tile / (NB / 2)) & 1, abort_flag) &&
+                mbar_wait_warp<true>(bar_full(seq % NB), (seq / NB) & 1, abort_flag);
+        if (alive) {
+          fence_proxy_async_smem();
+          tc_fence_after();
+        }
+      };
       // frees a ring buffer in both CTAs (only while somebody will fill it again)
       auto release = [&](int seq) {
         if (seq + NB <= last_seq) tc_commit_pair(bar_empty(seq % NB));
@@ -545,7 +553,10 @@ __global__ void __launch_bounds__(PairShape<HD, PAGED>::kThreads, 1)
         const bool do_pv = j >= 0, do_s = j + LA < ntiles;
         const int sv = ring_seq_v<LA>(j), sk = ring_seq_k<LA>(j + LA);
         const int sb = (j + LA) % LA;                       // buffer of P of tile j and of S of tile j + LA
-        if (do_pv) acquire(sv);
+        if (do_pv) {
+          if constexpr (PAGED) acquire(sv);
+          else acquire_written(sv, j);
+        }
         if (alive && do_s) acquire(sk);
         if (alive && do_pv) {
           alive = mbar_wait_warp(bar_p(sb), (j / LA) & 1, abort_flag);
@@ -578,6 +589,21 @@ __global__ void __launch_bounds__(PairShape<HD, PAGED>::kThreads, 1)
           }
         }
         __syncwarp();
+      }
+      if (!alive && p.status && lane == 0) atomicExch(p.status, 1);
+    } else if (!PAGED && warp == Shape::kMmaWarp) {
+      // =========================================================== relay of the peer's V copies
+      // The release at cluster scope that ordinary writes need in front of the leader's MMAs.  A warp without
+      // copies of its own gives it: a release waits for its thread's copies in flight (given by the copying
+      // warps, behind the next tile's copies, it took 414 us instead of 280 on 1024 tokens over 16000 at
+      // head_dim 256, 455 instead of 394 on the gated prompts).
+      const uint32_t full0 = cluster_addr(bar_full(0), 0);
+      bool alive = true;
+#pragma unroll 1
+      for (int t = 0; t < ntiles && alive; ++t) {
+        alive = mbar_wait_warp(bar_v(t), (t / (NB / 2)) & 1, abort_flag);
+        fence_proxy_async_smem();
+        if (alive && lane == 0) mbar_arrive_release_cluster(full0 + ring_seq_v<LA>(t) % NB * 8, 2 * NKW);
       }
       if (!alive && p.status && lane == 0) atomicExch(p.status, 1);
     }
