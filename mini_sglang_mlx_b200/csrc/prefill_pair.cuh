@@ -162,13 +162,16 @@ __device__ __forceinline__ uint32_t idesc_m256(uint32_t n, uint32_t b_mn) {
   return (idesc_m128<T>(n, b_mn) & ~(0x1fu << 24)) | ((256u >> 4) << 24);
 }
 
-__device__ __forceinline__ uint2 ld_shared_volatile2(uint32_t addr) {
-  uint2 v;
-  asm volatile("ld.volatile.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(addr) : "memory");
-  return v;
+// A value and its tag as one 64-bit access: whoever sees the tag sees its value.  (The elements of a vector
+// access of two words are accesses of their own, in no given order.)
+__device__ __forceinline__ uint2 ld_shared_tagged(uint32_t addr) {
+  uint64_t v;
+  asm volatile("ld.volatile.shared.b64 %0, [%1];" : "=l"(v) : "r"(addr) : "memory");
+  return make_uint2(static_cast<uint32_t>(v), static_cast<uint32_t>(v >> 32));
 }
-__device__ __forceinline__ void st_shared_volatile2(uint32_t addr, uint2 v) {
-  asm volatile("st.volatile.shared.v2.u32 [%0], {%1, %2};" ::"r"(addr), "r"(v.x), "r"(v.y) : "memory");
+__device__ __forceinline__ void st_shared_tagged(uint32_t addr, uint32_t value, uint32_t tag) {
+  asm volatile("st.volatile.shared.b64 [%0], %1;" ::"r"(addr), "l"(static_cast<uint64_t>(tag) << 32 | value)
+               : "memory");
 }
 // Barrier of all threads of the CTA that may be reached from several places in the code.
 template <int N>
@@ -679,10 +682,10 @@ __global__ void __launch_bounds__(PairShape<HD, PAGED>::kThreads, 1)
         if (j > 0) {
           // (a value tagged with its tile: the reader polls its own row, no barrier in between)
           const uint32_t at = smem_u32(&s_mref[((j - 1) & 1) * ROWS + r]);
-          uint2 got = ld_shared_volatile2(at);
+          uint2 got = ld_shared_tagged(at);
           if (got.y != static_cast<uint32_t>(j - 1)) {
             const long long t0 = clock64();
-            while ((got = ld_shared_volatile2(at)).y != static_cast<uint32_t>(j - 1)) {
+            while ((got = ld_shared_tagged(at)).y != static_cast<uint32_t>(j - 1)) {
               if (*abort_flag != 0 || clock64() - t0 > kTcWaitCycles) {
                 *abort_flag = 1;
                 alive = false;
@@ -697,7 +700,7 @@ __global__ void __launch_bounds__(PairShape<HD, PAGED>::kThreads, 1)
       }
       const float m_new = mt > m_old + 8.f ? mt : m_old;
       if constexpr (NG == 2) {
-        st_shared_volatile2(smem_u32(&s_mref[(j & 1) * ROWS + r]), make_uint2(__float_as_uint(m_new), j));
+        st_shared_tagged(smem_u32(&s_mref[(j & 1) * ROWS + r]), __float_as_uint(m_new), j);
       }
       if (m_new != m_ref && m_ref != -INFINITY) alpha = fast_exp2(m_ref - m_new);
       const bool resc = m_new != m_old && m_old != -INFINITY;

@@ -36,3 +36,31 @@ def test_v_copied_by_the_peers_threads_is_what_the_leader_multiplies(n, keys):
         assert torch.equal(a, b)
     ref = O.paged_prefill_attention_oracle(q, kc, vc, qo, kvp, slots, pre, sc)
     assert (a.float().cpu() - ref).abs().max() <= 2e-2
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("n,keys,cross", [(200, 250, False), (300, 1000, False), (300, 1024, True)])
+def test_a_reference_maximum_that_grows_with_every_tile(n, keys, cross, dtype):
+    """At head_dim 128 the two softmax groups of a pair pass every row's reference maximum from tile to tile,
+    with the tile's number.  Scores that rise by up to 40 (base 2) a tile, fall, or stay, row by row: a maximum
+    of another tile would scale the row's sum and its accumulator differently.  (A key range this short is
+    not split, and few items run as pairs.)"""
+    from mini_sglang_mlx_b200 import paged_prefill_attention_p16
+    hkv, hq, d = 2, 8, 128
+    kc, vc, pip, pidx, slots = make_pool([keys], 16, hkv, seed=keys + n, d=d, dtype=dtype)
+    g = torch.Generator(device="cuda").manual_seed(n)
+    # score of row i and key t, base 2: slope_i * t / 128 plus noise of size 1
+    slope = torch.empty(n, hq, device="cuda").uniform_(-40, 40, generator=g)
+    unit = math.sqrt(d) / 8 * math.log(2)             # one in q's first column times 8 in K's: one, base 2
+    q = torch.empty(n, hq, d, device="cuda").normal_(generator=g)
+    q[..., 0] = slope * unit
+    kc[slots.long(), :, 0] = (torch.arange(keys, device="cuda") / 16.0).to(dtype)[:, None]
+    vc.uniform_(-1, 1, generator=g)
+    q = q.to(dtype)
+    qo, kvp, lens, pre = _i32([0, n]), _i32([0, keys]), _i32([keys]), _i32([keys - n])
+    sc = 1 / math.sqrt(d)
+    out = paged_prefill_attention_p16(q, kc, vc, qo, pip, pidx, lens, pre, sc, n, page_size=16,
+                                      is_cross_attention=cross)
+    ref = O.paged_prefill_attention_oracle(q, kc, vc, qo, kvp, slots, pre, sc, is_cross_attention=cross)
+    # |V| <= 1: probabilities and output rounded to 8 bits of mantissa, 2^-9 each; the scores (up to 320) in fp32
+    assert (out.float().cpu() - ref).abs().max() <= 2 ** -8 + 1e-3
