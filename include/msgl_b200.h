@@ -310,7 +310,8 @@ int msgl_build_attn_metadata(const int32_t* req, const int32_t* page_table, int6
  * The same arrays with the requests' numbers in HOST memory: `req_host` (3 * batch int32, same order)
  * is read before the call returns and travels as kernel parameters, so a step needs no copy, no
  * staging buffer and no event.  batch <= MSGL_METADATA_HOST_MAX.  Also writes kv_lens (batch), the KV
- * lengths, which the page-granular operators read.
+ * lengths, which the page-granular operators read.  Lengths whose sum does not fit 32 bits are refused
+ * (MSGL_BAD_SHAPE) before anything is launched.
  */
 #define MSGL_METADATA_HOST_MAX 1024
 int msgl_build_attn_metadata_host(const int32_t* req_host, const int32_t* page_table,

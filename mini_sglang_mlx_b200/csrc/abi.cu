@@ -1537,6 +1537,15 @@ int msgl_build_attn_metadata_host(const int32_t* req_host, const int32_t* page_t
   p.page_indptr = page_indptr;
   p.page_indices = page_indptr ? page_indices : nullptr;
   p.status = static_cast<int*>(status_word);
+  // Sums that 32 bits do not hold are refused: a wrapped one can pass the kernel's checks against the sizes of
+  // its outputs and would put entries in front of them.  (Pages: no more than KV tokens.)
+  int64_t sum_q = 0, sum_kv = 0;
+  for (int b = 0; b < batch; ++b) {
+    sum_q += std::max(req_host[b], 0);
+    sum_kv += std::max(req_host[batch + b], 0);
+  }
+  if (sum_q >= (1ll << 31) || sum_kv >= (1ll << 31))
+    return fail(MSGL_BAD_SHAPE, std::string(op) + "the sums of the lengths must be < 2^31");
   // entries the longest request writes decide how many CTAs each request gets
   int64_t widest = 0;
   auto launch = [&](auto tag) -> cudaError_t {

@@ -165,3 +165,16 @@ def test_page_granular_workspace_queries_are_host_arithmetic():
     op = lib.msgl_prefill_workspace_bytes(4, 2048, 16000, 32, 8, 128, 512, 0)
     both = lib.msgl_prefill_workspace_bytes_p16(4, 2048, 1000, 16, 32, 8, 128, 512, 0)
     assert both == (op + 255) // 256 * 256 + idx
+
+
+@pytest.mark.parametrize("lens", [[(1 << 31) - 1, 64], [1 << 30] * 3 + [64], [(1 << 31) - 1] * 3 + [64]], ids=str)
+@pytest.mark.parametrize("which", ["extend", "kv"])
+def test_metadata_refuses_sums_that_wrap(lens, which):
+    """A wrapped sum is negative, or small, and passes for a place inside the outputs.  Pointers are only
+    compared here: the check comes before any CUDA call."""
+    n, ok = len(lens), 0x10000
+    extend, kv = (lens, [64] * n) if which == "extend" else ([1] * n, lens)
+    req = (ctypes.c_int32 * (3 * n))(*extend, *kv, *([0] * n))
+    rc = _lib.lib().msgl_build_attn_metadata_host(
+        req, ok, 128, 4, 128, n, 16, 0, 32, 256, 256, 16, ok, ok, ok, ok, ok, ok, ok, ok, ok, None, None)
+    assert rc == 1 and "build_attn_metadata: the sums of the lengths must be < 2^31" in _lib.last_error()
