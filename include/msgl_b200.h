@@ -400,6 +400,7 @@ int64_t msgl_fast_compare_key(const void* a, const void* b, int64_t len_a, int64
  * cache_row_stride elements per slot.  head_dim 128 or 256; rotary_dim = head_dim, head_dim/2
  * or head_dim/4 (the first rotary_dim elements of a head are rotated, the rest pass through).
  * Tokens whose out_loc is outside [0, num_slots) get their q processed and their k/v dropped.
+ * All rows are 8-byte aligned (16 at head_dim 256), the norm weights 8.
  */
 int msgl_qk_norm_rope_store(void* q, const void* k, const void* v, const void* q_weight,
                             const void* k_weight, const int32_t* positions,

@@ -1216,7 +1216,7 @@ int msgl_qk_norm_rope_store(void* q, const void* k, const void* v, const void* q
   if (n_tokens == 0) return MSGL_OK;
   if (!q || !k || !v || !positions || !out_loc || !k_cache || !v_cache)
     return fail(MSGL_BAD_ARG, std::string(op) + "null tensor pointer");
-  const int va = head_dim == 256 ? 16 : 8;   // bytes of one lane's access
+  const int va = head_dim == 256 ? 16 : 8;   // (a lane's access takes 8 bytes at either head_dim)
   auto aligned = [va](const void* ptr) { return reinterpret_cast<uintptr_t>(ptr) % va == 0; };
   const int64_t ve = va / 2;
   if (!aligned(q) || !aligned(k) || !aligned(v) || !aligned(k_cache) || !aligned(v_cache) ||
@@ -1224,6 +1224,8 @@ int msgl_qk_norm_rope_store(void* q, const void* k, const void* v, const void* q
       cache_row_stride % ve != 0)
     return fail(MSGL_BAD_ARG, std::string(op) + "q, k, v and cache rows must be 8-byte aligned "
                                                 "(16-byte at head_dim 256)");
+  if (reinterpret_cast<uintptr_t>(q_weight) % 8 != 0 || reinterpret_cast<uintptr_t>(k_weight) % 8 != 0)
+    return fail(MSGL_BAD_ARG, std::string(op) + "the norm weights must be 8-byte aligned");
   msgl::QkNormRopeParams p{};
   p.q = q;
   p.k = k;

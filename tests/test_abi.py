@@ -178,3 +178,16 @@ def test_metadata_refuses_sums_that_wrap(lens, which):
     rc = _lib.lib().msgl_build_attn_metadata_host(
         req, ok, 128, 4, 128, n, 16, 0, 32, 256, 256, 16, ok, ok, ok, ok, ok, ok, ok, ok, ok, None, None)
     assert rc == 1 and "build_attn_metadata: the sums of the lengths must be < 2^31" in _lib.last_error()
+
+
+@pytest.mark.parametrize("head_dim", [128, 256])
+@pytest.mark.parametrize("which", [3, 4], ids=["q_weight", "k_weight"])
+def test_qk_norm_rope_store_rejects_misaligned_norm_weights(which, head_dim):
+    """A weight that is a slice of a larger parameter may start at any element; lanes read it 8 bytes at a
+    time.  Pointers are only compared here."""
+    ok, row = 0x10000, 8 * head_dim
+    args = [ok, ok, ok, ok, ok, ok, ok, ok, ok, 4, 16, 8, head_dim, head_dim, 1e6, 1e-6, 64, 2 * row, row, row, row, 0,
+            None]
+    args[which] = ok + 2
+    assert _lib.lib().msgl_qk_norm_rope_store(*args) == 5
+    assert "qk_norm_rope_store: the norm weights must be 8-byte aligned" in _lib.last_error()
