@@ -10,6 +10,7 @@ op-prefixed messages.
 """
 from __future__ import annotations
 
+import threading
 from typing import Dict, Optional, Tuple
 
 import torch
@@ -37,6 +38,10 @@ _DTYPES = {torch.bfloat16: _lib.DTYPE_BF16, torch.float16: _lib.DTYPE_F16}
 # it, and never shared between operators.
 _workspaces: Dict[Tuple[int, int, str], torch.Tensor] = {}
 _retired: list = []   # outgrown buffers stay alive: work queued on their stream may still use them
+# The native calls keep a buffer's address, so a buffer that was handed out once must stay in one of
+# the two: threads that ask for the same scratch at the same time (an allocation lets others run)
+# take turns.
+_workspaces_lock = threading.Lock()
 
 
 _raw_current_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
@@ -76,18 +81,19 @@ def _on_device(device: torch.device):
 def _workspace(nbytes: int, device: torch.device, stream_handle: int, kind: str) -> torch.Tensor:
     index = device.index if device.index is not None else torch.cuda.current_device()
     key = (index, stream_handle, kind)
-    ws = _workspaces.get(key)
-    if ws is None or ws.numel() < nbytes:
-        if ws is not None:
-            _retired.append(ws)
-        # allocated and zero-filled on the stream the kernels will run on, so that the fill is
-        # ordered before them even when that stream is not torch's current one
-        with torch.cuda.stream(torch.cuda.ExternalStream(stream_handle, device=device)):
-            # (a power of two: the need of a decode batch grows with its tokens, and the outgrown
-            # buffers of a doubling series together stay below the buffer in use)
-            size = 1 << (max(nbytes, 1 << 20) - 1).bit_length()
-            ws = torch.zeros(size, dtype=torch.uint8, device=device)
-        _workspaces[key] = ws
+    with _workspaces_lock:
+        ws = _workspaces.get(key)
+        if ws is None or ws.numel() < nbytes:
+            # allocated and zero-filled on the stream the kernels will run on, so that the fill is
+            # ordered before them even when that stream is not torch's current one
+            with torch.cuda.stream(torch.cuda.ExternalStream(stream_handle, device=device)):
+                # (a power of two: the need of a decode batch grows with its tokens, and the outgrown
+                # buffers of a doubling series together stay below the buffer in use)
+                size = 1 << (max(nbytes, 1 << 20) - 1).bit_length()
+                grown = torch.zeros(size, dtype=torch.uint8, device=device)
+            if ws is not None:
+                _retired.append(ws)
+            _workspaces[key] = ws = grown
     return ws
 
 
