@@ -133,10 +133,10 @@ def _again(op: str, fn, device: torch.device, *args):
 def device_status(device=None) -> int:
     """Synchronise and return the OR of the device status words of every
     workspace on ``device`` (0 = no kernel reported an out-of-range slot),
-    clearing them."""
+    clearing them.  (Outgrown buffers count: what was reported before a buffer grew is not lost.)"""
     torch.cuda.synchronize(device)
     status = 0
-    for ws in _workspaces.values():
+    for ws in [*_workspaces.values(), *_retired]:
         word = ws[:4].view(torch.int32)
         status |= int(word.item())
         word.zero_()

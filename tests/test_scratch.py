@@ -56,3 +56,13 @@ def test_growth_that_finds_no_memory_leaves_the_buffer_in_use(host_scratch, monk
     assert K._workspace(100, dev, 7, "decode") is first and K._retired == []
     grown = K._workspace(first.numel() + 1, dev, 7, "decode")
     assert grown.numel() == 2 * first.numel() and K._retired == [first]
+
+
+def test_a_report_from_before_a_buffer_grew_is_not_lost(host_scratch, monkeypatch):
+    monkeypatch.setattr(torch.cuda, "synchronize", lambda device=None: None)
+    dev = torch.device("cuda", 0)
+    first = K._workspace(100, dev, 7, "decode")
+    first[:4].view(torch.int32).fill_(2)              # (a kernel met a slot outside the pool)
+    K._workspace(first.numel() + 1, dev, 7, "decode")
+    assert K.device_status() == 2
+    assert K.device_status() == 0
