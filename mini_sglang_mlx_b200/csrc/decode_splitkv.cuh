@@ -320,7 +320,9 @@ __global__ void __launch_bounds__(NWARPS * 32, HD == 256 ? 1 : 2)
   constexpr int BATCH = PAGED ? 32 : 2;
   struct Batch {
     int count, t0, len;  // groups; token of the first one; tokens there are
-    int y;               // PAGED: lane j, group j: first pool row; else lane 16 j + r: slot of row r; -1: zeros
+    // PAGED: lane j, group j: first pool row, num_slots if the page is outside the pool (rows behind the pool
+    // read as zeros); else lane 16 j + r: slot of row r, -1: zeros
+    int y;
   };
   Segment ps;
   int pb = b0, pg = warp;
@@ -343,7 +345,10 @@ __global__ void __launch_bounds__(NWARPS * 32, HD == 256 ? 1 : 2)
       const int64_t row = static_cast<int64_t>(id) * per + t % per;
       const int rows = PAGED ? min(kDecodeGroupTokens, w.len - t) : 1;
       if (id >= 0 && row + rows <= p.num_slots) w.y = static_cast<int>(row);
-      else if (p.status) atomicExch(p.status, 2);   // page or slot outside the pool: zeros
+      else {                                        // page or slot outside the pool: zeros
+        if (PAGED) w.y = static_cast<int>(p.num_slots);
+        if (p.status) atomicExch(p.status, 2);
+      }
     }
   };
   auto bar_of = [&](int stage) { return smem_u32(&s_bar[PAGED ? warp * NSTAGES + stage : 0]); };
@@ -377,7 +382,7 @@ __global__ void __launch_bounds__(NWARPS * 32, HD == 256 ? 1 : 2)
     if constexpr (PAGED) {
       const uint32_t bar = bar_of(stage);
       const int y = __shfl_sync(0xffffffffu, cur.y, ck);
-      const int n = y < 0 ? 0 : min(kDecodeGroupTokens, cur.len - cur.t0 - ck * (NWARPS * kDecodeGroupTokens));
+      const int n = min(kDecodeGroupTokens, cur.len - cur.t0 - ck * (NWARPS * kDecodeGroupTokens));
       if (n == kDecodeGroupTokens) {
         if (lane == 0) {
           mbar_arrive_expect_tx(bar, 2 * TILE_BYTES);
@@ -388,13 +393,13 @@ __global__ void __launch_bounds__(NWARPS * 32, HD == 256 ? 1 : 2)
           }
         }
       } else {
-        // ragged last page of the sequence (or a page outside the pool): valid rows by 16-byte
-        // copies, the rest zeros; the barrier completes when the copies of all lanes have landed
+        // ragged last page of the sequence: valid rows by 16-byte copies, the rest zeros; the barrier
+        // completes when the copies of all lanes have landed
 #pragma unroll 4
         for (int k = 0; k < kDecodeGroupTokens * CH / 32; ++k) {
           const int e = k * 32 + lane;
           const int row = e / CH, chunk = e % CH;
-          const bool ok = row < n;
+          const bool ok = row < n && y < p.num_slots;
           const int64_t off =
               (ok ? static_cast<int64_t>(y + row) * slot_stride + head_off : 0) + chunk * 16;
           cp_async_16(kdst + toff(row, chunk), kbase + off, ok ? 16 : 0);
@@ -618,6 +623,8 @@ __global__ void __launch_bounds__(NWARPS * 32, HD == 256 ? 1 : 2)
     cg -= cs.ng;
 
     wait_in_front();     // (a warp without groups)
+    // (a sequence's ragged last page came by ordinary copies, and its stage is filled by TMA next)
+    if (PAGED && cs.t_hi % kDecodeGroupTokens != 0) fence_proxy_async_smem();
     // ---- end of the segment: the warps' partials are merged, four heads at a time, a warp per head
     // and a lane per VPL consecutive columns
     const bool whole = cs.beg >= r0 && cs.end <= r1;     // (positions of its groups, not of the padding)

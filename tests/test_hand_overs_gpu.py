@@ -6,6 +6,7 @@ import pytest
 import torch
 
 from oracle import paged_attention_oracle as O
+from tests.helpers import assert_close_to_oracle
 from tests.test_page_granular_gpu import make_pool
 
 pytestmark = pytest.mark.gpu
@@ -64,3 +65,37 @@ def test_a_reference_maximum_that_grows_with_every_tile(n, keys, cross, dtype):
     ref = O.paged_prefill_attention_oracle(q, kc, vc, qo, kvp, slots, pre, sc, is_cross_attention=cross)
     # |V| <= 1: probabilities and output rounded to 8 bits of mantissa, 2^-9 each; the scores (up to 320) in fp32
     assert (out.float().cpu() - ref).abs().max() <= 2 ** -8 + 1e-3
+
+
+@pytest.mark.parametrize("d", [128, 256])
+@pytest.mark.parametrize("bad", [False, True], ids=["pages", "pages outside the pool"])
+def test_a_ring_stage_changes_between_ordinary_and_bulk_copies(d, bad):
+    """Decode rings run on across sequences: the stage that held a ragged last page (ordinary copies) is filled
+    by TMA next, over and over, and the pool changes from call to call.  The per-token form copies every
+    row the ordinary way and runs the same shares, so it gives the same bits; rows of a page outside the
+    pool are zeros in both."""
+    from mini_sglang_mlx_b200 import paged_decode_attention, paged_decode_attention_p16
+    from mini_sglang_mlx_b200.kernel import device_status
+    hkv, hq, splits = 2, 8, 4
+    kv_lens = [1 + 37 * i % 113 for i in range(300)] + [1999, 4001]
+    kc, vc, pip, pidx, slots = make_pool(kv_lens, 16, hkv, seed=d, d=d)
+    g = torch.Generator(device="cuda").manual_seed(d)
+    if bad:                                           # every third page
+        pidx[::3] += kc.shape[0]
+        page = torch.repeat_interleave(torch.arange(pidx.numel()).cuda(), 16)
+        own = torch.cat([torch.arange(l) + 16 * int(a) for l, a in zip(kv_lens, pip.tolist())]).cuda()
+        slots[page[own] % 3 == 0] = -1
+    q = torch.empty(len(kv_lens), hq, d, dtype=torch.bfloat16, device="cuda").normal_(generator=g)
+    kvp, lens, n = _i32(O.build_indptr(kv_lens).tolist()), _i32(kv_lens), _i32([splits] * len(kv_lens))
+    sc = 1 / math.sqrt(d)
+    device_status()
+    for _ in range(4):
+        kc.normal_(generator=g)
+        vc.normal_(generator=g)
+        a = paged_decode_attention_p16(q, kc, vc, pip, pidx, lens, n, sc, splits, page_size=16)
+        b = paged_decode_attention(q, kc, vc, kvp, slots, n, sc, splits)
+        assert torch.equal(a, b)
+    assert device_status() == (2 if bad else 0)
+    if not bad:
+        ref = O.paged_decode_attention_oracle(q, kc, vc, kvp, slots, sc)
+        assert_close_to_oracle(a, ref, "pages")
