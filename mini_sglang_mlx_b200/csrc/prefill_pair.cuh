@@ -247,6 +247,7 @@ __global__ void __launch_bounds__(PairShape<HD, PAGED>::kThreads, 1)
   ItemCoord it;
   const bool have_item = find_item<Shape::kThreads>(p, static_cast<int>(blockIdx.x) / 2, BM,
                                                     reinterpret_cast<int*>(smem_raw), it);
+  fence_proxy_async_smem();     // (Q comes to where the item search had its counts)
   if (p.early) grid_dependency_wait();
   grid_dependency_launch();
   tc_fence_before();

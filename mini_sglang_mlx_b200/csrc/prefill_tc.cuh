@@ -543,6 +543,7 @@ __global__ void __launch_bounds__(TcShape<NSUB, HD, PAGED>::kThreads,
   ItemCoord it;
   const bool have_item =
       find_item<kTcThreads>(p, static_cast<int>(blockIdx.x), BM, reinterpret_cast<int*>(smem_raw), it);
+  if (PAGED) fence_proxy_async_smem();   // (Q comes by bulk copies to where the item search had its counts)
   if (p.early) grid_dependency_wait();   // the item is found while the K/V store drains
   grid_dependency_launch();
   tc_fence_before();
