@@ -32,7 +32,8 @@
  *   kv_indptr, qo_indptr   (batch + 1) int32, CSR row pointers
  *   kv_indices             (kv_indptr[batch]) int32, slot id of every KV token
  *   prefix_lens            (batch) int32, absolute position of a sequence's first query row
- *   num_kv_splits          (batch) int32, split-KV hint per sequence
+ *   num_kv_splits          (batch) int32, the reference's split-KV hint per sequence; not read (the
+ *                          decode op cuts the batch into equal shares), may be NULL
  * Grouped-query mapping: kv_head = q_head / (num_q_heads / num_kv_heads).
  * q, out, gate, the pools and every workspace must be 16-byte aligned (the
  * kernels move them in 16-byte pieces); the attention ops return MSGL_BAD_ARG
@@ -107,8 +108,9 @@ size_t msgl_decode_workspace_bytes_full(int batch, int num_q_heads, int num_kv_h
  * (mini-sglang-mlx-kernel/csrc/paged_decode_attention.cpp:15-73, binding
  * csrc/bindings.cpp:36-44) and its two Metal stages
  * (csrc/paged_decode_attention.metal:313-506, 512-586).
- * num_kv_splits may be NULL (then every sequence uses max_kv_splits capped by
- * its length).  Sequences of length 0 produce zeros.
+ * The work split does not follow num_kv_splits (not read); max_kv_splits sets the
+ * least scratch that a call takes (msgl_decode_workspace_bytes).  Sequences of
+ * length 0 produce zeros.
  */
 int msgl_paged_decode_attention(
     const void* q, const void* k_cache, const void* v_cache,

@@ -17,10 +17,10 @@ Differences, all inside the boundary:
   (``page_indptr`` / ``page_indices`` / ``kv_lens``) and, when the page size is a
   multiple of 16, attention runs through the page-granular operators whose kernels
   fetch K/V as TMA boxes.
-* ``num_kv_splits`` is chosen for a 148-SM part from the batch's total work
-  (``compute_num_kv_splits``); ``policy="reference"`` keeps the reference rule
-  ``min(32, max(1, ceil(L/128)))`` (lines 304-307).  The result of the decode
-  op does not depend on the choice beyond fp32 rounding.
+* ``num_kv_splits`` is filled in for callers that read it (``compute_num_kv_splits``;
+  ``policy="reference"`` keeps the reference rule ``min(32, max(1, ceil(L/128)))``, lines
+  304-307).  The decode op does not: it cuts the batch into equal shares, and takes from
+  ``max_kv_splits`` only the least scratch of a call.
 """
 from __future__ import annotations
 
@@ -84,7 +84,7 @@ AttnMetadata = PrefillMetadata | DecodeMetadata
 
 def compute_num_kv_splits(kv_lens: Sequence[int], num_kv_heads: int, *, sm_count: int = 148,
                           max_kv_splits: int = MAX_KV_SPLITS, policy: str = "b200") -> List[int]:
-    """Per-sequence split count of the decode op.
+    """Per-sequence split count, the hint that ``DecodeMetadata.num_kv_splits`` carries.
 
     ``reference``: ``min(max, max(1, ceil(L/128)))`` (reference lines 304-307).
     ``b200``: one split per ``chunk`` tokens (``split_chunk_tokens``).
@@ -97,13 +97,12 @@ def compute_num_kv_splits(kv_lens: Sequence[int], num_kv_heads: int, *, sm_count
 
 def split_chunk_tokens(total_kv: int, num_kv_heads: int, *, sm_count: int = 148, batch: int = 0,
                        policy: str = "b200") -> int:
-    """Tokens per split of the decode op for a batch with ``total_kv`` KV tokens.
+    """Tokens per split in the hints of a batch with ``total_kv`` KV tokens.
 
-    ``b200``: the batch's ``total_kv * num_kv_heads`` token-heads spread over about 16 CTAs per
-    SM, clamped to [256, 4096] tokens: enough CTAs to fill the SMs, small enough that a long
-    sequence does not leave a tail.  A small batch that would then need a little more than one
-    wave of CTAs (two are resident per SM) gets the chunk that makes it exactly one: a CTA of
-    such a batch is a chain of memory latencies, and a second, partial wave doubles it."""
+    ``b200``, for a grid of one CTA per (sequence, head, split): the batch's ``total_kv *
+    num_kv_heads`` token-heads spread over about 16 CTAs per SM, clamped to [256, 4096] tokens; a
+    small batch that would need a little more than one wave of CTAs (two are resident per SM) gets
+    the chunk that makes it exactly one."""
     if policy == "reference":
         return 128
     chunk = -(-total_kv * num_kv_heads // (sm_count * 16))
@@ -317,9 +316,8 @@ class AttnBackend:
                                    batch=len(packed) // 12, policy=self.split_policy)
         _, kvp, prefix, splits, _, lens, ids, page_indptr, page_ids = self._index_arrays(
             packed, total_q, total_kv, pages, chunk)
-        # the split dimension of the launch grid: what the longest sequence needs, not the cap
-        # (CTAs of split slots no sequence uses would only start, look up a length and leave)
-        # (the reference policy keeps the reference's constant, backend.py:293)
+        # the largest entry of num_kv_splits, which the least scratch of a call is sized by (the
+        # reference policy keeps the reference's constant, backend.py:293)
         max_splits = MAX_KV_SPLITS
         if self.split_policy != "reference":
             max_splits = min(MAX_KV_SPLITS, max(1, -(-max_kv // chunk)))

@@ -152,7 +152,7 @@ template <typename T>
 __device__ __forceinline__ T apply_gate(float out, T gate) {
   const float o = to_f32(MmaOp<T>::from_float(out));
   // (a fast division, two units in the last place of fp32, in front of a rounding to 16 bits: the exact one
-  // took most of a 128-row epilogue, 38 us at head_dim 256)
+  // took most of a 128-row epilogue, 38 us at head_dim 256.  Below 2^-126 it gives zero.)
   const float s = to_f32(MmaOp<T>::from_float(__fdividef(1.f, 1.f + __expf(-to_f32(gate)))));
   return MmaOp<T>::from_float(o * s);
 }
@@ -296,13 +296,6 @@ __device__ __forceinline__ void bulk_commit() {
 __device__ __forceinline__ void bulk_wait_all() {
   asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
 }
-// global -> shared, the bytes are counted on `bar` as they land:
-__device__ __forceinline__ void bulk_load(uint32_t sdst, const void* gsrc, uint32_t bytes, uint32_t bar) {
-  asm volatile(
-      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-      ::"r"(sdst), "l"(gsrc), "r"(bytes), "r"(bar)
-      : "memory");
-}
 // orders this thread's accesses through the generic proxy with those of the async proxy
 // (bulk copies), in every state space
 __device__ __forceinline__ void fence_proxy_async_all() {
@@ -317,12 +310,17 @@ __device__ __forceinline__ void fence_proxy_async_smem() {
 __device__ __forceinline__ void fence_mbar_init() {
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
-// Programmatic dependent launch.  Every kernel here is launched so that its CTAs may be resident
-// while the kernel in front of it in the stream drains: it sets up what is its own (shared memory,
-// barriers, tensor memory), then grid_dependency_wait() blocks until the kernel in front has
-// finished and its writes are visible (no-op when launched without the attribute), and only then
-// does it touch global memory or let the kernel behind it in (grid_dependency_launch).  So a kernel
-// that has started knows that everything but the one kernel in front of it is complete.
+// Programmatic dependent launch.  The kernels of a layer (K/V store, norm + rotary + store, decode,
+// prefill and its merge) are launched so that their CTAs may be resident while the kernel in front in
+// the stream drains: they set up what is their own (shared memory, barriers, tensor memory), then
+// grid_dependency_wait() blocks until the kernel in front has finished and its writes are visible
+// (no-op when launched without the attribute).  A kernel lets the one behind it in
+// (grid_dependency_launch) only after its own wait, so one that has started knows that everything but
+// the kernel in front of it is complete.  That is what a layer call's attention builds on: the kernel in
+// front is its own store, and everything older may be read before the wait.  In decode a CTA without
+// work leaves without waiting; the first CTA of every head always waits, so the grid does.
+// The kernels that make index arrays (metadata, gather, page expansion) are launched plainly: they start
+// when everything in front is complete, and nothing starts before they are.
 __device__ __forceinline__ void grid_dependency_wait() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }

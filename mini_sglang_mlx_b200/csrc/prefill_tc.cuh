@@ -40,18 +40,19 @@
 // Page-granular form (PAGED): the pool is addressed by pages of 16 tokens (or a multiple), so
 // the 16 token rows of a page are contiguous in the pool and one TMA box copy
 // (cp.async.bulk.tensor.2d, 16 rows x 64 elements, 128-byte swizzle = exactly the tile layout
-// above) moves a quarter of a 64-key tile's K or V half.  One lane per page issues the copies
-// straight from the page ids, completion is counted in bytes on the tile's mbarrier; the seven
-// copying warps and the per-token id staging go away.  Only the ragged last page of a sequence
-// (and the pages of a tile past the sequence's end) are filled with 16-byte cp.async copies, so
-// that rows past the sequence's length are zeros rather than whatever the pool holds there.
+// above) moves a quarter of a 64-key tile's K or V half.  Three producer warps issue a tile's boxes
+// between them, one elected lane each, straight from the page ids; completion is counted in bytes on the
+// tile's mbarrier; the seven copying warps and the per-token id staging go away.  Only the ragged last
+// page of a sequence (and the pages of a tile past the sequence's end) are filled with 16-byte cp.async
+// copies, so that rows past the sequence's length are zeros rather than whatever the pool holds there.
 //
 // Key-range splits (few query tiles: verify, draft blocks, short chunks over long prefixes): a
 // CTA writes an unnormalised fp32 partial (O rows and their (max, sum)) to scratch; the
-// partials of a (sequence, query tile, head) unit are reduced row by row straight from scratch
-// (merge_kv_splits), either by the CTA that arrives last at the unit's arrival counter, inside
-// the same launch, or -- units whose partials exceed 64 KB -- by prefill_merge_kernel, a second
-// launch chained with programmatic stream serialization that spreads the rows over the grid.
+// partials of a (sequence, query tile, head) unit are merged either by the CTA that arrives last at the
+// unit's arrival counter, inside the same launch (through its shared memory, merge_kv_splits_cta), or --
+// units whose partials exceed 64 KB -- row by row straight from scratch (merge_kv_splits) by
+// prefill_merge_kernel, a second launch chained with programmatic stream serialization that spreads the
+// rows over the grid.
 #pragma once
 
 #include <type_traits>
@@ -67,8 +68,7 @@ constexpr int kTcSub = 128;       // rows per sub-tile (= MMA M)
 // CTAs per SM (short query blocks are bandwidth-bound: two independent pipelines per SM
 // keep more copies in flight).
 //
-// PAGED: the softmax warps, the MMA warp and three producer warps (the first issues the TMA
-// copies, all three load Q): 4*NSUB + 4 warps.
+// PAGED: the softmax warps, the MMA warp and three producer warps: 4*NSUB + 4 warps.
 template <int NSUB, int HD = 128, bool PAGED = false>
 struct TcShape {
   static_assert(HD == 128 || (HD == 256 && NSUB == 1), "head_dim 256 runs the one-sub-tile shape");

@@ -18,9 +18,10 @@
 // the four half a row further on (8-byte accesses), so with rotary_dim == head_dim
 // both members of a rotary pair sit in the same lane (with a smaller rotary_dim the partner
 // is a lane of the same group).  (Half a warp per 256-wide row took 110 registers, two CTAs per SM, and
-// 3.5 TB/s on 3269 tokens of 24 + 4 heads, 30.5 us; with a warp it is 64 registers and four CTAs.)  The rotary frequencies of a lane are constants; the
-// angles are recomputed per row from the token's position (cheaper than keeping a token's
-// rows together: what this kernel needs is many independent rows in flight).
+// 32.8 us on 3269 tokens of 24 + 4 heads, 3.3 TB/s; a warp takes 64, four CTAs per SM, and 20.9 us.)
+// The rotary frequencies of a lane are constants; the angles are recomputed per item from the token's
+// position (cheaper than keeping a token's rows together: what this kernel needs is many independent
+// rows in flight).
 #pragma once
 
 #include "common.cuh"
@@ -28,11 +29,11 @@
 namespace msgl {
 
 struct QkNormRopeParams {
-  void* q;                 // (n, hq, 128), normalised and rotated in place
-  const void* k;           // (n, hkv, 128)
-  const void* v;           // (n, hkv, 128)
-  const void* q_weight;    // (128) or null: no q norm
-  const void* k_weight;    // (128) or null: no k norm
+  void* q;                 // (n, hq, head_dim), normalised and rotated in place
+  const void* k;           // (n, hkv, head_dim)
+  const void* v;           // (n, hkv, head_dim)
+  const void* q_weight;    // (head_dim) or null: no q norm
+  const void* k_weight;    // (head_dim) or null: no k norm
   const int32_t* positions;
   const int32_t* out_loc;  // slot of each token's K/V row
   void* k_cache;
