@@ -66,3 +66,33 @@ def test_a_report_from_before_a_buffer_grew_is_not_lost(host_scratch, monkeypatc
     K._workspace(first.numel() + 1, dev, 7, "decode")
     assert K.device_status() == 2
     assert K.device_status() == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("max_splits", [1, 2, 3, 32])
+@pytest.mark.parametrize("kv_lens", [[5000], [1, 0, 700, 3000, 64], [40] * 50 + [2500] * 3], ids=lambda x: f"{len(x)}x{sum(x)}")
+def test_decode_with_the_least_scratch_that_a_call_takes(kv_lens, max_splits):
+    """Fewer partials than the op would like: fewer shares, down to a share per sequence (max_splits 1 and
+    2: no room for a partial per share and sequence).  Bytes behind the scratch stay as they were."""
+    import math
+
+    from mini_sglang_mlx_b200 import _lib
+    from oracle import paged_attention_oracle as O
+    from tests.helpers import assert_close_to_oracle
+    from tests.test_page_granular_gpu import make_pool
+    hkv, hq, d, batch = 2, 8, 128, len(kv_lens)
+    kc, vc, _, _, slots = make_pool(kv_lens, 16, hkv, seed=batch, d=d)
+    q = torch.randn(batch, hq, d, generator=torch.Generator().manual_seed(1)).bfloat16().cuda()
+    kvp = torch.from_numpy(O.build_indptr(kv_lens)).cuda()
+    lib, sc = _lib.lib(), 1 / math.sqrt(d)
+    need = lib.msgl_decode_workspace_bytes(batch, hq, d, max_splits)
+    ws = torch.full((need + 4096,), 255, dtype=torch.uint8, device="cuda")
+    ws[:65792] = 0
+    out = torch.empty_like(q)
+    for _ in range(2):
+        _lib.check(lib.msgl_paged_decode_attention_sized(
+            q.data_ptr(), kc.data_ptr(), vc.data_ptr(), kvp.data_ptr(), slots.data_ptr(), None, out.data_ptr(),
+            ws.data_ptr(), need, batch, hq, hkv, d, kc.shape[0], 0, sc, max_splits, sum(kv_lens),
+            torch.cuda.current_stream().cuda_stream))
+        assert_close_to_oracle(out, O.paged_decode_attention_oracle(q, kc, vc, kvp, slots, sc))
+    assert int(ws[:65792].sum()) == 0 and bool((ws[need:] == 255).all())
