@@ -645,6 +645,12 @@ constexpr int kDecMaxShare = 512;    // (256 / 384 / 512 on 32 sequences of 2000
 // A segment's end (merge of the warps, partial, next Q) takes about as long as two groups of each of
 // the four warps, five at head_dim 256 with its twice as long rows and one CTA per SM.
 constexpr int kDecPad128 = 8, kDecPad256 = 20;
+// A row in the last arriver's merge against a group in the loop (50 ns and about 0.2 us at head_dim 256, 25 ns
+// and 0.13 us at 128).  Steps of two layers, one sequence, 32 query over 2 KV heads of 256: 8191 tokens 137 us
+// without the balance, 82 / 82 / 76 with 0.15 / 0.2 / 0.3; 32767 tokens 176, 125 / 127 / 131; 131071 tokens 244,
+// 223 / 223 / 231; 32 over 4 heads of 128, 8191 tokens: 77, 43 / 43 / 45.  Batches whose pieces fit the ring at
+// once keep their shares: with the balance everywhere 2000 tokens of 16 over 2 heads of 256 went from 38.9 to 41.0.
+constexpr float kDecMergeRow = 0.2f;
 
 // Shares per KV head that fill the GPU's CTA slots once (two CTAs per SM, one at head_dim 256) ...
 int decode_wave(int num_kv_heads, int head_dim, int sms) {
@@ -790,6 +796,7 @@ static int decode_impl(const void* q, const void* k_cache, const void* v_cache,
   p.min_share = kDecMinShare;
   p.max_share = kDecMaxShare;
   p.pad = head_dim == 256 ? kDecPad256 : kDecPad128;
+  p.merge_row = kDecMergeRow;
   p.wave = decode_wave(num_kv_heads, head_dim, sms);
   unsigned char* ws = static_cast<unsigned char*>(workspace);
   p.status = reinterpret_cast<int*>(ws);

@@ -112,6 +112,11 @@ __device__ __forceinline__ float fast_exp2(float x) {
   asm volatile("ex2.approx.ftz.f32 %0, %1;\n" : "=f"(y) : "f"(x));
   return y;
 }
+__device__ __forceinline__ float fast_sqrt(float x) {
+  float y;
+  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
 
 // Packed two-float arithmetic (one instruction for two lanes of a register pair).
 __device__ __forceinline__ uint64_t pack_f32x2(float lo, float hi) {

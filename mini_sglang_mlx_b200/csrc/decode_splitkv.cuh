@@ -63,6 +63,7 @@ struct DecodeParams {
   int wave;          // shares per head that fill the GPU once
   int min_share, max_share;  // groups a share holds at least; at most, while num_shares allows another wave
   int pad;           // what the end of a segment costs, in groups
+  float merge_row;   // what a row of a piece costs in the merge, in groups
   int64_t num_slots;
   float scale_log2;  // sm_scale * log2(e)
   // The call's own K/V store is the kernel in front in the stream: it writes the pool rows
@@ -119,6 +120,7 @@ __global__ void __launch_bounds__(NWARPS * 32, HD == 256 ? 1 : 2)
   constexpr int NT = HD / 8;                              // output n-tiles
   constexpr int MROW = decode_merge_row_floats(HD);
   constexpr int PROW = decode_partial_floats(HD);
+  constexpr int kRing = NWARPS * NSTAGES * 2 * TILE_BYTES;
   static_assert(CH == 16 || CH == 32, "head_dim must be 128 or 256");
   static_assert(NWARPS == kDecodeMergeHeads, "a warp merges a head");
 
@@ -224,23 +226,34 @@ __global__ void __launch_bounds__(NWARPS * 32, HD == 256 ? 1 : 2)
   } else {
     // a lane sums a run of consecutive sequences; with at most 32 of them that is the window itself
     const int run = (B + 31) / 32;
-    int sum = 0, n1 = 0, kvb1 = 0, len1 = 0;
+    int sum = 0, n1 = 0, kvb1 = 0, len1 = 0, longest = 0;
     if (run == 1) {
       if (lane < B) n1 = length(lane, kvb1, len1);
       sum = padded(n1);
+      longest = n1;
     } else {
       for (int j = 0; j < run; ++j) {
         int kvb, len;
         const int b = lane * run + j;
-        if (b < B) sum += padded(length(b, kvb, len));
+        if (b >= B) break;
+        const int n = length(b, kvb, len);
+        sum += padded(n);
+        longest = max(longest, n);
       }
     }
+    longest = __reduce_max_sync(0xffffffffu, longest);
     int incl = scan(sum);
     int total = __shfl_sync(0xffffffffu, incl, 31);
     // whole waves of CTAs: 1.2 waves of equal shares take as long as two
     const int waves = max(1, min(ceil_div(total, p.wave * p.max_share), p.num_shares / p.wave));
     share = max(ceil_div(total, p.wave * waves), p.min_share);
     share = max(share, ceil_div(total, p.num_shares));
+    // The pieces of a sequence are merged by one CTA, a row per piece and query head.  Where they do not fit
+    // its ring at once the merge is as long as the loop and longer; share + longest / share * G * merge_row is
+    // least where the two are equal.
+    const int most = ceil_div(longest, share);
+    if (most > 32 || most * G * (PROW * 4) > kRing)
+      share = max(share, static_cast<int>(fast_sqrt(static_cast<float>(longest) * static_cast<float>(G) * p.merge_row)));
     share = ceil_div(share, NWARPS) * NWARPS;
     if (run == 1) {
       const int pieces = ceil_div(n1, share);
@@ -734,7 +747,6 @@ __global__ void __launch_bounds__(NWARPS * 32, HD == 256 ? 1 : 2)
     // 7 us.  (Copies by all threads, not bulk copies: those would need a proxy fence, 0.7 us, and one
     // thread to issue them.)  Pieces that do not fit at once come four heads and a ring's worth of
     // pieces at a time.
-    constexpr int kRing = NWARPS * NSTAGES * 2 * TILE_BYTES;
     constexpr int ROW16 = PROW / 4;                             // 16-byte chunks of a row
 #pragma unroll 1
     for (int k = 0; k < pending; ++k) {

@@ -99,3 +99,22 @@ def test_a_ring_stage_changes_between_ordinary_and_bulk_copies(d, bad):
     if not bad:
         ref = O.paged_decode_attention_oracle(q, kc, vc, kvp, slots, sc)
         assert_close_to_oracle(a, ref, "pages")
+
+
+@pytest.mark.parametrize("d,hkv,hq,limit", [(256, 2, 32, 11 * 128), (128, 2, 32, 11 * 128), (256, 1, 2, 32 * 128),
+                                            (128, 8, 16, 32 * 128)])
+@pytest.mark.parametrize("past", [-15, 0, 1, 5000])
+@pytest.mark.parametrize("others", [0, 40])
+def test_pieces_around_what_the_merge_holds_at_once(d, hkv, hq, limit, past, others):
+    """A share is 8 groups at least; up to `limit` tokens the pieces of one sequence fit the merging CTA's ring
+    (or 32 of them), beyond it the shares grow."""
+    from mini_sglang_mlx_b200 import paged_decode_attention, paged_decode_attention_p16
+    kv_lens = [limit + past] + [1 + i % 3 for i in range(others)]
+    kc, vc, pip, pidx, slots = make_pool(kv_lens, 16, hkv, seed=d + 100 + past, d=d)
+    g = torch.Generator(device="cuda").manual_seed(limit)
+    q = torch.empty(len(kv_lens), hq, d, dtype=torch.bfloat16, device="cuda").normal_(generator=g)
+    kvp, lens, n = _i32(O.build_indptr(kv_lens).tolist()), _i32(kv_lens), _i32([1] * len(kv_lens))
+    sc = 1 / math.sqrt(d)
+    out = paged_decode_attention_p16(q, kc, vc, pip, pidx, lens, n, sc, 1, page_size=16)
+    assert_close_to_oracle(out, O.paged_decode_attention_oracle(q, kc, vc, kvp, slots, sc))
+    assert torch.equal(paged_decode_attention(q, kc, vc, kvp, slots, n, sc, 1), out)
