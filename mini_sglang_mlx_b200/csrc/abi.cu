@@ -645,12 +645,14 @@ constexpr int kDecMaxShare = 512;    // (256 / 384 / 512 on 32 sequences of 2000
 // A segment's end (merge of the warps, partial, next Q) takes about as long as two groups of each of
 // the four warps, five at head_dim 256 with its twice as long rows and one CTA per SM.
 constexpr int kDecPad128 = 8, kDecPad256 = 20;
-// A row in the last arriver's merge against a group in the loop (50 ns and about 0.2 us at head_dim 256, 25 ns
-// and 0.13 us at 128).  Steps of two layers, one sequence, 32 query over 2 KV heads of 256: 8191 tokens 137 us
-// without the balance, 82 / 82 / 76 with 0.15 / 0.2 / 0.3; 32767 tokens 176, 125 / 127 / 131; 131071 tokens 244,
-// 223 / 223 / 231; 32 over 4 heads of 128, 8191 tokens: 77, 43 / 43 / 45.  Batches whose pieces fit the ring at
-// once keep their shares: with the balance everywhere 2000 tokens of 16 over 2 heads of 256 went from 38.9 to 41.0.
-constexpr float kDecMergeRow = 0.2f;
+// Merging a piece of a sequence (a warp per query head, eight pieces in flight) against a group in the loop, for
+// every four query heads of a KV head.  Beyond kDecMaxPieces pieces the shares grow to balance the two.  Steps of
+// two layers in us with 0.3 / 0.6 / 1.2: one sequence, 32 query over 2 KV heads of 256, 8191 tokens 61 / 62 / 68 (90
+// without the balance), 131071 tokens 211 / 196 / 204; three sequences of 20000 tokens there 123 / 98 / 99; 32
+// over 4 heads of 128, 32767 tokens 63 / 62 / 68; 16 over 8 heads, 4000 tokens 26.4 / 26.8 / 28.6.  With 32 pieces
+// instead of 16 the three sequences of 20000 tokens take 124; with 8, 2000 tokens of 16 over 2 heads 34.9 for 33.4.
+constexpr float kDecMergeRow = 0.6f;
+constexpr int kDecMaxPieces = 16;
 
 // Shares per KV head that fill the GPU's CTA slots once (two CTAs per SM, one at head_dim 256) ...
 int decode_wave(int num_kv_heads, int head_dim, int sms) {
@@ -796,8 +798,10 @@ static int decode_impl(const void* q, const void* k_cache, const void* v_cache,
   p.min_share = kDecMinShare;
   p.max_share = kDecMaxShare;
   p.pad = head_dim == 256 ? kDecPad256 : kDecPad128;
-  p.merge_row = kDecMergeRow;
+  p.merge_row = kDecMergeRow * static_cast<float>((p.group + kDecWarps - 1) / kDecWarps);
+  p.max_pieces = kDecMaxPieces;
   p.wave = decode_wave(num_kv_heads, head_dim, sms);
+  p.inv_wave = std::nextafter(1.f / static_cast<float>(p.wave), 2.f);
   unsigned char* ws = static_cast<unsigned char*>(workspace);
   p.status = reinterpret_cast<int*>(ws);
   const size_t own_tickets = decode_ticket_bytes(batch, num_q_heads);
@@ -826,6 +830,7 @@ static int decode_impl(const void* q, const void* k_cache, const void* v_cache,
   if (std::max<int64_t>(shares, batch) * num_kv_heads > 0x7fffffffLL)
     return fail(MSGL_BAD_SHAPE, std::string(op) + "problem too large for one launch");
   p.num_shares = static_cast<int>(shares);
+  p.max_waves = p.num_shares / p.wave;
   p.part = reinterpret_cast<float*>(ws + kStatusBytes + own_tickets);
   if (dtype == MSGL_DTYPE_BF16) return launch_decode<__nv_bfloat16>(p, head_dim, s, tm_k, tm_v);
   return launch_decode<__half>(p, head_dim, s, tm_k, tm_v);

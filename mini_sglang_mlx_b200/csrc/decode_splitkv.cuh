@@ -16,10 +16,16 @@
 // leave 7/8 of a 128-row tile idle.)
 //
 // A part of a sequence that a share holds is a segment.  At its end the warps' (max, sum, O) are
-// merged through shared memory; a segment that is a whole sequence writes the final rows, any other
-// (the first and the last of a share at most) writes a normalised fp32 partial and its log-sum-exp to
-// scratch.  A CTA that is through with its share arrives at those sequences' counters, and the one
-// that arrives last merges the partials; there is no second launch.
+// merged through shared memory, a warp per query head; a segment that is a whole sequence writes the final
+// rows, any other (the first and the last of a share at most) writes an fp32 partial (sum of the weighted rows,
+// maximum, sum of the weights) to scratch.  A warp of a CTA that is through with its share arrives at the
+// counters of the heads whose partials it wrote, and the one that arrives last at a head merges its pieces;
+// there is no second launch and no barrier.
+//
+// What bounds a small call is none of the chip's rates but the chain of a CTA's instructions, each of which
+// waits for the one in front (one warp per scheduler: 7.9 cycles per instruction, 2975 of them on 700 tokens of one
+// sequence; memory 10 % of it).  So the search for the share has no divisions and one scan, new rows' slots are
+// held in registers, and the merge of the pieces reads them straight into registers.
 //
 // Per-token form: K and V rows (256 or 512 bytes per token and head) are gathered through the slot
 // ids with 16-byte cp.async copies.  Page-granular form (PAGED): a group is one page (or a 16-row
@@ -53,17 +59,20 @@ struct DecodeParams {
   int page_size;
   void* out;
   const void* gate;  // (batch, hq, D) or null: out *= sigmoid(gate)
-  float* part;       // (slots, group, decode_partial_floats(D)): normalised partials, log-sum-exp behind each
-  // (batch, hkv) arrival counters of a (sequence, KV head)'s segments: the CTA that arrives last
+  float* part;       // (slots, group, decode_partial_floats(D)): partials, each with (maximum, sum) behind it
+  // (batch, hq) arrival counters of a (sequence, query head)'s segments: the warp that arrives last
   // merges the partials and puts the counter back to zero.  Zero before the first launch.
   int* tickets;
   int* status;       // device status word (0 = ok); may be null
   int batch, hq, hkv, group;
   int num_shares;    // shares per head at most (= gridDim.x / hkv); 0: a share is a whole sequence
   int wave;          // shares per head that fill the GPU once
+  float inv_wave;    // 1 / wave, not below it
+  int max_waves;     // num_shares / wave
   int min_share, max_share;  // groups a share holds at least; at most, while num_shares allows another wave
   int pad;           // what the end of a segment costs, in groups
-  float merge_row;   // what a row of a piece costs in the merge, in groups
+  int max_pieces;    // pieces of a sequence up to which the shares do not grow with the merge
+  float merge_row;   // what merging a piece costs, in groups
   int64_t num_slots;
   float scale_log2;  // sm_scale * log2(e)
   // The call's own K/V store is the kernel in front in the stream: it writes the pool rows
@@ -120,13 +129,11 @@ __global__ void __launch_bounds__(NWARPS * 32, HD == 256 ? 1 : 2)
   constexpr int NT = HD / 8;                              // output n-tiles
   constexpr int MROW = decode_merge_row_floats(HD);
   constexpr int PROW = decode_partial_floats(HD);
-  constexpr int kRing = NWARPS * NSTAGES * 2 * TILE_BYTES;
   static_assert(CH == 16 || CH == 32, "head_dim must be 128 or 256");
   static_assert(NWARPS == kDecodeMergeHeads, "a warp merges a head");
 
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ uint64_t s_bar[PAGED ? NWARPS * NSTAGES : 1];
-  __shared__ int s_last[2];
 
   const int h = static_cast<int>(blockIdx.x) % p.hkv;
   const int share_id = static_cast<int>(blockIdx.x) / p.hkv;
@@ -157,7 +164,6 @@ __global__ void __launch_bounds__(NWARPS * 32, HD == 256 ? 1 : 2)
       prefetch_tensormap(&tm_v);
       fence_mbar_init();
     }
-    __syncthreads();
   }
   // Behind its own K/V store the kernel starts early: it looks its share up and has the first groups
   // on their way (those without a row that the store writes) before the store is through.
@@ -169,6 +175,12 @@ __global__ void __launch_bounds__(NWARPS * 32, HD == 256 ? 1 : 2)
     grid_dependency_launch();
   };
   if (p.num_new < 0) wait_in_front();
+  // the rows that the store writes, 32 of them a register
+  constexpr int kNewRegs = kDecodeNewMax / 32;
+  int fresh[kNewRegs];
+#pragma unroll
+  for (int i = 0; i < kNewRegs; ++i)
+    fresh[i] = i * 32 + lane < p.num_new ? __ldg(after_wait(p.new_slots) + i * 32 + lane) : -1;
   const int32_t* indptr = after_wait(p.indptr);
   const int32_t* kv_lens = after_wait(p.kv_lens);
 
@@ -179,6 +191,14 @@ __global__ void __launch_bounds__(NWARPS * 32, HD == 256 ? 1 : 2)
   // (`aligned`): every CTA then has one segment.
   const int B = p.batch;
   int share = 0x7fffffff;
+  float inv_share = 0.f;
+  // n / share for n >= 0: the approximate quotient is off by one at most (quotients are below 2^20)
+  auto over_share = [&](int n) -> int {
+    int q = static_cast<int>(static_cast<float>(n) * inv_share);
+    const int r = n - q * share;
+    q += r < 0 ? -1 : r >= share ? 1 : 0;
+    return q;
+  };
   bool aligned = false;
   struct Window {        // 32 sequences from `base` on, in shared memory:
     int base;            // {first position, groups, first page / token of the index list, tokens}
@@ -200,7 +220,7 @@ __global__ void __launch_bounds__(NWARPS * 32, HD == 256 ? 1 : 2)
     }
     return x;
   };
-  auto padded = [&](int n) -> int { return n == 0 ? 0 : aligned ? ceil_div(n, share) * share : n + p.pad; };
+  auto padded = [&](int n) -> int { return n == 0 ? 0 : aligned ? (over_share(n - 1) + 1) * share : n + p.pad; };
   auto load_window = [&](Window& w, int base, int first) {
     int kvb = 0, len = 0;
     const int n = base + lane < B ? length(base + lane, kvb, len) : 0;
@@ -242,60 +262,75 @@ __global__ void __launch_bounds__(NWARPS * 32, HD == 256 ? 1 : 2)
       }
     }
     longest = __reduce_max_sync(0xffffffffu, longest);
-    int incl = scan(sum);
-    int total = __shfl_sync(0xffffffffu, incl, 31);
+    int total = __reduce_add_sync(0xffffffffu, sum);
     // whole waves of CTAs: 1.2 waves of equal shares take as long as two
-    const int waves = max(1, min(ceil_div(total, p.wave * p.max_share), p.num_shares / p.wave));
-    share = max(ceil_div(total, p.wave * waves), p.min_share);
-    share = max(share, ceil_div(total, p.num_shares));
-    // The pieces of a sequence are merged by one CTA, a row per piece and query head.  Where they do not fit
-    // its ring at once the merge is as long as the loop and longer; share + longest / share * G * merge_row is
-    // least where the two are equal.
-    const int most = ceil_div(longest, share);
-    if (most > 32 || most * G * (PROW * 4) > kRing)
-      share = max(share, static_cast<int>(fast_sqrt(static_cast<float>(longest) * static_cast<float>(G) * p.merge_row)));
-    share = ceil_div(share, NWARPS) * NWARPS;
+    if (total <= p.wave * p.max_share || p.max_waves <= 1) {
+      share = __float2int_ru(static_cast<float>(total) * p.inv_wave);     // (inv_wave is rounded up: one too many at most,
+      share -= (share - 1) * p.wave >= total ? 1 : 0;                     // or too few of a total beyond 2^24, see below)
+    } else {
+      share = ceil_div(total, p.wave * min(ceil_div(total, p.wave * p.max_share), p.max_waves));
+    }
+    share = max(share, p.min_share);
+    if (static_cast<int64_t>(share) * p.num_shares < total) share = ceil_div(total, p.num_shares);
+    // The pieces of a sequence's head are merged by one warp, a row per piece.  Where there are many of them
+    // the merge is as long as the loop and longer; share + longest / share * merge_row is least where the two
+    // are equal.
+    if (longest > p.max_pieces * share)
+      share = max(share, static_cast<int>(fast_sqrt(static_cast<float>(longest) * p.merge_row)));
+    share = (share + NWARPS - 1) / NWARPS * NWARPS;
+    inv_share = __fdividef(1.f, static_cast<float>(share));
     if (run == 1) {
-      const int pieces = ceil_div(n1, share);
+      const int pieces = n1 == 0 ? 0 : over_share(n1 - 1) + 1;
       aligned = __reduce_add_sync(0xffffffffu, pieces) <= min(p.wave, p.num_shares);
       if (aligned) {
         sum = pieces * share;
-        incl = scan(sum);
-        total = __shfl_sync(0xffffffffu, incl, 31);
+        total = __reduce_add_sync(0xffffffffu, sum);
       }
-      pw.at[lane] = make_int4(incl - sum, n1, kvb1, len1);
     }
     const int64_t start = static_cast<int64_t>(share_id) * share;
     if (start >= total && share_id > 0) return;
     r0 = static_cast<int>(start);
     tail = start + share >= total;
     r1 = tail ? total : r0 + share;
-    // first sequence that starts at r0 or holds it: in the first run that reaches r0, or right behind
-    const int l = __ffs(__ballot_sync(0xffffffffu, incl >= r0)) - 1;
-    int found = l * run + run, at = incl;    // (broadcast from lane l)
-    if (lane == l) {
-      int pos = incl - sum;
-      for (int j = 0; j < run; ++j) {
-        int kvb, len;
-        const int b = l * run + j;
-        if (b >= B) break;
-        const int n = run == 1 ? sum : padded(length(b, kvb, len));
-        if (pos >= r0 || pos + n > r0) {
-          found = b;
-          at = pos;
-          break;
+    // first sequence that starts at r0 or holds it
+    const int incl = scan(sum);
+    if (run == 1) {
+      pw.at[lane] = make_int4(incl - sum, n1, kvb1, len1);
+      const uint32_t m = __ballot_sync(0xffffffffu, lane < B && (incl - sum >= r0 || incl > r0));
+      b0 = m != 0u ? __ffs(m) - 1 : B;
+    } else {
+      // in the first run that reaches r0, or right behind
+      const int l = __ffs(__ballot_sync(0xffffffffu, incl >= r0)) - 1;
+      int found = l * run + run, at = incl;    // (broadcast from lane l)
+      if (lane == l) {
+        int pos = incl - sum;
+        for (int j = 0; j < run; ++j) {
+          int kvb, len;
+          const int b = l * run + j;
+          if (b >= B) break;
+          const int n = padded(length(b, kvb, len));
+          if (pos >= r0 || pos + n > r0) {
+            found = b;
+            at = pos;
+            break;
+          }
+          pos += n;
         }
-        pos += n;
       }
+      b0 = __shfl_sync(0xffffffffu, found, l);
+      at = __shfl_sync(0xffffffffu, at, l);
+      load_window(pw, b0, at);
     }
-    b0 = __shfl_sync(0xffffffffu, found, l);
-    at = __shfl_sync(0xffffffffu, at, l);
-    if (run > 1) load_window(pw, b0, at);
   }
   __syncwarp();
   cw.base = pw.base;
-  cw.at[lane] = pw.at[lane];
-  __syncwarp();
+  if (B <= 32) {
+    cw.at = pw.at;             // (all sequences: neither moves on)
+  } else {
+    cw.at[lane] = pw.at[lane];
+    __syncwarp();
+  }
+  if constexpr (PAGED) __syncthreads();     // the ring's barriers exist
 
   const unsigned char* __restrict__ kbase = static_cast<const unsigned char*>(p.k_cache);
   const unsigned char* __restrict__ vbase = static_cast<const unsigned char*>(p.v_cache);
@@ -336,6 +371,7 @@ __global__ void __launch_bounds__(NWARPS * 32, HD == 256 ? 1 : 2)
     // PAGED: lane j, group j: first pool row, num_slots if the page is outside the pool (rows behind the pool
     // read as zeros); else lane 16 j + r: slot of row r, -1: zeros
     int y;
+    uint32_t fresh;      // per-token form, before the wait
   };
   Segment ps;
   int pb = b0, pg = warp;
@@ -353,14 +389,26 @@ __global__ void __launch_bounds__(NWARPS * 32, HD == 256 ? 1 : 2)
     const int j = PAGED ? lane : lane / kDecodeGroupTokens;
     const int t = w.t0 + j * (NWARPS * kDecodeGroupTokens) + (PAGED ? 0 : lane % kDecodeGroupTokens);
     if (j < w.count && t < w.len) {
+      // (pages of 16 tokens: no division)
       const int per = PAGED ? p.page_size : 1;
-      const int id = __ldg(p.indices + ps.kvb + t / per);
-      const int64_t row = static_cast<int64_t>(id) * per + t % per;
+      const int page = PAGED && per != kDecodeGroupTokens ? t / per : PAGED ? t / kDecodeGroupTokens : t;
+      const int id = __ldg(p.indices + ps.kvb + page);
+      const int64_t row = static_cast<int64_t>(id) * per + (t - page * per);
       const int rows = PAGED ? min(kDecodeGroupTokens, w.len - t) : 1;
       if (id >= 0 && row + rows <= p.num_slots) w.y = static_cast<int>(row);
       else {                                        // page or slot outside the pool: zeros
         if (PAGED) w.y = static_cast<int>(p.num_slots);
         if (p.status) atomicExch(p.status, 2);
+      }
+    }
+    if constexpr (!PAGED) {
+      w.fresh = 0u;
+      if (!waited) {       // lanes whose row the kernel in front writes
+        bool hit = false;
+#pragma unroll
+        for (int i = 0; i < kNewRegs; ++i)
+          for (int k = 0; k < min(32, p.num_new - 32 * i); ++k) hit |= w.y == __shfl_sync(0xffffffffu, fresh[i], k);
+        w.fresh = __ballot_sync(0xffffffffu, hit);
       }
     }
   };
@@ -381,12 +429,10 @@ __global__ void __launch_bounds__(NWARPS * 32, HD == 256 ? 1 : 2)
       bool hit = false;
       if constexpr (PAGED) {
         const int y = __shfl_sync(0xffffffffu, cur.y, ck);
-        for (int k = lane; k < p.num_new; k += 32) {
-          const int slot = __ldg(p.new_slots + k);
-          hit |= slot >= y && slot < y + kDecodeGroupTokens;
-        }
+#pragma unroll
+        for (int i = 0; i < kNewRegs; ++i) hit |= fresh[i] >= y && fresh[i] < y + kDecodeGroupTokens;
       } else {
-        for (int k = 0; k < p.num_new; ++k) hit |= cur.y == __ldg(p.new_slots + k);
+        hit = (cur.fresh >> (ck * kDecodeGroupTokens) & 0xffffu) != 0u;
       }
       if (__any_sync(0xffffffffu, hit)) wait_in_front();
     }
@@ -683,7 +729,6 @@ __global__ void __launch_bounds__(NWARPS * 32, HD == 256 ? 1 : 2)
           wgt[w] = (M == -INFINITY) ? 0.f : fast_exp2(sm_m[w * 16 + g] - M);
           den += wgt[w] * sm_l[w * 16 + g];
         }
-        const float inv = den > 0.f ? 1.f / den : 0.f;
         float num[VPL];
 #pragma unroll
         for (int e = 0; e < VPL; ++e) num[e] = 0.f;
@@ -699,9 +744,10 @@ __global__ void __launch_bounds__(NWARPS * 32, HD == 256 ? 1 : 2)
             num[4 * e4 + 3] += wgt[w] * x.w;
           }
         }
-#pragma unroll
-        for (int e = 0; e < VPL; ++e) num[e] *= inv;
         if (whole) {
+          const float inv = den > 0.f ? 1.f / den : 0.f;
+#pragma unroll
+          for (int e = 0; e < VPL; ++e) num[e] *= inv;
           write_decode_row<T, VPL>(out, gate, hq_idx * HD + lane * VPL, num);
         } else {
           float* row = p.part + (slot * G + g) * PROW;
@@ -709,7 +755,7 @@ __global__ void __launch_bounds__(NWARPS * 32, HD == 256 ? 1 : 2)
           for (int e4 = 0; e4 < NV; ++e4)
             *reinterpret_cast<float4*>(row + lane * VPL + 4 * e4) =
                 make_float4(num[4 * e4], num[4 * e4 + 1], num[4 * e4 + 2], num[4 * e4 + 3]);
-          if (lane == 0) row[HD] = den > 0.f ? M * kLn2 + __logf(den) : -INFINITY;
+          if (lane == 0) *reinterpret_cast<float2*>(row + HD) = make_float2(M, den);
         }
       }
       __syncthreads();   // the rows may be written again
@@ -717,107 +763,86 @@ __global__ void __launch_bounds__(NWARPS * 32, HD == 256 ? 1 : 2)
     if (!whole) {        // at most the first and the last segment of the share
       if (pending > 0) part0 = part1;
       part1.b = b;
-      part1.first = cs.beg / share;
-      part1.count = (cs.end - 1) / share - part1.first + 1;
+      part1.first = over_share(cs.beg);
+      part1.count = over_share(cs.end - 1) - part1.first + 1;
       ++pending;
     }
   }
   cp_async_wait<0>();
 
-  // ---- the CTA that arrives last at a sequence's counter merges its partials:
-  // out = sum_s e^(lse_s - M) O_s / sum_s e^(lse_s - M)  (the second stage of the reference,
-  // paged_decode_attention.metal:512-586, without a launch)
+  // ---- the warp that arrives last at a (sequence, head)'s counter merges its partials:
+  // out = sum_s 2^(M_s - M) O_s / sum_s 2^(M_s - M) l_s  (the second stage of the reference,
+  // paged_decode_attention.metal:512-586, without a launch).  A warp arrives for the heads that it wrote, all
+  // at once; per CTA instead (a barrier, one thread's arrivals, the pieces through shared memory) the tail of a
+  // small call took 4.1 us, and a sequence's heads were all merged by one CTA.
   if (pending > 0) {
-    // (every warp is past its writes of partials, and done with the ring)
-    if (threadIdx.x < 2) {
-      int last = 0;
-      if (threadIdx.x < pending) {
-        const Partial& part = threadIdx.x == 0 ? part1 : part0;
-        int* ticket = p.tickets + static_cast<int64_t>(part.b) * p.hkv + h;
-        // the CTA's partials are visible device-wide before the arrival, the others' after it
-        last = atomic_add_acq_rel(ticket, 1) == part.count - 1 ? 1 : 0;
-        if (last) *ticket = 0;
-      }
-      s_last[threadIdx.x] = last;
+    const int mine = (G - warp + NWARPS - 1) / NWARPS;     // heads warp, warp + NWARPS, ... (none: <= 0)
+    __syncwarp();
+    bool last = false;
+    if (lane < pending * 8 && (lane & 7) < mine) {         // (at most four heads: 16 / NWARPS)
+      const Partial& part = lane < 8 ? part1 : part0;
+      int* ticket = p.tickets + static_cast<int64_t>(part.b) * p.hq + h * G + warp + (lane & 7) * NWARPS;
+      // the warp's partials are visible device-wide before the arrival, the others' after it
+      last = atomic_add_acq_rel(ticket, 1) == part.count - 1;
+      if (last) *ticket = 0;
     }
-    __syncthreads();
-    // The rows of a piece's heads are contiguous in scratch, each with its log-sum-exp behind it.
-    // They are copied into the ring, all pieces in flight together, then a warp merges a head: read
-    // into registers instead, eight pieces in flight, a sequence of 12 pieces x 8 heads of 256 took
-    // 7 us.  (Copies by all threads, not bulk copies: those would need a proxy fence, 0.7 us, and one
-    // thread to issue them.)  Pieces that do not fit at once come four heads and a ring's worth of
-    // pieces at a time.
-    constexpr int ROW16 = PROW / 4;                             // 16-byte chunks of a row
+    uint32_t todo = __ballot_sync(0xffffffffu, last);
+    __syncwarp();
 #pragma unroll 1
-    for (int k = 0; k < pending; ++k) {
-      if (s_last[k] == 0) continue;
-      const int b = k == 0 ? part1.b : part0.b;
-      const int first = k == 0 ? part1.first : part0.first, count = k == 0 ? part1.count : part0.count;
-      const int64_t slot0 = (static_cast<int64_t>(first) + b) * p.hkv + h;   // piece j: + j * hkv
-      const bool all = count <= 32 && static_cast<int64_t>(count) * G * (PROW * 4) <= kRing;
-      const int hl = all ? G : min(G, NWARPS);                // heads of a copy
-      const int fit = min(32, kRing / (hl * PROW * 4));
+    for (; todo != 0u; todo &= todo - 1) {
+      const int l = __ffs(todo) - 1;
+      const Partial& part = l < 8 ? part1 : part0;
+      const int g = warp + (l & 7) * NWARPS;
+      const int64_t oi = (static_cast<int64_t>(part.b) * p.hq + static_cast<int64_t>(h) * G + g) * HD + lane * VPL;
+      GateVec<T, VPL> gate;
+      gate.load(static_cast<const T*>(p.gate), oi);
+      const float* rows = p.part + ((static_cast<int64_t>(part.first) + part.b) * p.hkv + h) * G * PROW + g * PROW;
+      const int64_t pitch = static_cast<int64_t>(p.hkv) * G * PROW;     // from piece to piece
+      constexpr int FLY = 8;                                            // pieces in flight
+      float M = -INFINITY, den = 0.f, num[VPL];
+#pragma unroll
+      for (int e = 0; e < VPL; ++e) num[e] = 0.f;
 #pragma unroll 1
-      for (int hb = 0; hb < G; hb += hl) {
-        const int hn = min(hl, G - hb);
-        float M = -INFINITY, den = 0.f, num[VPL];
-#pragma unroll 1
-        for (int j0 = 0; j0 < count; j0 += fit) {
-          const int m = min(fit, count - j0);
-          for (int j = 0; j < m; ++j) {
-            const float* src = p.part + ((slot0 + static_cast<int64_t>(j0 + j) * p.hkv) * G + hb) * PROW;
-            const uint32_t dst = smem_u32(smem_al) + j * hl * (PROW * 4);
-            for (int c = threadIdx.x; c < hn * ROW16; c += NWARPS * 32) cp_async_16(dst + c * 16, src + c * 4, 16);
+      for (int j0 = 0; j0 < part.count; j0 += FLY, rows += FLY * pitch) {
+        const int m = min(FLY, part.count - j0);
+        float4 x[FLY][NV];
+        float2 ml = make_float2(-INFINITY, 0.f);                        // of piece lane % FLY
+        if (lane % FLY < m) ml = __ldcg(reinterpret_cast<const float2*>(rows + (lane % FLY) * pitch + HD));
+#pragma unroll
+        for (int j = 0; j < FLY; ++j)
+#pragma unroll
+          for (int e4 = 0; e4 < NV; ++e4)
+            x[j][e4] = j < m ? __ldcg(reinterpret_cast<const float4*>(rows + j * pitch + lane * VPL) + e4)
+                             : make_float4(0.f, 0.f, 0.f, 0.f);
+        float mx = ml.x;
+#pragma unroll
+        for (int o2 = FLY / 2; o2 > 0; o2 >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o2));
+        mx = fmaxf(mx, M);
+        const float old = M == -INFINITY ? 0.f : fast_exp2(M - mx);
+        const float w = ml.x == -INFINITY ? 0.f : fast_exp2(ml.x - mx);
+        M = mx;
+        float d = w * ml.y;
+#pragma unroll
+        for (int o2 = FLY / 2; o2 > 0; o2 >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o2);
+        den = den * old + d;
+#pragma unroll
+        for (int e = 0; e < VPL; ++e) num[e] *= old;
+#pragma unroll
+        for (int j = 0; j < FLY; ++j) {
+          const float wj = __shfl_sync(0xffffffffu, w, j);
+#pragma unroll
+          for (int e4 = 0; e4 < NV; ++e4) {
+            num[4 * e4 + 0] += wj * x[j][e4].x;
+            num[4 * e4 + 1] += wj * x[j][e4].y;
+            num[4 * e4 + 2] += wj * x[j][e4].z;
+            num[4 * e4 + 3] += wj * x[j][e4].w;
           }
-          cp_async_wait_all();
-          __syncthreads();
-#pragma unroll 1
-          for (int g = warp; g < hn; g += NWARPS) {           // (one head, unless everything fits)
-            const int64_t oi = (static_cast<int64_t>(b) * p.hq + static_cast<int64_t>(h) * G + hb + g) * HD + lane * VPL;
-            GateVec<T, VPL> gate;
-            if (j0 + m == count) gate.load(static_cast<const T*>(p.gate), oi);
-            if (j0 == 0) {
-              M = -INFINITY;
-              den = 0.f;
-#pragma unroll
-              for (int e = 0; e < VPL; ++e) num[e] = 0.f;
-            }
-            const float* rows = reinterpret_cast<const float*>(smem_al) + g * PROW;
-            const int pitch = hl * PROW;
-            const float ls = lane < m ? rows[lane * pitch + HD] : -INFINITY;
-            float mx = ls;
-#pragma unroll
-            for (int o2 = 16; o2 > 0; o2 >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o2));
-            mx = fmaxf(mx, M);
-            const float old = M == -INFINITY ? 0.f : __expf(M - mx);
-            const float w = ls == -INFINITY ? 0.f : __expf(ls - mx);
-            M = mx;
-            den *= old;
-#pragma unroll
-            for (int e = 0; e < VPL; ++e) num[e] *= old;
-#pragma unroll 4
-            for (int j = 0; j < m; ++j) {
-              const float wj = __shfl_sync(0xffffffffu, w, j);
-              den += wj;
-#pragma unroll
-              for (int e4 = 0; e4 < NV; ++e4) {
-                const float4 x = *reinterpret_cast<const float4*>(rows + j * pitch + lane * VPL + 4 * e4);
-                num[4 * e4 + 0] += wj * x.x;
-                num[4 * e4 + 1] += wj * x.y;
-                num[4 * e4 + 2] += wj * x.z;
-                num[4 * e4 + 3] += wj * x.w;
-              }
-            }
-            if (j0 + m == count) {
-              const float inv = den > 0.f ? 1.f / den : 0.f;
-#pragma unroll
-              for (int e = 0; e < VPL; ++e) num[e] *= inv;
-              write_decode_row<T, VPL>(out, gate, oi, num);
-            }
-          }
-          __syncthreads();                   // the ring may be filled again
         }
       }
+      const float inv = den > 0.f ? 1.f / den : 0.f;
+#pragma unroll
+      for (int e = 0; e < VPL; ++e) num[e] *= inv;
+      write_decode_row<T, VPL>(out, gate, oi, num);
     }
   }
   if (!alive && p.status && lane == 0) atomicExch(p.status, 1);   // a wait ran out

@@ -105,9 +105,8 @@ def test_a_ring_stage_changes_between_ordinary_and_bulk_copies(d, bad):
                                             (128, 8, 16, 32 * 128)])
 @pytest.mark.parametrize("past", [-15, 0, 1, 5000])
 @pytest.mark.parametrize("others", [0, 40])
-def test_pieces_around_what_the_merge_holds_at_once(d, hkv, hq, limit, past, others):
-    """A share is 8 groups at least; up to `limit` tokens the pieces of one sequence fit the merging CTA's ring
-    (or 32 of them), beyond it the shares grow."""
+def test_pieces_of_a_long_sequence_beside_short_ones(d, hkv, hq, limit, past, others):
+    """A share is 8 groups at least: 11 or 32 pieces of one sequence, one more or less, and many."""
     from mini_sglang_mlx_b200 import paged_decode_attention, paged_decode_attention_p16
     kv_lens = [limit + past] + [1 + i % 3 for i in range(others)]
     kc, vc, pip, pidx, slots = make_pool(kv_lens, 16, hkv, seed=d + 100 + past, d=d)
@@ -118,3 +117,26 @@ def test_pieces_around_what_the_merge_holds_at_once(d, hkv, hq, limit, past, oth
     out = paged_decode_attention_p16(q, kc, vc, pip, pidx, lens, n, sc, 1, page_size=16)
     assert_close_to_oracle(out, O.paged_decode_attention_oracle(q, kc, vc, kvp, slots, sc))
     assert torch.equal(paged_decode_attention(q, kc, vc, kvp, slots, n, sc, 1), out)
+
+
+@pytest.mark.parametrize("d,hkv,hq", [(128, 2, 2), (128, 2, 6), (256, 1, 5), (128, 1, 16), (256, 2, 8)])
+@pytest.mark.parametrize("kv_lens", [[128 * k + 5 for k in (1, 2, 7, 8, 9)], [128 * 16], [128 * 17 + 1, 300], [128 * 33],
+                                     [200] * 33 + [2100, 0, 2300]], ids=lambda x: f"{len(x)}x{sum(x)}")
+def test_a_warp_merges_the_pieces_of_its_heads(d, hkv, hq, kv_lens):
+    """A warp per query head, eight pieces at a time, whichever CTA arrives last at the head: heads that leave
+    warps without one, one to 33 pieces, two partials of a share (a sequence's end and the next one's start), and
+    the counters back at zero (a second call gives the same bits)."""
+    from mini_sglang_mlx_b200 import paged_decode_attention
+    kc, vc, _, _, slots = make_pool([max(l, 1) for l in kv_lens], 16, hkv, seed=hq, d=d)
+    slots = torch.cat([s[:l] for s, l in zip(slots.split([max(l, 1) for l in kv_lens]), kv_lens)])
+    g = torch.Generator(device="cuda").manual_seed(hq)
+    q, gate = (torch.empty(len(kv_lens), hq, d, dtype=torch.bfloat16, device="cuda").normal_(generator=g)
+               for _ in range(2))
+    kvp, n = _i32(O.build_indptr(kv_lens).tolist()), _i32([1] * len(kv_lens))
+    sc = 1 / math.sqrt(d)
+    ref = O.paged_decode_attention_oracle(q, kc, vc, kvp, slots, sc)
+    out = paged_decode_attention(q, kc, vc, kvp, slots, n, sc, 1)
+    assert_close_to_oracle(out, ref)
+    assert torch.equal(paged_decode_attention(q, kc, vc, kvp, slots, n, sc, 1), out)
+    gated = paged_decode_attention(q, kc, vc, kvp, slots, n, sc, 1, gate=gate)
+    assert_close_to_oracle(gated, out.float().cpu() * torch.sigmoid(gate.float()).cpu(), "gate")
