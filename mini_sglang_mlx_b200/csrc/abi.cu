@@ -1053,6 +1053,9 @@ static int prefill_impl(const void* q, const void* k_cache, const void* v_cache,
   p.is_cross = is_cross_attention ? 1 : 0;
   p.window = sliding_window_size;
   p.kv_chunk = pl.kv_chunk;
+  p.group_recip = msgl::reciprocal(p.group);
+  p.page_recip = msgl::reciprocal(p.page_size);
+  p.chunk_recip = msgl::reciprocal(p.kv_chunk);
   p.early = behind_store ? 1 : 0;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
 

@@ -112,6 +112,12 @@ __device__ __forceinline__ float fast_exp2(float x) {
   asm volatile("ex2.approx.ftz.f32 %0, %1;\n" : "=f"(y) : "f"(x));
   return y;
 }
+// (the same where the compiler may move it)
+__device__ __forceinline__ float exp2_approx(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
 __device__ __forceinline__ float fast_sqrt(float x) {
   float y;
   asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -160,6 +166,34 @@ __device__ __forceinline__ T apply_gate(float out, T gate) {
   // took most of a 128-row epilogue, 38 us at head_dim 256.  Below 2^-126 it gives zero.)
   const float s = to_f32(MmaOp<T>::from_float(__fdividef(1.f, 1.f + __expf(-to_f32(gate)))));
   return MmaOp<T>::from_float(o * s);
+}
+
+// Two elements of a row that is rounded already.  The product of two 16-bit numbers is exact in fp32, so one
+// 16-bit multiplication rounds as apply_gate does.  (10 instructions a pair, 4 of them special-function, for 32.)
+__device__ __forceinline__ uint32_t mul_pair(__nv_bfloat16, uint32_t a, uint32_t b) {
+  const __nv_bfloat162 r = __hmul2(*reinterpret_cast<__nv_bfloat162*>(&a), *reinterpret_cast<__nv_bfloat162*>(&b));
+  return *reinterpret_cast<const uint32_t*>(&r);
+}
+__device__ __forceinline__ uint32_t mul_pair(__half, uint32_t a, uint32_t b) {
+  const __half2 r = __hmul2(*reinterpret_cast<__half2*>(&a), *reinterpret_cast<__half2*>(&b));
+  return *reinterpret_cast<const uint32_t*>(&r);
+}
+__device__ __forceinline__ float2 unpack_pair(__nv_bfloat16, uint32_t v) {
+  return make_float2(__uint_as_float(v << 16), __uint_as_float(v & 0xffff0000u));
+}
+__device__ __forceinline__ float2 unpack_pair(__half, uint32_t v) { return __half22float2(*reinterpret_cast<__half2*>(&v)); }
+__device__ __forceinline__ float rcp_approx(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+template <typename T>
+__device__ __forceinline__ uint32_t apply_gate_pair(uint32_t out, uint32_t gate) {
+  const float2 g = unpack_pair(T{}, gate);
+  float x0, x1;
+  unpack_f32x2(mul_f32x2(pack_f32x2(g.x, g.y), pack_f32x2(-kLog2e, -kLog2e)), x0, x1);
+  unpack_f32x2(add_f32x2(pack_f32x2(exp2_approx(x0), exp2_approx(x1)), pack_f32x2(1.f, 1.f)), x0, x1);
+  return mul_pair(T{}, out, MmaOp<T>::pack(rcp_approx(x0), rcp_approx(x1)));
 }
 
 // Reduce over the four lanes that share a row of an m16n8 accumulator.

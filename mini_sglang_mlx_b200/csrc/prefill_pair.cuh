@@ -204,6 +204,7 @@ __global__ void __launch_bounds__(PairShape<HD, PAGED>::kThreads, 1)
   __shared__ PairBarriers bars;
   __shared__ uint32_t s_tmem_base;
   __shared__ int s_abort;
+  __shared__ FoundItem found;
   __shared__ float2 s_ml[NG == 2 ? 2 * ROWS : 1];        // (reference maximum, sum) of the rows, per group
   // reference maxima after the even / odd tiles, each with its tile's number
   __shared__ __align__(16) uint2 s_mref[NG == 2 ? 2 * ROWS : 1];
@@ -222,44 +223,58 @@ __global__ void __launch_bounds__(PairShape<HD, PAGED>::kThreads, 1)
   // (every second buffer of the ring holds V tiles, so a barrier's next use is behind the buffer's)
   auto bar_v = [&](int tile) { return smem_u32(&bars.v_here[tile % (NB / 2)]); };
 
-  if (tid == 0) {
-    s_abort = 0;
-    mbar_init(bar_q, 2 * 2 * NKW);
-    for (int bf = 0; bf < NB; ++bf) {
-      mbar_init(bar_full(bf), 2 * NKW);      // both CTAs' producers (V of per-token slots: the peer's relay)
-      mbar_init(bar_empty(bf), 1);
-    }
-    if (!PAGED)
-      for (int i = 0; i < NB / 2; ++i) mbar_init(smem_u32(&bars.v_here[i]), Shape::kVWarps * 32);
-    for (int b = 0; b < LA; ++b) {
-      mbar_init(bar_s(b), 1);
-      mbar_init(bar_p(b), 2 * (ROWS / 32));
-      mbar_init(bar_pv(b), 1);
-    }
-    fence_mbar_init();
-  }
-  if (NG == 2 && tid < 2 * ROWS) s_mref[tid] = make_uint2(0u, 0xffffffffu);
+  // ---- set-up, a warp for each part of it
   if (warp == Shape::kMmaWarp) {
     tmem_alloc_pair(smem_u32(&s_tmem_base), 512);
     tmem_relinquish_pair();
   }
+  if (warp == 1) {
+    // a barrier per lane
+    auto init = [&](uint64_t* first, int n, int count) {
+      if (lane < n) mbar_init(smem_u32(first + lane), count);
+    };
+    init(&bars.q_full, 1, 2 * 2 * NKW);
+    init(bars.full, NB, 2 * NKW);            // both CTAs' producers (V of per-token slots: the peer's relay)
+    init(bars.empty, NB, 1);
+    if (!PAGED) init(bars.v_here, NB / 2, Shape::kVWarps * 32);
+    init(bars.s_full, LA, 1);
+    init(bars.p_full, LA, 2 * (ROWS / 32));
+    init(bars.pv_done, LA, 1);
+    if (lane == 0) s_abort = 0;
+    fence_mbar_init();
+  }
+  if (NG == 2 && tid < 2 * ROWS) s_mref[tid] = make_uint2(0u, 0xffffffffu);
   if (!p.early) grid_dependency_wait();
-  ItemCoord it;
-  const bool have_item = find_item<Shape::kThreads>(p, static_cast<int>(blockIdx.x) / 2, BM,
-                                                    reinterpret_cast<int*>(smem_raw), it);
-  fence_proxy_async_smem();     // (Q comes to where the item search had its counts)
-  if (p.early) grid_dependency_wait();
-  grid_dependency_launch();
+  if (p.batch <= kWarpBatchMax) {
+    if (warp == 0) find_item_warp(p, static_cast<int>(blockIdx.x) / 2, BM, &found);
+  } else {
+    ItemCoord at;
+    const bool have = find_item<Shape::kThreads>(p, static_cast<int>(blockIdx.x) / 2, BM,
+                                                 reinterpret_cast<int*>(smem_raw), at);
+    fence_proxy_async_smem();   // (Q comes to where the item search had its counts)
+    if (tid == 0) {
+      found.have = have;
+      if (have) {
+        found.at = at;
+        found.seq = load_seq_shape(p, at.b, BM);
+      }
+    }
+  }
   tc_fence_before();
   cluster_sync_all();           // the barriers of both CTAs exist (and the CTA's own set-up is done)
   tc_fence_after();
   const uint32_t tmem = s_tmem_base;
-  if (!have_item) {             // the same in both CTAs: a launch rank past the last item
+  const bool producer = warp >= Shape::kProducerWarp0 && warp < Shape::kProducerWarp0 + NKW + Shape::kVWarps;
+  if (p.early && !(producer && found.have)) grid_dependency_wait();   // (producers: once they know their first copies)
+  if (!p.early || warp == 0) grid_dependency_launch();
+  if (!found.have) {            // the same in both CTAs: a launch rank past the last item
     if (warp == Shape::kMmaWarp) tmem_dealloc_pair(tmem, 512);
     return;
   }
+  const ItemCoord it = found.at;
   const int h = it.h;
-  const SeqShape sq = load_seq_shape(p, it.b, BM);
+  const SeqShape sq = found.seq;
+  auto over_group = [&](int x) { return divide_by(x, p.group_recip); };
   if (PAGED && it.first && rank == 0 && tid == 0 && p.status) {
     // a length that is negative or exceeds the sequence's pages was clamped: report it
     const int64_t cap = static_cast<int64_t>(p.page_indptr[it.b + 1] - p.page_indptr[it.b]) * p.page_size;
@@ -271,8 +286,8 @@ __global__ void __launch_bounds__(PairShape<HD, PAGED>::kThreads, 1)
   const int pk0 = it.qt * BM;
   const int rows_pair = min(BM, sq.tq * G - pk0);                       // >= 1
   const int rows_valid = max(0, min(ROWS, rows_pair - rank * ROWS));
-  const int tok_first = pk0 / G;
-  const int tok_last = (pk0 + rows_pair - 1) / G;
+  const int tok_first = over_group(pk0);
+  const int tok_last = over_group(pk0 + rows_pair - 1);
   int kv_lo = p.window > 0 ? max(0, sq.prefix + tok_first - p.window + 1) : 0;
   kv_lo = (kv_lo / BN) * BN;
   const int kv_hi = p.is_cross ? sq.L : min(sq.L, sq.prefix + tok_last + 1);   // keys from here on are never read
@@ -284,40 +299,45 @@ __global__ void __launch_bounds__(PairShape<HD, PAGED>::kThreads, 1)
   volatile int* abort_flag = &s_abort;
 
   // Output rows are packed in the Q buffer (free then: every S MMA is done; chunk c of row r sits at chunk
-  // position c ^ (r & 15)) and leave as whole rows, by all warps of the CTA: the gate's reads and
-  // exponentials took four softmax warps 20000 cycles at head_dim 256.
+  // position c ^ (r & 15)) and leave as whole rows, by all warps of the CTA, each with four of the gate's reads
+  // in flight from before the last PV is done.  (Of 53000 cycles of a gated pair at head_dim 256, 12400 went here with
+  // two reads at a time and one element per instruction.)
   constexpr int RB = HD * 2;
   unsigned char* stage = smem_raw + (q_smem - smem_u32(smem_raw));
+  constexpr int RPI = 32 / CH;                                // rows of a warp's access
+  constexpr int STEP = Shape::kWarps * RPI, FLY = 4;          // the gate's reads run FLY accesses ahead
+  uint4 gv[FLY];
+  auto row_offset = [&](int row) -> int64_t {
+    const int pk = pk0 + rank * ROWS + row;
+    const int tl = over_group(pk), g = pk - tl * G;
+    return (static_cast<int64_t>(sq.q_begin + tl) * p.hq + static_cast<int64_t>(h) * G + g) * HD + lane % CH * 8;
+  };
+  auto read_gate = [&](int row, uint4& g) {
+    if (p.gate && row < rows_valid) g = *reinterpret_cast<const uint4*>(static_cast<const T*>(p.gate) + row_offset(row));
+  };
+  auto first_gates = [&]() {
+#pragma unroll
+    for (int f = 0; f < FLY; ++f) read_gate(warp * RPI + lane / CH + f * STEP, gv[f]);
+  };
   auto write_rows = [&]() {
     cta_threads_sync<Shape::kThreads>();
     if (s_abort != 0) return;
-    constexpr int RPI = 32 / CH;                              // rows of a warp's access
-    constexpr int STEP = Shape::kWarps * RPI;
-    constexpr int FLY = 2;                                    // accesses in flight
     const int chunk = lane % CH;
 #pragma unroll 1
     for (int r0 = warp * RPI + lane / CH; r0 < rows_valid; r0 += FLY * STEP) {
-      T* dst[FLY];
-      uint4 w[FLY], gv[FLY];
 #pragma unroll
-      for (int k = 0; k < FLY; ++k) {
-        const int row = min(r0 + k * STEP, rows_valid - 1);   // (the last row again instead of a row behind it)
-        const int pk = pk0 + rank * ROWS + row;
-        const int tl = pk / G, g = pk - tl * G;
-        const int64_t off = (static_cast<int64_t>(sq.q_begin + tl) * p.hq + static_cast<int64_t>(h) * G + g) * HD + chunk * 8;
-        dst[k] = static_cast<T*>(p.out) + off;
-        if (p.gate) gv[k] = *reinterpret_cast<const uint4*>(static_cast<const T*>(p.gate) + off);
-        w[k] = *reinterpret_cast<const uint4*>(stage + row * RB + ((chunk ^ (row & 15)) << 4));
-      }
-#pragma unroll
-      for (int k = 0; k < FLY; ++k) {
+      for (int f = 0; f < FLY; ++f) {
+        const int row = r0 + f * STEP;
+        if (row >= rows_valid) break;
+        uint4 w = *reinterpret_cast<const uint4*>(stage + row * RB + ((chunk ^ (row & 15)) << 4));
         if (p.gate) {
-          T* wo = reinterpret_cast<T*>(&w[k]);
-          const T* wg = reinterpret_cast<const T*>(&gv[k]);
-#pragma unroll
-          for (int e = 0; e < 8; ++e) wo[e] = apply_gate<T>(to_f32(wo[e]), wg[e]);
+          w.x = apply_gate_pair<T>(w.x, gv[f].x);
+          w.y = apply_gate_pair<T>(w.y, gv[f].y);
+          w.z = apply_gate_pair<T>(w.z, gv[f].z);
+          w.w = apply_gate_pair<T>(w.w, gv[f].w);
+          read_gate(row + FLY * STEP, gv[f]);
         }
-        *reinterpret_cast<uint4*>(dst[k]) = w[k];
+        *reinterpret_cast<uint4*>(static_cast<T*>(p.out) + row_offset(row)) = w;
       }
     }
   };
@@ -335,10 +355,17 @@ __global__ void __launch_bounds__(PairShape<HD, PAGED>::kThreads, 1)
         prefetch_tensormap(is_k ? &tg_k : &tg_v);
         if (PAGED) prefetch_tensormap(is_k ? &tm_k : &tm_v);
       }
+      bool waited = !p.early;
+      auto wait_in_front = [&]() {
+        if (waited) return;
+        waited = true;
+        grid_dependency_wait();
+      };
       // ---- Q, dealt to all producers: boxes of 64 columns x 128 rows where a box holds whole tokens
       // (rows past the sequence's last query token hold a neighbour's rows then: computed on, never
       // written), else four rows at a time
-      if (ntiles > 0 && pid < 2 * NKW) {
+      auto load_q = [&]() {
+        if (pid >= 2 * NKW) return;
         if (p.q_tma) {
           if (elect_one()) {
             int mine = 0;
@@ -354,11 +381,12 @@ __global__ void __launch_bounds__(PairShape<HD, PAGED>::kThreads, 1)
           for (int e = 0; e < 4; ++e) {
             const int row = lane * 4 + e;
             const int pk = pk0 + rank * ROWS + row;
-            const int tl = pk / G, g = pk - tl * G;
+            const int tl = over_group(pk), g = pk - tl * G;
             rows[e] = row < rows_valid ? (sq.q_begin + tl) * p.hq + h * G + g : p.total_q * p.hq;
           }
           if (elect_one()) mbar_arrive_expect_tx_cluster(q_bar, (32 - pid + 2 * NKW - 1) / (2 * NKW) * (HD * 8));
           __syncwarp();
+#pragma unroll 1
           for (int l = pid; l < 32; l += 2 * NKW) {
             int r4[4];
 #pragma unroll
@@ -372,7 +400,7 @@ __global__ void __launch_bounds__(PairShape<HD, PAGED>::kThreads, 1)
           }
         }
         __syncwarp();
-      }
+      };
       // ---- key tiles.  K: this CTA's 64 keys, all columns; V: all 128 keys, its half of the columns.
       const int absent = static_cast<int>(p.num_slots);
       const int32_t* ids = (PAGED ? p.page_indices : p.kv_indices) + sq.kv_begin;
@@ -401,8 +429,9 @@ __global__ void __launch_bounds__(PairShape<HD, PAGED>::kThreads, 1)
             d.n = 0;
             const int t = t0 + lane * kTmaBoxRows;
             if (lane * kTmaBoxRows < RT && tile < ntiles && t < kv_hi) {
-              const int pg = __ldg(ids + t / p.page_size);
-              const int64_t row0 = static_cast<int64_t>(pg) * p.page_size + t % p.page_size;
+              const int page = divide_by(t, p.page_recip);
+              const int pg = __ldg(ids + page);
+              const int64_t row0 = static_cast<int64_t>(pg) * p.page_size + (t - page * p.page_size);
               const int nv = min(kTmaBoxRows, sq.L - t);
               if (pg < 0 || row0 + nv > p.num_slots) {
                 if (p.status) atomicExch(p.status, 2);     // page outside the pool: rows read as zeros
@@ -426,6 +455,8 @@ __global__ void __launch_bounds__(PairShape<HD, PAGED>::kThreads, 1)
         };
         Ids cur, nxt;
         fetch(0, cur);
+        wait_in_front();
+        if (!K && ntiles > 0) load_q();
 #pragma unroll 1
         for (int t = 0; t < ntiles; ++t) {
           fetch(t + 1, nxt);                                      // in flight while this tile's copies are issued
@@ -471,6 +502,7 @@ __global__ void __launch_bounds__(PairShape<HD, PAGED>::kThreads, 1)
             __syncwarp();
           }
           cur = nxt;
+          if (K && t == 0) load_q();      // (behind the first tile, whose page ids were on their way longer)
         }
       };
       if (is_k) {
@@ -498,6 +530,8 @@ __global__ void __launch_bounds__(PairShape<HD, PAGED>::kThreads, 1)
           return slot;
         };
         int slot = slot_of(0);
+        wait_in_front();
+        if (ntiles > 0) load_q();
 #pragma unroll 1
         for (int t = 0; t < ntiles; ++t) {
           const int next = slot_of(t + 1);
@@ -612,6 +646,7 @@ __global__ void __launch_bounds__(PairShape<HD, PAGED>::kThreads, 1)
       if (!alive && p.status && lane == 0) atomicExch(p.status, 1);
     }
     __syncwarp();
+    first_gates();
     write_rows();
   } else {
     // =========================================================== softmax
@@ -621,7 +656,7 @@ __global__ void __launch_bounds__(PairShape<HD, PAGED>::kThreads, 1)
     const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
     const uint32_t s_tm = tmem + lane_base;
     const uint32_t o_tm = tmem + lane_base + Shape::kOCol;
-    const int tl = (pk0 + rank * ROWS + r) / G;
+    const int tl = over_group(pk0 + rank * ROWS + r);
     const int pos = sq.prefix + tl;
     const int vhi = p.is_cross ? sq.L - 1 : min(pos, sq.L - 1);
     const int vlo = p.window > 0 ? pos - p.window + 1 : 0;
@@ -635,7 +670,7 @@ __global__ void __launch_bounds__(PairShape<HD, PAGED>::kThreads, 1)
     if (p.gate) {
       for (int e = warp * 32 + lane; e < rows_valid * (HD / 64); e += NG * ROWS) {
         const int pk = pk0 + rank * ROWS + e / (HD / 64);
-        const int tle = pk / G, g = pk - tle * G;
+        const int tle = over_group(pk), g = pk - tle * G;
         prefetch_l2(static_cast<const T*>(p.gate) +
                     (static_cast<int64_t>(sq.q_begin + tle) * p.hq + static_cast<int64_t>(h) * G + g) * HD +
                     e % (HD / 64) * 64);
@@ -661,10 +696,25 @@ __global__ void __launch_bounds__(PairShape<HD, PAGED>::kThreads, 1)
         for (int e = 0; e < BN; ++e) v[e] = __float_as_uint(__uint_as_float(v[e]) * p.scale_log2);
       }
       if (need_mask) {
+        if constexpr (HD == 128) {
+          // visible keys as bits, 32 at a time: predicates from a register, not two comparisons per key (six short
+          // prompts, 8 layers: 106.7 us for 112.1; at head_dim 256 it is the other way round, 159 for 147)
+          const int hi = vhi - k0, lo = vlo - k0;             // lo <= e <= hi
 #pragma unroll
-        for (int e = 0; e < BN; ++e) {
-          const int kpos = k0 + e;
-          if (!(kpos >= vlo && kpos <= vhi)) v[e] = 0xff800000u;  // -inf
+          for (int c = 0; c < BN / 32; ++c) {
+            const int h32 = hi - 32 * c, l32 = lo - 32 * c;
+            const uint32_t below = h32 >= 31 ? ~0u : h32 < 0 ? 0u : (2u << h32) - 1u;
+            const uint32_t from = l32 <= 0 ? ~0u : l32 > 31 ? 0u : ~0u << l32;
+            const uint32_t seen = below & from;
+#pragma unroll
+            for (int e = 0; e < 32; ++e) v[32 * c + e] = seen >> e & 1u ? v[32 * c + e] : 0xff800000u;  // -inf
+          }
+        } else {
+#pragma unroll
+          for (int e = 0; e < BN; ++e) {
+            const int kpos = k0 + e;
+            if (!(kpos >= vlo && kpos <= vhi)) v[e] = 0xff800000u;  // -inf
+          }
         }
       }
       float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
@@ -757,6 +807,7 @@ __global__ void __launch_bounds__(PairShape<HD, PAGED>::kThreads, 1)
 
     // ---- epilogue
     const bool any = ntiles > 0;
+    first_gates();
     if (alive && any) {
       alive = mbar_wait_warp(bar_pv((ntiles - 1) % LA), ((ntiles - 1) / LA) & 1, abort_flag);
       if (alive) tc_fence_after();

@@ -57,3 +57,29 @@ def test_decode_with_gate(d):
     _same_up_to_one_rounding(out, _gated(plain.cpu().float(), gate))
     with pytest.raises(RuntimeError, match="gate must match q"):
         paged_decode_attention(*args, gate=gate.cuda()[:2])
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("d", [128, 256])
+def test_gate_of_prefill_pairs_at_the_ends_of_its_range(dtype, d):
+    """Pairs of elements at a time: gates of any size, infinite and not a number.  Output, sigmoid and product are each
+    rounded to 16 bits, and the sigmoid's fp32 error may move its rounding by one unit: two in the product."""
+    from mini_sglang_mlx_b200 import paged_prefill_attention
+    n, hq, hkv = 150, 8, 2
+    g = torch.Generator(device="cuda").manual_seed(d)
+    q, gate = (torch.empty(n, hq, d, dtype=dtype, device="cuda").normal_(generator=g) for _ in range(2))
+    kc, vc = (torch.empty(n, hkv, d, dtype=dtype, device="cuda").normal_(generator=g) for _ in range(2))
+    ends = [float("inf"), -float("inf"), float("nan"), 0.0, -0.0, 6e4, -6e4, 87.0, -87.0, -89.0, 16.0, -16.0, 1e-7, -1e-7]
+    gate.view(-1)[: 512 * len(ends)] = torch.tensor(ends * 512, device="cuda").to(dtype)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32).cuda()
+    args = (q, kc, vc, i32([0, n]), i32([0, n]), torch.arange(n, dtype=torch.int32, device="cuda"), i32([0]), d ** -0.5, n)
+    out = paged_prefill_attention(*args).float()
+    got = paged_prefill_attention(*args, gate=gate).float()
+    want = out * torch.sigmoid(gate.float()).to(dtype).float()
+    assert torch.equal(got.isnan(), want.isnan())
+    unit = 2.0 ** (-8 if dtype == torch.bfloat16 else -11)
+    least = 2.0 ** -24                                        # (the smallest step of f16)
+    ok = (got - want).abs() <= 2 * 2 * unit * want.abs() + 2 * least
+    assert bool((ok | want.isnan()).all())
+    assert torch.equal(got[gate == float("inf")], out[gate == float("inf")])
+    assert bool((got[gate == -float("inf")] == 0).all())

@@ -121,3 +121,28 @@ def _separate(be, pool, q, k, v, i, b, w):
                            rope_base=1e6)
     torch.cuda.synchronize()
     return be._attend(q, pool.k_cache(i), pool.v_cache(i), md, False, 0)
+
+
+@pytest.mark.parametrize("batch", [31, 32, 33])
+@pytest.mark.parametrize("d,hkv,hq,q_hi,window", [(128, 2, 6, 90, 0), (256, 1, 4, 90, 0), (128, 2, 8, 12, 0), (128, 1, 8, 16, 100)])
+def test_items_of_up_to_32_sequences_and_of_more(batch, d, hkv, hq, q_hi, window):
+    """Up to 32 sequences one warp finds a CTA's work item, beyond that the whole CTA does: pairs and one-CTA
+    tiles, key ranges split or not, sequences without queries or keys, lengths that tie."""
+    from mini_sglang_mlx_b200 import paged_prefill_attention, paged_prefill_attention_p16
+    q_lens = [0 if i % 7 == 3 else 1 + (i * 37) % q_hi for i in range(batch)]
+    prefixes = [0 if i % 3 == 0 else (i * 211) % 700 for i in range(batch)]
+    q, _, kc, vc, pip, pidx, slots, kv_lens = _problem([max(n, 1) for n in q_lens], prefixes, hkv, hq, d, batch)
+    kept, at = [], 0
+    for n, x in zip(q_lens, kv_lens):                # (a sequence without queries has its cached tokens only)
+        kept.append(slots[at:at + x - (n == 0)])
+        at += x
+    kv_lens = [x - (n == 0) for n, x in zip(q_lens, kv_lens)]
+    slots, q = torch.cat(kept), q[:sum(q_lens)].contiguous()
+    qo, kvp, pre = _i32(O.build_indptr(q_lens).tolist()), _i32(O.build_indptr(kv_lens).tolist()), _i32(prefixes)
+    sc, n = 1 / math.sqrt(d), max(q_lens)
+    ref = O.paged_prefill_attention_oracle(q, kc, vc, qo, kvp, slots, pre, sc, sliding_window_size=window)
+    out = paged_prefill_attention_p16(q, kc, vc, qo, pip, pidx, _i32(kv_lens), pre, sc, n, page_size=16,
+                                      sliding_window_size=window)
+    assert_close_to_oracle(out, ref, "pages")
+    out = paged_prefill_attention(q, kc, vc, qo, kvp, slots, pre, sc, n, sliding_window_size=window)
+    assert_close_to_oracle(out, ref, "slots")
