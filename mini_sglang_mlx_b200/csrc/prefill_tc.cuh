@@ -284,6 +284,7 @@ struct MergeArgs {
   void* out;
   const void* gate;
   int hq, group;
+  uint64_t group_recip;
 };
 template <typename T, int HD, int NSW, int BM, int RU, int SU>
 __device__ __noinline__ void merge_kv_splits(const MergeArgs p, int nsp, int64_t slot0,
@@ -364,7 +365,7 @@ __device__ __noinline__ void merge_kv_splits(const MergeArgs p, int nsp, int64_t
       if (r0 + k >= row_hi) break;
       const float invd = L[k] > 0.f ? 1.f / L[k] : 0.f;
       const int pkr = pk0 + r0 + k;
-      const int tlr = pkr / G, gr = pkr - tlr * G;
+      const int tlr = divide_by(pkr, p.group_recip), gr = pkr - tlr * G;
       const int64_t oi =
           (static_cast<int64_t>(q_begin + tlr) * p.hq + static_cast<int64_t>(h) * G + gr) * HD +
           lane * VPL;
@@ -443,7 +444,7 @@ __device__ __noinline__ void merge_kv_splits_cta(const MergeArgs p, int nsp, int
       }
       const float inv = L > 0.f ? 1.f / L : 0.f;
       const int pk = pk0 + r0 + r;
-      const int tl = pk / G, g = pk - tl * G;
+      const int tl = divide_by(pk, p.group_recip), g = pk - tl * G;
       const int64_t oi =
           (static_cast<int64_t>(q_begin + tl) * p.hq + static_cast<int64_t>(h) * G + g) * HD + lane * VPL;
       alignas(16) T vals[VPL];
@@ -489,6 +490,7 @@ __global__ void __launch_bounds__(TcShape<NSUB, HD, PAGED>::kThreads,
   __shared__ TcBarriers bars;
   __shared__ uint32_t s_tmem_base;
   __shared__ int s_abort;
+  __shared__ FoundItem found;
   __shared__ int s_slots[(LA + 1) * BN];  // slot ids of the key tiles being copied / next to copy
 
   const int tid = threadIdx.x;
@@ -513,25 +515,21 @@ __global__ void __launch_bounds__(TcShape<NSUB, HD, PAGED>::kThreads,
   // of two), else as 16-byte copies by the producer threads
   const bool q_tma = PAGED && p.q_tma != 0;
 
-  if (tid == 0) {
-    s_abort = 0;
-    mbar_init(bar_q, q_tma ? 1 : NPROD);
-    mbar_init(smem_u32(&bars.idx_sync), NPROD);
-    for (int bf = 0; bf < kTcBufs; ++bf) {
-      // PAGED: per copying warp its 32 lanes (their cp.async arrivals) + the arrival that
-      // announces the TMA bytes
-      mbar_init(bar_full(bf), PAGED ? (NPROD / 32) * 33 : NPROD);
-      mbar_init(bar_empty(bf), 1);
-    }
-    for (int i = 0; i < NSUB; ++i) {
-      mbar_init(smem_u32(&bars.stage[i]), SUB / 32);     // one arrival per warp of the group
-      mbar_init(bar_sf(i, 0), 1);
-      mbar_init(bar_sf(i, 1), 1);
-      mbar_init(bar_pf(i, 0), SUB / 32);
-      mbar_init(bar_pf(i, 1), SUB / 32);
-      mbar_init(bar_pv(i, 0), 1);
-      mbar_init(bar_pv(i, 1), 1);
-    }
+  if (warp == 1) {
+    // a barrier per lane.  (PAGED: per copying warp its 32 lanes, their cp.async arrivals, and the arrival that
+    // announces the TMA bytes)
+    auto init = [&](uint64_t* first, int n, int count) {
+      if (lane < n) mbar_init(smem_u32(first + lane), count);
+    };
+    init(&bars.q_full, 1, q_tma ? 1 : NPROD);
+    init(&bars.idx_sync, 1, NPROD);
+    init(bars.full, kTcBufs, PAGED ? (NPROD / 32) * 33 : NPROD);
+    init(bars.empty, kTcBufs, 1);
+    init(bars.stage, NSUB, SUB / 32);                  // one arrival per warp of the group
+    init(&bars.s_full[0][0], 2 * NSUB, 1);
+    init(&bars.p_full[0][0], 2 * NSUB, SUB / 32);
+    init(&bars.pv_done[0][0], 2 * NSUB, 1);
+    if (lane == 0) s_abort = 0;
     fence_mbar_init();
   }
   if (warp == kMmaWarp) {
@@ -540,23 +538,39 @@ __global__ void __launch_bounds__(TcShape<NSUB, HD, PAGED>::kThreads,
   }
 
   if (!p.early) grid_dependency_wait();
-  ItemCoord it;
-  const bool have_item =
-      find_item<kTcThreads>(p, static_cast<int>(blockIdx.x), BM, reinterpret_cast<int*>(smem_raw), it);
-  if (PAGED) fence_proxy_async_smem();   // (Q comes by bulk copies to where the item search had its counts)
-  if (p.early) grid_dependency_wait();   // the item is found while the K/V store drains
-  grid_dependency_launch();
+  const bool by_warp = p.batch <= kWarpBatchMax;
+  if (by_warp) {
+    if (warp == 0) find_item_warp(p, static_cast<int>(blockIdx.x), BM, &found);
+  } else {
+    ItemCoord at;
+    const bool have = find_item<kTcThreads>(p, static_cast<int>(blockIdx.x), BM, reinterpret_cast<int*>(smem_raw), at);
+    if (PAGED) fence_proxy_async_smem();   // (Q comes by bulk copies to where the item search had its counts)
+    if (tid == 0) {
+      found.have = have;
+      if (have) {
+        found.at = at;
+        found.seq = load_seq_shape(p, at.b, BM);
+      }
+    }
+  }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  const bool have_item = found.have;
+  // (producers wait for the K/V store once they know their first copies)
+  if (p.early && !(warp >= kTcProducerWarp0 && have_item)) grid_dependency_wait();
+  if (!p.early || warp == 0) grid_dependency_launch();
   if (!have_item) {  // block-uniform: a launch rank past the last item
     if (warp == kMmaWarp) tmem_dealloc(s_tmem_base, Shape::kTmemCols);
     return;
   }
+  const ItemCoord it = found.at;
   const int h = it.h;
-  const SeqShape sq = load_seq_shape(p, it.b, BM);
+  const SeqShape sq = found.seq;
   const int qt = it.qt, split = it.split;
   const int slot_item = it.base + qt * sq.nsplit + split;   // where this item's kv-split partial goes
+  // (the two-sub-tile per-token form is at its register limit: with the reciprocals its tile loop takes 2 % longer)
+  auto over_group = [&](int x) { return NSUB == 2 && !PAGED ? x / G : divide_by(x, p.group_recip); };
   if (PAGED && it.first && tid == 0 && p.status) {
     // a length that is negative or exceeds the sequence's pages was clamped: report it
     const int64_t cap = static_cast<int64_t>(p.page_indptr[it.b + 1] - p.page_indptr[it.b]) * p.page_size;
@@ -568,7 +582,7 @@ __global__ void __launch_bounds__(TcShape<NSUB, HD, PAGED>::kThreads,
   const int pk0 = qt * BM;
   const int rows_valid = min(BM, sq.tq * G - pk0);              // >= 1
   const int nsub = (NSUB == 2 && rows_valid > SUB) ? 2 : 1;
-  const int tok_first = pk0 / G;
+  const int tok_first = over_group(pk0);
   const int s_lo = p.kv_chunk > 0 ? sq.lo + split * p.kv_chunk : 0;
   const int s_hi = p.kv_chunk > 0 ? sq.lo + (split + 1) * p.kv_chunk : 0x7fffffff;  // exclusive
   int kv_lo = p.window > 0 ? max(0, sq.prefix + tok_first - p.window + 1) : 0;
@@ -578,14 +592,14 @@ __global__ void __launch_bounds__(TcShape<NSUB, HD, PAGED>::kThreads,
 #pragma unroll
   for (int i = 0; i < NSUB; ++i) {
     const int last_row = min(rows_valid, (i + 1) * SUB) - 1;     // last valid row of the sub-tile
-    const int tok_last = (pk0 + last_row) / G;
+    const int tok_last = over_group(pk0 + last_row);
     int hi = p.is_cross ? sq.L : min(sq.L, sq.prefix + tok_last + 1);
     hi = min(hi, s_hi);
     ntiles_sub[i] = (i < nsub && hi > kv_lo) ? ceil_div(hi - kv_lo, BN) : 0;
   }
   const int ntiles = max(ntiles_sub[0], ntiles_sub[1]);
   // keys past kv_hi_load are never fetched (zero rows in the tile)
-  int kv_hi_load = p.is_cross ? sq.L : min(sq.L, sq.prefix + (pk0 + rows_valid - 1) / G + 1);
+  int kv_hi_load = p.is_cross ? sq.L : min(sq.L, sq.prefix + over_group(pk0 + rows_valid - 1) + 1);
   kv_hi_load = min(kv_hi_load, s_hi);
 
   // ---- shared-memory carve-up (1024-byte aligned tiles)
@@ -617,6 +631,10 @@ __global__ void __launch_bounds__(TcShape<NSUB, HD, PAGED>::kThreads,
     const int64_t slot_stride = static_cast<int64_t>(p.hkv) * (HD * 2);
     const int64_t head_off = static_cast<int64_t>(h) * (HD * 2);
 
+    // The first page / slot ids are on their way before the wait, Q and the tiles behind it.
+    auto load_q = [&]() {
+    if (p.early) grid_dependency_wait();
+    if (ntiles == 0) return;      // (the epilogue's zeros are staged where Q would land)
     if (q_tma) {
       // Q: one box per sub-tile and 64-element column block.  The tensor map is
       // (head_dim, query heads, tokens) with a box of 64 x G x 128/G, so the rows land in
@@ -638,7 +656,7 @@ __global__ void __launch_bounds__(TcShape<NSUB, HD, PAGED>::kThreads,
         const int row = i * PROWS + rsub;  // 0..255
         if (row >= nsub * SUB) break;
         const int pk = pk0 + row;
-        const int tl = pk / G, g = pk - tl * G;
+        const int tl = over_group(pk), g = pk - tl * G;
         const bool ok = row < rows_valid;
         const int64_t off =
             ok ? ((static_cast<int64_t>(sq.q_begin + tl) * p.hq + static_cast<int64_t>(h) * G + g) * HD)
@@ -648,6 +666,7 @@ __global__ void __launch_bounds__(TcShape<NSUB, HD, PAGED>::kThreads,
       }
       cp_async_mbar_arrive(bar_q);
     }
+    };
 
     bool alive = true;
     if constexpr (PAGED) {
@@ -676,8 +695,9 @@ __global__ void __launch_bounds__(TcShape<NSUB, HD, PAGED>::kThreads,
           n = 0;
           const int t0 = kv_lo + tile * BN + lane * kTmaBoxRows;
           if (lane < PPT && tile < ntiles && t0 < kv_hi_load) {
-            const int pg = __ldg(pages + t0 / p.page_size);
-            const int64_t row0 = static_cast<int64_t>(pg) * p.page_size + t0 % p.page_size;
+            const int page = divide_by(t0, p.page_recip);
+            const int pg = __ldg(pages + page);
+            const int64_t row0 = static_cast<int64_t>(pg) * p.page_size + (t0 - page * p.page_size);
             const int nv = min(kTmaBoxRows, sq.L - t0);
             if (pg < 0 || row0 + nv > p.num_slots) {
               if (p.status) atomicExch(p.status, 2);   // page outside the pool: rows read as zeros
@@ -741,6 +761,7 @@ __global__ void __launch_bounds__(TcShape<NSUB, HD, PAGED>::kThreads,
         int wy[LA + 1], wn[LA + 1];
 #pragma unroll
         for (int t = 0; t <= LA; ++t) fetch_box(t, wy[t], wn[t]);
+        load_q();
 #pragma unroll
         for (int t = 0; t < LA; ++t)
           if (t < ntiles && alive) produce(ring_seq_k<LA>(t), &tm_k, kbase, wy[t], wn[t]);
@@ -820,6 +841,7 @@ __global__ void __launch_bounds__(TcShape<NSUB, HD, PAGED>::kThreads,
       };
   #pragma unroll
       for (int t = 0; t <= LA; ++t) stage_slot(t, fetch_slot(t));
+      load_q();
       producers_sync();
       for (int t = 0; t < LA && t < ntiles && alive; ++t) produce(ring_seq_k<LA>(t), kbase, t);
   #pragma unroll 1
@@ -948,7 +970,7 @@ __global__ void __launch_bounds__(TcShape<NSUB, HD, PAGED>::kThreads,
     const uint32_t o_tm = tmem + lane_base + kOCol + i * HD;
     const int row = i * SUB + r;
     const int pk = pk0 + row;
-    const int tl = pk / G;
+    const int tl = over_group(pk);
     const bool valid = row < rows_valid;
     const int pos = sq.prefix + tl;
     const int vhi = min(p.is_cross ? sq.L - 1 : min(pos, sq.L - 1), s_hi - 1);
@@ -1109,7 +1131,7 @@ __global__ void __launch_bounds__(TcShape<NSUB, HD, PAGED>::kThreads,
             const int prow = i * SUB + rloc;
             if (prow < rows_valid) {
               const int pkr = pk0 + prow;
-              const int tlr = pkr / G, gr = pkr - tlr * G;
+              const int tlr = over_group(pkr), gr = pkr - tlr * G;
               T* dst = static_cast<T*>(p.out) +
                        (static_cast<int64_t>(sq.q_begin + tlr) * p.hq + static_cast<int64_t>(h) * G + gr) * HD;
               uint4 w =
@@ -1118,10 +1140,10 @@ __global__ void __launch_bounds__(TcShape<NSUB, HD, PAGED>::kThreads,
                 const T* grow = static_cast<const T*>(p.gate) + (dst - static_cast<T*>(p.out));
                 const uint4 gv = *reinterpret_cast<const uint4*>(
                     reinterpret_cast<const unsigned char*>(grow) + chunk * 16);
-                T* wo = reinterpret_cast<T*>(&w);
-                const T* wg = reinterpret_cast<const T*>(&gv);
-#pragma unroll
-                for (int e = 0; e < 8; ++e) wo[e] = apply_gate<T>(to_f32(wo[e]), wg[e]);
+                w.x = apply_gate_pair<T>(w.x, gv.x);
+                w.y = apply_gate_pair<T>(w.y, gv.y);
+                w.z = apply_gate_pair<T>(w.z, gv.z);
+                w.w = apply_gate_pair<T>(w.w, gv.w);
               }
               *reinterpret_cast<uint4*>(reinterpret_cast<unsigned char*>(dst) + chunk * 16) = w;
             }
@@ -1238,7 +1260,7 @@ __global__ void __launch_bounds__(TcShape<NSUB, HD, PAGED>::kThreads,
     constexpr int kMergers = Shape::kRebalanceRegs ? kMmaWarp : Shape::kWarps;
     if (s_last != 0 && warp < kMergers) {
       // the softmax warps merge (functions of their own: their registers do not weigh on the main loop)
-      const MergeArgs ma{p.part_o, p.part_ml, p.out, p.gate, p.hq, p.group};
+      const MergeArgs ma{p.part_o, p.part_ml, p.out, p.gate, p.hq, p.group, p.group_recip};
       // (rows x 2 splits in flight per lane: what the register cap of the main kernel holds)
       constexpr int kMergeRows = (!Shape::kRebalanceRegs && HD == 128) ? 4 : 2;
       constexpr int kFree = Shape::kSmemBytes - 1024;       // Q and the ring
@@ -1279,7 +1301,7 @@ __global__ void __launch_bounds__(kMergeWarps * 32) prefill_merge_kernel(const P
   const int row_hi = min(rows_valid, row_lo + per);
   if (row_lo >= row_hi) return;
   const int64_t slot0 = static_cast<int64_t>(it.base + it.qt * nsp) * p.hkv + it.h;
-  const MergeArgs ma{p.part_o, p.part_ml, p.out, p.gate, p.hq, p.group};
+  const MergeArgs ma{p.part_o, p.part_ml, p.out, p.gate, p.hq, p.group, p.group_recip};
   merge_kv_splits<T, HD, kMergeWarps, BM, 2, 4>(ma, nsp, slot0, p.hkv, row_lo, row_hi, pk0, sq.q_begin,
                                                  it.h);
 }
