@@ -209,6 +209,12 @@ int msgl_paged_decode_attention_sized(const void* q, const void* k_cache, const 
 size_t msgl_prefill_workspace_bytes(int batch, int total_q, int64_t total_kv, int num_q_heads,
                                     int num_kv_heads, int head_dim, int max_len_extend,
                                     int sliding_window_size);
+/* As many bytes as a call with per-token kv_indices can use: with these it lays the K/V rows of a long prefill out
+ * as pages first (at most 256 MiB for them), with fewer (down to msgl_prefill_workspace_bytes) it gathers them row
+ * by row in the attention kernel. */
+size_t msgl_prefill_workspace_bytes_full(int batch, int total_q, int64_t total_kv, int num_q_heads,
+                                         int num_kv_heads, int head_dim, int max_len_extend,
+                                         int sliding_window_size);
 
 /*
  * Kernel launches one prefill call of this shape makes: 1, or 2 when the key

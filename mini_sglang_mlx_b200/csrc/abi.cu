@@ -279,6 +279,9 @@ bool prefill_pairs(int batch, int total_q, int64_t total_kv, int group, int num_
   return waves(sms / 2) * (17. + 1.9 * key_tiles) < waves(sms) * (20. + 4. * key_tiles);
 }
 
+bool prefill_gathers(int batch, int total_q, int64_t total_kv, int hq, int hkv, int head_dim, int max_len_extend,
+                     int window, int kv_chunk);
+
 PrefillPlan plan_prefill(int batch, int total_q, int64_t total_kv, int hq, int hkv, int head_dim,
                          int max_len_extend, int window, int sms) {
   // The key range is split only when the query tiles alone cannot give every CTA slot of the
@@ -639,6 +642,111 @@ __global__ void expand_page_indices_kernel(const int32_t* __restrict__ page_indp
   }
 }
 
+// ---- per-token K/V rows laid out as pages, in front of a long prefill.  Every 256-query tile reads its keys
+// again, and with per-token slots every one of those reads is a gather of 16-byte copies by seven warps of
+// the CTA, which bounds the kernel; copied once per call into pages (K and V rows of all heads, 16 tokens a page, a
+// sequence's first page at kv_indptr[b] / 16 + b, which leaves every sequence its last, partly filled one) they come by
+// TMA, and pairs of CTAs share them.  Bound by memory: rows are read once and written once, eight of a warp's
+// 16-byte accesses in flight per lane.  Slots outside the pool become zero rows, as in the attention kernels.
+struct GatherRowsParams {
+  const unsigned char *k, *v;
+  const int32_t *kv_indptr, *kv_indices;
+  unsigned char *k_rows, *v_rows;
+  int32_t *page_indptr, *page_indices, *kv_lens;
+  int batch, row_chunks;       // 16-byte chunks of a token's row of all heads
+  int max_pages;
+  int64_t num_slots;
+  int* status;
+};
+constexpr int kGatherTokens = 8;   // of a warp
+
+__global__ void __launch_bounds__(256) gather_rows_kernel(const GatherRowsParams p) {
+  msgl::grid_dependency_wait();
+  msgl::grid_dependency_launch();
+  const int b = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int32_t* indptr = msgl::after_wait(p.kv_indptr);
+  const int begin = indptr[b];
+  const int page0 = begin / msgl::kTmaBoxRows + b;
+  const bool bad = begin < 0 || page0 >= p.max_pages;
+  const int room = bad ? 0 : (p.max_pages - page0) * msgl::kTmaBoxRows;
+  const int len = bad ? 0 : min(max(indptr[b + 1] - begin, 0), room);
+  const int pages = (len + msgl::kTmaBoxRows - 1) / msgl::kTmaBoxRows;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    p.page_indptr[b] = bad ? 0 : page0;
+    p.kv_lens[b] = len;
+    if (b == p.batch - 1) p.page_indptr[p.batch] = bad ? 0 : page0 + pages;
+  }
+  for (int i = blockIdx.x * 256 + threadIdx.x; i < pages; i += gridDim.x * 256) p.page_indices[page0 + i] = page0 + i;
+  const int64_t row_bytes = static_cast<int64_t>(p.row_chunks) * 16;
+  const int32_t* ids = msgl::after_wait(p.kv_indices) + begin;
+  const int64_t row0 = static_cast<int64_t>(page0) * msgl::kTmaBoxRows;
+  for (int t0 = (blockIdx.x * 8 + warp) * kGatherTokens; t0 < len; t0 += gridDim.x * 8 * kGatherTokens) {
+    int slot = -1;
+    if (lane < kGatherTokens && t0 + lane < len) {
+      slot = __ldg(ids + t0 + lane);
+      if (slot < -1 || slot >= p.num_slots) {
+        if (p.status) atomicExch(p.status, 2);
+        slot = -1;
+      }
+    }
+    const int n = min(kGatherTokens, len - t0);
+    int from[kGatherTokens];
+#pragma unroll
+    for (int i = 0; i < kGatherTokens; ++i) from[i] = __shfl_sync(0xffffffffu, slot, i);
+    for (int c = lane; c < p.row_chunks; c += 32) {
+#pragma unroll
+      for (int h = 0; h < kGatherTokens; h += 4) {
+        uint4 x[4], y[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          x[i] = y[i] = make_uint4(0u, 0u, 0u, 0u);
+          if (from[h + i] >= 0) {
+            x[i] = __ldg(reinterpret_cast<const uint4*>(p.k + from[h + i] * row_bytes) + c);
+            y[i] = __ldg(reinterpret_cast<const uint4*>(p.v + from[h + i] * row_bytes) + c);
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          if (h + i >= n) break;
+          const int64_t to = (row0 + t0 + h + i) * row_bytes;
+          reinterpret_cast<uint4*>(p.k_rows + to)[c] = x[i];
+          reinterpret_cast<uint4*>(p.v_rows + to)[c] = y[i];
+        }
+      }
+    }
+  }
+}
+
+// The scratch that takes: behind the header the K rows, the V rows, the page ids, and room for the pointer array and
+// the lengths of any batch.
+constexpr size_t kGatherIndexBytes = 2 * 65537 * sizeof(int32_t) + 256;
+constexpr size_t kGatherBytesMax = 256u << 20;
+constexpr double kGatherWorth = 4.5;
+size_t gather_page_bytes(int num_kv_heads) {
+  return static_cast<size_t>(msgl::kTmaBoxRows) * num_kv_heads * 128 * 2 * 2 + sizeof(int32_t);
+}
+size_t gather_bytes(int batch, int64_t total_kv, int num_kv_heads) {
+  return kGatherIndexBytes + static_cast<size_t>(total_kv / msgl::kTmaBoxRows + batch + 1) * gather_page_bytes(num_kv_heads);
+}
+
+// Pays where the attention takes several times what the copies do, by a rough model of both.  Steps of two layers in us,
+// gathered by the attention kernel / laid out first, and the model's ratio: 3 sequences of 300 to 2000 tokens over up
+// to 8000, 32 over 4 heads 1039 / 779 (14); 4000 tokens, 32 over 8 heads 442 / 390 (9.9); 1000 over 16000 664 / 546 (6.8);
+// 2000 over 5000, 16 over 8 298 / 280 (5.1); two prompts of up to 4000 288 / 276 (4.7); eight of up to 2938, 16 over 8
+// 556 / 545 (3.3); four chunks of 512 over up to 4096, 32 over 8 284 / 285 (3.0); 16 over 8 192 / 219 (1.5).
+bool prefill_gathers(int batch, int total_q, int64_t total_kv, int hq, int hkv, int head_dim, int max_len_extend,
+                     int window, int kv_chunk) {
+  if (head_dim != 128 || kv_chunk != 0 || prefill_short_q(max_len_extend, hq / hkv, head_dim) || batch > 65535 ||
+      tensor_map_encoder() == nullptr)
+    return false;
+  if (total_kv <= 0 || gather_bytes(batch, total_kv, hkv) > kGatherBytesMax) return false;
+  double keys = std::max(1., static_cast<double>(total_kv) / batch - 0.5 * total_q / batch);
+  if (window > 0) keys = std::min<double>(keys, window);
+  const double attend_us = 4. * head_dim * hq * static_cast<double>(total_q) * keys / 1e9;    // at 1 PFLOP/s
+  const double copy_us = 5. + static_cast<double>(total_kv) * hkv * head_dim * 8. / 4e6;      // at 4 TB/s
+  return attend_us > kGatherWorth * copy_us;
+}
+
 // ---- decode scheduling (shared by the workspace query and the launch), in groups of 16 tokens
 constexpr int kDecMinShare = 8;      // below, a warp has one group or two and the merge dominates
 constexpr int kDecMaxShare = 512;    // (256 / 384 / 512 on 32 sequences of 2000 to 20000 tokens: 248 / 238 / 238 us)
@@ -959,11 +1067,27 @@ int msgl_prefill_launch_count(int batch, int total_q, int64_t total_kv, int num_
       num_q_heads % num_kv_heads != 0)
     return 1;
   const int sms = sm_count_cached();
-  (void)page_granular;   // both index granularities split alike
   const PrefillPlan pl = plan_prefill(batch, total_q, total_kv, num_q_heads, num_kv_heads,
                                       head_dim, max_len_extend, sliding_window_size,
                                       sms > 0 ? sms : 148);
+  if (!page_granular && prefill_gathers(batch, total_q, total_kv, num_q_heads, num_kv_heads, head_dim, max_len_extend,
+                                        sliding_window_size, pl.kv_chunk))
+    return 2;            // (with the scratch of msgl_prefill_workspace_bytes_full)
   return (pl.kv_chunk > 0 && !pl.fused_merge) ? 2 : 1;
+}
+
+size_t msgl_prefill_workspace_bytes_full(int batch, int total_q, int64_t total_kv, int num_q_heads, int num_kv_heads,
+                                         int head_dim, int max_len_extend, int sliding_window_size) {
+  const size_t least = msgl_prefill_workspace_bytes(batch, total_q, total_kv, num_q_heads, num_kv_heads, head_dim,
+                                                    max_len_extend, sliding_window_size);
+  if (batch <= 0 || total_q <= 0 || num_q_heads <= 0 || num_kv_heads <= 0 || num_q_heads % num_kv_heads != 0) return least;
+  const int sms = sm_count_cached();
+  const PrefillPlan pl = plan_prefill(batch, total_q, total_kv, num_q_heads, num_kv_heads, head_dim, max_len_extend,
+                                      sliding_window_size, sms > 0 ? sms : 148);
+  if (!prefill_gathers(batch, total_q, total_kv, num_q_heads, num_kv_heads, head_dim, max_len_extend, sliding_window_size,
+                       pl.kv_chunk))
+    return least;
+  return std::max(least, kStatusBytes + gather_bytes(batch, total_kv, num_kv_heads));
 }
 
 static int prefill_impl(const void* q, const void* k_cache, const void* v_cache,
@@ -1000,6 +1124,47 @@ static int prefill_impl(const void* q, const void* k_cache, const void* v_cache,
                                                 "16-byte aligned");
   const int sms = sm_count_cached();
   if (sms <= 0) return fail(MSGL_CUDA_ERROR, std::string(op) + "cannot query the device");
+  const PrefillPlan pl = plan_prefill(batch, total_q, total_kv, num_q_heads, num_kv_heads,
+                                      head_dim, max_len_extend, sliding_window_size, sms);
+  const size_t need = kStatusBytes + pl.plan_bytes + pl.part_ml_bytes + pl.part_o_bytes;
+  if (!workspace || workspace_bytes < need)
+    return fail(MSGL_BAD_ARG, std::string(op) + "workspace too small");
+  PageIndex laid_out;
+  if (!pages && num_slots > 0 &&
+      prefill_gathers(batch, total_q, total_kv, num_q_heads, num_kv_heads, head_dim, max_len_extend, sliding_window_size,
+                      pl.kv_chunk) &&
+      workspace_bytes >= kStatusBytes + gather_bytes(batch, total_kv, num_kv_heads)) {
+    // (the pool's tensor maps are kept by address and size: as many pages as the scratch holds, whatever the call)
+    GatherRowsParams g{};
+    const int64_t cap = static_cast<int64_t>((workspace_bytes - kStatusBytes - kGatherIndexBytes) / gather_page_bytes(num_kv_heads));
+    g.max_pages = static_cast<int>(std::min<int64_t>(cap, (1ll << 31) / msgl::kTmaBoxRows - 1));
+    const size_t rows_bytes = static_cast<size_t>(g.max_pages) * msgl::kTmaBoxRows * num_kv_heads * head_dim * 2;
+    unsigned char* at = static_cast<unsigned char*>(workspace) + kStatusBytes;
+    g.k_rows = at;
+    g.v_rows = at + rows_bytes;
+    g.page_indices = reinterpret_cast<int32_t*>(at + 2 * rows_bytes);
+    g.page_indptr = g.page_indices + g.max_pages;
+    g.kv_lens = g.page_indptr + batch + 1;
+    g.k = static_cast<const unsigned char*>(k_cache);
+    g.v = static_cast<const unsigned char*>(v_cache);
+    g.kv_indptr = kv_indptr;
+    g.kv_indices = kv_indices;
+    g.batch = batch;
+    g.row_chunks = num_kv_heads * head_dim / 8;
+    g.num_slots = num_slots;
+    g.status = static_cast<int*>(workspace);
+    const int64_t per_seq = total_kv / batch + 1;
+    const unsigned gx = static_cast<unsigned>(std::max<int64_t>(1, std::min<int64_t>((per_seq + 63) / 64, 4096)));
+    const cudaError_t err = launch_dependent(gather_rows_kernel, dim3(gx, batch), dim3(256), 0,
+                                             static_cast<cudaStream_t>(stream), g);
+    if (err != cudaSuccess) return cuda_fail("paged_prefill_attention", err);
+    laid_out = PageIndex{g.page_indptr, g.page_indices, g.kv_lens, msgl::kTmaBoxRows};
+    pages = &laid_out;
+    k_cache = g.k_rows;
+    v_cache = g.v_rows;
+    num_slots = static_cast<int64_t>(g.max_pages) * msgl::kTmaBoxRows;
+    behind_store = false;      // (the index arrays are this kernel's)
+  }
   CUtensorMap tm_k, tm_v;
   std::memset(&tm_k, 0, sizeof(tm_k));
   std::memset(&tm_v, 0, sizeof(tm_v));
@@ -1010,11 +1175,6 @@ static int prefill_impl(const void* q, const void* k_cache, const void* v_cache,
   std::memset(&tm_q, 0, sizeof(tm_q));
   const bool q_tma = pages && make_query_tensor_map(&tm_q, q, total_q, num_q_heads,
                                                     num_q_heads / num_kv_heads, head_dim, dtype);
-  const PrefillPlan pl = plan_prefill(batch, total_q, total_kv, num_q_heads, num_kv_heads,
-                                      head_dim, max_len_extend, sliding_window_size, sms);
-  const size_t need = kStatusBytes + pl.plan_bytes + pl.part_ml_bytes + pl.part_o_bytes;
-  if (!workspace || workspace_bytes < need)
-    return fail(MSGL_BAD_ARG, std::string(op) + "workspace too small");
   if (pl.items * num_kv_heads > 0x7fffffffLL || num_q_heads > 65535)
     return fail(MSGL_BAD_SHAPE, std::string(op) + "problem too large for one launch");
 

@@ -280,7 +280,7 @@ PyObject* prefill(PyObject*, PyObject* const* a, Py_ssize_t n) {
   size_t ws_bytes;
   if (!stream_of(a[12], s.device, &stream) ||
       !scratch_for(s.device, stream, kPrefill,
-                   msgl_prefill_workspace_bytes(batch, s.n, total_kv, s.hq, s.hkv, s.d,
+                   msgl_prefill_workspace_bytes_full(batch, s.n, total_kv, s.hq, s.hkv, s.d,
                                                 static_cast<int>(max_ext), static_cast<int>(window)),
                    &ws, &ws_bytes))
     return nullptr;
@@ -560,7 +560,8 @@ PyObject* prefill_layer(PyObject*, PyObject* const* a, Py_ssize_t n) {
   size_t ws_bytes;
   if (!stream_of(Py_None, s.device, &stream) ||
       !scratch_for(s.device, stream, kPrefill,
-                   msgl_prefill_workspace_bytes(batch, s.n, lens ? total * page_size : total, s.hq, s.hkv, s.d,
+                   (lens ? msgl_prefill_workspace_bytes : msgl_prefill_workspace_bytes_full)(
+                                                batch, s.n, lens ? total * page_size : total, s.hq, s.hkv, s.d,
                                                 static_cast<int>(max_ext), static_cast<int>(window)),
                    &ws, &ws_bytes))
     return nullptr;

@@ -146,3 +146,56 @@ def test_items_of_up_to_32_sequences_and_of_more(batch, d, hkv, hq, q_hi, window
     assert_close_to_oracle(out, ref, "pages")
     out = paged_prefill_attention(q, kc, vc, qo, kvp, slots, pre, sc, n, sliding_window_size=window)
     assert_close_to_oracle(out, ref, "slots")
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("hkv,hq,q_lens,prefixes,kw", [
+    (1, 32, [2600, 37, 0, 300], [100, 500, 64, 900], {}), (4, 32, [2300], [1], {}),
+    (3, 48, [17, 1800], [0, 700], dict(sliding_window_size=900)), (2, 32, [2300, 1100], [3, 0], dict(is_cross_attention=True))],
+    ids=lambda x: str(x)[:30])
+def test_long_prefill_over_per_token_slots(hkv, hq, q_lens, prefixes, kw, dtype):
+    """Rows laid out as pages first, with room for them in the scratch: the page-granular call's bits; slots outside
+    the pool are zeros and reported.  With the least scratch the attention kernel gathers them itself."""
+    from mini_sglang_mlx_b200 import _lib, paged_prefill_attention, paged_prefill_attention_p16
+    from mini_sglang_mlx_b200.kernel import device_status
+    d, lib = 128, _lib.lib()
+    need = [max(n, 1) for n in q_lens]
+    q, _, kc, vc, pip, pidx, slots, kv_lens = _problem(need, prefixes, hkv, hq, d, sum(q_lens), dtype=dtype)
+    kept, at = [], 0
+    for n, x in zip(q_lens, kv_lens):
+        kept.append(slots[at:at + x - (n == 0)])
+        at += x
+    kv_lens = [x - (n == 0) for n, x in zip(q_lens, kv_lens)]
+    slots, q = torch.cat(kept), q[:sum(q_lens)].contiguous()
+    qo, kvp, pre = _i32(O.build_indptr(q_lens).tolist()), _i32(O.build_indptr(kv_lens).tolist()), _i32(prefixes)
+    sc, n, batch, tq, tkv = 1 / math.sqrt(d), max(q_lens), len(q_lens), sum(q_lens), sum(kv_lens)
+    window, cross = kw.get("sliding_window_size", 0), kw.get("is_cross_attention", False)
+    shape = (batch, tq, tkv, hq, hkv, d, n, window)
+    assert lib.msgl_prefill_launch_count(*shape, 0) == 2          # (the rows are laid out)
+    args = (qo, kvp, slots, pre, sc, n)
+    device_status()
+    out = paged_prefill_attention(q, kc, vc, *args, **kw)
+    paged = paged_prefill_attention_p16(q, kc, vc, qo, pip, pidx, _i32(kv_lens), pre, sc, n, page_size=16, **kw)
+    assert torch.equal(out, paged) and device_status() == 0
+    ref = O.paged_prefill_attention_oracle(q, kc, vc, qo, kvp, slots, pre, sc, **kw)
+    assert_close_to_oracle(out, ref, "laid out")
+    least, full = lib.msgl_prefill_workspace_bytes(*shape), lib.msgl_prefill_workspace_bytes_full(*shape)
+    assert least < full <= least + (256 << 20)
+    for size in (least, full - 1, full):
+        ws = torch.full((size + 4096,), 255, dtype=torch.uint8, device="cuda")
+        ws[:65792] = 0
+        got = torch.empty_like(q)
+        _lib.check(lib.msgl_paged_prefill_attention(
+            q.data_ptr(), kc.data_ptr(), vc.data_ptr(), qo.data_ptr(), kvp.data_ptr(), slots.data_ptr(), pre.data_ptr(),
+            got.data_ptr(), ws.data_ptr(), size, batch, tq, tkv, hq, hkv, d, kc.shape[0], int(dtype == torch.float16), sc, n,
+            int(cross), window, torch.cuda.current_stream().cuda_stream))
+        assert_close_to_oracle(got, ref, str(size))
+        assert torch.equal(got, out) or size < full
+        assert int(ws[:65792].sum()) == 0 and bool((ws[size:] == 255).all())
+    bad = slots.clone()
+    bad[::5], bad[1::7] = -1, kc.shape[0] + 3
+    out = paged_prefill_attention(q, kc, vc, qo, kvp, bad, pre, sc, n, **kw)
+    assert device_status() == 2
+    kz, vz = torch.cat([kc, torch.zeros_like(kc[:1])]), torch.cat([vc, torch.zeros_like(vc[:1])])
+    zeros = torch.where((bad < 0) | (bad >= kc.shape[0]), kc.shape[0], bad)
+    assert_close_to_oracle(out, O.paged_prefill_attention_oracle(q, kz, vz, qo, kvp, zeros, pre, sc, **kw), "zeros")
