@@ -164,6 +164,44 @@ bool make_pool_tensor_map(CUtensorMap* out, const void* base, int64_t num_slots,
   return true;
 }
 
+// 3-D map over a pool for the decode kernel: (64 elements, slots, blocks of 64 elements of a row), so that one box is 16
+// token rows x all head_dim elements of one head, a block of columns after the other, as the kernel's tiles lie in
+// shared memory.  (A copy instruction costs its warp 67 cycles whatever its size: one per tile instead of two or four.)
+bool make_pool_group_map(CUtensorMap* out, const void* base, int64_t num_slots, int num_kv_heads, int head_dim,
+                         int dtype) {
+  struct Cached {
+    const void* base;
+    int64_t num_slots;
+    int hkv, hd, dtype;
+    CUtensorMap map;
+  };
+  static thread_local Cached cache[256] = {};
+  const uintptr_t key = reinterpret_cast<uintptr_t>(base) >> 8;
+  Cached& c = cache[(key ^ (key >> 8) ^ (key >> 16) ^ (key >> 24)) % 256];
+  if (c.base == base && c.num_slots == num_slots && c.hkv == num_kv_heads && c.hd == head_dim && c.dtype == dtype &&
+      base != nullptr) {
+    *out = c.map;
+    return true;
+  }
+  EncodeTiledFn enc = tensor_map_encoder();
+  if (!enc || num_slots <= 0 || num_slots >= (1ll << 32) || reinterpret_cast<uintptr_t>(base) % 16 != 0) return false;
+  const cuuint64_t dims[3] = {64, static_cast<cuuint64_t>(num_slots),
+                              static_cast<cuuint64_t>(num_kv_heads) * head_dim / 64};
+  const cuuint64_t strides[2] = {static_cast<cuuint64_t>(num_kv_heads) * head_dim * 2, 128};
+  const cuuint32_t box[3] = {64, static_cast<cuuint32_t>(msgl::kTmaBoxRows), static_cast<cuuint32_t>(head_dim / 64)};
+  const cuuint32_t elem_strides[3] = {1, 1, 1};
+  CUtensorMap m;
+  const CUresult r = enc(&m, dtype == MSGL_DTYPE_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16
+                                                      : CU_TENSOR_MAP_DATA_TYPE_FLOAT16,
+                         3, const_cast<void*>(base), dims, strides, box, elem_strides,
+                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                         CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return false;
+  c = Cached{base, num_slots, num_kv_heads, head_dim, dtype, m};
+  *out = m;
+  return true;
+}
+
 // 3-D map over the query tensor (tokens, query heads, head_dim): a box is 64 elements x the
 // `group` heads of one KV head x 128 / group tokens, i.e. the 128 packed rows of a query
 // sub-tile in the order the kernel numbers them.  Needs a group that divides 128.
@@ -877,8 +915,8 @@ static int decode_impl(const void* q, const void* k_cache, const void* v_cache,
   CUtensorMap tm_k, tm_v;
   std::memset(&tm_k, 0, sizeof(tm_k));
   std::memset(&tm_v, 0, sizeof(tm_v));
-  if (pages && (!make_pool_tensor_map(&tm_k, k_cache, num_slots, num_kv_heads, head_dim, dtype) ||
-                !make_pool_tensor_map(&tm_v, v_cache, num_slots, num_kv_heads, head_dim, dtype)))
+  if (pages && (!make_pool_group_map(&tm_k, k_cache, num_slots, num_kv_heads, head_dim, dtype) ||
+                !make_pool_group_map(&tm_v, v_cache, num_slots, num_kv_heads, head_dim, dtype)))
     return fail(MSGL_CUDA_ERROR, std::string(op) + "cannot build the tensor maps of the K/V pool");
   const size_t need = msgl_decode_workspace_bytes(batch, num_q_heads, head_dim, max_kv_splits);
   if (!workspace || workspace_bytes < need)

@@ -29,8 +29,8 @@
 //
 // Per-token form: K and V rows (256 or 512 bytes per token and head) are gathered through the slot
 // ids with 16-byte cp.async copies.  Page-granular form (PAGED): a group is one page (or a 16-row
-// slice of a larger page), contiguous in the pool, so lane 0 fetches it with TMA box copies
-// (cp.async.bulk.tensor.2d, 16 rows x 64 elements, 128-byte swizzle) straight from the page id and
+// slice of a larger page), contiguous in the pool, so lane 0 fetches it with a TMA box copy each for K and V
+// (cp.async.bulk.tensor.3d: HD / 64 blocks of 16 rows x 64 elements, 128-byte swizzle) straight from the page id and
 // the warp waits on the stage's mbarrier; only a sequence's ragged last page is copied row by row
 // (rows past the length are zero-filled).
 //
@@ -445,11 +445,8 @@ __global__ void __launch_bounds__(NWARPS * 32, HD == 256 ? 1 : 2)
       if (n == kDecodeGroupTokens) {
         if (lane == 0) {
           mbar_arrive_expect_tx(bar, 2 * TILE_BYTES);
-#pragma unroll
-          for (int c = 0; c < HD / 64; ++c) {
-            tma_load_2d(kdst + c * (kDecodeGroupTokens * 128), &tm_k, h * HD + c * 64, y, bar);
-            tma_load_2d(vdst + c * (kDecodeGroupTokens * 128), &tm_v, h * HD + c * 64, y, bar);
-          }
+          tma_load_3d(kdst, &tm_k, 0, y, h * (HD / 64), bar);
+          tma_load_3d(vdst, &tm_v, 0, y, h * (HD / 64), bar);
         }
       } else {
         // ragged last page of the sequence: valid rows by 16-byte copies, the rest zeros; the barrier
