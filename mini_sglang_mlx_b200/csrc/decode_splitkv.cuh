@@ -406,9 +406,12 @@ __global__ void __launch_bounds__(NWARPS * 32, HD == 256 ? 1 : 2)
       if (!waited) {       // lanes whose row the kernel in front writes
         bool hit = false;
 #pragma unroll
-        for (int i = 0; i < kNewRegs; ++i)
-          for (int k = 0; k < min(32, p.num_new - 32 * i); ++k) hit |= w.y == __shfl_sync(0xffffffffu, fresh[i], k);
-        w.fresh = __ballot_sync(0xffffffffu, hit);
+        for (int i = 0; i < kNewRegs; ++i) {
+          if (i * 32 >= p.num_new) break;
+#pragma unroll 16
+          for (int k = 0; k < 32; ++k) hit |= w.y == __shfl_sync(0xffffffffu, fresh[i], k);
+        }
+        w.fresh = __ballot_sync(0xffffffffu, hit && w.y >= 0);
       }
     }
   };
@@ -795,10 +798,11 @@ __global__ void __launch_bounds__(NWARPS * 32, HD == 256 ? 1 : 2)
       gate.load(static_cast<const T*>(p.gate), oi);
       const float* rows = p.part + ((static_cast<int64_t>(part.first) + part.b) * p.hkv + h) * G * PROW + g * PROW;
       const int64_t pitch = static_cast<int64_t>(p.hkv) * G * PROW;     // from piece to piece
-      constexpr int FLY = 8;                                            // pieces in flight
       float M = -INFINITY, den = 0.f, num[VPL];
 #pragma unroll
       for (int e = 0; e < VPL; ++e) num[e] = 0.f;
+      auto add_pieces = [&](auto fly) {
+      constexpr int FLY = decltype(fly)::value;                         // pieces in flight
 #pragma unroll 1
       for (int j0 = 0; j0 < part.count; j0 += FLY, rows += FLY * pitch) {
         const int m = min(FLY, part.count - j0);
@@ -836,6 +840,10 @@ __global__ void __launch_bounds__(NWARPS * 32, HD == 256 ? 1 : 2)
           }
         }
       }
+      };
+      // (16 pieces of a head are three reads of L2 in a row otherwise)
+      if (part.count > 8) add_pieces(std::integral_constant<int, 16>{});
+      else add_pieces(std::integral_constant<int, 8>{});
       const float inv = den > 0.f ? 1.f / den : 0.f;
 #pragma unroll
       for (int e = 0; e < VPL; ++e) num[e] *= inv;
