@@ -788,9 +788,11 @@ bool prefill_gathers(int batch, int total_q, int64_t total_kv, int hq, int hkv, 
 // ---- decode scheduling (shared by the workspace query and the launch), in groups of 16 tokens
 constexpr int kDecMinShare = 8;      // below, a warp has one group or two and the merge dominates
 constexpr int kDecMaxShare = 512;    // (256 / 384 / 512 on 32 sequences of 2000 to 20000 tokens: 248 / 238 / 238 us)
-// A segment's end (merge of the warps, partial, next Q) takes about as long as two groups of each of
-// the four warps, five at head_dim 256 with its twice as long rows and one CTA per SM.
-constexpr int kDecPad128 = 8, kDecPad256 = 20;
+// A segment's end (merge of the warps, partial, next Q) takes about as long as three groups of each of
+// the four warps, five at head_dim 256 with its twice as long rows and one CTA per SM.  (Steps of four layers with 8 / 12 /
+// 16: 12 requests of 1000 to 8000 tokens 221 / 218 / 217 us, 37 in per-token slots 148 / 146.6 / 146.9, 3 of 500 to 3000
+// 50.3 / 50.3 / 52.1; 19 of 512 to 16384 at head_dim 256 with 12 / 16 / 20: 199 / 195 / 186.)
+constexpr int kDecPad128 = 12, kDecPad256 = 20;
 // Merging a piece of a sequence (a warp per query head, eight pieces in flight) against a group in the loop, for
 // every four query heads of a KV head.  Beyond kDecMaxPieces pieces the shares grow to balance the two.  Steps of
 // two layers in us with 0.3 / 0.6 / 1.2: one sequence, 32 query over 2 KV heads of 256, 8191 tokens 61 / 62 / 68 (90

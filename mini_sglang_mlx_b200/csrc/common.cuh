@@ -13,7 +13,6 @@
 namespace msgl {
 
 constexpr float kLog2e = 1.4426950408889634f;
-constexpr float kLn2 = 0.6931471805599453f;
 
 // ---------------------------------------------------------------- addresses
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
