@@ -759,7 +759,7 @@ __global__ void __launch_bounds__(256) gather_rows_kernel(const GatherRowsParams
 // the lengths of any batch.
 constexpr size_t kGatherIndexBytes = 2 * 65537 * sizeof(int32_t) + 256;
 constexpr size_t kGatherBytesMax = 256u << 20;
-constexpr double kGatherWorth = 4.5;
+constexpr double kGatherWorth = 2.9;
 size_t gather_page_bytes(int num_kv_heads) {
   return static_cast<size_t>(msgl::kTmaBoxRows) * num_kv_heads * 128 * 2 * 2 + sizeof(int32_t);
 }

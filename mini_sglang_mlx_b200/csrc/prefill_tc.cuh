@@ -538,7 +538,10 @@ __global__ void __launch_bounds__(TcShape<NSUB, HD, PAGED>::kThreads,
   }
 
   if (!p.early) grid_dependency_wait();
-  const bool by_warp = p.batch <= kWarpBatchMax;
+  // (The two-sub-tile shape is at its register limit: with these the tile loop of its page-granular form takes 2 %
+  // longer, 512 tokens over 32768 282 -> 288 us, so that one keeps the general search and its divisions.)
+  constexpr bool kGeneral = NSUB == 2 && PAGED;
+  const bool by_warp = !kGeneral && p.batch <= kWarpBatchMax;
   if (by_warp) {
     if (warp == 0) find_item_warp(p, static_cast<int>(blockIdx.x), BM, &found);
   } else {
@@ -566,11 +569,10 @@ __global__ void __launch_bounds__(TcShape<NSUB, HD, PAGED>::kThreads,
   }
   const ItemCoord it = found.at;
   const int h = it.h;
-  const SeqShape sq = found.seq;
+  const SeqShape sq = kGeneral ? load_seq_shape(p, it.b, BM) : found.seq;
   const int qt = it.qt, split = it.split;
   const int slot_item = it.base + qt * sq.nsplit + split;   // where this item's kv-split partial goes
-  // (the two-sub-tile per-token form is at its register limit: with the reciprocals its tile loop takes 2 % longer)
-  auto over_group = [&](int x) { return NSUB == 2 && !PAGED ? x / G : divide_by(x, p.group_recip); };
+  auto over_group = [&](int x) { return NSUB == 2 ? x / G : divide_by(x, p.group_recip); };
   if (PAGED && it.first && tid == 0 && p.status) {
     // a length that is negative or exceeds the sequence's pages was clamped: report it
     const int64_t cap = static_cast<int64_t>(p.page_indptr[it.b + 1] - p.page_indptr[it.b]) * p.page_size;
@@ -668,6 +670,7 @@ __global__ void __launch_bounds__(TcShape<NSUB, HD, PAGED>::kThreads,
     }
     };
 
+    if constexpr (kGeneral) load_q();
     bool alive = true;
     if constexpr (PAGED) {
       // ------------------------------------------------ page-granular: TMA boxes from the page ids
@@ -695,7 +698,7 @@ __global__ void __launch_bounds__(TcShape<NSUB, HD, PAGED>::kThreads,
           n = 0;
           const int t0 = kv_lo + tile * BN + lane * kTmaBoxRows;
           if (lane < PPT && tile < ntiles && t0 < kv_hi_load) {
-            const int page = divide_by(t0, p.page_recip);
+            const int page = kGeneral ? t0 / p.page_size : divide_by(t0, p.page_recip);
             const int pg = __ldg(pages + page);
             const int64_t row0 = static_cast<int64_t>(pg) * p.page_size + (t0 - page * p.page_size);
             const int nv = min(kTmaBoxRows, sq.L - t0);
@@ -761,7 +764,7 @@ __global__ void __launch_bounds__(TcShape<NSUB, HD, PAGED>::kThreads,
         int wy[LA + 1], wn[LA + 1];
 #pragma unroll
         for (int t = 0; t <= LA; ++t) fetch_box(t, wy[t], wn[t]);
-        load_q();
+        if constexpr (!kGeneral) load_q();
 #pragma unroll
         for (int t = 0; t < LA; ++t)
           if (t < ntiles && alive) produce(ring_seq_k<LA>(t), &tm_k, kbase, wy[t], wn[t]);
@@ -1140,10 +1143,17 @@ __global__ void __launch_bounds__(TcShape<NSUB, HD, PAGED>::kThreads,
                 const T* grow = static_cast<const T*>(p.gate) + (dst - static_cast<T*>(p.out));
                 const uint4 gv = *reinterpret_cast<const uint4*>(
                     reinterpret_cast<const unsigned char*>(grow) + chunk * 16);
-                w.x = apply_gate_pair<T>(w.x, gv.x);
-                w.y = apply_gate_pair<T>(w.y, gv.y);
-                w.z = apply_gate_pair<T>(w.z, gv.z);
-                w.w = apply_gate_pair<T>(w.w, gv.w);
+                if constexpr (kGeneral) {
+                  T* wo = reinterpret_cast<T*>(&w);
+                  const T* wg = reinterpret_cast<const T*>(&gv);
+#pragma unroll
+                  for (int e = 0; e < 8; ++e) wo[e] = apply_gate<T>(to_f32(wo[e]), wg[e]);
+                } else {
+                  w.x = apply_gate_pair<T>(w.x, gv.x);
+                  w.y = apply_gate_pair<T>(w.y, gv.y);
+                  w.z = apply_gate_pair<T>(w.z, gv.z);
+                  w.w = apply_gate_pair<T>(w.w, gv.w);
+                }
               }
               *reinterpret_cast<uint4*>(reinterpret_cast<unsigned char*>(dst) + chunk * 16) = w;
             }
