@@ -552,7 +552,7 @@ __global__ void __launch_bounds__(TcShape<NSUB, HD, PAGED>::kThreads,
       found.have = have;
       if (have) {
         found.at = at;
-        found.seq = load_seq_shape(p, at.b, BM);
+        if (!kGeneral) found.seq = load_seq_shape(p, at.b, BM);
       }
     }
   }
