@@ -18,7 +18,9 @@
  * kernels leave the counters at zero, but they must BE zero at the first call:
  * clear at least the header once after allocating a workspace
  * (cudaMemsetAsync), use one workspace per stream, and let nothing else write
- * to the header.  After a call that reported status 1 clear it again.
+ * to the header.  After a call that reported status 1 clear it again.  A call
+ * can be several launches that hand data over through the workspace: threads
+ * that share a stream and its workspace make their calls in turn.
  *
  * Each function replaces one operator of the reference extension
  * `mini_sglang_mlx_kernel` (mini-sglang-mlx-kernel/csrc/bindings.cpp); the

@@ -23,8 +23,9 @@
 
 #include <algorithm>
 #include <cmath>
+#include <deque>
+#include <mutex>
 #include <string>
-#include <vector>
 
 #include "../../include/msgl_b200.h"
 
@@ -33,47 +34,51 @@ namespace {
 using at::Tensor;
 
 // ------------------------------------------------------------------ scratch
-// Address and size of the scratch of (device, stream, operator), as the Python side made it; asked
-// for again (which grows it) when a call needs more.
+// Address and size of the scratch of a stream's operators, as the Python side made it; asked for again
+// (which grows it) when a call needs more.
 enum Kind { kDecode = 0, kPrefill = 1 };
 const char* const kKindNames[] = {"decode", "prefill"};
 
-struct Scratch {
+struct StreamScratch {
   int device;
   int64_t stream;
-  int kind;
+  // Held while a call queues its launches.  An attention call can be several of them that hand data over
+  // through the scratch (slot ids or counters written in front, partials merged behind), and other Python
+  // threads run while it queues them: two calls in turn keep each its own.
+  std::mutex launches;
+  void* ptr[2] = {};
+  size_t bytes[2] = {};
+  StreamScratch(int d, int64_t s) : device(d), stream(s) {}
+};
+// guarded by the GIL, but for `launches`; entries keep their place and are never destroyed (a thread may hold one at exit)
+std::deque<StreamScratch>& g_scratch = *new std::deque<StreamScratch>;
+PyObject* g_make_workspace = nullptr;  // Python: (nbytes, device index, stream handle, kind) -> tensor
+
+// The scratch a call got: it stays valid when the stream's scratch grows meanwhile (the Python side keeps
+// outgrown buffers).
+struct Scratch {
+  StreamScratch* of;
   void* ptr;
   size_t bytes;
 };
-std::vector<Scratch> g_scratch;        // guarded by the GIL
-PyObject* g_make_workspace = nullptr;  // Python: (nbytes, device index, stream handle, kind) -> tensor
 
-bool scratch_for(int device, int64_t stream, int kind, size_t need, void** ptr, size_t* bytes) {
-  Scratch* found = nullptr;
-  for (Scratch& s : g_scratch)
-    if (s.stream == stream && s.kind == kind && s.device == device) {
+bool scratch_for(int device, int64_t stream, int kind, size_t need, Scratch* out) {
+  StreamScratch* found = nullptr;
+  for (StreamScratch& s : g_scratch)
+    if (s.stream == stream && s.device == device) {
       found = &s;
       break;
     }
-  if (found == nullptr || found->bytes < need) {
-    // (the Python side keeps the tensor alive)
+  if (found == nullptr) found = &g_scratch.emplace_back(device, stream);
+  if (found->bytes[kind] < need) {
     THPObjectPtr t(PyObject_CallFunction(g_make_workspace, "niLs", static_cast<Py_ssize_t>(need), device,
                                          static_cast<long long>(stream), kKindNames[kind]));
     if (!t) return false;
     const Tensor& ws = THPVariable_Unpack(t.get());
-    const Scratch s{device, stream, kind, ws.data_ptr(), static_cast<size_t>(ws.numel())};
-    found = nullptr;
-    for (Scratch& e : g_scratch)
-      if (e.stream == stream && e.kind == kind && e.device == device) found = &e;
-    if (found == nullptr) {
-      g_scratch.push_back(s);
-      found = &g_scratch.back();
-    } else {
-      *found = s;
-    }
+    found->ptr[kind] = ws.data_ptr();
+    found->bytes[kind] = static_cast<size_t>(ws.numel());
   }
-  *ptr = found->ptr;
-  *bytes = found->bytes;
+  *out = Scratch{found, found->ptr[kind], found->bytes[kind]};
   return true;
 }
 
@@ -92,12 +97,21 @@ const int32_t* i32(const Tensor& t) { return static_cast<const int32_t*>(t.data_
 
 // A call of the C ABI without the GIL: a launch waits when the stream's queue is full.  (Its error
 // message is per thread.)  The GIL is taken back however the call ends.
+struct NoGil {
+  PyThreadState* state = PyEval_SaveThread();
+  ~NoGil() { PyEval_RestoreThread(state); }
+};
 template <typename F>
 int unlocked(F&& call) {
-  struct NoGil {
-    PyThreadState* state = PyEval_SaveThread();
-    ~NoGil() { PyEval_RestoreThread(state); }
-  } no_gil;
+  NoGil no_gil;
+  return call();
+}
+// The same for a call whose launches share scratch: calls on one stream take turns.  (Waited for without the
+// GIL, which the thread whose turn it is wants back at its end.)
+template <typename F>
+int in_turn(const Scratch& ws, F&& call) {
+  NoGil no_gil;
+  std::lock_guard<std::mutex> turn(ws.of->launches);
   return call();
 }
 
@@ -198,18 +212,17 @@ PyObject* decode(PyObject*, PyObject* const* a, Py_ssize_t n) {
   ARG_FLOAT(scale, a[6]);
   ARG_INT(max_splits, a[7]);
   int64_t stream;
-  void* ws;
-  size_t ws_bytes;
+  Scratch ws;
   if (!stream_of(a[9], s.device, &stream) ||
       !scratch_for(s.device, stream, kDecode,
                    msgl_decode_workspace_bytes_full(s.n, s.hq, s.hkv, s.d, static_cast<int>(max_splits),
                                                     indices.numel()),
-                   &ws, &ws_bytes))
+                   &ws))
     return nullptr;
   Tensor out = empty_like_rows(q);
-  const int rc = unlocked([&] {
+  const int rc = in_turn(ws, [&] {
     return msgl_paged_decode_attention_sized(
-      q.data_ptr(), kc.data_ptr(), vc.data_ptr(), i32(indptr), i32(indices), gate, out.data_ptr(), ws, ws_bytes,
+      q.data_ptr(), kc.data_ptr(), vc.data_ptr(), i32(indptr), i32(indices), gate, out.data_ptr(), ws.ptr, ws.bytes,
       s.n, s.hq, s.hkv, s.d, s.num_slots, s.dtype, static_cast<float>(scale), static_cast<int>(max_splits),
       indices.numel(), reinterpret_cast<void*>(stream));
   });
@@ -240,15 +253,14 @@ PyObject* decode_paged(PyObject*, PyObject* const* a, Py_ssize_t n) {
                                         total_pages * page_size) + 255) / 256 * 256 +
       msgl_page_index_workspace_bytes(s.n, total_pages, static_cast<int>(page_size));
   int64_t stream;
-  void* ws;
-  size_t ws_bytes;
-  if (!stream_of(a[11], s.device, &stream) || !scratch_for(s.device, stream, kDecode, need, &ws, &ws_bytes))
+  Scratch ws;
+  if (!stream_of(a[11], s.device, &stream) || !scratch_for(s.device, stream, kDecode, need, &ws))
     return nullptr;
   Tensor out = empty_like_rows(q);
-  const int rc = unlocked([&] {
+  const int rc = in_turn(ws, [&] {
     return msgl_paged_decode_attention_p16(
       q.data_ptr(), kc.data_ptr(), vc.data_ptr(), i32(indptr), i32(pages), i32(lens), i32(splits), gate,
-      out.data_ptr(), ws, ws_bytes, s.n, s.hq, s.hkv, s.d, s.num_slots, s.dtype, static_cast<float>(scale),
+      out.data_ptr(), ws.ptr, ws.bytes, s.n, s.hq, s.hkv, s.d, s.num_slots, s.dtype, static_cast<float>(scale),
       static_cast<int>(max_splits), static_cast<int>(page_size), total_pages, reinterpret_cast<void*>(stream));
   });
   return rc ? raise_status(rc) : THPVariable_Wrap(std::move(out));
@@ -276,24 +288,23 @@ PyObject* prefill(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const int batch = static_cast<int>(prefix.numel());
   const int64_t total_kv = indices.numel();
   int64_t stream;
-  void* ws;
-  size_t ws_bytes;
+  Scratch ws;
   if (!stream_of(a[12], s.device, &stream) ||
       !scratch_for(s.device, stream, kPrefill,
                    msgl_prefill_workspace_bytes_full(batch, s.n, total_kv, s.hq, s.hkv, s.d,
                                                 static_cast<int>(max_ext), static_cast<int>(window)),
-                   &ws, &ws_bytes))
+                   &ws))
     return nullptr;
   Tensor out = empty_like_rows(q);
   void* st = reinterpret_cast<void*>(stream);
-  const int rc = unlocked([&] {
+  const int rc = in_turn(ws, [&] {
     return gate ? msgl_paged_prefill_attention_gated(q.data_ptr(), kc.data_ptr(), vc.data_ptr(), i32(qo), i32(indptr),
-                                                i32(indices), i32(prefix), gate, out.data_ptr(), ws, ws_bytes,
+                                                i32(indices), i32(prefix), gate, out.data_ptr(), ws.ptr, ws.bytes,
                                                 batch, s.n, total_kv, s.hq, s.hkv, s.d, s.num_slots, s.dtype,
                                                 static_cast<float>(scale), static_cast<int>(max_ext), cross,
                                                 static_cast<int>(window), st)
            : msgl_paged_prefill_attention(q.data_ptr(), kc.data_ptr(), vc.data_ptr(), i32(qo), i32(indptr),
-                                          i32(indices), i32(prefix), out.data_ptr(), ws, ws_bytes, batch, s.n,
+                                          i32(indices), i32(prefix), out.data_ptr(), ws.ptr, ws.bytes, batch, s.n,
                                           total_kv, s.hq, s.hkv, s.d, s.num_slots, s.dtype,
                                           static_cast<float>(scale), static_cast<int>(max_ext), cross,
                                           static_cast<int>(window), st);
@@ -327,20 +338,19 @@ PyObject* prefill_paged(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const int batch = static_cast<int>(prefix.numel());
   const int64_t total_pages = pages.numel();
   int64_t stream;
-  void* ws;
-  size_t ws_bytes;
+  Scratch ws;
   if (!stream_of(a[14], s.device, &stream) ||
       !scratch_for(s.device, stream, kPrefill,
                    msgl_prefill_workspace_bytes_p16(batch, s.n, total_pages, static_cast<int>(page_size), s.hq,
                                                     s.hkv, s.d, static_cast<int>(max_ext),
                                                     static_cast<int>(window)),
-                   &ws, &ws_bytes))
+                   &ws))
     return nullptr;
   Tensor out = empty_like_rows(q);
-  const int rc = unlocked([&] {
+  const int rc = in_turn(ws, [&] {
     return msgl_paged_prefill_attention_p16(
       q.data_ptr(), kc.data_ptr(), vc.data_ptr(), i32(qo), i32(indptr), i32(pages), i32(lens), i32(prefix), gate,
-      out.data_ptr(), ws, ws_bytes, batch, s.n, s.hq, s.hkv, s.d, s.num_slots, s.dtype, static_cast<float>(scale),
+      out.data_ptr(), ws.ptr, ws.bytes, batch, s.n, s.hq, s.hkv, s.d, s.num_slots, s.dtype, static_cast<float>(scale),
       static_cast<int>(max_ext), cross, static_cast<int>(window), static_cast<int>(page_size), total_pages,
       reinterpret_cast<void*>(stream));
   });
@@ -368,14 +378,13 @@ PyObject* store_kv(PyObject*, PyObject* const* a, Py_ssize_t n) {
       kc.stride(0) != vc.stride(0) || c10::cuda::current_device() != dev.index())
     Py_RETURN_NONE;
   int64_t stream;
-  void* ws;
-  size_t ws_bytes;
-  if (!stream_of(a[5], dev.index(), &stream) || !scratch_for(dev.index(), stream, kDecode, 256, &ws, &ws_bytes))
+  Scratch ws;
+  if (!stream_of(a[5], dev.index(), &stream) || !scratch_for(dev.index(), stream, kDecode, 256, &ws))
     return nullptr;
   const int rc = unlocked([&] {
     return msgl_store_kv_cache(kc.data_ptr(), vc.data_ptr(), i32(idx), k.data_ptr(), v.data_ptr(),
                                      static_cast<int>(len), static_cast<int>(hkv), static_cast<int>(d), kc.size(0),
-                                     kc.stride(0), k.stride(0), dt, ws, reinterpret_cast<void*>(stream));
+                                     kc.stride(0), k.stride(0), dt, ws.ptr, reinterpret_cast<void*>(stream));
   });
   if (rc) return raise_status(rc);
   Py_RETURN_TRUE;
@@ -503,18 +512,17 @@ PyObject* decode_layer(PyObject*, PyObject* const* a, Py_ssize_t n) {
   ARG_INT(page_size, a[12]);
   const int64_t total = indices.numel();
   int64_t stream;
-  void* ws;
-  size_t ws_bytes;
+  Scratch ws;
   if (!stream_of(Py_None, s.device, &stream) ||
       !scratch_for(s.device, stream, kDecode,
                    msgl_decode_workspace_bytes_full(s.n, s.hq, s.hkv, s.d, static_cast<int>(max_splits),
                                                     lens ? total * page_size : total),
-                   &ws, &ws_bytes))
+                   &ws))
     return nullptr;
   Tensor out = empty_like_rows(q);
-  const int rc = unlocked([&] {
+  const int rc = in_turn(ws, [&] {
     return msgl_decode_layer(&rows, q.data_ptr(), kc.data_ptr(), vc.data_ptr(), i32(indptr), i32(indices),
-                                   lens, gate, out.data_ptr(), ws, ws_bytes, s.n, s.hq, s.hkv, s.d, s.num_slots,
+                                   lens, gate, out.data_ptr(), ws.ptr, ws.bytes, s.n, s.hq, s.hkv, s.d, s.num_slots,
                                    s.dtype, static_cast<float>(scale), static_cast<int>(max_splits),
                                    static_cast<int>(page_size), total, reinterpret_cast<void*>(stream));
   });
@@ -556,20 +564,19 @@ PyObject* prefill_layer(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (cross < 0) return nullptr;
   const int64_t total = indices.numel();
   int64_t stream;
-  void* ws;
-  size_t ws_bytes;
+  Scratch ws;
   if (!stream_of(Py_None, s.device, &stream) ||
       !scratch_for(s.device, stream, kPrefill,
                    (lens ? msgl_prefill_workspace_bytes : msgl_prefill_workspace_bytes_full)(
                                                 batch, s.n, lens ? total * page_size : total, s.hq, s.hkv, s.d,
                                                 static_cast<int>(max_ext), static_cast<int>(window)),
-                   &ws, &ws_bytes))
+                   &ws))
     return nullptr;
   Tensor out = empty_like_rows(q);
-  const int rc = unlocked([&] {
+  const int rc = in_turn(ws, [&] {
     return msgl_prefill_layer(
       &rows, q.data_ptr(), kc.data_ptr(), vc.data_ptr(), i32(qo), i32(indptr), i32(indices), lens, i32(prefix), gate,
-      out.data_ptr(), ws, ws_bytes, batch, s.n, s.hq, s.hkv, s.d, s.num_slots, s.dtype, static_cast<float>(scale),
+      out.data_ptr(), ws.ptr, ws.bytes, batch, s.n, s.hq, s.hkv, s.d, s.num_slots, s.dtype, static_cast<float>(scale),
       static_cast<int>(max_ext), cross, static_cast<int>(window), static_cast<int>(page_size), total,
       reinterpret_cast<void*>(stream));
   });
@@ -690,9 +697,8 @@ PyObject* index_arrays(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (tq < 0 || tkv < 0 || tp < 0) Py_RETURN_NONE;
   const int dev = table.device().index();
   int64_t stream;
-  void* ws;
-  size_t ws_bytes;
-  if (!stream_of(a[9], dev, &stream) || !scratch_for(dev, stream, kDecode, 256, &ws, &ws_bytes)) return nullptr;
+  Scratch ws;
+  if (!stream_of(a[9], dev, &stream) || !scratch_for(dev, stream, kDecode, 256, &ws)) return nullptr;
   const bool paged = ps > 1;
   const int64_t size[9] = {batch + 1, batch + 1, batch, batch, tq, batch, per_token ? tkv : 0,
                            paged ? batch + 1 : 0, paged ? tp : 0};
@@ -710,7 +716,7 @@ PyObject* index_arrays(PyObject*, PyObject* const* a, Py_ssize_t n) {
       table.size(1), static_cast<int>(batch), static_cast<int>(ps), static_cast<int>(chunk),
       static_cast<int>(max_splits), tq, tkv, paged ? tp : 0, p + off[0], p + off[1], p + off[2], p + off[3],
       tq ? p + off[4] : nullptr, p + off[5], size[6] ? p + off[6] : nullptr, paged ? p + off[7] : nullptr,
-      size[8] ? p + off[8] : nullptr, ws, reinterpret_cast<void*>(stream));
+      size[8] ? p + off[8] : nullptr, ws.ptr, reinterpret_cast<void*>(stream));
   });
   if (rc) return raise_status(rc);
   THPObjectPtr out(PyTuple_New(9));
