@@ -217,13 +217,19 @@ size_t msgl_prefill_workspace_bytes(int batch, int total_q, int64_t total_kv, in
 size_t msgl_prefill_workspace_bytes_full(int batch, int total_q, int64_t total_kv, int num_q_heads,
                                          int num_kv_heads, int head_dim, int max_len_extend,
                                          int sliding_window_size);
+/* The part of it that those pages take, 0 where a call does not lay its rows out: msgl_prefill_layer_pages takes
+ * it as memory of its own, which belongs to the call alone and can go elsewhere once its launches are queued. */
+size_t msgl_prefill_kv_pages_bytes(int batch, int total_q, int64_t total_kv, int num_q_heads, int num_kv_heads,
+                                   int head_dim, int max_len_extend, int sliding_window_size);
 
 /*
  * Kernel launches one prefill call of this shape makes: 1, or 2 when the key
  * range is split and a (sequence, query tile, head) unit is too large for the
  * CTA that finishes last to merge (the merge is then a second launch, chained
- * to the first with programmatic stream serialization).  page_granular != 0
- * asks for the *_p16 entry points.  No counterpart in the reference.
+ * to the first with programmatic stream serialization), or when a call with
+ * per-token kv_indices lays its K/V rows out as pages first (given the memory
+ * of msgl_prefill_kv_pages_bytes; else 1).  page_granular != 0 asks for the
+ * *_p16 entry points.  No counterpart in the reference.
  */
 int msgl_prefill_launch_count(int batch, int total_q, int64_t total_kv, int num_q_heads,
                               int num_kv_heads, int head_dim, int max_len_extend,
@@ -461,6 +467,19 @@ int msgl_prefill_layer(const msgl_new_rows* rows, void* q, void* k_cache, void* 
                        int num_kv_heads, int head_dim, int64_t num_slots, int dtype, float sm_scale,
                        int max_len_extend, int is_cross_attention, int sliding_window_size,
                        int page_size, int64_t total, void* stream);
+
+/*
+ * msgl_prefill_layer with memory for the pages of a long call over per-token kv_indices
+ * (msgl_prefill_kv_pages_bytes; NULL: none but the workspace's).  rows NULL: nothing to store.
+ */
+int msgl_prefill_layer_pages(const msgl_new_rows* rows, void* q, void* k_cache, void* v_cache,
+                             const int32_t* qo_indptr, const int32_t* indptr, const int32_t* indices,
+                             const int32_t* kv_lens, const int32_t* prefix_lens, const void* gate, void* out,
+                             void* workspace, size_t workspace_bytes, void* kv_pages, size_t kv_pages_bytes,
+                             int batch, int total_q, int num_q_heads, int num_kv_heads, int head_dim,
+                             int64_t num_slots, int dtype, float sm_scale, int max_len_extend,
+                             int is_cross_attention, int sliding_window_size, int page_size, int64_t total,
+                             void* stream);
 
 #ifdef __cplusplus
 }

@@ -40,6 +40,7 @@ SIGNATURES = {
     "msgl_read_status": (_i, [_vp, _i, _vp, _vp]),
     "msgl_prefill_workspace_bytes": (_sz, [_i, _i, _i64, _i, _i, _i, _i, _i]),
     "msgl_prefill_workspace_bytes_full": (_sz, [_i, _i, _i64, _i, _i, _i, _i, _i]),
+    "msgl_prefill_kv_pages_bytes": (_sz, [_i, _i, _i64, _i, _i, _i, _i, _i]),
     "msgl_selftest_bounded_wait": (_i, [_vp, _i, _vp]),
     "msgl_prefill_launch_count": (_i, [_i, _i, _i64, _i, _i, _i, _i, _i, _i]),
     "msgl_page_index_workspace_bytes": (_sz, [_i, _i64, _i]),
@@ -65,6 +66,9 @@ SIGNATURES = {
     "msgl_prefill_layer": (
         _i, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _sz, _i, _i, _i, _i, _i, _i64, _i,
              _f, _i, _i, _i, _i, _i64, _vp]),
+    "msgl_prefill_layer_pages": (
+        _i, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _sz, _vp, _sz, _i, _i, _i, _i, _i,
+             _i64, _i, _f, _i, _i, _i, _i, _i64, _vp]),
     "msgl_store_kv_cache": (_i, [_vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i64, _i64, _i64, _i, _vp, _vp]),
     "msgl_gather_kv_indices": (_i, [_vp, _i64, _vp, _vp, _vp, _i, _i64, _i64, _i64, _vp, _vp]),
     "msgl_fast_compare_key": (_i64, [_vp, _vp, _i64, _i64, _i]),

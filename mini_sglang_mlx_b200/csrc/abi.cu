@@ -755,8 +755,9 @@ __global__ void __launch_bounds__(256) gather_rows_kernel(const GatherRowsParams
   }
 }
 
-// The scratch that takes: behind the header the K rows, the V rows, the page ids, and room for the pointer array and
-// the lengths of any batch.
+// The memory that takes: the K rows, the V rows, the page ids, and room for the pointer array and the lengths of any
+// batch.  It is the call's own (the host module takes it from torch's allocator and gives it back behind the launches): a
+// buffer kept per stream would hold up to 256 MiB for good on a device whose memory is the K/V pool's.
 constexpr size_t kGatherIndexBytes = 2 * 65537 * sizeof(int32_t) + 256;
 constexpr size_t kGatherBytesMax = 256u << 20;
 constexpr double kGatherWorth = 2.9;
@@ -1112,22 +1113,28 @@ int msgl_prefill_launch_count(int batch, int total_q, int64_t total_kv, int num_
                                       sms > 0 ? sms : 148);
   if (!page_granular && prefill_gathers(batch, total_q, total_kv, num_q_heads, num_kv_heads, head_dim, max_len_extend,
                                         sliding_window_size, pl.kv_chunk))
-    return 2;            // (with the scratch of msgl_prefill_workspace_bytes_full)
+    return 2;            // (given the memory of msgl_prefill_kv_pages_bytes)
   return (pl.kv_chunk > 0 && !pl.fused_merge) ? 2 : 1;
 }
 
-size_t msgl_prefill_workspace_bytes_full(int batch, int total_q, int64_t total_kv, int num_q_heads, int num_kv_heads,
-                                         int head_dim, int max_len_extend, int sliding_window_size) {
-  const size_t least = msgl_prefill_workspace_bytes(batch, total_q, total_kv, num_q_heads, num_kv_heads, head_dim,
-                                                    max_len_extend, sliding_window_size);
-  if (batch <= 0 || total_q <= 0 || num_q_heads <= 0 || num_kv_heads <= 0 || num_q_heads % num_kv_heads != 0) return least;
+size_t msgl_prefill_kv_pages_bytes(int batch, int total_q, int64_t total_kv, int num_q_heads, int num_kv_heads,
+                                   int head_dim, int max_len_extend, int sliding_window_size) {
+  if (batch <= 0 || total_q <= 0 || num_q_heads <= 0 || num_kv_heads <= 0 || num_q_heads % num_kv_heads != 0) return 0;
   const int sms = sm_count_cached();
   const PrefillPlan pl = plan_prefill(batch, total_q, total_kv, num_q_heads, num_kv_heads, head_dim, max_len_extend,
                                       sliding_window_size, sms > 0 ? sms : 148);
   if (!prefill_gathers(batch, total_q, total_kv, num_q_heads, num_kv_heads, head_dim, max_len_extend, sliding_window_size,
                        pl.kv_chunk))
-    return least;
-  return std::max(least, kStatusBytes + gather_bytes(batch, total_kv, num_kv_heads));
+    return 0;
+  return gather_bytes(batch, total_kv, num_kv_heads);
+}
+
+size_t msgl_prefill_workspace_bytes_full(int batch, int total_q, int64_t total_kv, int num_q_heads, int num_kv_heads,
+                                         int head_dim, int max_len_extend, int sliding_window_size) {
+  return std::max(msgl_prefill_workspace_bytes(batch, total_q, total_kv, num_q_heads, num_kv_heads, head_dim,
+                                               max_len_extend, sliding_window_size),
+                  kStatusBytes + msgl_prefill_kv_pages_bytes(batch, total_q, total_kv, num_q_heads, num_kv_heads, head_dim,
+                                                             max_len_extend, sliding_window_size));
 }
 
 static int prefill_impl(const void* q, const void* k_cache, const void* v_cache,
@@ -1137,7 +1144,8 @@ static int prefill_impl(const void* q, const void* k_cache, const void* v_cache,
                         int64_t total_kv, int num_q_heads, int num_kv_heads, int head_dim,
                         int64_t num_slots, int dtype, float sm_scale, int max_len_extend,
                         int is_cross_attention, int sliding_window_size, void* stream,
-                        const PageIndex* pages = nullptr, bool behind_store = false) {
+                        const PageIndex* pages = nullptr, bool behind_store = false, void* kv_pages = nullptr,
+                        size_t kv_pages_bytes = 0) {
   const char* op = "paged_prefill_attention: ";
   if (total_q < 0 || num_q_heads <= 0 || num_kv_heads <= 0 || num_slots < 0 || total_kv < 0)
     return fail(MSGL_BAD_SHAPE,
@@ -1159,7 +1167,7 @@ static int prefill_impl(const void* q, const void* k_cache, const void* v_cache,
       (!pages && (!kv_indptr || !kv_indices)))
     return fail(MSGL_BAD_ARG, std::string(op) + "null tensor pointer");
   if (!aligned16(q) || !aligned16(k_cache) || !aligned16(v_cache) || !aligned16(out) ||
-      !aligned16(gate) || !aligned16(workspace))
+      !aligned16(gate) || !aligned16(workspace) || !aligned16(kv_pages))
     return fail(MSGL_BAD_ARG, std::string(op) + "q, the pools, out, gate and the workspace must be "
                                                 "16-byte aligned");
   const int sms = sm_count_cached();
@@ -1170,16 +1178,20 @@ static int prefill_impl(const void* q, const void* k_cache, const void* v_cache,
   if (!workspace || workspace_bytes < need)
     return fail(MSGL_BAD_ARG, std::string(op) + "workspace too small");
   PageIndex laid_out;
+  if (!kv_pages) {   // (a call whose key range is not split uses no more than the header)
+    kv_pages = static_cast<unsigned char*>(workspace) + kStatusBytes;
+    kv_pages_bytes = workspace_bytes - kStatusBytes;
+  }
   if (!pages && num_slots > 0 &&
       prefill_gathers(batch, total_q, total_kv, num_q_heads, num_kv_heads, head_dim, max_len_extend, sliding_window_size,
                       pl.kv_chunk) &&
-      workspace_bytes >= kStatusBytes + gather_bytes(batch, total_kv, num_kv_heads)) {
-    // (the pool's tensor maps are kept by address and size: as many pages as the scratch holds, whatever the call)
+      kv_pages_bytes >= gather_bytes(batch, total_kv, num_kv_heads)) {
+    // (the pool's tensor maps are kept by address and size: as many pages as there is room for, whatever the call)
     GatherRowsParams g{};
-    const int64_t cap = static_cast<int64_t>((workspace_bytes - kStatusBytes - kGatherIndexBytes) / gather_page_bytes(num_kv_heads));
+    const int64_t cap = static_cast<int64_t>((kv_pages_bytes - kGatherIndexBytes) / gather_page_bytes(num_kv_heads));
     g.max_pages = static_cast<int>(std::min<int64_t>(cap, (1ll << 31) / msgl::kTmaBoxRows - 1));
     const size_t rows_bytes = static_cast<size_t>(g.max_pages) * msgl::kTmaBoxRows * num_kv_heads * head_dim * 2;
-    unsigned char* at = static_cast<unsigned char*>(workspace) + kStatusBytes;
+    unsigned char* at = static_cast<unsigned char*>(kv_pages);
     g.k_rows = at;
     g.v_rows = at + rows_bytes;
     g.page_indices = reinterpret_cast<int32_t*>(at + 2 * rows_bytes);
@@ -1852,6 +1864,33 @@ int msgl_decode_layer(const msgl_new_rows* rows, void* q, void* k_cache, void* v
                      rows->n_tokens > 0 ? rows : nullptr);
 }
 
+int msgl_prefill_layer_pages(const msgl_new_rows* rows, void* q, void* k_cache, void* v_cache,
+                             const int32_t* qo_indptr, const int32_t* indptr, const int32_t* indices,
+                             const int32_t* kv_lens, const int32_t* prefix_lens, const void* gate, void* out,
+                             void* workspace, size_t workspace_bytes, void* kv_pages, size_t kv_pages_bytes,
+                             int batch, int total_q, int num_q_heads, int num_kv_heads, int head_dim,
+                             int64_t num_slots, int dtype, float sm_scale, int max_len_extend,
+                             int is_cross_attention, int sliding_window_size, int page_size, int64_t total,
+                             void* stream) {
+  if (total < 0) return fail(MSGL_BAD_SHAPE, "paged_prefill_attention: negative size");
+  if (kv_lens && (page_size <= 0 || page_size % msgl::kTmaBoxRows != 0 || total * page_size >= (1ll << 31)))
+    return fail(MSGL_BAD_ARG, "paged_prefill_attention: page_size must be a multiple of 16, with fewer than 2^31 "
+                              "tokens in all pages");
+  if (kv_lens && batch > 0 && (!indptr || (total > 0 && !indices)))
+    return fail(MSGL_BAD_ARG, "paged_prefill_attention: null tensor pointer");
+  if (rows) {
+    const int rc = store_new_rows(rows, q, k_cache, v_cache, num_q_heads, num_kv_heads, head_dim, num_slots, dtype,
+                                  workspace, stream);
+    if (rc != MSGL_OK) return rc;
+  }
+  const PageIndex pages{indptr, indices, kv_lens, page_size};
+  return prefill_impl(q, k_cache, v_cache, qo_indptr, indptr, indices, prefix_lens, gate, out, workspace,
+                      workspace_bytes, batch, total_q, kv_lens ? total * page_size : total, num_q_heads,
+                      num_kv_heads, head_dim, num_slots, dtype, sm_scale, max_len_extend, is_cross_attention,
+                      sliding_window_size, stream, kv_lens ? &pages : nullptr, rows && rows->n_tokens > 0,
+                      kv_pages, kv_pages_bytes);
+}
+
 int msgl_prefill_layer(const msgl_new_rows* rows, void* q, void* k_cache, void* v_cache,
                        const int32_t* qo_indptr, const int32_t* indptr, const int32_t* indices,
                        const int32_t* kv_lens, const int32_t* prefix_lens, const void* gate, void* out,
@@ -1860,20 +1899,10 @@ int msgl_prefill_layer(const msgl_new_rows* rows, void* q, void* k_cache, void* 
                        int max_len_extend, int is_cross_attention, int sliding_window_size, int page_size,
                        int64_t total, void* stream) {
   if (!rows) return fail(MSGL_BAD_ARG, "paged_prefill_attention: null rows");
-  if (total < 0) return fail(MSGL_BAD_SHAPE, "paged_prefill_attention: negative size");
-  if (kv_lens && (page_size <= 0 || page_size % msgl::kTmaBoxRows != 0 || total * page_size >= (1ll << 31)))
-    return fail(MSGL_BAD_ARG, "paged_prefill_attention: page_size must be a multiple of 16, with fewer than 2^31 "
-                              "tokens in all pages");
-  if (kv_lens && batch > 0 && (!indptr || (total > 0 && !indices)))
-    return fail(MSGL_BAD_ARG, "paged_prefill_attention: null tensor pointer");
-  const int rc = store_new_rows(rows, q, k_cache, v_cache, num_q_heads, num_kv_heads, head_dim, num_slots, dtype,
-                                workspace, stream);
-  if (rc != MSGL_OK) return rc;
-  const PageIndex pages{indptr, indices, kv_lens, page_size};
-  return prefill_impl(q, k_cache, v_cache, qo_indptr, indptr, indices, prefix_lens, gate, out, workspace,
-                      workspace_bytes, batch, total_q, kv_lens ? total * page_size : total, num_q_heads,
-                      num_kv_heads, head_dim, num_slots, dtype, sm_scale, max_len_extend, is_cross_attention,
-                      sliding_window_size, stream, kv_lens ? &pages : nullptr, rows->n_tokens > 0);
+  return msgl_prefill_layer_pages(rows, q, k_cache, v_cache, qo_indptr, indptr, indices, kv_lens, prefix_lens, gate, out,
+                                  workspace, workspace_bytes, nullptr, 0, batch, total_q, num_q_heads, num_kv_heads,
+                                  head_dim, num_slots, dtype, sm_scale, max_len_extend, is_cross_attention,
+                                  sliding_window_size, page_size, total, stream);
 }
 
 }  // extern "C"

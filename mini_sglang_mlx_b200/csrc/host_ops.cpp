@@ -53,6 +53,7 @@ struct StreamScratch {
 // guarded by the GIL, but for `launches`; entries keep their place and are never destroyed (a thread may hold one at exit)
 std::deque<StreamScratch>& g_scratch = *new std::deque<StreamScratch>;
 PyObject* g_make_workspace = nullptr;  // Python: (nbytes, device index, stream handle, kind) -> tensor
+PyObject* g_make_pages = nullptr;      // Python: (nbytes, device index, stream handle) -> tensor or None
 
 // The scratch a call got: it stays valid when the stream's scratch grows meanwhile (the Python side keeps
 // outgrown buffers).
@@ -79,6 +80,25 @@ bool scratch_for(int device, int64_t stream, int kind, size_t need, Scratch* out
     found->bytes[kind] = static_cast<size_t>(ws.numel());
   }
   *out = Scratch{found, found->ptr[kind], found->bytes[kind]};
+  return true;
+}
+
+// Memory of one call for the pages of its K/V rows, asked for after the call's output and given back when the call
+// has queued its launches.  Without it (no memory, or none made) the attention kernel gathers the rows itself.
+struct Pages {
+  THPObjectPtr tensor;
+  void* ptr = nullptr;
+  size_t bytes = 0;
+};
+bool pages_for(int device, int64_t stream, size_t bytes, Pages* out) {
+  if (bytes == 0 || g_make_pages == nullptr) return true;
+  out->tensor = PyObject_CallFunction(g_make_pages, "niL", static_cast<Py_ssize_t>(bytes), device,
+                                      static_cast<long long>(stream));
+  if (!out->tensor) return false;
+  if (out->tensor.get() == Py_None) return true;
+  const Tensor& t = THPVariable_Unpack(out->tensor.get());
+  out->ptr = t.data_ptr();
+  out->bytes = static_cast<size_t>(t.numel());
   return true;
 }
 
@@ -289,25 +309,25 @@ PyObject* prefill(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const int64_t total_kv = indices.numel();
   int64_t stream;
   Scratch ws;
+  Pages pages;
   if (!stream_of(a[12], s.device, &stream) ||
       !scratch_for(s.device, stream, kPrefill,
-                   msgl_prefill_workspace_bytes_full(batch, s.n, total_kv, s.hq, s.hkv, s.d,
-                                                static_cast<int>(max_ext), static_cast<int>(window)),
+                   msgl_prefill_workspace_bytes(batch, s.n, total_kv, s.hq, s.hkv, s.d, static_cast<int>(max_ext),
+                                                static_cast<int>(window)),
                    &ws))
     return nullptr;
   Tensor out = empty_like_rows(q);
-  void* st = reinterpret_cast<void*>(stream);
+  if (!pages_for(s.device, stream,
+                 msgl_prefill_kv_pages_bytes(batch, s.n, total_kv, s.hq, s.hkv, s.d, static_cast<int>(max_ext),
+                                             static_cast<int>(window)),
+                 &pages))
+    return nullptr;
   const int rc = in_turn(ws, [&] {
-    return gate ? msgl_paged_prefill_attention_gated(q.data_ptr(), kc.data_ptr(), vc.data_ptr(), i32(qo), i32(indptr),
-                                                i32(indices), i32(prefix), gate, out.data_ptr(), ws.ptr, ws.bytes,
-                                                batch, s.n, total_kv, s.hq, s.hkv, s.d, s.num_slots, s.dtype,
-                                                static_cast<float>(scale), static_cast<int>(max_ext), cross,
-                                                static_cast<int>(window), st)
-           : msgl_paged_prefill_attention(q.data_ptr(), kc.data_ptr(), vc.data_ptr(), i32(qo), i32(indptr),
-                                          i32(indices), i32(prefix), out.data_ptr(), ws.ptr, ws.bytes, batch, s.n,
-                                          total_kv, s.hq, s.hkv, s.d, s.num_slots, s.dtype,
-                                          static_cast<float>(scale), static_cast<int>(max_ext), cross,
-                                          static_cast<int>(window), st);
+    return msgl_prefill_layer_pages(
+      nullptr, q.data_ptr(), kc.data_ptr(), vc.data_ptr(), i32(qo), i32(indptr), i32(indices), nullptr, i32(prefix),
+      gate, out.data_ptr(), ws.ptr, ws.bytes, pages.ptr, pages.bytes, batch, s.n, s.hq, s.hkv, s.d, s.num_slots,
+      s.dtype, static_cast<float>(scale), static_cast<int>(max_ext), cross, static_cast<int>(window), 1, total_kv,
+      reinterpret_cast<void*>(stream));
   });
   return rc ? raise_status(rc) : THPVariable_Wrap(std::move(out));
 }
@@ -565,20 +585,26 @@ PyObject* prefill_layer(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const int64_t total = indices.numel();
   int64_t stream;
   Scratch ws;
+  Pages pages;
+  const int64_t tokens = lens ? total * page_size : total;
   if (!stream_of(Py_None, s.device, &stream) ||
       !scratch_for(s.device, stream, kPrefill,
-                   (lens ? msgl_prefill_workspace_bytes : msgl_prefill_workspace_bytes_full)(
-                                                batch, s.n, lens ? total * page_size : total, s.hq, s.hkv, s.d,
-                                                static_cast<int>(max_ext), static_cast<int>(window)),
+                   msgl_prefill_workspace_bytes(batch, s.n, tokens, s.hq, s.hkv, s.d, static_cast<int>(max_ext),
+                                                static_cast<int>(window)),
                    &ws))
     return nullptr;
   Tensor out = empty_like_rows(q);
+  if (!pages_for(s.device, stream,
+                 lens ? 0 : msgl_prefill_kv_pages_bytes(batch, s.n, tokens, s.hq, s.hkv, s.d, static_cast<int>(max_ext),
+                                                        static_cast<int>(window)),
+                 &pages))
+    return nullptr;
   const int rc = in_turn(ws, [&] {
-    return msgl_prefill_layer(
+    return msgl_prefill_layer_pages(
       &rows, q.data_ptr(), kc.data_ptr(), vc.data_ptr(), i32(qo), i32(indptr), i32(indices), lens, i32(prefix), gate,
-      out.data_ptr(), ws.ptr, ws.bytes, batch, s.n, s.hq, s.hkv, s.d, s.num_slots, s.dtype, static_cast<float>(scale),
-      static_cast<int>(max_ext), cross, static_cast<int>(window), static_cast<int>(page_size), total,
-      reinterpret_cast<void*>(stream));
+      out.data_ptr(), ws.ptr, ws.bytes, pages.ptr, pages.bytes, batch, s.n, s.hq, s.hkv, s.d, s.num_slots, s.dtype,
+      static_cast<float>(scale), static_cast<int>(max_ext), cross, static_cast<int>(window),
+      static_cast<int>(page_size), total, reinterpret_cast<void*>(stream));
   });
   return rc ? raise_status(rc) : THPVariable_Wrap(std::move(out));
 }
@@ -735,11 +761,12 @@ PyObject* index_arrays(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return out.release();
 }
 
-// (callable): how scratch is made, see g_make_workspace
-PyObject* set_workspace_maker(PyObject*, PyObject* fn) {
+// (callable): how scratch is made, see g_make_workspace and g_make_pages
+template <PyObject** MAKER>
+PyObject* set_maker(PyObject*, PyObject* fn) {
   Py_INCREF(fn);
-  Py_XDECREF(g_make_workspace);
-  g_make_workspace = fn;
+  Py_XDECREF(*MAKER);
+  *MAKER = fn;
   Py_RETURN_NONE;
 }
 
@@ -749,7 +776,8 @@ PyMethodDef kMethods[] = {FAST(decode),       FAST(decode_paged),       FAST(pre
                           FAST(prefill_paged), FAST(store_kv),          FAST(qk_norm_rope_store),
                           FAST(decode_layer), FAST(prefill_layer),     FAST(collect_lens),
                           FAST(index_arrays),
-                          {"set_workspace_maker", set_workspace_maker, METH_O, nullptr},
+                          {"set_workspace_maker", set_maker<&g_make_workspace>, METH_O, nullptr},
+                          {"set_pages_maker", set_maker<&g_make_pages>, METH_O, nullptr},
                           {nullptr, nullptr, 0, nullptr}};
 PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_host", "Host side of the operators.", -1, kMethods,
                        nullptr, nullptr, nullptr, nullptr};

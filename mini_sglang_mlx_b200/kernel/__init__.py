@@ -88,9 +88,13 @@ def _workspace(nbytes: int, device: torch.device, stream_handle: int, kind: str)
             # ordered before them even when that stream is not torch's current one
             with torch.cuda.stream(torch.cuda.ExternalStream(stream_handle, device=device)):
                 # (a power of two: the need of a decode batch grows with its tokens, and the outgrown
-                # buffers of a doubling series together stay below the buffer in use)
+                # buffers of a doubling series together stay below the buffer in use; as it is where
+                # that finds no memory)
                 size = 1 << (max(nbytes, 1 << 20) - 1).bit_length()
-                grown = torch.zeros(size, dtype=torch.uint8, device=device)
+                try:
+                    grown = torch.zeros(size, dtype=torch.uint8, device=device)
+                except torch.OutOfMemoryError:
+                    grown = torch.zeros(nbytes, dtype=torch.uint8, device=device)
             if ws is not None:
                 _retired.append(ws)
             _workspaces[key] = ws = grown
@@ -101,12 +105,38 @@ def _make_workspace(nbytes: int, index: int, stream_handle: int, kind: str) -> t
     return _workspace(nbytes, torch.device("cuda", index), stream_handle, kind)
 
 
+# Calls of a device that are not asked for page memory after one that found none: an attempt that
+# fails makes torch wait for the device and give its cached blocks back, so it is not made in every layer.
+_PAGES_PAUSE = 256
+_pages_pause: Dict[int, int] = {}
+
+
+def _make_pages(nbytes: int, index: int, stream_handle: int) -> Optional[torch.Tensor]:
+    """Memory for the K/V rows that one long prefill over per-token slots lays out as pages, or None where
+    the device has none left (a pool may fill it): the call then gathers the rows as it goes.  Of the call's
+    stream, so that it can be given back as soon as the launches are queued."""
+    pause = _pages_pause.get(index, 0)
+    if pause > 0:
+        _pages_pause[index] = pause - 1
+        return None
+    device = torch.device("cuda", index)
+    try:
+        if _stream_handle(None, device) == stream_handle:
+            return torch.empty(nbytes, dtype=torch.uint8, device=device)
+        with torch.cuda.stream(torch.cuda.ExternalStream(stream_handle, device=device)):
+            return torch.empty(nbytes, dtype=torch.uint8, device=device)
+    except torch.OutOfMemoryError:
+        _pages_pause[index] = _PAGES_PAUSE
+        return None
+
+
 class _HostOps:
     """The native operators (``csrc/host_ops.cpp``), told at their first use how scratch is made."""
 
     def __getattr__(self, name):
         fn = getattr(_lib.host, name)
         _lib.host.set_workspace_maker(_make_workspace)
+        _lib.host.set_pages_maker(_make_pages)
         setattr(self, name, fn)
         return fn
 

@@ -40,8 +40,11 @@ inline CUDAStream getCurrentCUDAStream(int) { return {}; }
 RECORDER = """
 #include <unistd.h>
 #include <atomic>
+#include <cstddef>
 #include <cstdint>
 namespace {
+size_t g_workspace, g_pages;
+bool g_have_pages;
 std::atomic<int> g_next{0}, g_at{0};
 int g_log[4096];
 int note() {
@@ -61,7 +64,19 @@ ENTRY(msgl_paged_prefill_attention)
 ENTRY(msgl_paged_prefill_attention_gated)
 ENTRY(msgl_paged_prefill_attention_p16)
 ENTRY(msgl_decode_layer)
-ENTRY(msgl_prefill_layer)
+// 5 MB of pages for every call of more than 100 query tokens
+size_t msgl_prefill_kv_pages_bytes(int, int total_q, int64_t, int, int, int, int, int) {
+  return total_q > 100 ? 5000000 : 0;
+}
+int msgl_prefill_layer_pages(const void*, void*, void*, void*, const void*, const void*, const void*, const void*,
+                             const void*, const void*, void*, void*, size_t workspace, void* pages, size_t bytes) {
+  g_workspace = workspace;
+  g_have_pages = pages != nullptr;
+  g_pages = bytes;
+  return note();
+}
+size_t last_workspace() { return g_workspace; }
+size_t last_pages() { return g_have_pages ? g_pages : 0; }
 }
 """
 
@@ -79,14 +94,16 @@ def host(tmp_path_factory):
     cmd[cmd.index("-O2")] = "-O0"
     first = next(i for i, a in enumerate(cmd) if a.startswith("-I"))
     cmd[first:first] = [f"-I{at}", "-include", str(at / "on_cpu.h")]
-    recorder = at / "recorder.o"
+    entries = at / "recorder.o"
     subprocess.run([shutil.which("g++") or "g++", "-std=c++17", "-fPIC", "-c", str(at / "recorder.cpp"), "-o",
-                    str(recorder)], check=True)
-    subprocess.run([*cmd, str(recorder), "-Wl,-Bsymbolic", f"-Wl,-rpath,{B.PKG_DIR}", "-o", str(lib)], check=True)
+                    str(entries)], check=True)
+    subprocess.run([*cmd, str(entries), "-Wl,-Bsymbolic", f"-Wl,-rpath,{B.PKG_DIR}", "-o", str(lib)], check=True)
     loader = importlib.machinery.ExtensionFileLoader("_host", str(lib))
     module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_host", loader))
     loader.exec_module(module)
-    return module, ctypes.CDLL(str(lib))
+    recorder = ctypes.CDLL(str(lib))
+    recorder.last_workspace.restype = recorder.last_pages.restype = ctypes.c_size_t
+    return module, recorder
 
 
 def _calls(m):
@@ -133,6 +150,48 @@ def test_calls_on_one_stream_queue_their_launches_in_turn(host):
     seen = [log.recorded(i) for i in range(2 * n)]
     assert sorted(seen) == sorted([*range(1, n + 1), *range(-n, 0)])
     assert all(seen[i] > 0 and seen[i + 1] == -seen[i] for i in range(0, 2 * n, 2)), seen
+
+
+@pytest.mark.parametrize("layer", [False, True], ids=["operator", "layer"])
+def test_a_long_prefill_goes_without_page_memory_that_nobody_has(host, monkeypatch, layer):
+    """The rows' pages are memory of the call's own: the scratch that stays is the least one, and where the
+    pages find no memory the call runs without them (and the next ones do not ask again)."""
+    from mini_sglang_mlx_b200 import kernel as K
+    m, log = host
+    asked, kept = [], []
+
+    def workspace(nbytes, index, stream, kind):
+        kept.append(nbytes)
+        return torch.zeros(nbytes, dtype=torch.uint8)
+
+    m.set_workspace_maker(workspace)
+    n = 200
+    q, kc, k = torch.zeros(n, 2, 128).bfloat16(), torch.zeros(64, 1, 128).bfloat16(), torch.zeros(1, 1, 128).bfloat16()
+    two, one = torch.zeros(2, dtype=torch.int32), torch.zeros(1, dtype=torch.int32)
+
+    def call():
+        if layer:
+            return m.prefill_layer(q, k, k, kc, kc, one, None, two, two, two, None, one, 0.1, n, 1, False, 0, None)
+        return m.prefill(q, kc, kc, two, two, two, one, 0.1, n, False, 0, None, 7)
+
+    m.set_pages_maker(lambda nbytes, index, stream: asked.append(nbytes) or torch.empty(nbytes, dtype=torch.uint8))
+    assert isinstance(call(), torch.Tensor) and asked == [5000000] and log.last_pages() == 5000000
+    assert sum(kept) < 1000000 and log.last_workspace() < 1000000
+
+    def none_left(*a, **kw):
+        asked.append(a)
+        raise torch.OutOfMemoryError("no memory")
+
+    monkeypatch.setattr(torch, "empty", none_left)
+    monkeypatch.setattr(K, "_stream_handle", lambda stream, device: 7)
+    monkeypatch.setattr(K, "_pages_pause", {})
+    m.set_pages_maker(lambda nbytes, index, stream: K._make_pages(nbytes, 0, stream))
+    asked.clear()
+    for _ in range(K._PAGES_PAUSE + 1):
+        assert K._make_pages(100, 0, 7) is None
+    assert len(asked) == 1
+    for asks in (2, 2):
+        assert isinstance(call(), torch.Tensor) and len(asked) == asks and log.last_pages() == 0
 
 
 def test_calls_on_other_streams_do_not_wait(host):

@@ -58,6 +58,18 @@ def test_growth_that_finds_no_memory_leaves_the_buffer_in_use(host_scratch, monk
     assert grown.numel() == 2 * first.numel() and K._retired == [first]
 
 
+def test_growth_asks_for_what_it_needs_where_a_power_of_two_finds_no_memory(host_scratch, monkeypatch):
+    dev, real, limit = torch.device("cuda", 0), torch.zeros, (1 << 20) + 5000
+
+    def small(n, *a, **k):
+        if n > limit:
+            raise torch.OutOfMemoryError("no memory")
+        return real(n, *a, **k)
+
+    monkeypatch.setattr(torch, "zeros", small)
+    assert K._workspace((1 << 20) + 4096, dev, 7, "prefill").numel() == (1 << 20) + 4096
+
+
 def test_a_report_from_before_a_buffer_grew_is_not_lost(host_scratch, monkeypatch):
     monkeypatch.setattr(torch.cuda, "synchronize", lambda device=None: None)
     dev = torch.device("cuda", 0)
@@ -96,3 +108,49 @@ def test_decode_with_the_least_scratch_that_a_call_takes(kv_lens, max_splits):
             torch.cuda.current_stream().cuda_stream))
         assert_close_to_oracle(out, O.paged_decode_attention_oracle(q, kc, vc, kvp, slots, sc))
     assert int(ws[:65792].sum()) == 0 and bool((ws[need:] == 255).all())
+
+
+@pytest.mark.gpu
+def test_a_long_prefill_over_token_slots_keeps_no_memory_and_does_without(monkeypatch):
+    """Its K/V rows are laid out as pages in memory of the call's own, given back behind it; on a device
+    without room for them it gathers the rows as it goes."""
+    import math
+
+    from mini_sglang_mlx_b200 import _lib
+    from oracle import paged_attention_oracle as O
+    from tests.helpers import assert_close_to_oracle
+    from tests.test_page_granular_gpu import make_pool
+    n, hkv, hq, d = 2300, 4, 32, 128
+    kc, vc, _, _, slots = make_pool([n], 16, hkv, seed=4, d=d)
+    q = torch.randn(n, hq, d, generator=torch.Generator().manual_seed(4)).bfloat16().cuda()
+    ends, prefix = torch.tensor([0, n], dtype=torch.int32, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+    pages = _lib.lib().msgl_prefill_kv_pages_bytes(1, n, n, hq, hkv, d, n, 0)
+    assert pages > 1 << 20
+    monkeypatch.setattr(K, "_pages_pause", {})
+
+    def call():
+        return K.paged_prefill_attention(q, kc, vc, ends, ends, slots, prefix, 1 / math.sqrt(d), n)
+
+    out = call()
+    held = torch.cuda.memory_allocated()
+    again = call()
+    assert torch.cuda.memory_allocated() - held <= 2 * again.numel() + 512 and K._pages_pause == {}
+    assert torch.equal(out, again)
+    del again
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    room, hold = torch.empty(2 * out.numel(), dtype=torch.uint8, device="cuda"), []
+    total = torch.cuda.get_device_properties(0).total_memory
+    try:
+        torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + (64 << 20)) / total)
+        with pytest.raises(torch.OutOfMemoryError):
+            for _ in range(1000):
+                hold.append(torch.empty(pages - 4096, dtype=torch.uint8, device="cuda"))
+        del room                               # (room for the output)
+        without = call()
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    assert K._pages_pause == {0: K._PAGES_PAUSE}
+    ref = O.paged_prefill_attention_oracle(q, kc, vc, ends, ends, slots, prefix, 1 / math.sqrt(d))
+    assert_close_to_oracle(out, ref, "laid out")
+    assert_close_to_oracle(without, ref, "gathered")
