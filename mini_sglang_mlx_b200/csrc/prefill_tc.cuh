@@ -636,7 +636,7 @@ __global__ void __launch_bounds__(TcShape<NSUB, HD, PAGED>::kThreads,
     // The first page / slot ids are on their way before the wait, Q and the tiles behind it.
     auto load_q = [&]() {
     if (p.early) grid_dependency_wait();
-    if (ntiles == 0) return;      // (the epilogue's zeros are staged where Q would land)
+    if (NSUB == 1 && ntiles == 0) return;      // (the epilogue's zeros are staged where Q would land)
     if (q_tma) {
       // Q: one box per sub-tile and 64-element column block.  The tensor map is
       // (head_dim, query heads, tokens) with a box of 64 x G x 128/G, so the rows land in
@@ -1088,7 +1088,12 @@ __global__ void __launch_bounds__(TcShape<NSUB, HD, PAGED>::kThreads,
 #ifdef MSGL_TRACE
     if (tid == 0) MSGL_TR(6, clock64());               // last P handed over
 #endif
-    // ---- epilogue
+    // ---- epilogue.  Of two sub-tiles the first can be without key tiles where the second has some: its zero rows are
+    // staged where its Q lands, so behind Q.  (Q is loaded there whatever the tiles: with a branch in front of it the
+    // per-token form's copying warps took 1 to 5 % longer for their loop, 81 to 331 tokens over up to 11644 of seven
+    // sequences 876 us against 836; with one sub-tile the branch costs nothing, and without it twelve-token verify blocks
+    // took 211 us for 209.)
+    if (NSUB == 2 && my_tiles == 0) alive = mbar_wait_warp(bar_q, 0, abort_flag);
     if (alive && my_tiles > 0) {
       alive = mbar_wait_warp(bar_pv(i, (my_tiles - 1) % LA), ((my_tiles - 1) / LA) & 1, abort_flag);
       if (alive) tc_fence_after();

@@ -199,3 +199,35 @@ def test_long_prefill_over_per_token_slots(hkv, hq, q_lens, prefixes, kw, dtype)
     kz, vz = torch.cat([kc, torch.zeros_like(kc[:1])]), torch.cat([vc, torch.zeros_like(vc[:1])])
     zeros = torch.where((bad < 0) | (bad >= kc.shape[0]), kc.shape[0], bad)
     assert_close_to_oracle(out, O.paged_prefill_attention_oracle(q, kz, vz, qo, kvp, zeros, pre, sc, **kw), "zeros")
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("hkv,hq,q_lens,prefixes,launches", [
+    (2, 8, [64], [4 * 1024 - 40], 2), (2, 12, [43, 86], [3 * 1024 - 20, 1024 - 70], 2), (1, 8, [16], [2 * 1024 - 9], 2),
+    (2, 8, [300, 131, 217] * 12, [-300, 5, -217] * 6 + [0, -131, 40] * 6, 1)], ids=lambda x: str(x)[:30])
+def test_sub_tiles_without_keys(hkv, hq, q_lens, prefixes, launches, dtype):
+    """Key ranges cut inside the new tokens, so that the first rows of an item have no key in a piece and the last ones
+    do, and sequences without any key: zero rows and empty partials are staged where the queries land."""
+    from mini_sglang_mlx_b200 import _lib, paged_prefill_attention, paged_prefill_attention_p16
+    d, n = 128, max(q_lens)
+    kv_lens = [a + b for a, b in zip(q_lens, prefixes)]
+    kc, vc, pip, pidx, slots = make_pool([max(x, 1) for x in kv_lens], 16, hkv, seed=hq, d=d, dtype=dtype)
+    keep, at = [], 0
+    for x in kv_lens:
+        keep.append(slots[at:at + x])
+        at += max(x, 1)
+    slots, q = torch.cat(keep), torch.randn(sum(q_lens), hq, d, generator=torch.Generator().manual_seed(hq)).to(dtype).cuda()
+    shape = (len(q_lens), sum(q_lens), sum(kv_lens), hq, hkv, d, n, 0)
+    assert _lib.lib().msgl_prefill_launch_count(*shape, 0) == launches
+    qo, kvp, pre = (_i32(x) for x in (O.build_indptr(q_lens).tolist(), O.build_indptr(kv_lens).tolist(),
+                                      [max(x, 0) for x in prefixes]))
+    sc = 1 / math.sqrt(d)
+    ref = O.paged_prefill_attention_oracle(q, kc, vc, qo, kvp, slots, pre, sc)
+    out = paged_prefill_attention(q, kc, vc, qo, kvp, slots, pre, sc, n)
+    assert_close_to_oracle(out, ref, "slots")
+    paged = paged_prefill_attention_p16(q, kc, vc, qo, pip, pidx, _i32(kv_lens), pre, sc, n, page_size=16)
+    assert_close_to_oracle(paged, ref, "pages")
+    for b, x in enumerate(kv_lens):
+        if x == 0:
+            rows = slice(sum(q_lens[:b]), sum(q_lens[:b + 1]))
+            assert not out[rows].any() and not paged[rows].any()
