@@ -538,10 +538,7 @@ __global__ void __launch_bounds__(TcShape<NSUB, HD, PAGED>::kThreads,
   }
 
   if (!p.early) grid_dependency_wait();
-  // (The two-sub-tile shape is at its register limit: with these the tile loop of its page-granular form takes 2 %
-  // longer, 512 tokens over 32768 282 -> 288 us, so that one keeps the general search and its divisions.)
-  constexpr bool kGeneral = NSUB == 2 && PAGED;
-  const bool by_warp = !kGeneral && p.batch <= kWarpBatchMax;
+  const bool by_warp = p.batch <= kWarpBatchMax;
   if (by_warp) {
     if (warp == 0) find_item_warp(p, static_cast<int>(blockIdx.x), BM, &found);
   } else {
@@ -552,7 +549,7 @@ __global__ void __launch_bounds__(TcShape<NSUB, HD, PAGED>::kThreads,
       found.have = have;
       if (have) {
         found.at = at;
-        if (!kGeneral) found.seq = load_seq_shape(p, at.b, BM);
+        found.seq = load_seq_shape(p, at.b, BM);
       }
     }
   }
@@ -569,7 +566,7 @@ __global__ void __launch_bounds__(TcShape<NSUB, HD, PAGED>::kThreads,
   }
   const ItemCoord it = found.at;
   const int h = it.h;
-  const SeqShape sq = kGeneral ? load_seq_shape(p, it.b, BM) : found.seq;
+  const SeqShape sq = found.seq;
   const int qt = it.qt, split = it.split;
   const int slot_item = it.base + qt * sq.nsplit + split;   // where this item's kv-split partial goes
   auto over_group = [&](int x) { return NSUB == 2 ? x / G : divide_by(x, p.group_recip); };
@@ -633,7 +630,11 @@ __global__ void __launch_bounds__(TcShape<NSUB, HD, PAGED>::kThreads,
     const int64_t slot_stride = static_cast<int64_t>(p.hkv) * (HD * 2);
     const int64_t head_off = static_cast<int64_t>(h) * (HD * 2);
 
-    // The first page / slot ids are on their way before the wait, Q and the tiles behind it.
+    // The first page / slot ids are on their way before the wait, Q and the tiles behind it.  In the two-sub-tile
+    // page-granular form Q goes first, and the gate is applied an element at a time: that shape is at its register
+    // limit, and its tile loop moves with what is around it (us with ids first and the gate by pairs / this way: 512 tokens
+    // over 32768 286 / 274, 128 over 2048 39.6 / 37.9, twelve prompts of 500 398 / 394).
+    constexpr bool kQFirst = NSUB == 2 && PAGED;
     auto load_q = [&]() {
     if (p.early) grid_dependency_wait();
     if (NSUB == 1 && ntiles == 0) return;      // (the epilogue's zeros are staged where Q would land)
@@ -670,7 +671,7 @@ __global__ void __launch_bounds__(TcShape<NSUB, HD, PAGED>::kThreads,
     }
     };
 
-    if constexpr (kGeneral) load_q();
+    if constexpr (kQFirst) load_q();
     bool alive = true;
     if constexpr (PAGED) {
       // ------------------------------------------------ page-granular: TMA boxes from the page ids
@@ -698,7 +699,7 @@ __global__ void __launch_bounds__(TcShape<NSUB, HD, PAGED>::kThreads,
           n = 0;
           const int t0 = kv_lo + tile * BN + lane * kTmaBoxRows;
           if (lane < PPT && tile < ntiles && t0 < kv_hi_load) {
-            const int page = kGeneral ? t0 / p.page_size : divide_by(t0, p.page_recip);
+            const int page = divide_by(t0, p.page_recip);
             const int pg = __ldg(pages + page);
             const int64_t row0 = static_cast<int64_t>(pg) * p.page_size + (t0 - page * p.page_size);
             const int nv = min(kTmaBoxRows, sq.L - t0);
@@ -764,7 +765,7 @@ __global__ void __launch_bounds__(TcShape<NSUB, HD, PAGED>::kThreads,
         int wy[LA + 1], wn[LA + 1];
 #pragma unroll
         for (int t = 0; t <= LA; ++t) fetch_box(t, wy[t], wn[t]);
-        if constexpr (!kGeneral) load_q();
+        if constexpr (!kQFirst) load_q();
 #pragma unroll
         for (int t = 0; t < LA; ++t)
           if (t < ntiles && alive) produce(ring_seq_k<LA>(t), &tm_k, kbase, wy[t], wn[t]);
@@ -1148,7 +1149,7 @@ __global__ void __launch_bounds__(TcShape<NSUB, HD, PAGED>::kThreads,
                 const T* grow = static_cast<const T*>(p.gate) + (dst - static_cast<T*>(p.out));
                 const uint4 gv = *reinterpret_cast<const uint4*>(
                     reinterpret_cast<const unsigned char*>(grow) + chunk * 16);
-                if constexpr (kGeneral) {
+                if constexpr (NSUB == 2 && PAGED) {   // (see kQFirst)
                   T* wo = reinterpret_cast<T*>(&w);
                   const T* wg = reinterpret_cast<const T*>(&gv);
 #pragma unroll
