@@ -760,7 +760,7 @@ __global__ void __launch_bounds__(256) gather_rows_kernel(const GatherRowsParams
 // buffer kept per stream would hold up to 256 MiB for good on a device whose memory is the K/V pool's.
 constexpr size_t kGatherIndexBytes = 2 * 65537 * sizeof(int32_t) + 256;
 constexpr size_t kGatherBytesMax = 256u << 20;
-constexpr double kGatherWorth = 2.9;
+constexpr double kGatherWorth = 3.0;
 size_t gather_page_bytes(int num_kv_heads) {
   return static_cast<size_t>(msgl::kTmaBoxRows) * num_kv_heads * 128 * 2 * 2 + sizeof(int32_t);
 }
@@ -768,11 +768,13 @@ size_t gather_bytes(int batch, int64_t total_kv, int num_kv_heads) {
   return kGatherIndexBytes + static_cast<size_t>(total_kv / msgl::kTmaBoxRows + batch + 1) * gather_page_bytes(num_kv_heads);
 }
 
-// Pays where the attention takes several times what the copies do, by a rough model of both.  Steps of two layers in us,
-// gathered by the attention kernel / laid out first, and the model's ratio: 3 sequences of 300 to 2000 tokens over up
-// to 8000, 32 over 4 heads 1039 / 779 (14); 4000 tokens, 32 over 8 heads 442 / 390 (9.9); 1000 over 16000 664 / 546 (6.8);
-// 2000 over 5000, 16 over 8 298 / 280 (5.1); two prompts of up to 4000 288 / 276 (4.7); eight of up to 2938, 16 over 8
-// 556 / 545 (3.3); four chunks of 512 over up to 4096, 32 over 8 284 / 285 (3.0); 16 over 8 192 / 219 (1.5).
+// Pays where the attention takes several times what the copies do, by a rough model of both.  Hundred shapes (one to twelve
+// sequences, 30 to 4096 new tokens, 0 to 16000 cached, windows among them), time with the rows gathered by the attention
+// kernel over time with them laid out first, by the model's ratio: below 1 0.45 to 1.05; 1 to 2 0.85 to 1.13, in the mean
+// 0.97; 2 to 3 0.91 to 1.08, 1.01; 3 to 3.3 0.97 to 1.14, 1.03; above 3.3 1.01 to 1.49 on all 35, 1.11.  So 3: below it the
+// mean gains nothing that the page memory would be worth.  (Steps of two layers in us: four chunks of 512 over up to 4096, 32
+// over 8 heads 258 / 248 (3.0); four of 512 over up to 6000 323 / 332 (3.3); two of 1200 over up to 7000, 16 over 8 494 / 356
+// (3.7); three prompts of up to 2413 383 / 347 (5.5); two of 700 over 16000 1183 / 849 (5.1).)
 bool prefill_gathers(int batch, int total_q, int64_t total_kv, int hq, int hkv, int head_dim, int max_len_extend,
                      int window, int kv_chunk) {
   if (head_dim != 128 || kv_chunk != 0 || prefill_short_q(max_len_extend, hq / hkv, head_dim) || batch > 65535 ||
