@@ -124,80 +124,51 @@ EncodeTiledFn tensor_map_encoder() {
   return fn;
 }
 
-// 2-D map over a pool (num_slots rows of num_kv_heads * head_dim 16-bit elements): a box is
-// box_rows (16, or 1 for tile::gather4) token rows x 64 elements (128 bytes) of one head, written to shared memory with the
-// 128-byte swizzle, i.e. in the layout the tensor-core descriptors of the kernels expect.
-// Rows outside the pool read as zeros.  The maps are kept per thread, one per hash of the pool's
-// address: a model's layers each have two pools and go through them in turn.
-bool make_pool_tensor_map(CUtensorMap* out, const void* base, int64_t num_slots, int num_kv_heads,
-                          int head_dim, int dtype, int box_rows = msgl::kTmaBoxRows) {
-  struct Cached {
-    const void* base;
-    int64_t num_slots;
-    int hkv, hd, dtype, rows;
-    CUtensorMap map;
-  };
-  static thread_local Cached cache[256] = {};
-  const uintptr_t key = reinterpret_cast<uintptr_t>(base) >> 8;
-  Cached& c = cache[(key ^ (key >> 8) ^ (key >> 16) ^ (key >> 24) ^ (box_rows * 8)) % 256];
-  if (c.base == base && c.num_slots == num_slots && c.hkv == num_kv_heads && c.hd == head_dim &&
-      c.dtype == dtype && c.rows == box_rows && base != nullptr) {
-    *out = c.map;
-    return true;
-  }
-  EncodeTiledFn enc = tensor_map_encoder();
-  if (!enc || num_slots <= 0 || reinterpret_cast<uintptr_t>(base) % 16 != 0) return false;
-  const cuuint64_t dims[2] = {static_cast<cuuint64_t>(num_kv_heads) * head_dim,
-                              static_cast<cuuint64_t>(num_slots)};
-  const cuuint64_t strides[1] = {static_cast<cuuint64_t>(num_kv_heads) * head_dim * 2};
-  const cuuint32_t box[2] = {64, static_cast<cuuint32_t>(box_rows)};
-  const cuuint32_t elem_strides[2] = {1, 1};
-  CUtensorMap m;
-  const CUresult r = enc(&m, dtype == MSGL_DTYPE_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16
-                                                      : CU_TENSOR_MAP_DATA_TYPE_FLOAT16,
-                         2, const_cast<void*>(base), dims, strides, box, elem_strides,
-                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                         CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) return false;
-  c = Cached{base, num_slots, num_kv_heads, head_dim, dtype, box_rows, m};
-  *out = m;
-  return true;
-}
-
-// 3-D map over a pool for the decode kernel: (64 elements, slots, blocks of 64 elements of a row), so that one box is 16
-// token rows x all head_dim elements of one head, a block of columns after the other, as the kernel's tiles lie in
-// shared memory.  (A copy instruction costs its warp 67 cycles whatever its size: one per tile instead of two or four.)
-bool make_pool_group_map(CUtensorMap* out, const void* base, int64_t num_slots, int num_kv_heads, int head_dim,
-                         int dtype) {
+// Maps over a pool (num_slots rows of num_kv_heads * head_dim 16-bit elements).  A copy lands in shared memory with the
+// 128-byte swizzle, i.e. in the layout the tensor-core descriptors of the kernels expect; rows outside the pool read as
+// zeros.  The maps are kept per thread, one per hash of the pool's address and the form: a model's layers each have two
+// pools and go through them in turn.
+enum class PoolBox {
+  kPage,   // 2-D, 16 token rows x 64 elements (128 bytes) of one head
+  kRow,    // 2-D, one row of those, for tile::gather4
+  kHead,   // 3-D (64 elements, slots, blocks of 64 elements of a row): 16 token rows x all head_dim elements of one head, a block
+           // of columns after the other, as the decode kernel's tiles lie in shared memory.  (A copy instruction costs
+           // its warp 67 cycles whatever its size: one per tile instead of two or four.)
+};
+bool make_pool_map(CUtensorMap* out, PoolBox form, const void* base, int64_t num_slots, int num_kv_heads, int head_dim,
+                   int dtype) {
   struct Cached {
     const void* base;
     int64_t num_slots;
     int hkv, hd, dtype;
+    PoolBox form;
     CUtensorMap map;
   };
-  static thread_local Cached cache[256] = {};
+  static thread_local Cached cache[512] = {};
   const uintptr_t key = reinterpret_cast<uintptr_t>(base) >> 8;
-  Cached& c = cache[(key ^ (key >> 8) ^ (key >> 16) ^ (key >> 24)) % 256];
+  Cached& c = cache[(key ^ (key >> 8) ^ (key >> 16) ^ (key >> 24) ^ (static_cast<unsigned>(form) * 136)) % 512];
   if (c.base == base && c.num_slots == num_slots && c.hkv == num_kv_heads && c.hd == head_dim && c.dtype == dtype &&
-      base != nullptr) {
+      c.form == form && base != nullptr) {
     *out = c.map;
     return true;
   }
   EncodeTiledFn enc = tensor_map_encoder();
   if (!enc || num_slots <= 0 || num_slots >= (1ll << 32) || reinterpret_cast<uintptr_t>(base) % 16 != 0) return false;
-  const cuuint64_t dims[3] = {64, static_cast<cuuint64_t>(num_slots),
-                              static_cast<cuuint64_t>(num_kv_heads) * head_dim / 64};
-  const cuuint64_t strides[2] = {static_cast<cuuint64_t>(num_kv_heads) * head_dim * 2, 128};
-  const cuuint32_t box[3] = {64, static_cast<cuuint32_t>(msgl::kTmaBoxRows), static_cast<cuuint32_t>(head_dim / 64)};
+  const cuuint64_t row = static_cast<cuuint64_t>(num_kv_heads) * head_dim, slots = static_cast<cuuint64_t>(num_slots);
+  const bool head = form == PoolBox::kHead;
+  const cuuint64_t dims[3] = {head ? 64 : row, slots, row / 64};
+  const cuuint64_t strides[2] = {row * 2, 128};
+  const cuuint32_t box[3] = {64, form == PoolBox::kRow ? 1u : static_cast<cuuint32_t>(msgl::kTmaBoxRows),
+                             static_cast<cuuint32_t>(head_dim / 64)};
   const cuuint32_t elem_strides[3] = {1, 1, 1};
   CUtensorMap m;
   const CUresult r = enc(&m, dtype == MSGL_DTYPE_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16
                                                       : CU_TENSOR_MAP_DATA_TYPE_FLOAT16,
-                         3, const_cast<void*>(base), dims, strides, box, elem_strides,
+                         head ? 3 : 2, const_cast<void*>(base), dims, strides, box, elem_strides,
                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                          CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return false;
-  c = Cached{base, num_slots, num_kv_heads, head_dim, dtype, m};
+  c = Cached{base, num_slots, num_kv_heads, head_dim, dtype, form, m};
   *out = m;
   return true;
 }
@@ -920,8 +891,8 @@ static int decode_impl(const void* q, const void* k_cache, const void* v_cache,
   CUtensorMap tm_k, tm_v;
   std::memset(&tm_k, 0, sizeof(tm_k));
   std::memset(&tm_v, 0, sizeof(tm_v));
-  if (pages && (!make_pool_group_map(&tm_k, k_cache, num_slots, num_kv_heads, head_dim, dtype) ||
-                !make_pool_group_map(&tm_v, v_cache, num_slots, num_kv_heads, head_dim, dtype)))
+  if (pages && (!make_pool_map(&tm_k, PoolBox::kHead, k_cache, num_slots, num_kv_heads, head_dim, dtype) ||
+                !make_pool_map(&tm_v, PoolBox::kHead, v_cache, num_slots, num_kv_heads, head_dim, dtype)))
     return fail(MSGL_CUDA_ERROR, std::string(op) + "cannot build the tensor maps of the K/V pool");
   const size_t need = msgl_decode_workspace_bytes(batch, num_q_heads, head_dim, max_kv_splits);
   if (!workspace || workspace_bytes < need)
@@ -1222,8 +1193,8 @@ static int prefill_impl(const void* q, const void* k_cache, const void* v_cache,
   CUtensorMap tm_k, tm_v;
   std::memset(&tm_k, 0, sizeof(tm_k));
   std::memset(&tm_v, 0, sizeof(tm_v));
-  if (pages && (!make_pool_tensor_map(&tm_k, k_cache, num_slots, num_kv_heads, head_dim, dtype) ||
-                !make_pool_tensor_map(&tm_v, v_cache, num_slots, num_kv_heads, head_dim, dtype)))
+  if (pages && (!make_pool_map(&tm_k, PoolBox::kPage, k_cache, num_slots, num_kv_heads, head_dim, dtype) ||
+                !make_pool_map(&tm_v, PoolBox::kPage, v_cache, num_slots, num_kv_heads, head_dim, dtype)))
     return fail(MSGL_CUDA_ERROR, std::string(op) + "cannot build the tensor maps of the K/V pool");
   CUtensorMap tm_q;
   std::memset(&tm_q, 0, sizeof(tm_q));
@@ -1280,8 +1251,8 @@ static int prefill_impl(const void* q, const void* k_cache, const void* v_cache,
   CUtensorMap tg_k, tg_v;
   if (pair) {
     // everything by TMA: boxes of pages, rows of pools and queries by gather
-    pair = make_pool_tensor_map(&tg_k, k_cache, num_slots, num_kv_heads, head_dim, dtype, 1) &&
-           make_pool_tensor_map(&tg_v, v_cache, num_slots, num_kv_heads, head_dim, dtype, 1);
+    pair = make_pool_map(&tg_k, PoolBox::kRow, k_cache, num_slots, num_kv_heads, head_dim, dtype) &&
+           make_pool_map(&tg_v, PoolBox::kRow, v_cache, num_slots, num_kv_heads, head_dim, dtype);
     if (pair && !pages)
       p.q_tma = make_query_tensor_map(&tm_q, q, total_q, num_q_heads, p.group, head_dim, dtype) ? 1 : 0;
     if (pair && !p.q_tma) pair = make_query_row_map(&tm_q, q, total_q, num_q_heads, head_dim, dtype);

@@ -111,6 +111,9 @@ constexpr int kPrefillTickets = 1024;   // arrival counters the prefill op may u
 // visible key length, longest first, and inside a (sequence, head) the last (causally
 // longest) q tile comes first; larger batches keep the natural order, reversed.
 // `scratch` is block-shared memory the caller does not need yet (4*kSortedBatchMax ints).
+// (find_item_warp below numbers a batch of up to 32 sequences in the same way, down to the order of equal lengths: an
+// attention kernel may take its item from either, and prefill_merge_kernel, which takes it from this one, reads the
+// partials at the slots that `base` and `qt_base` give.)
 template <int NTHREADS>
 __device__ __forceinline__ bool find_item(const PrefillParams& p, int rank, int BM, int* scratch,
                                           ItemCoord& out) {
@@ -230,9 +233,10 @@ __device__ __forceinline__ bool find_item(const PrefillParams& p, int rank, int 
   return out.b >= 0;
 }
 
-// The same for at most 32 sequences, a lane each, by one warp, with the sequence's shape: no barrier, no second
-// look at the index arrays and no division on the way of a CTA that has nothing else to do yet (2400 + 1800 cycles
-// before its first copies in the general form).  (Quotients here are below 2^20: an approximate one is off by one.)
+// The same (order, ties and numbers as find_item) for at most 32 sequences, a lane each, by one warp, with the sequence's
+// shape: no barrier, no second look at the index arrays and no division on the way of a CTA that has nothing else to do
+// yet (2400 + 1800 cycles before its first copies in the general form).  (Quotients here are below 2^20: an approximate
+// one is off by one.)
 struct FoundItem {
   ItemCoord at;
   SeqShape seq;

@@ -203,7 +203,7 @@ def test_long_prefill_over_per_token_slots(hkv, hq, q_lens, prefixes, kw, dtype)
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("hkv,hq,q_lens,prefixes,launches", [
-    (2, 8, [64], [4 * 1024 - 40], 2), (2, 12, [43, 86], [3 * 1024 - 20, 1024 - 70], 2), (1, 8, [16], [2 * 1024 - 9], 2),
+    (2, 8, [64], [4 * 1024 - 40], 2), (2, 8, [64] * 3, [2 * 1024 - 40] * 3, 2), (2, 12, [43, 86], [3 * 1024 - 20, 1024 - 70], 2), (1, 8, [16], [2 * 1024 - 9], 2),
     (2, 8, [300, 131, 217] * 12, [-300, 5, -217] * 6 + [0, -131, 40] * 6, 1)], ids=lambda x: str(x)[:30])
 def test_sub_tiles_without_keys(hkv, hq, q_lens, prefixes, launches, dtype):
     """Key ranges cut inside the new tokens, so that the first rows of an item have no key in a piece and the last ones
