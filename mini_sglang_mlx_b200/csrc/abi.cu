@@ -669,39 +669,63 @@ struct GatherRowsParams {
 };
 constexpr int kGatherTokens = 8;   // of a warp
 
+// The tokens of all sequences are dealt to the warps in one row, whatever the lengths (a row of CTAs per sequence, as many
+// as an average one needs, left a long sequence among short ones to a few of them: two of 10200 and 14900 tokens among six of
+// 200 over 4 KV heads 28.4 -> 19.2 us, one of 8700 among three of 800 to 1200 over 8 29.9 -> 23.4, three of 3200 to 9200
+// 21.5 -> 17.5).  A token's sequence is the number of those that end at or before it.
 __global__ void __launch_bounds__(256) gather_rows_kernel(const GatherRowsParams p) {
   msgl::grid_dependency_wait();
   msgl::grid_dependency_launch();
-  const int b = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int thread = blockIdx.x * 256 + threadIdx.x, threads = gridDim.x * 256;
   const int32_t* indptr = msgl::after_wait(p.kv_indptr);
-  const int begin = indptr[b];
-  const int page0 = begin / msgl::kTmaBoxRows + b;
-  const bool bad = begin < 0 || page0 >= p.max_pages;
-  const int room = bad ? 0 : (p.max_pages - page0) * msgl::kTmaBoxRows;
-  const int len = bad ? 0 : min(max(indptr[b + 1] - begin, 0), room);
-  const int pages = (len + msgl::kTmaBoxRows - 1) / msgl::kTmaBoxRows;
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
+  const int rows = p.max_pages * msgl::kTmaBoxRows;
+  const int last = min(indptr[p.batch], rows);
+  for (int b = thread; b < p.batch; b += threads) {
+    const int begin = indptr[b], page0 = begin / msgl::kTmaBoxRows + b;
+    const bool bad = begin < 0 || page0 >= p.max_pages;
+    const int room = bad ? 0 : (p.max_pages - page0) * msgl::kTmaBoxRows;
+    const int len = bad ? 0 : min(max(indptr[b + 1] - begin, 0), room);
     p.page_indptr[b] = bad ? 0 : page0;
     p.kv_lens[b] = len;
-    if (b == p.batch - 1) p.page_indptr[p.batch] = bad ? 0 : page0 + pages;
+    if (b == p.batch - 1)
+      p.page_indptr[p.batch] = bad ? 0 : page0 + (len + msgl::kTmaBoxRows - 1) / msgl::kTmaBoxRows;
   }
-  for (int i = blockIdx.x * 256 + threadIdx.x; i < pages; i += gridDim.x * 256) p.page_indices[page0 + i] = page0 + i;
+  const int pages = min(max(last, 0) / msgl::kTmaBoxRows + p.batch + 1, p.max_pages);
+  for (int i = thread; i < pages; i += threads) p.page_indices[i] = i;
   const int64_t row_bytes = static_cast<int64_t>(p.row_chunks) * 16;
-  const int32_t* ids = msgl::after_wait(p.kv_indices) + begin;
-  const int64_t row0 = static_cast<int64_t>(page0) * msgl::kTmaBoxRows;
-  for (int t0 = (blockIdx.x * 8 + warp) * kGatherTokens; t0 < len; t0 += gridDim.x * 8 * kGatherTokens) {
-    int slot = -1;
-    if (lane < kGatherTokens && t0 + lane < len) {
-      slot = __ldg(ids + t0 + lane);
-      if (slot < -1 || slot >= p.num_slots) {
-        if (p.status) atomicExch(p.status, 2);
-        slot = -1;
+  const int32_t* ids = msgl::after_wait(p.kv_indices);
+  for (int64_t at = static_cast<int64_t>(blockIdx.x * 8 + warp) * kGatherTokens; at < last;
+       at += static_cast<int64_t>(gridDim.x) * 8 * kGatherTokens) {
+    const int t0 = static_cast<int>(at);
+    int seq = 0;                     // lane i: sequence of token t0 + i
+    for (int b0 = 0; b0 < p.batch; b0 += 32) {
+      const int end = b0 + lane < p.batch ? indptr[b0 + lane + 1] : 0x7fffffff;
+#pragma unroll
+      for (int i = 0; i < kGatherTokens; ++i) {
+        const int before = __popc(__ballot_sync(0xffffffffu, end <= t0 + i));
+        if (lane == i) seq += before;
       }
     }
-    const int n = min(kGatherTokens, len - t0);
-    int from[kGatherTokens];
+    int slot = -1, row = -1;
+    if (lane < kGatherTokens && t0 + lane < last && seq < p.batch) {
+      const int begin = indptr[seq];
+      const int64_t to = (static_cast<int64_t>(begin) / msgl::kTmaBoxRows + seq) * msgl::kTmaBoxRows + (t0 + lane - begin);
+      if (begin >= 0 && begin <= t0 + lane && to < rows) {
+        row = static_cast<int>(to);
+        slot = __ldg(ids + t0 + lane);
+        if (slot < -1 || slot >= p.num_slots) {
+          if (p.status) atomicExch(p.status, 2);
+          slot = -1;
+        }
+      }
+    }
+    int from[kGatherTokens], to[kGatherTokens];
 #pragma unroll
-    for (int i = 0; i < kGatherTokens; ++i) from[i] = __shfl_sync(0xffffffffu, slot, i);
+    for (int i = 0; i < kGatherTokens; ++i) {
+      from[i] = __shfl_sync(0xffffffffu, slot, i);
+      to[i] = __shfl_sync(0xffffffffu, row, i);
+    }
     for (int c = lane; c < p.row_chunks; c += 32) {
 #pragma unroll
       for (int h = 0; h < kGatherTokens; h += 4) {
@@ -716,10 +740,9 @@ __global__ void __launch_bounds__(256) gather_rows_kernel(const GatherRowsParams
         }
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          if (h + i >= n) break;
-          const int64_t to = (row0 + t0 + h + i) * row_bytes;
-          reinterpret_cast<uint4*>(p.k_rows + to)[c] = x[i];
-          reinterpret_cast<uint4*>(p.v_rows + to)[c] = y[i];
+          if (to[h + i] < 0) continue;
+          reinterpret_cast<uint4*>(p.k_rows + to[h + i] * row_bytes)[c] = x[i];
+          reinterpret_cast<uint4*>(p.v_rows + to[h + i] * row_bytes)[c] = y[i];
         }
       }
     }
@@ -745,7 +768,9 @@ size_t gather_bytes(int batch, int64_t total_kv, int num_kv_heads) {
 // 0.97; 2 to 3 0.91 to 1.08, 1.01; 3 to 3.3 0.97 to 1.14, 1.03; above 3.3 1.01 to 1.49 on all 35, 1.11.  So 3: below it the
 // mean gains nothing that the page memory would be worth.  (Steps of two layers in us: four chunks of 512 over up to 4096, 32
 // over 8 heads 258 / 248 (3.0); four of 512 over up to 6000 323 / 332 (3.3); two of 1200 over up to 7000, 16 over 8 494 / 356
-// (3.7); three prompts of up to 2413 383 / 347 (5.5); two of 700 over 16000 1183 / 849 (5.1).)
+// (3.7); three prompts of up to 2413 383 / 347 (5.5); two of 700 over 16000 1183 / 849 (5.1).)  The lengths of the single
+// sequences are not known here: where the longest one's pairs are a little more than a wave it can lose (8700 tokens,
+// 700 of them new, among three of 800 to 1200, 32 over 8 heads: 365 / 379).
 bool prefill_gathers(int batch, int total_q, int64_t total_kv, int hq, int hkv, int head_dim, int max_len_extend,
                      int window, int kv_chunk) {
   if (head_dim != 128 || kv_chunk != 0 || prefill_short_q(max_len_extend, hq / hkv, head_dim) || batch > 65535 ||
@@ -1178,9 +1203,8 @@ static int prefill_impl(const void* q, const void* k_cache, const void* v_cache,
     g.row_chunks = num_kv_heads * head_dim / 8;
     g.num_slots = num_slots;
     g.status = static_cast<int*>(workspace);
-    const int64_t per_seq = total_kv / batch + 1;
-    const unsigned gx = static_cast<unsigned>(std::max<int64_t>(1, std::min<int64_t>((per_seq + 63) / 64, 4096)));
-    const cudaError_t err = launch_dependent(gather_rows_kernel, dim3(gx, batch), dim3(256), 0,
+    const unsigned ctas = static_cast<unsigned>(std::min<int64_t>((total_kv + 63) / 64, 8192));
+    const cudaError_t err = launch_dependent(gather_rows_kernel, dim3(ctas), dim3(256), 0,
                                              static_cast<cudaStream_t>(stream), g);
     if (err != cudaSuccess) return cuda_fail("paged_prefill_attention", err);
     laid_out = PageIndex{g.page_indptr, g.page_indices, g.kv_lens, msgl::kTmaBoxRows};

@@ -231,3 +231,23 @@ def test_sub_tiles_without_keys(hkv, hq, q_lens, prefixes, launches, dtype):
         if x == 0:
             rows = slice(sum(q_lens[:b]), sum(q_lens[:b + 1]))
             assert not out[rows].any() and not paged[rows].any()
+
+
+@pytest.mark.parametrize("lens", [[(8000, 6000)] + [(3, 5 * i) for i in range(39)], [(1, 0)] * 33 + [(8000, 6000)],
+                                  [(7, 9)] * 2 + [(8000, 4001)] + [(0, 0)] * 3 + [(1, 6)]], ids=lambda x: str(len(x)))
+def test_rows_of_a_long_sequence_among_short_ones_are_laid_out(lens):
+    """Tokens are dealt to the copying warps across sequences: more than a warp's 32 of them, ends inside a warp's eight
+    tokens, sequences without keys."""
+    from mini_sglang_mlx_b200 import _lib, paged_prefill_attention, paged_prefill_attention_p16
+    from mini_sglang_mlx_b200.kernel import device_status
+    q_lens, prefixes = [a for a, _ in lens], [p for _, p in lens]
+    hkv, hq, d, n, kv_lens = 1, 32, 128, max(q_lens), [a + p for a, p in lens]
+    assert _lib.lib().msgl_prefill_launch_count(len(lens), sum(q_lens), sum(kv_lens), hq, hkv, d, n, 0, 0) == 2
+    kc, vc, pip, pidx, slots = make_pool([max(x, 1) for x in kv_lens], 16, hkv, seed=len(lens), d=d)
+    slots = torch.cat([s[:x] for s, x in zip(slots.split([max(x, 1) for x in kv_lens]), kv_lens)])
+    q = torch.empty(sum(q_lens), hq, d, dtype=torch.bfloat16, device="cuda").normal_(generator=torch.Generator("cuda").manual_seed(1))
+    qo, kvp, pre = _i32(O.build_indptr(q_lens).tolist()), _i32(O.build_indptr(kv_lens).tolist()), _i32(prefixes)
+    device_status()
+    out = paged_prefill_attention(q, kc, vc, qo, kvp, slots, pre, 0.1, n)
+    paged = paged_prefill_attention_p16(q, kc, vc, qo, pip, pidx, _i32(kv_lens), pre, 0.1, n, page_size=16)
+    assert torch.equal(out, paged) and device_status() == 0
