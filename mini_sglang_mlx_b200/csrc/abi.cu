@@ -671,7 +671,7 @@ constexpr int kGatherTokens = 8;   // of a warp
 
 // The tokens of all sequences are dealt to the warps in one row, whatever the lengths (a row of CTAs per sequence, as many
 // as an average one needs, left a long sequence among short ones to a few of them: two of 10200 and 14900 tokens among six of
-// 200 over 4 KV heads 28.4 -> 19.2 us, one of 8700 among three of 800 to 1200 over 8 29.9 -> 23.4, three of 3200 to 9200
+// 200 over 4 KV heads 28.4 -> 19.2 us, one of 8700 among three of 800 to 1200 over 8 29.9 -> 23.4, three of 5900 to 8200
 // 21.5 -> 17.5).  A token's sequence is the number of those that end at or before it.
 __global__ void __launch_bounds__(256) gather_rows_kernel(const GatherRowsParams p) {
   msgl::grid_dependency_wait();

@@ -112,6 +112,74 @@ def test_a_layer_call_equals_store_then_attention(phase, batch, page_size):
     assert torch.equal(got[0][1], got[1][1])
 
 
+@pytest.mark.parametrize("page_size", [1, 16])
+@pytest.mark.parametrize("d,hkv,hq,new,cached,mask,launches", [
+    (128, 2, 8, [16] * 16, 3000, dict(sliding_window_size=1024), 1),                        # draft blocks
+    (128, 2, 8, [8] * 70, 1500, {}, 1),                  # verification, key ranges split, merged by the last CTA
+    (128, 2, 8, [8] * 5, 6000, {}, 2), (128, 2, 8, [128], 9000, {}, 2),       # merged by a second launch
+    (128, 2, 6, [64 + i % 9 for i in range(40)], 500, {}, 1),       # more sequences than a warp finds its item among
+    (256, 2, 16, [600, 33, 570], 900, {}, 1), (256, 2, 12, [9] * 3, 2000, {}, None), (256, 1, 6, [130] * 33, 90, {}, 1),
+    (128, 1, 32, [2300, 40], 1500, {}, {1: 2, 16: 1}),              # per-token rows laid out as pages first
+], ids=lambda x: str(x)[:24])
+def test_a_layer_call_equals_store_then_attention_in_every_prefill_form(d, hkv, hq, new, cached, mask, launches, page_size):
+    """Attention that starts while the layer's own store still writes, in the forms of prefill, against separate calls with a
+    wait for the device between them: layers back to back, again with other rows over another pool."""
+    from mini_sglang_mlx_b200 import _lib
+    from mini_sglang_mlx_b200.attention import AttnBackend
+    from mini_sglang_mlx_b200.core import Batch, BatchPhase, Req
+    from mini_sglang_mlx_b200.kernel import qk_norm_rope_store
+    from mini_sglang_mlx_b200.kvcache import MHAKVCache
+
+    class WaitingPool(MHAKVCache):
+        def store_kv(self, *args, **kw):
+            super().store_kv(*args, **kw)
+            torch.cuda.synchronize()
+
+    class Cfg:
+        head_dim, num_kv_heads = d, hkv
+
+    g = torch.Generator().manual_seed(len(new) + d)
+    batch, most = len(new), -(-(cached + max(new)) // page_size)
+    lens = torch.randint(cached // 2, cached + 1, (batch,), generator=g).tolist()
+    pages = torch.randperm(batch * most, generator=g).int().view(batch, -1)
+    table = (pages[:, :, None] * page_size + torch.arange(page_size, dtype=torch.int32)).reshape(batch, -1).cuda()
+    loc = torch.cat([table[i, c:c + x] for i, (c, x) in enumerate(zip(lens, new))])
+    if launches is not None:
+        total = sum(lens) + sum(new) if page_size == 1 else sum(-(-(c + x) // 16) * 16 for c, x in zip(lens, new))
+        assert _lib.lib().msgl_prefill_launch_count(
+            batch, sum(new), total, hq, hkv, d, max(new), mask.get("sliding_window_size", 0), int(page_size > 1)) == (
+                launches if isinstance(launches, int) else launches[page_size])
+    pools = [cls(hkv, 4, d, table.numel(), torch.bfloat16) for cls in (MHAKVCache, WaitingPool)]
+    w = [torch.randn(d, generator=g).bfloat16().cuda() for _ in range(2)]
+    dev = torch.Generator("cuda").manual_seed(d)
+    for _ in range(3):
+        x = [[torch.empty(sum(new), h, d, dtype=torch.bfloat16, device="cuda").normal_(generator=dev) for h in (hq, hkv, hkv)]
+             for _ in range(4)]
+        rows, got = torch.empty_like(pools[0]._buffer).normal_(generator=dev), []
+        for pool in pools:
+            pool._buffer.copy_(rows)
+            be = AttnBackend(Cfg, pool, table, page_size=page_size)
+            b = Batch(reqs=[Req(table_idx=i, cached_len=c, device_len=c + n) for i, (c, n) in enumerate(zip(lens, new))],
+                      phase=BatchPhase.PREFILL, out_loc=loc)
+            be.prepare_metadata(b)
+            outs, qs = [], [q.clone() for q, _, _ in x]
+            for i, (q, (_, k, v)) in enumerate(zip(qs, x)):
+                if i % 2:
+                    outs.append(be.forward(q, k, v, i, b, **mask))
+                elif type(pool) is MHAKVCache:
+                    outs.append(be.forward_from_projections(q, k, v, i, b, q_norm_weight=w[0], k_norm_weight=w[1],
+                                                            rope_base=1e6, **mask))
+                else:
+                    q = qk_norm_rope_store(q, k, v, *w, b.attn_metadata.positions, loc, pool.k_cache(i), pool.v_cache(i),
+                                           rope_base=1e6)
+                    torch.cuda.synchronize()
+                    outs.append(be._attend(q, pool.k_cache(i), pool.v_cache(i), b.attn_metadata, False,
+                                           mask.get("sliding_window_size", 0)))
+            got.append((outs, qs, pool._buffer.clone()))
+        assert all(torch.equal(a, c) for kind in (0, 1) for a, c in zip(got[0][kind], got[1][kind]))
+        assert torch.equal(got[0][2], got[1][2])
+
+
 def _separate(be, pool, q, k, v, i, b, w):
     from mini_sglang_mlx_b200.kernel import qk_norm_rope_store
     if i % 2:
@@ -238,7 +306,7 @@ def test_sub_tiles_without_keys(hkv, hq, q_lens, prefixes, launches, dtype):
 def test_rows_of_a_long_sequence_among_short_ones_are_laid_out(lens):
     """Tokens are dealt to the copying warps across sequences: more than a warp's 32 of them, ends inside a warp's eight
     tokens, sequences without keys."""
-    from mini_sglang_mlx_b200 import _lib, paged_prefill_attention, paged_prefill_attention_p16
+    from mini_sglang_mlx_b200 import _lib, kernel as K, paged_prefill_attention, paged_prefill_attention_p16
     from mini_sglang_mlx_b200.kernel import device_status
     q_lens, prefixes = [a for a, _ in lens], [p for _, p in lens]
     hkv, hq, d, n, kv_lens = 1, 32, 128, max(q_lens), [a + p for a, p in lens]
@@ -251,3 +319,11 @@ def test_rows_of_a_long_sequence_among_short_ones_are_laid_out(lens):
     out = paged_prefill_attention(q, kc, vc, qo, kvp, slots, pre, 0.1, n)
     paged = paged_prefill_attention_p16(q, kc, vc, qo, pip, pidx, _i32(kv_lens), pre, 0.1, n, page_size=16)
     assert torch.equal(out, paged) and device_status() == 0
+    made = []          # (what the memory held before is not read: NaN here)
+    _lib.host.set_pages_maker(lambda size, index, stream: made.append(torch.full(
+        (size,), 255, dtype=torch.uint8, device="cuda")) or made[-1])
+    try:
+        again = paged_prefill_attention(q, kc, vc, qo, kvp, slots, pre, 0.1, n)
+    finally:
+        _lib.host.set_pages_maker(K._make_pages)
+    assert made and torch.equal(again, paged)
