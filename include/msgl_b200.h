@@ -84,11 +84,12 @@ const char* msgl_last_error_string(void);
 int msgl_device_sm_count(void);
 
 /*
- * Bytes of scratch the decode op needs: the header, fp32 partial outputs
- * (batch, num_q_heads, max_kv_splits, head_dim) and fp32 log-sum-exp (batch,
- * num_q_heads, max_kv_splits); a batch of more than 16384 (sequence, head)
- * pairs gets a counter region of its own in front of the partials, which every
- * call clears.
+ * Bytes of scratch the decode op needs: the header and room for fp32 partial outputs
+ * (batch, num_q_heads, max_kv_splits, head_dim) with a float for each (batch,
+ * num_q_heads, max_kv_splits), as the reference's temporaries have it; the op
+ * fills it with rows of head_dim + 4 floats (weighted sum, maximum, sum of the
+ * weights).  A batch of more than 16384 (sequence, head) pairs gets a counter
+ * region of its own in front of the partials, which every call clears.
  * Replaces the two temporaries of PagedDecodeAttention::eval_gpu
  * (mini-sglang-mlx-kernel/csrc/paged_decode_attention.cpp:119-131).
  */
@@ -104,8 +105,8 @@ size_t msgl_decode_workspace_bytes_full(int batch, int num_q_heads, int num_kv_h
 
 /*
  * Paged decode attention: one query token per sequence over all of its KV
- * tokens, split over the KV range; the piece of a (sequence, KV head) that
- * finishes last merges the partials by log-sum-exp (one launch).
+ * tokens, split over the KV range; the warp that arrives last at a (sequence,
+ * query head) merges its pieces by their maxima and sums (one launch).
  * Replaces paged_decode_attention
  * (mini-sglang-mlx-kernel/csrc/paged_decode_attention.cpp:15-73, binding
  * csrc/bindings.cpp:36-44) and its two Metal stages

@@ -288,9 +288,6 @@ bool prefill_pairs(int batch, int total_q, int64_t total_kv, int group, int num_
   return waves(sms / 2) * (17. + 1.9 * key_tiles) < waves(sms) * (20. + 4. * key_tiles);
 }
 
-bool prefill_gathers(int batch, int total_q, int64_t total_kv, int hq, int hkv, int head_dim, int max_len_extend,
-                     int window, int kv_chunk);
-
 PrefillPlan plan_prefill(int batch, int total_q, int64_t total_kv, int hq, int hkv, int head_dim,
                          int max_len_extend, int window, int sms) {
   // The key range is split only when the query tiles alone cannot give every CTA slot of the
@@ -792,12 +789,12 @@ constexpr int kDecMaxShare = 512;    // (256 / 384 / 512 on 32 sequences of 2000
 // 16: 12 requests of 1000 to 8000 tokens 221 / 218 / 217 us, 37 in per-token slots 148 / 146.6 / 146.9, 3 of 500 to 3000
 // 50.3 / 50.3 / 52.1; 19 of 512 to 16384 at head_dim 256 with 12 / 16 / 20: 199 / 195 / 186.)
 constexpr int kDecPad128 = 12, kDecPad256 = 20;
-// Merging a piece of a sequence (a warp per query head, eight pieces in flight) against a group in the loop, for
+// Merging a piece of a sequence (a warp per query head, up to sixteen pieces in flight) against a group in the loop, for
 // every four query heads of a KV head.  Beyond kDecMaxPieces pieces the shares grow to balance the two.  Steps of
-// two layers in us with 0.3 / 0.6 / 1.2: one sequence, 32 query over 2 KV heads of 256, 8191 tokens 61 / 62 / 68 (90
-// without the balance), 131071 tokens 211 / 196 / 204; three sequences of 20000 tokens there 123 / 98 / 99; 32
-// over 4 heads of 128, 32767 tokens 63 / 62 / 68; 16 over 8 heads, 4000 tokens 26.4 / 26.8 / 28.6.  With 32 pieces
-// instead of 16 the three sequences of 20000 tokens take 124; with 8, 2000 tokens of 16 over 2 heads 34.9 for 33.4.
+// two layers in us with 0.3 / 0.6 / 1.2: one sequence, 32 query over 2 KV heads of 256, 8191 tokens 57.0 / 54.5 / 60.0,
+// 131071 tokens 198 / 179 / 176 (210 / 207 / 223 in per-token slots); three sequences of 20000 tokens there 110 / 94 / 87
+// (104 / 103 / 109); 32 over 4 heads of 128, 32767 tokens 56.7 / 57.7 / 63.5.  With 32 pieces instead of 16 the three
+// sequences of 20000 tokens take 109; with 8, 2000 tokens of 16 over 2 heads of 128 27.5 for 26.0.
 constexpr float kDecMergeRow = 0.6f;
 constexpr int kDecMaxPieces = 16;
 
@@ -845,12 +842,10 @@ struct PageIndex {
 
 }  // namespace
 
-// Arrival counters of the decode op: one per (sequence, KV head).  They sit in the workspace
-// header when there are at most kTicketSlots of them; a larger batch gets a region of its own
-// behind the header, cleared by every call (the workspace query is not told the KV head
-// count, so it sizes that region for the query heads).
 static bool aligned16(const void* ptr) { return reinterpret_cast<uintptr_t>(ptr) % 16 == 0; }
 
+// Arrival counters of the decode op: one per (sequence, query head).  They sit in the workspace header when there
+// are at most kTicketSlots of them; a larger batch gets a region of its own behind the header, cleared by every call.
 static size_t decode_ticket_bytes(int batch, int num_q_heads) {
   const size_t n = static_cast<size_t>(batch) * num_q_heads;
   return n <= kTicketSlots ? 0 : (n * sizeof(int) + 255) / 256 * 256;
@@ -1043,8 +1038,8 @@ int msgl_paged_decode_attention_static(const void* q, const void* k_cache, const
   const int rc = static_scratch_for_current_device(&scratch);
   if (rc != MSGL_OK) return rc;
   // What has to start at zero does: the array is zero when the library is loaded, the arrival
-  // counters behind the status word are put back to zero by the CTA that merges, every partial
-  // and log-sum-exp that a merge reads is written earlier in the same call, and the status
+  // counters behind the status word are put back to zero by the warp that merges, every partial, maximum
+  // and sum that a merge reads is written earlier in the same call, and the status
   // word at the head is sticky by design.
   return msgl_paged_decode_attention(q, k_cache, v_cache, kv_indptr, kv_indices, num_kv_splits, out,
                                      scratch, MSGL_STATIC_SCRATCH_BYTES, batch, num_q_heads,

@@ -23,8 +23,8 @@
 // there is no second launch and no barrier.
 //
 // What bounds a small call is none of the chip's rates but the chain of a CTA's instructions, each of which
-// waits for the one in front (one warp per scheduler: 7.9 cycles per instruction, 2975 of them on 700 tokens of one
-// sequence; memory 10 % of it).  So the search for the share has no divisions and one scan, new rows' slots are
+// waits for the one in front (one warp per scheduler: 8 to 10 cycles per instruction, 2320 of them on 700 tokens of one
+// sequence, 2975 before; memory 10 % of it).  So the search for the share has no divisions and one scan, new rows' slots are
 // held in registers, and the merge of the pieces reads them straight into registers.
 //
 // Per-token form: K and V rows (256 or 512 bytes per token and head) are gathered through the slot
@@ -36,9 +36,9 @@
 //
 // Semantics follow the reference stages
 // (mini-sglang-mlx-kernel/csrc/paged_decode_attention.metal:313-506 and
-// 512-586): slot addressing row = kv_indices[kv_indptr[b] + t], normalised
-// partials, lse in natural-log units, merge out = sum_s e^{lse_s-M} O_s /
-// sum_s e^{lse_s-M}.  The reference's split counts are hints; here the shares take their place
+// 512-586): slot addressing row = kv_indices[kv_indptr[b] + t]; its partials are normalised, each with a
+// log-sum-exp, here they carry (maximum in log2 units, sum) and are divided once, in the merge:
+// out = sum_s 2^{M_s-M} O_s / sum_s 2^{M_s-M} l_s.  The reference's split counts are hints; here the shares take their place
 // (its result does not depend on them).  Address arithmetic is 64-bit.
 #pragma once
 

@@ -123,7 +123,7 @@ def test_pieces_of_a_long_sequence_beside_short_ones(d, hkv, hq, limit, past, ot
 @pytest.mark.parametrize("kv_lens", [[128 * k + 5 for k in (1, 2, 7, 8, 9)], [128 * 16], [128 * 17 + 1, 300], [128 * 33],
                                      [200] * 33 + [2100, 0, 2300]], ids=lambda x: f"{len(x)}x{sum(x)}")
 def test_a_warp_merges_the_pieces_of_its_heads(d, hkv, hq, kv_lens):
-    """A warp per query head, eight pieces at a time, whichever CTA arrives last at the head: heads that leave
+    """A warp per query head, eight or sixteen pieces at a time, whichever CTA arrives last at the head: heads that leave
     warps without one, one to 33 pieces, two partials of a share (a sequence's end and the next one's start), and
     the counters back at zero (a second call gives the same bits)."""
     from mini_sglang_mlx_b200 import paged_decode_attention
