@@ -219,7 +219,8 @@ size_t msgl_prefill_workspace_bytes_full(int batch, int total_q, int64_t total_k
                                          int num_kv_heads, int head_dim, int max_len_extend,
                                          int sliding_window_size);
 /* The part of it that those pages take, 0 where a call does not lay its rows out: msgl_prefill_layer_pages takes
- * it as memory of its own, which belongs to the call alone and can go elsewhere once its launches are queued. */
+ * it as memory of its own, which belongs to the call alone and can go elsewhere once its launches are queued (of a
+ * captured call: once its graph is replayed no more). */
 size_t msgl_prefill_kv_pages_bytes(int batch, int total_q, int64_t total_kv, int num_q_heads, int num_kv_heads,
                                    int head_dim, int max_len_extend, int sliding_window_size);
 

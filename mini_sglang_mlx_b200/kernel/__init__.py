@@ -110,6 +110,20 @@ def _make_workspace(nbytes: int, index: int, stream_handle: int, kind: str) -> t
 _PAGES_PAUSE = 256
 _pages_pause: Dict[int, int] = {}
 
+# Page memory of captured calls by (device, stream), and what they outgrew: a graph writes there whenever it is
+# replayed, and a stream can be captured without torch's allocator knowing, so it stays, like the scratch.
+_captured_pages: Dict[Tuple[int, int], list] = {}
+
+
+def _pages_now(nbytes: int, device: torch.device, stream_handle: int) -> torch.Tensor:
+    """On torch's current stream."""
+    if not torch.cuda.is_current_stream_capturing():
+        return torch.empty(nbytes, dtype=torch.uint8, device=device)
+    kept = _captured_pages.setdefault((device.index, stream_handle), [])
+    if not kept or kept[-1].numel() < nbytes:
+        kept.append(torch.empty(1 << (nbytes - 1).bit_length(), dtype=torch.uint8, device=device))
+    return kept[-1]
+
 
 def _make_pages(nbytes: int, index: int, stream_handle: int) -> Optional[torch.Tensor]:
     """Memory for the K/V rows that one long prefill over per-token slots lays out as pages, or None where
@@ -122,9 +136,9 @@ def _make_pages(nbytes: int, index: int, stream_handle: int) -> Optional[torch.T
     device = torch.device("cuda", index)
     try:
         if _stream_handle(None, device) == stream_handle:
-            return torch.empty(nbytes, dtype=torch.uint8, device=device)
+            return _pages_now(nbytes, device, stream_handle)
         with torch.cuda.stream(torch.cuda.ExternalStream(stream_handle, device=device)):
-            return torch.empty(nbytes, dtype=torch.uint8, device=device)
+            return _pages_now(nbytes, device, stream_handle)
     except torch.OutOfMemoryError:
         _pages_pause[index] = _PAGES_PAUSE
         return None

@@ -84,3 +84,26 @@ def test_prefill_replays_on_new_contents(q_lens, prefix):
     assert torch.equal(out, call())
     assert_close_to_oracle(out, O.paged_prefill_attention_oracle(q, kc, vc, qo, kvp, slots, pre, scale),
                            f"prefill graph replay {q_lens}")
+
+
+def test_a_long_prefill_over_token_slots_replays_on_new_contents():
+    """Rows laid out as pages in memory that the graph keeps: between replays nothing else gets it."""
+    from mini_sglang_mlx_b200 import _lib, paged_prefill_attention
+    g = torch.Generator("cuda").manual_seed(7)
+    hkv, hq, d, q_lens, kv_lens = 4, 32, 128, [1500, 700], [2500, 700]
+    assert _lib.lib().msgl_prefill_kv_pages_bytes(2, 2200, 3200, hq, hkv, d, 1500, 0) > 0
+    kc, vc = (torch.empty(3300, hkv, d, dtype=torch.bfloat16, device="cuda").normal_(generator=g) for _ in range(2))
+    q = torch.empty(2200, hq, d, dtype=torch.bfloat16, device="cuda").normal_(generator=g)
+    slots = torch.randperm(3300, generator=g, device="cuda")[:3200].int()
+    qo, kvp = torch.from_numpy(O.build_indptr(q_lens)).cuda(), torch.from_numpy(O.build_indptr(kv_lens)).cuda()
+    pre = torch.tensor([1000, 0], dtype=torch.int32).cuda()
+    call = lambda: paged_prefill_attention(q, kc, vc, qo, kvp, slots, pre, 0.09, 1500)  # noqa: E731
+    graph, out = _capture(call)
+    for _ in range(2):
+        for x in (q, kc, vc):
+            x.normal_(generator=g)
+        want = call()
+        others = [torch.full((1 << 22,), float("nan"), device="cuda") for _ in range(8)]
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out, want) and all(bool(x.isnan().all()) for x in others)

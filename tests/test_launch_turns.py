@@ -184,6 +184,7 @@ def test_a_long_prefill_goes_without_page_memory_that_nobody_has(host, monkeypat
 
     monkeypatch.setattr(torch, "empty", none_left)
     monkeypatch.setattr(K, "_stream_handle", lambda stream, device: 7)
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
     monkeypatch.setattr(K, "_pages_pause", {})
     m.set_pages_maker(lambda nbytes, index, stream: K._make_pages(nbytes, 0, stream))
     asked.clear()

@@ -13,6 +13,7 @@ def host_scratch(monkeypatch):
     """The operators' scratch bookkeeping over host memory: no entry to begin with, none left behind."""
     monkeypatch.setattr(K, "_workspaces", {})
     monkeypatch.setattr(K, "_retired", [])
+    monkeypatch.setattr(K, "_captured_pages", {}, raising=False)
     monkeypatch.setattr(torch.cuda, "ExternalStream", lambda *a, **k: None)
     monkeypatch.setattr(torch.cuda, "stream", lambda s: contextlib.nullcontext())
     real = torch.zeros
@@ -68,6 +69,21 @@ def test_growth_asks_for_what_it_needs_where_a_power_of_two_finds_no_memory(host
 
     monkeypatch.setattr(torch, "zeros", small)
     assert K._workspace((1 << 20) + 4096, dev, 7, "prefill").numel() == (1 << 20) + 4096
+
+
+def test_page_memory_of_a_captured_call_stays(host_scratch, monkeypatch):
+    """A graph writes there whenever it is replayed, so the memory is neither given back nor taken twice; an
+    uncaptured call's is its own."""
+    real = torch.empty
+    monkeypatch.setattr(torch, "empty", lambda n, *, dtype, device: real(n, dtype=dtype))
+    monkeypatch.setattr(K, "_stream_handle", lambda stream, device: 7)
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
+    a, b = K._make_pages(5000, 0, 7), K._make_pages(5000, 0, 7)
+    assert a.data_ptr() != b.data_ptr()
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: True)
+    at = [K._make_pages(n, 0, stream).data_ptr() for n, stream in ((5000, 7), (4000, 7), (9000, 7), (9000, 7), (5000, 8))]
+    others = [K._make_pages(5000, 0, 9 + i).data_ptr() for i in range(8)]        # (memory given back would be handed out)
+    assert at[0] == at[1] != at[2] == at[3] and len({*at, *others}) == 3 + len(others)
 
 
 def test_a_report_from_before_a_buffer_grew_is_not_lost(host_scratch, monkeypatch):
